@@ -275,6 +275,8 @@ struct Layout {
     size_t coef, omega, snap_const, slot_first, item_first, partial, large, evec, hdw, total;
     int P, IP, max_items, T;
     bool phase_records;
+    bool fourier;  // the phase sum as a nonuniform Fourier transform
+    NufftShape nu;
 };
 
 static size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -339,6 +341,13 @@ static Layout powder_layout(const msp_powder_args *a) {
     const int has_pairs = a->mode != MSP_MODE_INTEGRAL;
     L.IP = phase_pairs_per_item(a->num_snap, L.P, a->precision);
     L.max_items = has_pairs ? phase_max_items(a->num_snap, a->num_slots, L.P, L.IP) : 0;
+    L.fourier = has_pairs && a->uniform &&
+                nufft_shape(a->num_snap, L.P, a->num_slots, L.T, a->precision,
+                            a->mode != MSP_MODE_FAST || a->t0 != 0.0, &L.nu);
+    if (L.fourier) {
+        L.IP = L.nu.ip;
+        L.max_items = L.nu.max_items;
+    }
     const size_t ce = a->precision == MSP_PREC_MIXED ? 8 : 16;
     size_t off = 0;
     L.coef = off;
@@ -355,7 +364,8 @@ static Layout powder_layout(const msp_powder_args *a) {
     L.item_first = off;
     off += align256((size_t)(a->num_slots + 1) * 4);
     L.partial = off;
-    off += align256((size_t)L.max_items * L.T * (L.phase_records ? 4 : 8));
+    off += align256(L.fourier ? L.nu.bytes
+                              : (size_t)L.max_items * L.T * (L.phase_records ? 4 : 8));
     L.evec = off;
     off += align256(snap_evec_bytes(a->n, a->num_snap, a->precision));
     // MIXED, n <= MSP_MAX_DIM: Hsys and Z as double-words (no FP64 in the
@@ -512,12 +522,19 @@ int msp_powder_run(const msp_powder_args *a) {
                     "msp_schedule");
     if (rc != MSP_OK) return rc;
     if (ev) cudaEventRecord(ev[3], st);
-    if (a->mode != MSP_MODE_INTEGRAL) {
+    if (L.fourier) {
+        rc = cuda_check(launch_nufft_spread(pa, L.nu, a->precision, ws + L.partial, st),
+                        "msp_nufft_spread");
+        if (rc != MSP_OK) return rc;
+    } else if (a->mode != MSP_MODE_INTEGRAL) {
         rc = cuda_check(launch_phase(pa, a->precision, L.max_items, a->uniform, st), "msp_phase");
         if (rc != MSP_OK) return rc;
     }
     if (ev) cudaEventRecord(ev[4], st);
-    rc = cuda_check(launch_reduce(pa, sa.snap_const, a->out, L.T, st), "msp_reduce");
+    rc = L.fourier ? cuda_check(launch_nufft_rows(pa, L.nu, a->precision, ws + L.partial,
+                                                  sa.snap_const, a->out, st),
+                                "msp_nufft_rows")
+                   : cuda_check(launch_reduce(pa, sa.snap_const, a->out, L.T, st), "msp_reduce");
     if (rc != MSP_OK) return rc;
     if (ev) cudaEventRecord(ev[5], st);
     return MSP_OK;

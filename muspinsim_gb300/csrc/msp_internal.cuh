@@ -141,6 +141,31 @@ struct PhaseArgs {
     int accumulate;       // reduce: out += sum instead of out = sum
 };
 
+// Pair range [begin, end) of work item `item`; begin = -1 when the item does
+// not exist.  item_first / slot_first are num_slots + 1 prefix arrays; the
+// items of a slot cover its pairs in runs of IP.
+__device__ __forceinline__ void phase_item_range(const PhaseArgs &a, int item, int *b, int *e) {
+    const int total = a.item_first[a.num_slots];
+    if (item >= total) {
+        *b = -1;
+        *e = -1;
+        return;
+    }
+    int lo = 0, hi = a.num_slots - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (a.item_first[mid] <= item)
+            lo = mid;
+        else
+            hi = mid - 1;
+    }
+    const int pb = a.slot_first[lo] * a.P + (item - a.item_first[lo]) * a.IP;
+    const int slot_end = a.slot_first[lo + 1] * a.P;
+    const int pe = pb + a.IP;
+    *b = pb;
+    *e = pe < slot_end ? pe : slot_end;
+}
+
 size_t snap_smem_bytes(int n, int mode, int precision, int fac_len);
 // Hsys (nh entries) and Z (nz entries) split into double-words into dst
 // (nh + nz float4: Hsys first), for SnapArgs::Hsys_dw / Z_dw.
@@ -180,6 +205,24 @@ cudaError_t launch_phase(const PhaseArgs &a, int precision, int max_items, int u
                          cudaStream_t st);
 cudaError_t launch_reduce(const PhaseArgs &a, const double *snap_const, double *out,
                           int num_times, cudaStream_t st);
+
+// Phase sum of a uniform grid as a nonuniform Fourier transform
+// (msp_nufft.cu) for rows that many pairs feed: its shape and workspace
+// (false: the direct sum is cheaper), the spreading stage and the reduction
+// and transform into the output rows.
+struct NufftShape {
+    int tiles, tt;   // time tiles, samples per tile
+    int n1, n2, m;   // grid of n1 n2 = 2 m angles
+    int two;         // sine terms too
+    int cols;        // cells per tile (cosine, then sine)
+    int ip, max_items;
+    size_t off_root, off_win, off_tab, off_partial, off_rows, off_spec, bytes;
+};
+bool nufft_shape(long long S, int P, int slots, int T, int precision, bool two, NufftShape *out);
+cudaError_t launch_nufft_spread(const PhaseArgs &a, const NufftShape &s, int precision, char *ws,
+                                cudaStream_t st);
+cudaError_t launch_nufft_rows(const PhaseArgs &a, const NufftShape &s, int precision, char *ws,
+                              const double *snap_const, double *out, cudaStream_t st);
 
 cudaError_t launch_fast_cos_sum(const double *times, int num_times, int d, const double *A,
                                 const double *W, int n, double *out, cudaStream_t st);

@@ -41,31 +41,6 @@ __device__ __forceinline__ void sincos_t(double x, float *s, float *c) {
     sincosf((float)x, s, c);
 }
 
-// Pair range [begin, end) of work item `item`; begin = -1 when the item does
-// not exist.  item_first / slot_first are num_slots + 1 prefix arrays; the
-// items of a slot cover its pairs in runs of IP.
-__device__ __forceinline__ void item_range(const PhaseArgs &a, int item, int *b, int *e) {
-    const int total = a.item_first[a.num_slots];
-    if (item >= total) {
-        *b = -1;
-        *e = -1;
-        return;
-    }
-    int lo = 0, hi = a.num_slots - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (a.item_first[mid] <= item)
-            lo = mid;
-        else
-            hi = mid - 1;
-    }
-    const int pb = a.slot_first[lo] * a.P + (item - a.item_first[lo]) * a.IP;
-    const int slot_end = a.slot_first[lo + 1] * a.P;
-    const int pe = pb + a.IP;
-    *b = pb;
-    *e = pe < slot_end ? pe : slot_end;
-}
-
 template <typename T>
 __global__ void __launch_bounds__(128) msp_phase_uniform_kernel(PhaseArgs a) {
     constexpr int K = 64, TM = PhaseCfg<T>::TM, TN = PhaseCfg<T>::TN, PS = PhaseCfg<T>::PS;
@@ -82,7 +57,7 @@ __global__ void __launch_bounds__(128) msp_phase_uniform_kernel(PhaseArgs a) {
     __shared__ int s_range[2];
 
     const int tid = threadIdx.x;
-    if (tid == 0) item_range(a, blockIdx.x, &s_range[0], &s_range[1]);
+    if (tid == 0) phase_item_range(a, blockIdx.x, &s_range[0], &s_range[1]);
     __syncthreads();
     const int pbeg = s_range[0], pend = s_range[1];
     if (pbeg < 0) return;
@@ -229,7 +204,7 @@ __global__ void __launch_bounds__(128, 4) msp_phase_uniform_f32_kernel(PhaseArgs
     __shared__ int s_range[2];
 
     const int tid = threadIdx.x;
-    if (tid == 0) item_range(a, blockIdx.x, &s_range[0], &s_range[1]);
+    if (tid == 0) phase_item_range(a, blockIdx.x, &s_range[0], &s_range[1]);
     __syncthreads();
     const int pbeg = s_range[0], pend = s_range[1];
     if (pbeg < 0) return;
@@ -619,7 +594,7 @@ __global__ void __launch_bounds__(MSP_TC_THREADS) msp_phase_tc_kernel(PhaseArgs 
 
     const int tid = threadIdx.x, warp = tid >> 5;
     if (tid == 0) {
-        item_range(a, blockIdx.x, &s_range[0], &s_range[1]);
+        phase_item_range(a, blockIdx.x, &s_range[0], &s_range[1]);
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&mbar[0])));
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&mbar[1])));
         asm volatile("fence.mbarrier_init.release.cluster;");
@@ -897,7 +872,7 @@ __global__ void __launch_bounds__(MSP_TCW_THREADS, 2) msp_phase_tcw_kernel(Phase
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (tid == 0) {
-        item_range(a, blockIdx.x, &s_range[0], &s_range[1]);
+        phase_item_range(a, blockIdx.x, &s_range[0], &s_range[1]);
         for (int t = 0; t < MSP_TCW_TABLES; ++t) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&tab_full[t])),
                          "r"(MSP_TCW_TABLE_THREADS / 32));
@@ -1116,7 +1091,7 @@ __global__ void __launch_bounds__(256) msp_phase_direct_kernel(PhaseArgs a) {
     __shared__ double sw[256];
     __shared__ int s_range[2];
     const int tid = threadIdx.x;
-    if (tid == 0) item_range(a, blockIdx.x, &s_range[0], &s_range[1]);
+    if (tid == 0) phase_item_range(a, blockIdx.x, &s_range[0], &s_range[1]);
     __syncthreads();
     const int pbeg = s_range[0], pend = s_range[1];
     if (pbeg < 0) return;
