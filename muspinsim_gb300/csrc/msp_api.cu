@@ -275,6 +275,7 @@ struct Layout {
     size_t coef, omega, snap_const, slot_first, item_first, partial, large, evec, hdw, total;
     int P, IP, max_items, T;
     bool phase_records;
+    bool two_stage, split;
     bool fourier;  // the phase sum as a nonuniform Fourier transform
     NufftShape nu;
 };
@@ -333,15 +334,19 @@ static int check_powder(const msp_powder_args *a) {
     return MSP_OK;
 }
 
-static Layout powder_layout(const msp_powder_args *a) {
+// Workspace of a run.  `lean` leaves out what only buys speed (the Fourier
+// form of the phase sum, and in FP64 the two-stage snapshots): for callers
+// with a fixed scratch.
+static Layout powder_layout(const msp_powder_args *a, bool lean = false) {
     Layout L;
+    const bool mixed = a->precision == MSP_PREC_MIXED;
     const size_t S = (size_t)a->num_snap;
     L.T = a->mode == MSP_MODE_INTEGRAL ? 1 : a->num_times;
     L.P = a->n * (a->n - 1) / 2;
     const int has_pairs = a->mode != MSP_MODE_INTEGRAL;
     L.IP = phase_pairs_per_item(a->num_snap, L.P, a->precision);
     L.max_items = has_pairs ? phase_max_items(a->num_snap, a->num_slots, L.P, L.IP) : 0;
-    L.fourier = has_pairs && a->uniform &&
+    L.fourier = has_pairs && a->uniform && !lean &&
                 nufft_shape(a->num_snap, L.P, a->num_slots, L.T, a->precision,
                             a->mode != MSP_MODE_FAST || a->t0 != 0.0, &L.nu);
     if (L.fourier) {
@@ -367,12 +372,12 @@ static Layout powder_layout(const msp_powder_args *a) {
     off += align256(L.fourier ? L.nu.bytes
                               : (size_t)L.max_items * L.T * (L.phase_records ? 4 : 8));
     L.evec = off;
-    off += align256(snap_evec_bytes(a->n, a->num_snap, a->precision));
-    // MIXED, n <= MSP_MAX_DIM: Hsys and Z as double-words (no FP64 in the
-    // snapshot kernels)
+    L.two_stage = snap_evec_bytes(a->n, a->num_snap) > 0 && (mixed || !lean);
+    off += align256(L.two_stage ? snap_evec_bytes(a->n, a->num_snap) : 0);
+    // n <= MSP_MAX_DIM: Hsys and Z as double-words for the FP32 stages
     L.hdw = off;
-    if (a->precision == MSP_PREC_MIXED && a->n <= MSP_MAX_DIM && a->num_snap > 0)
-        off += align256((size_t)4 * a->n * a->n * 16);
+    L.split = a->n <= MSP_MAX_DIM && a->num_snap > 0 && (mixed || !lean);
+    off += align256(L.split ? (size_t)4 * a->n * a->n * 16 : 0);
     L.large = off;
     if (a->n > MSP_MAX_DIM) {
         if (a->mode == MSP_MODE_FAST)
@@ -394,6 +399,17 @@ int msp_powder_workspace(const msp_powder_args *args, size_t *bytes) {
     return MSP_OK;
 }
 
+}  // extern "C"
+
+namespace msp {
+// Smallest workspace msp_powder_run accepts (0 when the arguments are bad).
+size_t powder_min_workspace(const msp_powder_args *args) {
+    return check_powder(args) == MSP_OK ? powder_layout(args, true).total : 0;
+}
+}  // namespace msp
+
+extern "C" {
+
 int msp_powder_run(const msp_powder_args *a) {
     int rc = check_powder(a);
     if (rc != MSP_OK) return rc;
@@ -407,7 +423,11 @@ int msp_powder_run(const msp_powder_args *a) {
         MSP_CHECK_PTR(a->slot);
         MSP_CHECK_PTR(a->status);
     }
-    const Layout L = powder_layout(a);
+    Layout L = powder_layout(a);
+    if (a->workspace != NULL && a->workspace_bytes < L.total) {
+        const Layout lean = powder_layout(a, true);
+        if (lean.total <= a->workspace_bytes) L = lean;
+    }
     if (L.total > 0) {
         if (a->workspace == NULL || a->workspace_bytes < L.total)
             return fail(MSP_ERR_WORKSPACE, "msp_powder_run: workspace %zu < %zu bytes",
@@ -454,7 +474,7 @@ int msp_powder_run(const msp_powder_args *a) {
     sa.snap_const = reinterpret_cast<double *>(ws + L.snap_const);
     sa.status = a->status;
     sa.coef_f32 = a->precision == MSP_PREC_MIXED;
-    sa.evec = snap_evec_bytes(a->n, a->num_snap, a->precision) > 0 ? ws + L.evec : NULL;
+    sa.evec = L.two_stage ? ws + L.evec : NULL;
 
     const bool large = a->n > MSP_MAX_DIM;
     if (!large) {
@@ -466,7 +486,7 @@ int msp_powder_run(const msp_powder_args *a) {
 
     cudaEvent_t *ev = timer_slot(a->timer);
     if (ev) cudaEventRecord(ev[0], st);
-    if (a->precision == MSP_PREC_MIXED && !large && a->num_snap > 0) {
+    if (L.split) {
         const size_t nn = (size_t)a->n * a->n;
         float4 *hdw = reinterpret_cast<float4 *>(ws + L.hdw);
         rc = cuda_check(launch_split_dw(a->Hsys, nn, a->Z, 3 * nn, hdw, st), "msp_split_dw");
@@ -474,15 +494,14 @@ int msp_powder_run(const msp_powder_args *a) {
         sa.Hsys_dw = hdw;
         sa.Z_dw = hdw + nn;
     }
-    // two-stage MIXED snapshots (n <= 32): the warp Jacobi is its own stage
-    const bool two_stage = !large && sa.evec != NULL && a->num_snap > 0;
-    if (two_stage) {
+    // two-stage snapshots (n <= 32): the FP32 eigenvectors are their own stage
+    if (L.two_stage) {
         rc = cuda_check(launch_jacobi_warp(sa, st), "msp_jacobi_warp");
         if (rc != MSP_OK) return rc;
     }
     if (ev) cudaEventRecord(ev[1], st);
-    if (two_stage)
-        rc = cuda_check(launch_snapshots_refine(sa, a->mode, st), "msp_snap");
+    if (L.two_stage)
+        rc = cuda_check(launch_snapshots_refine(sa, a->mode, a->precision, st), "msp_snap");
     else if (large && a->num_snap > 0 && a->mode == MSP_MODE_FAST)
         rc = cuda_check(launch_large_fast(sa, reinterpret_cast<double *>(ws + L.large),
                                           large_grid(a->num_snap, a->n, a->precision), st, 0,

@@ -176,9 +176,10 @@ static __device__ void oa_cluster_diagonal(const float2 *lam, const float *corr,
 // the corrected eigenvector matrix X (nrows x n, row stride ldx), and sets
 // the clusters' eigenvalues; the other levels get l_i + corr_i.  Returns
 // this thread's share of the step size.  Ends with a barrier.
+// Xl (optional, laid out like X): low words of X, zeroed in rotated columns.
 static __device__ float oa_resolve_clusters(cx<float> *X, int ldx, int nrows, float2 *lam,
                                      const float *corr, int n, const OaCluster &c,
-                                     float lscale) {
+                                     float lscale, cx<float> *Xl = nullptr) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int nwarps = (blockDim.x + 31) >> 5;
     const float noise = 4.0f * (float)n * 5.684341886080802e-14f * lscale;  // 4 n 2^-44 max|l|
@@ -222,6 +223,7 @@ static __device__ float oa_resolve_clusters(cx<float> *X, int ldx, int nrows, fl
                         const cx<float> x = X[(size_t)r * ldx + i], y = X[(size_t)r * ldx + j];
                         X[(size_t)r * ldx + i] = cadd(cscale(R.c, x), cscale(-1.0f, cmulc(s, y)));
                         X[(size_t)r * ldx + j] = cadd(cmul(s, x), cscale(R.c, y));
+                        if (Xl) Xl[(size_t)r * ldx + i] = Xl[(size_t)r * ldx + j] = mk<float>(0.f, 0.f);
                     }
                     __syncwarp();
                     if (lane == 0) {

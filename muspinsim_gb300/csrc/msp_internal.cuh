@@ -31,7 +31,7 @@ struct SnapArgs {
     int max_refine;  // MIXED refinement step cap
     const cx<double> *Hsys;
     const cx<double> *Z;
-    // MIXED (optional): Hsys and Z pre-split into double-words, one float4
+    // optional: Hsys and Z pre-split into double-words, one float4
     // (re_hi, im_hi, re_lo, im_lo) per entry, same indexing; NULL: the
     // kernels split the FP64 matrices themselves
     const float4 *Hsys_dw;
@@ -64,7 +64,7 @@ struct SnapArgs {
     double *snap_const;  // num_snap
     int *status;         // num_snap
     int coef_f32;        // n > 64 kernels: pair_coef holds float2 (MIXED) instead of double2
-    void *evec;          // MIXED, n <= 32: num_snap * n * n FP32 complex eigenvectors
+    void *evec;          // n <= 32: num_snap * n * n FP32 complex eigenvectors
                          // (row-major) from the warp Jacobi stage; NULL runs the
                          // single-kernel form
     // Heterogeneous batches (msp_multi_*): when num_seg > 0 the launch's
@@ -171,21 +171,28 @@ size_t snap_smem_bytes(int n, int mode, int precision, int fac_len);
 // (nh + nz float4: Hsys first), for SnapArgs::Hsys_dw / Z_dw.
 cudaError_t launch_split_dw(const double *Hsys, size_t nh, const double *Z, size_t nz,
                             float4 *dst, cudaStream_t st);
-// Two-stage MIXED snapshots (n <= 32): the warp-per-matrix FP32 Jacobi
+// Two-stage snapshots (n <= 32): the warp-per-matrix FP32 Jacobi
 // (msp_jacobi_warp.cu) writes eigenvectors to SnapArgs::evec; the snapshot
 // kernels refine them.  Bytes of that scratch for num_snap snapshots (0 when
 // the form does not apply).
 bool jacobi_warp_supported(int n);
-size_t snap_evec_bytes(int n, long long num_snap, int precision);
+size_t snap_evec_bytes(int n, long long num_snap);
 cudaError_t launch_jacobi_warp(const SnapArgs &a, cudaStream_t st);
 // Householder + QL alternative to the warp Jacobi (msp_ql_warp.cu), same
 // inputs and eigenvector scratch
 bool ql_warp_supported(int n);
 cudaError_t launch_ql_warp(const SnapArgs &a, cudaStream_t st);
-cudaError_t launch_snapshots_refine(const SnapArgs &a, int mode, cudaStream_t st, int threads = 0,
-                                    int grid = 0);
+cudaError_t launch_snapshots_refine(const SnapArgs &a, int mode, int precision, cudaStream_t st,
+                                    int threads = 0, int grid = 0);
 cudaError_t launch_snapshots(const SnapArgs &a, int mode, int precision, cudaStream_t st,
                              int threads = 0, int grid = 0);
+// FP64 snapshots and eigensolver, n <= 64 (msp_snap64.cu).
+size_t snap64_smem_bytes(int n, int fac_len, int threads);
+int snap64_occupancy(int n, int threads, bool pre);
+cudaError_t launch_snapshots64(const SnapArgs &a, int mode, bool pre, cudaStream_t st, int threads,
+                               int grid);
+cudaError_t launch_eigh64(const double *H, int n, int batch, int max_sweeps, double *evals,
+                          double *evecs, int *status, cudaStream_t st);
 // Threads per CTA of the snapshot kernels when the caller gives none.
 int snap_default_threads(int n);
 // CTAs of one snapshot kernel that fit on one SM with `threads` threads.

@@ -255,7 +255,7 @@ static int plan_layout(msp_multi_plan *p, const msp_multi_desc *d) {
         b.off_partial = off;
         off += al256((size_t)b.max_items * T * (records ? 4 : 8));
         b.off_evec = off;
-        off += al256(b.large ? 0 : snap_evec_bytes(b.n, (long long)S, p->precision));
+        off += al256(b.large ? 0 : snap_evec_bytes(b.n, (long long)S));
         b.off_large = off;
         if (b.large) {
             int g = p->sms * b.ctas_per_sm;
@@ -394,7 +394,7 @@ static int plan_enqueue(msp_multi_plan *p, const msp_multi_io *io, cudaStream_t 
             sa.snap_const = reinterpret_cast<double *>(ws + b.off_const);
             sa.status = io->status;
             sa.coef_f32 = mixed;
-            sa.evec = (!b.large && snap_evec_bytes(b.n, 1, p->precision) > 0) ? ws + b.off_evec
+            sa.evec = (!b.large && snap_evec_bytes(b.n, 1) > 0) ? ws + b.off_evec
                                                                                : NULL;
             sa.num_seg = c.num_seg;
             sa.seg_first = reinterpret_cast<const int *>(ws + c.seg_first);
