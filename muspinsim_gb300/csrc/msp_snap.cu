@@ -157,12 +157,14 @@ __global__ void __maxnreg__(64) msp_snap_fast_kernel(SnapArgs a) {
 // Mixed general path: every term C_jk = rho'_jk O'_kj (j >= k, O'_kj =
 // sum_i conj(U_ik) (O U)_ij): pair records (EVOLVE) or the decaying-integral
 // terms (INTEGRAL); returns this thread's share of the constant / integral
-// as a double-word.  NN > 0: n = NN at compile time.
+// as a double-word.  rho' comes from Y, or (hot) from O' itself: (delta_jk +
+// hot_scale O'_jk n) / n.  NN > 0: n = NN at compile time.
 template <bool INTEGRAL, int NN>
 __device__ __forceinline__ float2 rho_terms_mixed(const SnapArgs &a, const SnapSmem<float> &s,
                                                   const cx<float> *U, const cx<float> *OU,
                                                   const cx<float> *Y, int n_rt, int sn,
-                                                  float tau_f, float itau_f) {
+                                                  float tau_f, float itau_f, bool hot,
+                                                  float hot_scale) {
     const int n = NN > 0 ? NN : n_rt, ld = n + (n & 1) + 1;
     const int P = n * (n - 1) / 2, ntri = n * (n + 1) / 2;
     const float scale2 = 2.0f * (float)a.wscale[sn];
@@ -177,7 +179,9 @@ __device__ __forceinline__ float2 rho_terms_mixed(const SnapArgs &a, const SnapS
             orr += u.re * x.re + u.im * x.im;
             oii += u.re * x.im - u.im * x.re;
         }
-        const cx<float> r = Y[j * ld + k];
+        const cx<float> r =
+            hot ? mk<float>(fmaf(hot_scale, orr, j == k ? 1.0f / (float)n : 0.f), -hot_scale * oii)
+                : Y[j * ld + k];
         const float cr = r.re * orr - r.im * oii;
         const float ci = r.re * oii + r.im * orr;
         if (INTEGRAL) {
@@ -208,6 +212,8 @@ __device__ __forceinline__ float2 rho_terms_mixed(const SnapArgs &a, const SnapS
 // pair coefficients of <O>(t) = sum_ij rho'_ij O'_ji exp(-i w_ij t)
 // (muspinsim/hamiltonian.py:80-107); INTEGRAL writes the decaying integral
 // divided by tau (muspinsim/hamiltonian.py:150-164, experiment.py:492-496).
+// At T = inf rho' follows from O' (rho_is_hot), which leaves one eigenbasis
+// product instead of two and the digit products.
 // At most 96 registers (shared memory limits these CTAs to ~4 per SM at n =
 // 32 anyway).
 template <bool INTEGRAL, bool PRE>
@@ -221,25 +227,29 @@ __global__ void __maxnreg__(96) msp_snap_rho_kernel(SnapArgs a) {
     const float itau_f = INTEGRAL ? (float)(1.0 / a.tau) : 0.f;
 
     for (int sn = blockIdx.x; sn < a.num_snap; sn += gridDim.x) {
+        const bool hot = rho_is_hot(a, sn);
         if (a.rho_fac) {
             for (int e = tid; e < a.fac_len; e += nt)
                 s.fac[e] = a.rho_fac[(size_t)sn * a.fac_len + e];
-        } else {
+        } else if (!hot) {
             build_rho_factors(a, sn, s.fac);
         }
         load_hamiltonian<T, true, PRE>(a.Hsys, a.Z, a.Hsys_dw, a.Z_dw, a.field + 3 * (size_t)sn,
                                        n, m, s);
         // made visible by the eigensolve's barriers
-        for (int e = tid; e < a.fac_len; e += nt)
-            s.facf[e] = mk<float>((float)s.fac[e].re, (float)s.fac[e].im);
+        if (!hot)
+            for (int e = tid; e < a.fac_len; e += nt)
+                s.facf[e] = mk<float>((float)s.fac[e].re, (float)s.fac[e].im);
         int st = snap_eigvecs<T, PRE>(a, sn, sn, n, m, s);
         st |= eigenpairs(s, n, m, a.max_refine);
         const cx<T> *U = s.w.U;
 
-        // T1 = rho0 U by Kronecker factors: X ping-pongs between H and B2
-        const cx<T> *X = U;
-        cx<T> *Y = s.w.H;
-        {
+        const cx<T> *X = s.w.H;
+        cx<T> *Y = s.B2;
+        if (!hot) {
+            // rho0 U by Kronecker factors: X ping-pongs between H and B2
+            X = U;
+            Y = s.w.H;
             int off = 0;
             for (int sp = 0; sp < a.num_spins; ++sp) {
                 const int dim = a.dims[sp];
@@ -248,15 +258,15 @@ __global__ void __maxnreg__(96) msp_snap_rho_kernel(SnapArgs a) {
                 X = Y;
                 Y = (Y == s.w.H) ? s.B2 : s.w.H;
             }
+            // X holds rho0 U.  rho'_jk (j >= k) -> Y (the other buffer).
+            if (n == 24)
+                tri_conj_products<T, 24>(U, X, Y, n);
+            else if (n == 32)
+                tri_conj_products<T, 32>(U, X, Y, n);
+            else
+                tri_conj_products<T, 0>(U, X, Y, n);
+            __syncthreads();
         }
-        // X holds rho0 U.  rho'_jk (j >= k) -> Y (the other buffer).
-        if (n == 24)
-            tri_conj_products<T, 24>(U, X, Y, n);
-        else if (n == 32)
-            tri_conj_products<T, 32>(U, X, Y, n);
-        else
-            tri_conj_products<T, 0>(U, X, Y, n);
-        __syncthreads();
         // O U into the buffer X (free now): O = sum_a p_a S^a on the muon digit
         cx<T> *OU = const_cast<cx<T> *>(X);
         {
@@ -279,10 +289,11 @@ __global__ void __maxnreg__(96) msp_snap_rho_kernel(SnapArgs a) {
         }
         __syncthreads();
         // FP32 terms, double-word level gaps and sums
+        const float hs = hot ? (float)rho_hot_scale(a, sn) : 0.f;
         const float2 local =
-            n == 24   ? rho_terms_mixed<INTEGRAL, 24>(a, s, U, OU, Y, n, sn, tau_f, itau_f)
-            : n == 32 ? rho_terms_mixed<INTEGRAL, 32>(a, s, U, OU, Y, n, sn, tau_f, itau_f)
-                      : rho_terms_mixed<INTEGRAL, 0>(a, s, U, OU, Y, n, sn, tau_f, itau_f);
+            n == 24   ? rho_terms_mixed<INTEGRAL, 24>(a, s, U, OU, Y, n, sn, tau_f, itau_f, hot, hs)
+            : n == 32 ? rho_terms_mixed<INTEGRAL, 32>(a, s, U, OU, Y, n, sn, tau_f, itau_f, hot, hs)
+                      : rho_terms_mixed<INTEGRAL, 0>(a, s, U, OU, Y, n, sn, tau_f, itau_f, hot, hs);
         const double sum = dw_block_sum(local, reinterpret_cast<float2 *>(s.w.red));
         if (tid == 0) {
             a.snap_const[sn] = INTEGRAL ? a.wscale[sn] * sum / a.tau : a.wscale[sn] * sum;

@@ -630,6 +630,7 @@ __global__ void __maxnreg__(80) msp_snap64_fast_kernel(SnapArgs a) {
 // coefficients of <O>(t) = sum_ij rho'_ij O'_ji exp(-i w_ij t)
 // (muspinsim/hamiltonian.py:80-107); INTEGRAL writes the decaying integral
 // divided by tau (muspinsim/hamiltonian.py:150-164, experiment.py:492-496).
+// At T = inf rho' follows from O' (rho_is_hot).
 template <bool INTEGRAL, bool PRE>
 __global__ void __maxnreg__(96) msp_snap64_rho_kernel(SnapArgs a) {
     extern __shared__ __align__(16) char smem[];
@@ -640,10 +641,11 @@ __global__ void __maxnreg__(96) msp_snap64_rho_kernel(SnapArgs a) {
     double2 *coef = reinterpret_cast<double2 *>(a.pair_coef);
     const double twopi = 6.283185307179586476925;
     for (int sn = blockIdx.x; sn < a.num_snap; sn += gridDim.x) {
+        const bool hot = rho_is_hot(a, sn);
         if (a.rho_fac) {
             for (int e = tid; e < a.fac_len; e += nt)
                 s.fac[e] = a.rho_fac[(size_t)sn * a.fac_len + e];
-        } else {
+        } else if (!hot) {
             build_rho_factors(a, sn, s.fac);
         }
         SnapSource src;
@@ -654,20 +656,24 @@ __global__ void __maxnreg__(96) msp_snap64_rho_kernel(SnapArgs a) {
         src.Zdw = a.Z_dw;
         const int st = snapshot64<PRE>(a, src, sn, s, n, m, a.fac_len);
         const cx<double> *U = s.D0;
-        // rho0 U by Kronecker factors: X ping-pongs between D1 and D2
-        const cx<double> *X = U;
-        cx<double> *Y = s.D1;
-        int off = 0;
-        for (int sp = 0; sp < a.num_spins; ++sp) {
-            const int dim = a.dims[sp];
-            apply_digit<double>(s.fac + off, dim, a.strides[sp], X, Y, n, m);
-            off += dim * dim;
-            X = Y;
-            Y = (Y == s.D1) ? s.D2 : s.D1;
+        const cx<double> *X = s.D1;
+        cx<double> *Y = s.D2;
+        if (!hot) {
+            // rho0 U by Kronecker factors: X ping-pongs between D1 and D2
+            X = U;
+            Y = s.D1;
+            int off = 0;
+            for (int sp = 0; sp < a.num_spins; ++sp) {
+                const int dim = a.dims[sp];
+                apply_digit<double>(s.fac + off, dim, a.strides[sp], X, Y, n, m);
+                off += dim * dim;
+                X = Y;
+                Y = (Y == s.D1) ? s.D2 : s.D1;
+            }
+            // rho'_jk (j >= k) into the other buffer
+            tri_conj_products<double, 0>(U, X, Y, n);
+            __syncthreads();
         }
-        // rho'_jk (j >= k) into the other buffer
-        tri_conj_products<double, 0>(U, X, Y, n);
-        __syncthreads();
         // O U into the buffer X (free now): O = sum_a p_a S^a on the muon digit
         cx<double> *OU = const_cast<cx<double> *>(X);
         {
@@ -685,7 +691,7 @@ __global__ void __maxnreg__(96) msp_snap64_rho_kernel(SnapArgs a) {
             }
         }
         __syncthreads();
-        const double scale = a.wscale[sn];
+        const double scale = a.wscale[sn], hs = hot ? rho_hot_scale(a, sn) : 0.0;
         double local = 0.0;
         for (int e = tid; e < ntri; e += nt) {
             int j, k;
@@ -701,7 +707,9 @@ __global__ void __maxnreg__(96) msp_snap64_rho_kernel(SnapArgs a) {
                 h1 = fma(-u.im, x.re, h1);
             }
             const double orr = g0 + g1, oii = h0 + h1;
-            const cx<double> r = Y[j * ld + k];
+            // rho'_jk, at T = inf from O'_jk
+            const cx<double> r = hot ? mk<double>(fma(hs, orr, j == k ? 1.0 / n : 0.0), -hs * oii)
+                                     : Y[j * ld + k];
             // C_jk = rho'_jk O'_kj
             const double cr = r.re * orr - r.im * oii, ci = r.re * oii + r.im * orr;
             if (INTEGRAL) {

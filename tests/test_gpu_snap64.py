@@ -87,3 +87,40 @@ def test_snapshots_match_oracle(spins, orient, temperature):
         gammas=sy.gammas, temperature=None if np.isinf(temperature) else temperature)
     assert int(st.max().item()) == 0
     assert np.abs(out.cpu().numpy()[0] - oracle_powder(wl)).max() <= 1e-10
+
+
+# rho0 in its closed forms: T = inf, ground state and thermal snapshots of one
+# launch, a polarisation that is not a unit vector, the muon not first
+@pytest.mark.parametrize("prec,tol", [(_lib.PREC_FP64, 1e-10), (_lib.PREC_MIXED, 1e-6)])
+@pytest.mark.parametrize("mode", [_lib.MODE_EVOLVE, _lib.MODE_INTEGRAL])
+@pytest.mark.parametrize("length", [1.0, 0.5])
+def test_temperatures_of_one_launch(prec, tol, mode, length):
+    rng = np.random.default_rng(3)
+    spins = ["e", "mu", "N"]
+    coup = [("hyperfine", {"i": 2}, workloads.random_hyperfine(rng)),
+            ("hyperfine", {"i": 3}, workloads.random_hyperfine(rng))]
+    temps = np.array([np.inf, 2.0, 0.0, np.inf, 40.0])
+    times = np.linspace(0.0, 10.0, 40)
+    B = rng.normal(size=(5, 3)) * 0.05
+    B[3] = 0.0
+    p = rng.normal(size=(5, 3))
+    p /= np.linalg.norm(p, axis=1)[:, None]
+    wl = workloads.Workload("s", spins, coup, np.zeros((1, 3)), B[:1], p[0], times)
+    sy = wl.system()
+    out, st = kernels.powder_run(
+        12, sy.hamiltonian_matrix(), sy.zeeman_operators(), B, length * p, np.ones(5),
+        np.arange(5, dtype=np.int32), 5, times, mode=mode, precision=prec,
+        dims=list(sy.dimension), mu_index=1, gammas=sy.gammas, temperature=temps, tau=2.197)
+    assert int(st.max().item()) == 0
+    from oracle import port
+    from tests.helpers import oracle_system
+
+    osy = oracle_system(spins, coup)
+    Z = osy.zeeman_operators()
+    for k in range(5):
+        H = osy.hamiltonian() + np.einsum("a,aij->ij", B[k], Z)
+        rho = port.rho0(osy, B[k], p[k], temps[k])
+        op = osy.muon_operator(length * p[k])
+        ref = (port.evolve(H, rho, times, [op])[:, 0].real if mode == _lib.MODE_EVOLVE
+               else port.integrate_decaying(H, rho, 2.197, [op])[:1].real / 2.197)
+        assert np.abs(out[k].cpu().numpy() - ref).max() <= tol
