@@ -15,16 +15,16 @@
 //     Gaussian elimination with partial pivoting (the matrix is regular:
 //     Re lambda <= 0 for a Lindbladian and 1/tau > 0).
 // Same values up to rounding, and no ill-conditioned eigenvector matrix
-// when L is (nearly) defective.  All FP64: the plain drop-in path.
+// when L is (nearly) defective.  FP64 in both precisions.
 //
 // One CTA per superoperator problem; its N x N matrices (N = n^2) live in a
-// per-CTA slice of the caller's workspace (L2-resident for N <= 64).
+// per-CTA slice of the caller's workspace.  The driver's evolution on a
+// uniform grid with N <= 64 takes the real form further down instead.
 #include <math_constants.h>
 #include <string.h>
 
 #include <algorithm>
 
-#include "msp_dw.cuh"
 #include "msp_internal.cuh"
 #include "msp_rho.cuh"
 
@@ -387,8 +387,6 @@ struct LbArgs {
     double *res;             // num_snap x T (real part x wscale)
     zd *scratch;
     size_t scratch_entries;  // per CTA
-    int build_only;          // write L, rho0 and vec(O^T) per snapshot, do not propagate
-    zd *Lout, *vout, *oout;  // num_snap x N^2, N, N
 };
 
 // Two axes orthogonal to z (muspinsim/utils.py:71-93), z a unit vector.
@@ -531,16 +529,6 @@ __global__ void __launch_bounds__(MSP_LB_THREADS) msp_lindblad_kernel(LbArgs a) 
                 __syncthreads();
             }
         }
-        if (a.build_only) {
-            for (int e = tid; e < N * N; e += nt) a.Lout[(size_t)s * N * N + e] = w.L[e];
-            for (int e = tid; e < N; e += nt) {
-                a.vout[(size_t)s * N + e] = w.v[e];
-                a.oout[(size_t)s * N + e] = w.o[e];
-            }
-            if (tid == 0 && sa.status) sa.status[s] = MSP_ITEM_OK;
-            __syncthreads();
-            continue;
-        }
         const double weight = sa.wscale[s];
         double *res = a.res + (size_t)s * a.num_times;
         if (a.integral) {
@@ -555,309 +543,405 @@ __global__ void __launch_bounds__(MSP_LB_THREADS) msp_lindblad_kernel(LbArgs a) 
     }
 }
 
-// ---------------------------------------------------------------- double-word propagation
-// The mixed precision of the evolution mode on a uniform grid, N = n^2 <= 64:
-// L, the propagators and rho live in shared memory as double-word FP32
-// (hi + lo pairs, about 48 significant bits), and every product runs on the
-// FP32 pipe with the anchored compensated accumulation of the Celio kernels:
-// each sum starts at a power of two K >= 4 ||row|| ||column|| (Cauchy-
-// Schwarz bounds every partial sum), so fma(u, x, s), the exact s - t and
-// fma(u, x, s - t) give the sum and its rounding error.  GB300 runs FP64 at
-// 1/64 of the FP32 rate with a 64-cycle dependent-FMA latency; the FP64
-// kernel above stays the reference form.
-constexpr int LBW_MAXN = 64;
+// ---------------------------------------------------------------- real form
+// Evolution on a uniform grid, N = n^2 <= 64 (both precisions).  What bounds it
+// is the FP64 pipe (1/74 of the FP32 rate), so the form with the fewest FP64
+// operations is taken:
+//   * a Lindbladian maps Hermitian matrices to Hermitian ones, so in the
+//     orthonormal Hermitian basis (E_ii, (E_ij + E_ji) / sqrt 2, i (E_ij - E_ji) /
+//     sqrt 2) it is a REAL N x N matrix: one FMA per product term instead of
+//     four;
+//   * exp(A), ||A||_2 <= 0.9 after scaling, is the degree-16 Taylor polynomial
+//     (truncation 5e-16) in powers of A^4 (Paterson and Stockmeyer 1973): six
+//     products instead of thirteen or more;
+//   * samples come from y_{j b + i} = (o^T F^j) (E^i rho0), F = E^b by log2 b
+//     further squarings: b + T / b matrix-vector products instead of T.
+// One CTA per snapshot, everything in shared memory (six N x N matrices; ld =
+// N + 4 keeps the row-parallel matrix-vector product free of bank conflicts);
+// a product is 4 x 4 outputs per thread.  mu, e, 1H (N = 64), 200 snapshots x
+// 1000 times: 34.4 -> 2.4 ms (FP64 as above) and 4.3 -> 2.4 ms (double-word
+// FP32 propagation); 15 products' worth of FMAs on 200 CTAs over 152 SMs.
+constexpr int LBR_MAXN = 64, LBR_THREADS = 256, LBR_GIANTS = 128;
+constexpr int LBR_FAC = 96;  // rho0 factors: sum of d^2 for a product of d up to 8, and spins 0
+constexpr size_t LBR_SMEM_MAX = 224 * 1024;  // beside the kernel's static arrays (3 KB)
 
-constexpr int LBW_THREADS = 256;  // one CTA per SM (shared memory); 512 measured slower
-constexpr int LBW_CHUNK = 256;    // time steps recorded before they are measured
-
-struct LbDwArgs {
-    const zd *L, *v, *o;  // per snapshot: N x N, N, N (from the build-only pass)
-    int n, num_snap, num_times;
-    double t0, dt;
-    const double *wscale;
-    double *res;          // num_snap x T
-    float4 *hist;         // per CTA: LBW_CHUNK x N states awaiting measurement
+struct LbrShape {
+    int b, lg;  // samples per giant step, log2
 };
 
-// <O> of the recorded states hist[0 .. cnt) into res[k0 ..): two threads per
-// state, FP64 sums of the double-word values.
-__device__ void lbw_measure_chunk(const float4 *hist, const double2 *os, int N, int cnt,
-                                  double weight, double *res) {
-    const int tid = threadIdx.x, half = tid & 1, j = tid >> 1;
-    const int h = (N + 1) >> 1, e0 = half * h, e1 = min(N, e0 + h);
-    const int per = blockDim.x >> 1;  // states per pass; every thread runs every pass
-    for (int jj = j; jj < (cnt + per - 1) / per * per; jj += per) {
-        double acc = 0.0;
-        if (jj < cnt)
-            for (int e = e0; e < e1; ++e) {
-                const double2 r = dw_join(hist[(size_t)jj * N + e]), o = os[e];
-                acc = fma(o.x, r.x, fma(-o.y, r.y, acc));
-            }
-        acc += __shfl_xor_sync(0xffffffffu, acc, 1);
-        if (jj < cnt && half == 0) res[jj] = acc * weight;
-    }
-}
-
-// (h, l) * (ch, cl) for one real component, renormalised
-__device__ __forceinline__ void lbw_mul(float &h, float &l, float ch, float cl) {
-    const float p = h * ch;
-    float e = fmaf(h, ch, -p);
-    e = fmaf(h, cl, fmaf(l, ch, e));
-    h = p + e;
-    l = e - (h - p);
-}
-
-// (h, l) + 1 exactly to double-word precision
-__device__ __forceinline__ void lbw_add1(float &h, float &l) {
-    const float s = 1.0f + h;
-    const float bb = s - 1.0f;
-    const float err = (1.0f - (s - bb)) + (h - bb);
-    const float e = l + err;
-    h = s + e;
-    l = e - (h - s);
-}
-
-// Shared-memory position of matrix entry (i, k): odd rows are XOR-swizzled
-// by 4 entries (sw = 4 when N is a multiple of 8, else 0), so that the two
-// rows a quarter-warp reads in the matrix-vector product fall in disjoint
-// bank groups; a permutation inside every row.
-__device__ __forceinline__ int lbw_at(int i, int k, int N, int sw) {
-    return i * N + (k ^ ((i & 1) * sw));
-}
-
-__device__ __forceinline__ void lbw_step(u64 &s1, u64 &c1, u64 &s2, u64 &c2, float4 a, float4 b) {
-    const u64 R = f32x2(a.x, a.x), I = f32x2(a.y, a.y), lR = f32x2(a.z, a.z),
-              lI = f32x2(a.w, a.w);
-    const u64 xh = f32x2(b.x, b.y), xl = f32x2(b.z, b.w);
-    const u64 t1 = fma_f32x2(R, xh, s1);
-    const u64 t2 = fma_f32x2(I, xh, s2);
-    c1 = add2(c1, fma_f32x2(R, xh, sub2(s1, t1)));
-    c2 = add2(c2, fma_f32x2(I, xh, sub2(s2, t2)));
-    s1 = t1;
-    s2 = t2;
-    c1 = fma_f32x2(R, xl, c1);
-    c2 = fma_f32x2(I, xl, c2);
-    c1 = fma_f32x2(lR, xh, c1);
-    c2 = fma_f32x2(lI, xh, c2);
-}
-
-// C = A B (N x N, shared memory); rn, cn: scratch for row / column norms
-__device__ void lbw_gemm(float4 *C, const float4 *A, const float4 *B, int N, float *rn, float *cn,
-                         int sw) {
-    const int tid = threadIdx.x, nt = blockDim.x;
-    for (int q = tid; q < 2 * N; q += nt) {
-        float acc = 0.f;
-        if (q < N) {
-            for (int k = 0; k < N; ++k) {
-                const float4 a = A[q * N + k];  // a whole row, in any order
-                acc = fmaf(a.x, a.x, fmaf(a.y, a.y, acc));
-            }
-            rn[q] = sqrtf(acc);
-        } else {
-            const int j = q - N;
-            for (int k = 0; k < N; ++k) {
-                const float4 b = B[lbw_at(k, j, N, sw)];
-                acc = fmaf(b.x, b.x, fmaf(b.y, b.y, acc));
-            }
-            cn[j] = sqrtf(acc);
+// b = 2^lg minimises log2(b) N^3 + (b + T / b) N^2.
+__host__ __device__ inline LbrShape lbr_shape(int N, int T) {
+    LbrShape s = {1, 0};
+    double best = 1e300;
+    for (int lg = 0; lg <= 6; ++lg) {
+        const double b = (double)(1 << lg), c = lg * (double)N + b + (T + b - 1.0) / b;
+        if (c < best) {
+            best = c;
+            s.b = 1 << lg;
+            s.lg = lg;
         }
     }
-    __syncthreads();
-    // a task is row i and the columns jb, jb + W, jb + 2W, jb + 3W (W = N / 4
-    // rounded up): consecutive threads read consecutive columns of B
-    const int W = (N + 3) >> 2;
-    for (int task = tid; task < N * W; task += nt) {
-        const int i = task / W, jb = task - i * W;
-        u64 s1[4], s2[4], c1[4], c2[4], KK[4];
+    return s;
+}
+
+__host__ __device__ inline size_t lbr_smem_bytes(int n, int num_diss) {
+    const size_t N = (size_t)n * n, M = N * (N + 4);
+    // four matrices, later b + LBR_GIANTS vectors (stride N + 1); two more
+    // matrices; r, o and 3 N of scratch; K and the dissipators
+    const size_t vecs = (64 + (size_t)LBR_GIANTS) * (N + 1);
+    return ((4 * M > vecs ? 4 * M : vecs) + 2 * M + 5 * N) * 8 +
+           (1 + 2 * (size_t)num_diss) * N * 16;
+}
+
+// Row and column of basis element e of the Hermitian basis and its kind (0
+// diagonal, 1 symmetric, 2 antisymmetric): e = i n + j with the diagonal at i =
+// j, symmetric elements above and antisymmetric ones below it.
+__device__ __forceinline__ void lbr_basis(int e, int n, int &i, int &j, int &kind) {
+    const int r = e / n, c = e - r * n;
+    kind = r == c ? 0 : (r < c ? 1 : 2);
+    i = r < c ? r : c;
+    j = r < c ? c : r;
+}
+
+// L_{ij,kl} = K_ik delta_jl + delta_ik conj(K_jl) + sum_d g_d D_ik conj(D_jl).
+__device__ __forceinline__ zd lbr_entry(const zd *K, const zd *D, const double *g, int nd, int n,
+                                        int i, int j, int k, int l) {
+    zd v = mk<double>(0.0, 0.0);
+    if (j == l) v = K[i * n + k];
+    if (i == k) {
+        const zd c = K[j * n + l];
+        v.re += c.re;
+        v.im -= c.im;
+    }
+    for (int d = 0; d < nd; ++d) {
+        const zd a = cscale(g[d], D[(d * n + i) * n + k]), b = D[(d * n + j) * n + l];
+        v.re = fma(a.re, b.re, fma(a.im, b.im, v.re));
+        v.im = fma(a.im, b.re, fma(-a.re, b.im, v.im));
+    }
+    return v;
+}
+
+// f x the superoperator in the Hermitian basis into A (row stride ld).
+__device__ void lbr_matrix(double *A, const zd *K, const zd *D, const double *g, int nd, int n,
+                           int ld, double f) {
+    const int N = n * n;
+    const double r2 = 1.41421356237309504880, h2 = 0.70710678118654752440;
+    for (int e = threadIdx.x; e < N * N; e += blockDim.x) {
+        const int a = e / N, b = e - a * N;
+        int i, j, ka, k, l, kb;
+        lbr_basis(a, n, i, j, ka);
+        lbr_basis(b, n, k, l, kb);
+        // (L B_b)_ij
+        zd v = lbr_entry(K, D, g, nd, n, i, j, k, l);
+        if (kb) {
+            const zd w = lbr_entry(K, D, g, nd, n, i, j, l, k);
+            // symmetric: v + w; antisymmetric: i (v - w)
+            v = kb == 1 ? mk<double>(v.re + w.re, v.im + w.im) : mk<double>(w.im - v.im, v.re - w.re);
+        }
+        // rows: sqrt 2 Re, sqrt 2 Im; columns: 1 / sqrt 2
+        const double x = ka == 2 ? v.im : v.re;
+        A[a * ld + b] = f * x * (ka ? (kb ? 1.0 : r2) : (kb ? h2 : 1.0));
+    }
+}
+
+// C = A B, plus c0 I + c1 P1 + c2 P2 + c3 P3 when P1 is given; C aliases none
+// of A and B.
+__device__ void lbr_gemm(double *C, const double *A, const double *B, int N, int ld,
+                         const double *P1 = nullptr, const double *P2 = nullptr,
+                         const double *P3 = nullptr, double c0 = 0.0, double c1 = 0.0,
+                         double c2 = 0.0, double c3 = 0.0) {
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    const int R = (N + 15) >> 4;  // 16-row bands
+    double acc[4][4];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int j = jb + q * W < N ? jb + q * W : N - 1;
-            const float K = pow2_above(4.01f * rn[i] * cn[j]);
-            KK[q] = f32x2(K, K);
-            s1[q] = s2[q] = KK[q];
-            c1[q] = c2[q] = 0ull;
-        }
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[r][c] = 0.0;
+    if (R == 4) {
+#pragma unroll 2
         for (int k = 0; k < N; ++k) {
-            const float4 a = A[lbw_at(i, k, N, sw)];
+            double a[4], b[4];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int j = jb + q * W < N ? jb + q * W : N - 1;
-                lbw_step(s1[q], c1[q], s2[q], c2[q], a, B[lbw_at(k, j, N, sw)]);
+            for (int r = 0; r < 4; ++r) {
+                a[r] = ty + 16 * r < N ? A[(ty + 16 * r) * ld + k] : 0.0;
+                b[r] = tx + 16 * r < N ? B[k * ld + tx + 16 * r] : 0.0;
+            }
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) acc[r][c] = fma(a[r], b[c], acc[r][c]);
+        }
+    } else {
+        for (int k = 0; k < N; ++k) {
+#pragma unroll
+            for (int r = 0; r < 3; ++r) {
+                if (r >= R || ty + 16 * r >= N) continue;
+                const double a = A[(ty + 16 * r) * ld + k];
+#pragma unroll
+                for (int c = 0; c < 3; ++c)
+                    if (c < R && tx + 16 * c < N)
+                        acc[r][c] = fma(a, B[k * ld + tx + 16 * c], acc[r][c]);
             }
         }
+    }
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
-            if (jb + q * W < N)
-                C[lbw_at(i, jb + q * W, N, sw)] =
-                    dw_finish(sub2(s1[q], KK[q]), c1[q], sub2(s2[q], KK[q]), c2[q]);
-    }
-    __syncthreads();
-}
-
-// y = E x with P lanes per output (P the largest power of two <= 32 with
-// N P <= threads; lane p of an output takes k = p, p + P, ...); xb bounds
-// ||x||_2.
-__device__ void lbw_matvec(float4 *y, const float4 *E, const float4 *x, int N, const float *rE,
-                           float xb, int sw) {
-    const int tid = threadIdx.x, nt = blockDim.x;
-    int P = 1;
-    while (P < 32 && N * P * 2 <= nt) P *= 2;
-    const int part = tid & (P - 1);
-    for (int i0 = 0; i0 < N; i0 += nt / P) {
-        const int i = i0 + tid / P;
-        const bool active = i < N;
-        const int ii = active ? i : 0;
-        const float K = pow2_above(4.01f * rE[ii] * xb);
-        const u64 KK = f32x2(K, K);
-        u64 s1 = KK, s2 = KK, c1 = 0ull, c2 = 0ull;
-        if (active) {
-#pragma unroll 4
-            for (int k = part; k < N; k += P)
-                lbw_step(s1, c1, s2, c2, E[lbw_at(ii, k, N, sw)], x[k]);
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const int i = ty + 16 * r, j = tx + 16 * c;
+            if (i >= N || j >= N) continue;
+            const int o = i * ld + j;
+            double v = acc[r][c];
+            if (P1) v += fma(c1, P1[o], fma(c2, P2[o], fma(c3, P3[o], i == j ? c0 : 0.0)));
+            C[o] = v;
         }
-        s1 = sub2(s1, KK);
-        s2 = sub2(s2, KK);
-        for (int off = 1; off < P; off <<= 1) {
-            const u64 o1 = __shfl_xor_sync(0xffffffffu, s1, off);
-            const u64 o2 = __shfl_xor_sync(0xffffffffu, s2, off);
-            const u64 d1 = __shfl_xor_sync(0xffffffffu, c1, off);
-            const u64 d2 = __shfl_xor_sync(0xffffffffu, c2, off);
-            two_sum2(s1, o1, c1);
-            two_sum2(s2, o2, c2);
-            c1 = add2(c1, d1);
-            c2 = add2(c2, d2);
+    __syncthreads();
+}
+
+// y = E x, four lanes per row.
+__device__ void lbr_matvec(double *y, const double *E, const double *x, int N, int ld) {
+    const int part = threadIdx.x & 3;
+    for (int i = threadIdx.x >> 2; i < ((N + 7) & ~7); i += LBR_THREADS / 4) {
+        double s0 = 0.0, s1 = 0.0;
+        if (i < N)
+            for (int k = part; k < N; k += 8) {
+                s0 = fma(E[i * ld + k], x[k], s0);
+                if (k + 4 < N) s1 = fma(E[i * ld + k + 4], x[k + 4], s1);
+            }
+        s0 += s1;
+        s0 += __shfl_xor_sync(0xffffffffu, s0, 1);
+        s0 += __shfl_xor_sync(0xffffffffu, s0, 2);
+        if (i < N && part == 0) y[i] = s0;
+    }
+    __syncthreads();
+}
+
+// y = x^T F: columns across the lanes, four row groups (red: 3 N doubles).
+__device__ void lbr_vecmat(double *y, const double *F, const double *x, int N, int ld, double *red) {
+    const int j = threadIdx.x & 63, part = threadIdx.x >> 6;
+    double s0 = 0.0, s1 = 0.0;
+    if (j < N)
+        for (int k = part; k < N; k += 8) {
+            s0 = fma(F[k * ld + j], x[k], s0);
+            if (k + 4 < N) s1 = fma(F[(k + 4) * ld + j], x[k + 4], s1);
         }
-        if (active && part == 0) y[i] = dw_finish(s1, c1, s2, c2);
-    }
+    s0 += s1;
+    if (part > 0 && j < N) red[(part - 1) * N + j] = s0;
+    __syncthreads();
+    if (part == 0 && j < N) y[j] = ((s0 + red[j]) + (red[N + j] + red[2 * N + j]));
     __syncthreads();
 }
 
-// row 2-norms of a matrix (any order inside a row), slightly rounded up
-__device__ void lbw_row_norms(const float4 *E, int N, float *r) {
-    for (int i = threadIdx.x; i < N; i += blockDim.x) {
-        float q = 0.f;
-        for (int k = 0; k < N; ++k)
-            q = fmaf(E[i * N + k].x, E[i * N + k].x, fmaf(E[i * N + k].y, E[i * N + k].y, q));
-        r[i] = sqrtf(q) * 1.0001f;
+// exp of the matrix in W[0] (scaled in place); W: six matrices.  Returns the
+// one that holds the result; `spare` another, free one.
+__device__ double *lbr_expm(double *const *W, int N, int ld, double *red, double **spare) {
+    const int tid = threadIdx.x;
+    double *A = W[0];
+    // ||A||_2 <= sqrt(||A||_1 ||A||_inf)
+    double c1 = 0.0, ci = 0.0;
+    if (tid < N) {
+        for (int k = 0; k < N; ++k) {
+            c1 += fabs(A[k * ld + tid]);
+            ci += fabs(A[tid * ld + k]);
+        }
     }
-    __syncthreads();
-}
-
-// exp(f L) by scaling, Horner Taylor-13 and squaring; returns X or T
-__device__ float4 *lbw_expm(const float4 *Ls, float4 *X, float4 *T, int N, double f,
-                            double lnorm, float *rn, float *cn, int sw) {
-    const int tid = threadIdx.x, nt = blockDim.x, NN = N * N;
-    double nrm = lnorm * fabs(f);
+    c1 = lb_block_max(c1, red);
+    ci = lb_block_max(ci, red);
+    double nrm = sqrt(c1 * ci);
     int sq = 0;
-    while (nrm > 0.5 && sq < 64) {
+    while (nrm > 0.9 && sq < 64) {
         nrm *= 0.5;
         ++sq;
     }
-    const double g = ldexp(f, -sq);
-    // logical column of physical entry e: the swizzle is its own inverse
-    for (int e = tid; e < NN; e += nt) {
-        const int i = e / N, j = (e - i * N) ^ ((i & 1) * sw);
-        X[e] = make_float4(i == j ? 1.f : 0.f, 0.f, 0.f, 0.f);
+    const double g = ldexp(1.0, -sq);
+    for (int e = tid; e < N * ld; e += LBR_THREADS) A[e] *= g;
+    __syncthreads();
+    double *A2 = W[1], *A3 = W[2], *A4 = W[3], *X = W[4], *T = W[5];
+    lbr_gemm(A2, A, A, N, ld);
+    lbr_gemm(A3, A2, A, N, ld);
+    lbr_gemm(A4, A2, A2, N, ld);
+    // c_k = 1 / k!
+    double c[17];
+    c[0] = 1.0;
+#pragma unroll
+    for (int k = 1; k <= 16; ++k) c[k] = c[k - 1] / (double)k;
+    for (int e = tid; e < N * N; e += LBR_THREADS) {
+        const int i = e / N, j = e - i * N, o = i * ld + j;
+        X[o] = fma(c[16], A4[o], fma(c[15], A3[o], fma(c[14], A2[o], fma(c[13], A[o], i == j ? c[12] : 0.0))));
     }
     __syncthreads();
-    for (int k = 13; k >= 1; --k) {  // X <- I + (g / k) L X
-        lbw_gemm(T, Ls, X, N, rn, cn, sw);
-        const double c = g / (double)k;
-        const float ch = (float)c, cl = (float)(c - (double)ch);
-        for (int e = tid; e < NN; e += nt) {
-            const int i = e / N, j = (e - i * N) ^ ((i & 1) * sw);
-            float4 t = T[e];
-            lbw_mul(t.x, t.z, ch, cl);
-            lbw_mul(t.y, t.w, ch, cl);
-            if (i == j) lbw_add1(t.x, t.z);
-            X[e] = t;
-        }
-        __syncthreads();
-    }
-    float4 *P = X, *Q = T;
-    for (int q = 0; q < sq; ++q) {
-        lbw_gemm(Q, P, P, N, rn, cn, sw);
-        float4 *t = P;
+    lbr_gemm(T, A4, X, N, ld, A, A2, A3, c[8], c[9], c[10], c[11]);
+    lbr_gemm(X, A4, T, N, ld, A, A2, A3, c[4], c[5], c[6], c[7]);
+    lbr_gemm(T, A4, X, N, ld, A, A2, A3, c[0], c[1], c[2], c[3]);
+    double *P = T, *Q = X;
+    for (int s = 0; s < sq; ++s) {
+        lbr_gemm(Q, P, P, N, ld);
+        double *t = P;
         P = Q;
         Q = t;
     }
+    *spare = Q;
     return P;
 }
 
-__global__ void __launch_bounds__(LBW_THREADS) msp_lindblad_dw_kernel(LbDwArgs a) {
-    extern __shared__ __align__(16) unsigned char lbw_smem[];
+__global__ void __launch_bounds__(LBR_THREADS) msp_lindblad_real_kernel(LbArgs a) {
+    extern __shared__ __align__(16) unsigned char lbr_smem[];
     __shared__ double red[64];
-    const int n = a.n, N = n * n, NN = N * N, tid = threadIdx.x, nt = blockDim.x;
-    float4 *Ls = reinterpret_cast<float4 *>(lbw_smem);
-    float4 *X = Ls + NN, *T = X + NN, *x0 = T + NN, *x1 = x0 + N;
-    double2 *os = reinterpret_cast<double2 *>(x1 + N);
-    float *rn = reinterpret_cast<float *>(os + N), *cn = rn + N, *rE = cn + N;
-    const int sw = (N & 7) == 0 ? 4 : 0;
-    for (int s = blockIdx.x; s < a.num_snap; s += gridDim.x) {
-        const zd *Lg = a.L + (size_t)s * NN;
-        for (int e = tid; e < NN; e += nt) {
-            const int i = e / N, k = e - i * N;
-            Ls[lbw_at(i, k, N, sw)] = dw_split(make_double2(Lg[e].re, Lg[e].im));
+    __shared__ zd fac[LBR_FAC];
+    __shared__ double axes[6], rates[2 * MSP_MAX_SPINS];
+    const SnapArgs &sa = a.sa;
+    const int n = sa.n, N = n * n, ld = N + 4, tid = threadIdx.x, nt = LBR_THREADS;
+    const int s = blockIdx.x, nn = N, nd = 2 * a.num_diss;
+    const size_t M = (size_t)N * ld, vs = N + 1, vecs = (64 + LBR_GIANTS) * vs;
+    double *const base = reinterpret_cast<double *>(lbr_smem);
+    double *const top = base + (4 * M > vecs ? 4 * M : vecs);
+    double *const W[6] = {base, base + M, base + 2 * M, base + 3 * M, top, top + M};
+    double *r = top + 2 * M, *o = r + N, *tmp = o + N;
+    zd *K = reinterpret_cast<zd *>(tmp + 3 * N), *D = K + N;
+
+    const double *b = sa.field + 3 * (size_t)s, *p = sa.pol + 3 * (size_t)s;
+    const double Bn = sqrt(b[0] * b[0] + b[1] * b[1] + b[2] * b[2]);
+    const double Tk = sa.temperature ? sa.temperature[s] : CUDART_INF;
+    build_rho_factors(sa, s, fac);
+    if (tid == 32) {
+        double x[3] = {1.0, 0.0, 0.0}, y[3] = {0.0, 1.0, 0.0};
+        if (Bn != 0.0) {
+            const double z[3] = {b[0] / Bn, b[1] / Bn, b[2] / Bn};
+            lb_get_xy(z, x, y);
         }
-        for (int e = tid; e < N; e += nt) {
-            const zd v = a.v[(size_t)s * N + e], o = a.o[(size_t)s * N + e];
-            x0[e] = dw_split(make_double2(v.re, v.im));
-            os[e] = make_double2(o.re, o.im);
-        }
-        // ||L||_1 (largest column sum, FP64) and ||rho0||_2
-        double cmax = 0.0, v2 = 0.0;
-        for (int j = tid; j < N; j += nt) {
-            double c = 0.0;
-            for (int i = 0; i < N; ++i) c += sqrt(Lg[(size_t)i * N + j].re * Lg[(size_t)i * N + j].re +
-                                                  Lg[(size_t)i * N + j].im * Lg[(size_t)i * N + j].im);
-            cmax = fmax(cmax, c);
-            const zd v = a.v[(size_t)s * N + j];
-            v2 += v.re * v.re + v.im * v.im;
-        }
-        const double lnorm = lb_block_max(cmax, red);
-        const zd vs = lb_block_csum(mk<double>(v2, 0.0), red);
-        // a density matrix keeps ||vec(rho)||_2 = sqrt(Tr rho^2) <= 1
-        const float xb = (float)(fmax(1.0, sqrt(vs.re)) * 1.01);
-        float4 *cur = x0;
-        if (a.t0 != 0.0) {
-            float4 *E0 = lbw_expm(Ls, X, T, N, 2.0 * CUDART_PI * a.t0, lnorm, rn, cn, sw);
-            lbw_row_norms(E0, N, rE);
-            lbw_matvec(x1, E0, cur, N, rE, xb, sw);
-            cur = x1;
-        }
-        const double weight = a.wscale[s];
-        double *res = a.res + (size_t)s * a.num_times;
-        float4 *hist = a.hist + (size_t)blockIdx.x * LBW_CHUNK * N;
-        // state 0
-        for (int e = tid; e < N; e += nt) hist[e] = cur[e];
-        __syncthreads();
-        lbw_measure_chunk(hist, os, N, 1, weight, res);
-        __syncthreads();
-        if (a.num_times > 1) {
-            float4 *E = lbw_expm(Ls, X, T, N, 2.0 * CUDART_PI * a.dt, lnorm, rn, cn, sw);
-            lbw_row_norms(E, N, rE);
-            float4 *nxt = cur == x0 ? x1 : x0;
-            for (int k0 = 1; k0 < a.num_times; k0 += LBW_CHUNK) {
-                const int cnt = min(LBW_CHUNK, a.num_times - k0);
-                for (int q = 0; q < cnt; ++q) {
-                    lbw_matvec(nxt, E, cur, N, rE, xb, sw);
-                    float4 *t = cur;
-                    cur = nxt;
-                    nxt = t;
-                    // cur is only read until the next matvec, which writes nxt
-                    for (int e = tid; e < N; e += nt) hist[(size_t)q * N + e] = cur[e];
-                }
-                __syncthreads();
-                lbw_measure_chunk(hist, os, N, cnt, weight, res + k0);
-                __syncthreads();
-            }
+        for (int k = 0; k < 3; ++k) {
+            axes[k] = x[k];
+            axes[3 + k] = y[k];
         }
     }
-}
-
-static size_t lbw_smem_bytes(int n) {
-    const size_t N = (size_t)n * n;
-    return 3 * N * N * 16 + 2 * N * 16 + N * 16 + 3 * N * 4 + 64;
+    __syncthreads();
+    // S+ and S- about the field of each dissipative spin
+    for (int d = 0; d < a.num_diss; ++d) {
+        const int si = a.diss_spin[d];
+        const double rate = a.diss_rate[d];
+        double Zu = 0.0;
+        if (Tk > 0.0) Zu = exp(-6.62607015e-34 * sa.gammas[si] * Bn * 1e6 / (1.380649e-23 * Tk));
+        const double gp = rate * Zu / (CUDART_PI * (1.0 + Zu)), gm = rate / (CUDART_PI * (1.0 + Zu));
+        const zd *S = a.spin_ops + (size_t)si * 3 * nn;
+        for (int e = tid; e < nn; e += nt) {
+            double xr = 0, xi = 0, yr = 0, yi = 0;
+            for (int c = 0; c < 3; ++c) {
+                const zd sc = S[c * nn + e];
+                xr += axes[c] * sc.re;
+                xi += axes[c] * sc.im;
+                yr += axes[3 + c] * sc.re;
+                yi += axes[3 + c] * sc.im;
+            }
+            D[(2 * d) * nn + e] = mk<double>(xr - yi, xi + yr);
+            D[(2 * d + 1) * nn + e] = mk<double>(xr + yi, xi - yr);
+        }
+        if (tid == 0) {
+            rates[2 * d] = gp;
+            rates[2 * d + 1] = gm;
+        }
+    }
+    // rho0 and the observable in the Hermitian basis
+    const zd *Smu = a.spin_ops + (size_t)sa.mu_index * 3 * nn;
+    for (int e = tid; e < N; e += nt) {
+        int i, j, kind;
+        lbr_basis(e, n, i, j, kind);
+        int off = 0, ri = i, rj = j, stride = n;
+        zd v = mk<double>(1.0, 0.0);
+        for (int q = 0; q < sa.num_spins; ++q) {
+            const int dq = sa.dims[q];
+            stride /= dq;
+            const int di = ri / stride, dj = rj / stride;
+            ri -= di * stride;
+            rj -= dj * stride;
+            v = cmul(v, fac[off + di * dq + dj]);
+            off += dq * dq;
+        }
+        const int q = i * n + j;
+        const zd w = mk<double>(
+            p[0] * Smu[q].re + p[1] * Smu[nn + q].re + p[2] * Smu[2 * nn + q].re,
+            p[0] * Smu[q].im + p[1] * Smu[nn + q].im + p[2] * Smu[2 * nn + q].im);
+        const double r2 = kind ? 1.41421356237309504880 : 1.0;
+        r[e] = r2 * (kind == 2 ? v.im : v.re);
+        o[e] = r2 * (kind == 2 ? w.im : w.re);
+    }
+    __syncthreads();
+    // K = -i H - 1/2 sum_d g_d D^H D
+    for (int e = tid; e < nn; e += nt) {
+        const zd hs = sa.Hsys[e], z0 = sa.Z[e], z1 = sa.Z[nn + e], z2 = sa.Z[2 * nn + e];
+        const double hr = hs.re + b[0] * z0.re + b[1] * z1.re + b[2] * z2.re;
+        const double hi = hs.im + b[0] * z0.im + b[1] * z1.im + b[2] * z2.im;
+        const int i = e / n, j = e - i * n;
+        double kr = hi, ki = -hr;
+        for (int d = 0; d < nd; ++d) {
+            double mr = 0, mi = 0;
+            for (int k = 0; k < n; ++k) {
+                const zd x = D[(d * n + k) * n + i], y = D[(d * n + k) * n + j];
+                mr += x.re * y.re + x.im * y.im;
+                mi += x.re * y.im - x.im * y.re;
+            }
+            kr -= 0.5 * rates[d] * mr;
+            ki -= 0.5 * rates[d] * mi;
+        }
+        K[e] = mk<double>(kr, ki);
+    }
+    __syncthreads();
+    double *spare;
+    if (a.t0 != 0.0) {  // to the first sample
+        lbr_matrix(W[0], K, D, rates, nd, n, ld, 2.0 * CUDART_PI * a.t0);
+        __syncthreads();
+        const double *E0 = lbr_expm(W, N, ld, red, &spare);
+        lbr_matvec(tmp, E0, r, N, ld);
+        for (int e = tid; e < N; e += nt) r[e] = tmp[e];
+        __syncthreads();
+    }
+    const int Tn = a.num_times;
+    const LbrShape sh = lbr_shape(N, Tn);
+    lbr_matrix(W[0], K, D, rates, nd, n, ld, 2.0 * CUDART_PI * a.dt);
+    __syncthreads();
+    double *E = lbr_expm(W, N, ld, red, &spare);
+    // the result and the spare are W[4] and W[5]: vectors go below them
+    double *baby = base, *giant = baby + 64 * vs;
+    for (int e = tid; e < N; e += nt) baby[e] = r[e];
+    __syncthreads();
+    for (int i = 1; i < sh.b; ++i)
+        lbr_matvec(baby + i * vs, E, baby + (i - 1) * vs, N, ld);
+    for (int q = 0; q < sh.lg; ++q) {
+        lbr_gemm(spare, E, E, N, ld);
+        double *t = E;
+        E = spare;
+        spare = t;
+    }
+    const double weight = sa.wscale[s];
+    double *res = a.res + (size_t)s * Tn;
+    const int groups = (Tn + sh.b - 1) / sh.b;
+    for (int e = tid; e < N; e += nt) giant[e] = o[e];
+    __syncthreads();
+    for (int g0 = 0; g0 < groups; g0 += LBR_GIANTS) {
+        const int cnt = min(LBR_GIANTS, groups - g0);
+        if (g0 > 0) {  // continue from the last chunk's final vector
+            lbr_vecmat(o, E, giant + (LBR_GIANTS - 1) * vs, N, ld, tmp);
+            for (int e = tid; e < N; e += nt) giant[e] = o[e];
+            __syncthreads();
+        }
+        for (int j = 1; j < cnt; ++j)
+            lbr_vecmat(giant + j * vs, E, giant + (j - 1) * vs, N, ld, tmp);
+        for (int e = tid; e < cnt * sh.b; e += nt) {
+            const int j = e / sh.b, i = e - j * sh.b;
+            const int k = (g0 + j) * sh.b + i;
+            if (k >= Tn) continue;
+            const double *x = baby + i * vs, *y = giant + j * vs;
+            double s0 = 0.0, s1 = 0.0;
+            int q = 0;
+            for (; q + 1 < N; q += 2) {
+                s0 = fma(x[q], y[q], s0);
+                s1 = fma(x[q + 1], y[q + 1], s1);
+            }
+            if (q < N) s0 = fma(x[q], y[q], s0);
+            res[k] = (s0 + s1) * weight;
+        }
+        __syncthreads();
+    }
+    if (tid == 0 && sa.status) sa.status[s] = MSP_ITEM_OK;
 }
 
 // out[slot][t] = sum of the slot's snapshot results, in snapshot order
@@ -972,30 +1056,18 @@ static int check_lindblad(const msp_lindblad_args *a) {
     return MSP_OK;
 }
 
-// Upper bound of the double-word kernel's grid (SMs x 2): sizes the
-// per-CTA history buffers.
-static int lbw_grid_max() {
-    int dev = 0, sms = 152;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
-        cudaGetLastError();
-        sms = 152;
-    }
-    return 2 * sms;
-}
-
 struct LbLayout {
-    size_t res, slot_first, item_first, scratch, Lb, vb, ob, hb, total;
+    size_t res, slot_first, item_first, scratch, total;
     int T, grid;
-    bool dw;  // double-word propagation (mixed, evolve, uniform grid, n^2 <= 64)
+    bool real;  // the real form: evolution on a uniform grid, n^2 <= 64
 };
 
 static LbLayout lb_layout(const msp_lindblad_args *a) {
     LbLayout L;
     L.T = a->mode == MSP_MODE_INTEGRAL ? 1 : a->num_times;
     L.grid = lb_grid(a->num_snap);
-    L.dw = a->precision == MSP_PREC_MIXED && a->mode == MSP_MODE_EVOLVE && a->uniform &&
-           a->n * a->n <= LBW_MAXN;
+    L.real = a->mode == MSP_MODE_EVOLVE && a->uniform && a->n * a->n <= LBR_MAXN &&
+             lbr_smem_bytes(a->n, a->num_dissipative) <= LBR_SMEM_MAX;
     size_t off = 0;
     auto take = [&](size_t b) {
         const size_t o = off;
@@ -1005,15 +1077,7 @@ static LbLayout lb_layout(const msp_lindblad_args *a) {
     L.res = take((size_t)a->num_snap * L.T * 8);
     L.slot_first = take((size_t)(a->num_slots + 1) * 4);
     L.item_first = take((size_t)(a->num_slots + 1) * 4);
-    L.scratch = take(lb_entries(a->n, 1) * sizeof(zd) * L.grid);
-    L.Lb = L.vb = L.ob = L.hb = 0;
-    if (L.dw) {
-        const size_t N = (size_t)a->n * a->n;
-        L.Lb = take((size_t)a->num_snap * N * N * sizeof(zd));
-        L.vb = take((size_t)a->num_snap * N * sizeof(zd));
-        L.ob = take((size_t)a->num_snap * N * sizeof(zd));
-        L.hb = take((size_t)lbw_grid_max() * LBW_CHUNK * N * 16);
-    }
+    L.scratch = take(L.real ? 0 : lb_entries(a->n, 1) * sizeof(zd) * L.grid);
     L.total = off;
     return L;
 }
@@ -1073,46 +1137,12 @@ int msp_lindblad_run(const msp_lindblad_args *a) {
     la.res = reinterpret_cast<double *>(ws + Lo.res);
     la.scratch = reinterpret_cast<zd *>(ws + Lo.scratch);
     la.scratch_entries = lb_entries(a->n, 1);
-    if (a->num_snap > 0 && Lo.dw) {
-        la.build_only = 1;
-        la.Lout = reinterpret_cast<zd *>(ws + Lo.Lb);
-        la.vout = reinterpret_cast<zd *>(ws + Lo.vb);
-        la.oout = reinterpret_cast<zd *>(ws + Lo.ob);
-        msp_lindblad_kernel<<<Lo.grid, MSP_LB_THREADS, 0, st>>>(la);
-        rc = lb_cuda(cudaGetLastError());
-        if (rc != MSP_OK) return rc;
-        LbDwArgs da;
-        da.L = la.Lout;
-        da.v = la.vout;
-        da.o = la.oout;
-        da.n = a->n;
-        da.num_snap = a->num_snap;
-        da.num_times = Lo.T;
-        da.t0 = a->t0;
-        da.dt = a->dt;
-        da.wscale = a->wscale;
-        da.res = la.res;
-        da.hist = reinterpret_cast<float4 *>(ws + Lo.hb);
-        const size_t smem = lbw_smem_bytes(a->n);
-        rc = lb_cuda(cudaFuncSetAttribute(msp_lindblad_dw_kernel,
+    if (a->num_snap > 0 && Lo.real) {
+        const size_t smem = lbr_smem_bytes(a->n, a->num_dissipative);
+        rc = lb_cuda(cudaFuncSetAttribute(msp_lindblad_real_kernel,
                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         if (rc != MSP_OK) return rc;
-        int occ = 1;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, msp_lindblad_dw_kernel,
-                                                          LBW_THREADS, smem) != cudaSuccess ||
-            occ < 1) {
-            cudaGetLastError();
-            occ = 1;
-        }
-        int dev = 0, sms = 152;
-        if (cudaGetDevice(&dev) != cudaSuccess ||
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
-            cudaGetLastError();
-            sms = 152;
-        }
-        const int grid = (int)std::min<long long>(
-            a->num_snap, std::min<long long>((long long)sms * occ, lbw_grid_max()));
-        msp_lindblad_dw_kernel<<<grid, LBW_THREADS, smem, st>>>(da);
+        msp_lindblad_real_kernel<<<a->num_snap, LBR_THREADS, smem, st>>>(la);
         rc = lb_cuda(cudaGetLastError());
         if (rc != MSP_OK) return rc;
     } else if (a->num_snap > 0) {

@@ -302,10 +302,8 @@ class ExperimentRunner:
 
     def _run_lindblad(self, B_lab, p_lab, T, wscale, rows, nrows, times):
         """Dissipative snapshots on the GPU (msp_lindblad_run): every
-        snapshot's Lindbladian is built and propagated on the device, results
-        reduced into the output rows; the 'mixed' precision propagates in
-        double-word FP32 where that form applies (uniform time grid,
-        n^2 <= 64), FP64 otherwise."""
+        snapshot's Lindbladian is built and propagated on the device in
+        FP64, results reduced into the output rows."""
         from muspinsim_gb300 import _lib
         from muspinsim_gb300.powder import _rows_sorted
 

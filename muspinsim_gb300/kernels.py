@@ -649,9 +649,7 @@ def lindblad_run(n, Hsys, Z, spin_ops, dims, mu_index, gammas, dissipation, fiel
                  precision=_lib.PREC_FP64):
     """A batch of dissipative snapshots reduced into output rows
     (msp_lindblad_run).  ``dissipation``: {spin index: rate}; ``spin_ops``:
-    (num_spins, 3, n, n).  ``precision`` PREC_MIXED propagates in
-    double-word FP32 where it applies (evolution on a uniform grid,
-    n^2 <= 64).  Returns (out, status): out (num_slots, T) or (num_slots,)
+    (num_spins, 3, n, n).  Both precisions run in FP64.  Returns (out, status): out (num_slots, T) or (num_slots,)
     for MODE_INTEGRAL."""
     d = device()
     a = _lib.LindbladArgs()
