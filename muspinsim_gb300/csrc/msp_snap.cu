@@ -462,51 +462,55 @@ cudaError_t launch_assemble(const double *Hsys, const double *Z, const double *f
     return cudaGetLastError();
 }
 
-// out = U^dag M U (adjoint = 0) or U M U^dag (adjoint = 1), FP64, one CTA per
-// matrix, n <= 64: U and M staged in shared memory, T = M U (or M U^dag)
-// kept in shared memory, then out = U^dag T (or U T) written to global.
-__global__ void msp_basis_change_kernel(const cx<double> *__restrict__ U, long long u_stride,
-                                        const cx<double> *__restrict__ M, long long m_stride,
-                                        int n, int batch, int adjoint,
-                                        cx<double> *__restrict__ out) {
+// out = U^dag M U (adjoint = 0) or U M U^dag (adjoint = 1), FP64, n <= 64.  One
+// CTA per MSP_BC_COLS columns of a matrix (few matrices come per call: one
+// CTA for all of a 24 x 24 one took 53 us): T = M U (or M U^dag) for these
+// columns in shared memory, then U^dag T (or U T).
+#define MSP_BC_COLS 4
+__global__ void __launch_bounds__(128) msp_basis_change_kernel(
+    const cx<double> *__restrict__ U, long long u_stride, const cx<double> *__restrict__ M,
+    long long m_stride, int n, int batch, int adjoint, cx<double> *__restrict__ out) {
     extern __shared__ __align__(16) char smem[];
+    const int ld = n + 1;  // odd or even, rows and columns both spread over the banks
     cx<double> *sU = reinterpret_cast<cx<double> *>(smem);
-    cx<double> *sM = sU + n * n;
-    cx<double> *sT = sM + n * n;
+    cx<double> *sT = sU + n * ld;
     const int tid = threadIdx.x, nt = blockDim.x;
+    const int k0 = blockIdx.y * MSP_BC_COLS, kn = n - k0 < MSP_BC_COLS ? n - k0 : MSP_BC_COLS;
     for (int b = blockIdx.x; b < batch; b += gridDim.x) {
         const cx<double> *Ub = U + (size_t)b * u_stride;
         const cx<double> *Mb = M + (size_t)b * m_stride;
-        for (int e = tid; e < n * n; e += nt) {
-            sU[e] = Ub[e];
-            sM[e] = Mb[e];
-        }
+        if (u_stride != 0 || b == (int)blockIdx.x)
+            for (int e = tid; e < n * n; e += nt) sU[(e / n) * ld + e % n] = Ub[e];
         __syncthreads();
-        for (int e = tid; e < n * n; e += nt) {
-            const int i = FastDiv(n).div(e), k = e - i * n;
-            double tr = 0, ti = 0;
+        for (int e = tid; e < n * kn; e += nt) {
+            const int i = e / kn, k = k0 + e - (e / kn) * kn;
+            double r0 = 0, r1 = 0, i0 = 0, i1 = 0;
             for (int l = 0; l < n; ++l) {
-                const cx<double> mv = sM[i * n + l];
+                const cx<double> mv = Mb[i * n + l];
                 // adjoint: (U^dag)_lk = conj(U_kl)
-                const cx<double> uv = adjoint ? conj(sU[k * n + l]) : sU[l * n + k];
-                tr += mv.re * uv.re - mv.im * uv.im;
-                ti += mv.re * uv.im + mv.im * uv.re;
+                const cx<double> uv = adjoint ? conj(sU[k * ld + l]) : sU[l * ld + k];
+                r0 = fma(mv.re, uv.re, r0);
+                r1 = fma(-mv.im, uv.im, r1);
+                i0 = fma(mv.re, uv.im, i0);
+                i1 = fma(mv.im, uv.re, i1);
             }
-            sT[e] = mk<double>(tr, ti);
+            sT[e] = mk<double>(r0 + r1, i0 + i1);
         }
         __syncthreads();
         cx<double> *Ob = out + (size_t)b * n * n;
-        for (int e = tid; e < n * n; e += nt) {
-            const int j = FastDiv(n).div(e), k = e - j * n;
-            double tr = 0, ti = 0;
+        for (int e = tid; e < n * kn; e += nt) {
+            const int j = e / kn, q = e - (e / kn) * kn;
+            double r0 = 0, r1 = 0, i0 = 0, i1 = 0;
             for (int i = 0; i < n; ++i) {
                 // row j of U^dag = conj(U_ij); row j of U = U_ji
-                const cx<double> uv = adjoint ? sU[j * n + i] : conj(sU[i * n + j]);
-                const cx<double> tv = sT[i * n + k];
-                tr += uv.re * tv.re - uv.im * tv.im;
-                ti += uv.re * tv.im + uv.im * tv.re;
+                const cx<double> uv = adjoint ? sU[j * ld + i] : conj(sU[i * ld + j]);
+                const cx<double> tv = sT[i * kn + q];
+                r0 = fma(uv.re, tv.re, r0);
+                r1 = fma(-uv.im, tv.im, r1);
+                i0 = fma(uv.re, tv.im, i0);
+                i1 = fma(uv.im, tv.re, i1);
             }
-            Ob[e] = mk<double>(tr, ti);
+            Ob[(size_t)j * n + k0 + q] = mk<double>(r0 + r1, i0 + i1);
         }
         __syncthreads();
     }
@@ -582,12 +586,12 @@ cudaError_t launch_basis_change(const double *U, long long u_stride, const doubl
         }
         return cudaGetLastError();
     }
-    const size_t smem = (size_t)3 * n * n * sizeof(cx<double>);
+    const size_t smem = ((size_t)n * (n + 1) + (size_t)n * MSP_BC_COLS) * sizeof(cx<double>);
     cudaError_t e = cudaFuncSetAttribute(msp_basis_change_kernel,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    int grid = batch < 152 * 8 ? batch : 152 * 8;
-    msp_basis_change_kernel<<<grid, n <= 16 ? 64 : 256, smem, st>>>(
+    const dim3 grid(batch < 152 * 8 ? batch : 152 * 8, (n + MSP_BC_COLS - 1) / MSP_BC_COLS);
+    msp_basis_change_kernel<<<grid, 128, smem, st>>>(
         reinterpret_cast<const cx<double> *>(U), u_stride,
         reinterpret_cast<const cx<double> *>(M), m_stride, n, batch, adjoint,
         reinterpret_cast<cx<double> *>(out));
