@@ -30,11 +30,15 @@ int record_error(int code, const char *msg);
 static size_t adj_align(size_t x) { return (x + 255) & ~(size_t)255; }
 
 struct AdjointLayout {
-    size_t H, evecs, evals, Gh, Gd, total;
+    size_t H, evecs, evals, Gh, Gd, nufft, total;
+    bool fourier;  // G by a nonuniform Fourier transform (msp_nufft.cu)
+    NufftShape nu;
 };
 
-static AdjointLayout adjoint_layout(int n, int S) {
+// `lean`: without the transform's workspace (callers with a fixed scratch).
+static AdjointLayout adjoint_layout(const msp_adjoint_args *a, bool lean = false) {
     AdjointLayout L;
+    const int n = a->n, S = a->num_snap;
     const size_t mat = adj_align((size_t)S * n * n * 16);
     size_t off = 0;
     L.H = off;  // assembled H; later the per-snapshot gradients
@@ -47,6 +51,11 @@ static AdjointLayout adjoint_layout(int n, int S) {
     off += mat;
     L.Gd = off;
     off += mat;
+    L.nufft = off;
+    L.fourier = !lean && a->uniform &&
+                nufft_adjoint_shape((long long)S * (n * (n + 1) / 2), a->num_slots, a->num_times,
+                                    &L.nu);
+    if (L.fourier) off += adj_align(L.nu.bytes);
     L.total = off;
     return L;
 }
@@ -322,7 +331,7 @@ int msp_adjoint_workspace(const msp_adjoint_args *a, size_t *bytes) {
     const int rc = adj_check(a);
     if (rc != MSP_OK) return rc;
     if (bytes == NULL) return adj_fail(MSP_ERR_ARG, "msp_adjoint_workspace: bytes is NULL");
-    *bytes = adjoint_layout(a->n, a->num_snap).total;
+    *bytes = adjoint_layout(a).total;
     return MSP_OK;
 }
 
@@ -337,7 +346,8 @@ int msp_adjoint_fast(const msp_adjoint_args *a) {
     if (!a->Hsys || !a->Z || !a->field || !a->pol || !a->wscale || !a->slot || !a->grad_out ||
         !a->status)
         return adj_fail(MSP_ERR_ARG, "msp_adjoint: a required pointer is NULL");
-    const AdjointLayout L = adjoint_layout(n, S);
+    AdjointLayout L = adjoint_layout(a);
+    if (a->workspace_bytes < L.total) L = adjoint_layout(a, true);
     if (a->workspace == NULL || a->workspace_bytes < L.total)
         return adj_fail(MSP_ERR_WORKSPACE, "msp_adjoint: workspace too small");
     if (reinterpret_cast<uintptr_t>(a->workspace) & 255)
@@ -375,7 +385,12 @@ int msp_adjoint_fast(const msp_adjoint_args *a) {
         free(th);
     }
 
-    {
+    if (L.fourier) {
+        rc = adj_cuda(launch_nufft_adjoint(L.nu, ws + L.nufft, lam, n, S, a->slot, a->grad_out,
+                                           a->num_slots, a->t0, a->dt, Gh, Gd, st),
+                      "msp_adjoint transform");
+        if (rc != MSP_OK) return rc;
+    } else {
         const long long items = (long long)S * (n * (n + 1) / 2);
         long long blocks = (items + 7) / 8;
         if (blocks > 152 * 16) blocks = 152 * 16;

@@ -230,6 +230,11 @@ cudaError_t launch_nufft_spread(const PhaseArgs &a, const NufftShape &s, int pre
                                 cudaStream_t st);
 cudaError_t launch_nufft_rows(const PhaseArgs &a, const NufftShape &s, int precision, char *ws,
                               const double *snap_const, double *out, cudaStream_t st);
+// The adjoint's transform of a gradient row at every level difference.
+bool nufft_adjoint_shape(long long points, int slots, int T, NufftShape *out);
+cudaError_t launch_nufft_adjoint(const NufftShape &s, char *ws, const double *evals, int n, int S,
+                                 const int *slot, const double *g, int slots, double t0, double dt,
+                                 cx<double> *Gh, cx<double> *Gd, cudaStream_t st);
 
 cudaError_t launch_fast_cos_sum(const double *times, int num_times, int d, const double *A,
                                 const double *W, int n, double *out, cudaStream_t st);

@@ -36,6 +36,7 @@
 //      F[g1][q] = sum_g2 b e^{2 pi i g2 q / n2}, then
 //      f(k) = Re sum_g1 e^{2 pi i g1 k / G} F[g1][k mod n2].
 #include <math.h>
+#include <string.h>
 
 #include <type_traits>
 
@@ -673,6 +674,171 @@ NuArgs nu_args(const NufftShape &s, int precision, char *ws) {
     return na;
 }
 
+// ------------------------------------------------------------------ adjoint direction
+//
+// G(nu) = sum_k g_k e^{2 pi i nu t_k} and H(nu) = sum_k t_k g_k e^{2 pi i nu
+// t_k} of a row of samples g on t_k = t0 + k dt at many frequencies: with the
+// same window, U_j = sum_k (g_k / phi^(k)) e^{2 pi i j k / G} and
+// G(nu) = e^{2 pi i nu t0} sum_j phi(j - s) U_j, s = nu dt G mod G.  U is
+// conjugate-symmetric (g real): only j = 0 .. m is kept.
+
+struct __align__(16) NuCell {
+    double gr, gi, hr, hi;  // U of g and of t g
+};
+
+// F[k1][q] = sum_k2 h_{k1 + n1 k2} e^{2 pi i k2 q / n2}, q <= n2 / 2; one CTA per
+// (k1, which of g and t g, row).
+__global__ void __launch_bounds__(64) msp_nufft_adj_dft1_kernel(NuArgs na, const double *__restrict__ g,
+                                                                int T, double t0, double dt) {
+    extern __shared__ __align__(16) double sm[];
+    const int k1 = blockIdx.x, which = blockIdx.y, n1 = na.n1, n2 = na.n2, h = n2 / 2 + 1;
+    double2 *tw = reinterpret_cast<double2 *>(sm);
+    double *u = sm + 2 * n2;
+    const double *row = g + (size_t)blockIdx.z * T;
+    const int cnt = k1 < T ? (T - 1 - k1) / n1 + 1 : 0;
+    for (int i = threadIdx.x; i < n2; i += 64) tw[i] = na.root[(size_t)i * n1];
+    for (int i = threadIdx.x; i < cnt; i += 64) {
+        const int k = k1 + n1 * i;
+        u[i] = row[k] * na.win[k] * (which ? t0 + (double)k * dt : 1.0);
+    }
+    __syncthreads();
+    double2 *F = na.spec + (((size_t)blockIdx.z * 2 + which) * n1 + k1) * h;
+    for (int q = threadIdx.x; q < h; q += 64) {
+        double re[2] = {0.0, 0.0}, im[2] = {0.0, 0.0};
+        int idx = 0;
+        for (int i = 0; i < cnt; ++i) {
+            const double2 t = tw[idx];
+            re[i & 1] = fma(u[i], t.x, re[i & 1]);
+            im[i & 1] = fma(u[i], t.y, im[i & 1]);
+            idx += q;
+            if (idx >= n2) idx -= n2;
+        }
+        F[q] = make_double2(re[0] + re[1], im[0] + im[1]);
+    }
+}
+
+// U_j = sum_k1 e^{2 pi i j k1 / G} F[k1][j mod n2], j = 0 .. m, as (G, H) pairs:
+// 32 cells per CTA, 4 threads per cell and quantity.
+__global__ void __launch_bounds__(256) msp_nufft_adj_dft2_kernel(NuArgs na, NuCell *__restrict__ grid) {
+    __shared__ double2 red[8][32];
+    const int kk = threadIdx.x & 31, part = (threadIdx.x >> 5) & 3, which = threadIdx.x >> 7;
+    const int n1 = na.n1, n2 = na.n2, h = n2 / 2 + 1, G = 2 * na.m;
+    const int j = blockIdx.x * 32 + kk;
+    double c = 0.0, s = 0.0;
+    if (j <= na.m) {
+        const int qf = j % n2;
+        const bool mir = qf >= h;
+        const int q = mir ? n2 - qf : qf;
+        const double sg = mir ? -1.0 : 1.0;
+        const double2 *F = na.spec + ((size_t)blockIdx.y * 2 + which) * n1 * h + q;
+        long long x = (long long)part * j % G;
+        const long long step = 4LL * j % G;
+        for (int k1 = part; k1 < n1; k1 += 4) {
+            const double2 e = na.root[x], f = F[(size_t)k1 * h];
+            c = fma(e.x, f.x, fma(-sg * e.y, f.y, c));
+            s = fma(e.y, f.x, fma(sg * e.x, f.y, s));
+            x += step;
+            if (x >= G) x -= G;
+        }
+    }
+    red[which * 4 + part][kk] = make_double2(c, s);
+    __syncthreads();
+    if (threadIdx.x < 32 && j <= na.m) {
+        double2 v[2];
+#pragma unroll
+        for (int w = 0; w < 2; ++w) {
+            v[w] = make_double2(0.0, 0.0);
+#pragma unroll
+            for (int p = 0; p < 4; ++p) {
+                v[w].x += red[w * 4 + p][kk].x;
+                v[w].y += red[w * 4 + p][kk].y;
+            }
+        }
+        grid[(size_t)blockIdx.y * (na.m + 1) + j] = NuCell{v[0].x, v[0].y, v[1].x, v[1].y};
+    }
+}
+
+// One thread per (snapshot, a <= b): G and 2 pi i H at nu = l_b - l_a into the
+// full n x n tables (G(-nu) = conj G(nu), H likewise).
+__global__ void __launch_bounds__(128) msp_nufft_adj_eval_kernel(
+    NuArgs na, const NuCell *__restrict__ grid, const double *__restrict__ evals, int n, int S,
+    const int *__restrict__ slot, double t0, double dt, cx<double> *__restrict__ Gh,
+    cx<double> *__restrict__ Gd) {
+    extern __shared__ __align__(16) char smtab[];
+    constexpr int W = NU_W64;
+    for (int e = threadIdx.x; e < NU_TAB_BYTES / 16; e += 128)
+        reinterpret_cast<uint4 *>(smtab)[e] = reinterpret_cast<const uint4 *>(na.tab)[e];
+    __syncthreads();
+    const int ntri = n * (n + 1) / 2, m = na.m;
+    const long long items = (long long)S * ntri;
+    const double twopi = 6.283185307179586476925;
+    for (long long it = (long long)blockIdx.x * 128 + threadIdx.x; it < items;
+         it += (long long)gridDim.x * 128) {
+        const int s = (int)(it / ntri), e = (int)(it - (long long)s * ntri);
+        // e -> (b, a), b >= a, e = b (b + 1) / 2 + a
+        int b = (int)((sqrtf(8.0f * e + 1.0f) - 1.0f) * 0.5f);
+        while ((b + 1) * (b + 2) / 2 <= e) ++b;
+        while (b * (b + 1) / 2 > e) --b;
+        const int a = e - b * (b + 1) / 2;
+        const double nu = evals[(size_t)s * n + b] - evals[(size_t)s * n + a];
+        // cycles per sample, reduced to [-1/2, 1/2]
+        const double p = nu * dt;
+        double f = (p - rint(p)) + fma(nu, dt, -p);
+        const bool neg = f < 0.0;
+        f = fabs(f);
+        const double x = f * (2.0 * m) - 0.5 * W;
+        cx<double> hg = mk<double>(CUDART_NAN, CUDART_NAN), hd = hg;
+        if (x >= -W && x <= m) {
+            const double first = ceil(x), frac = first - x;
+            int k = (int)(frac * NU_SUB);
+            k = k < 0 ? 0 : (k > NU_SUB - 1 ? NU_SUB - 1 : k);
+            const double dl = frac - ((double)k + 0.5) * (1.0 / NU_SUB);
+            const float df = (float)dl;
+            const double *hi = reinterpret_cast<const double *>(smtab) + k * 4 * W;
+            const float4 *lo = reinterpret_cast<const float4 *>(smtab + NU_ENTRIES * 32) + k * W;
+            const NuCell *row = grid + (size_t)slot[s] * (m + 1);
+            double gr = 0.0, gi = 0.0, dr = 0.0, di = 0.0;
+#pragma unroll 4
+            for (int c = 0; c < W; ++c) {
+                const float4 t4 = lo[c];
+                const float t = fmaf(df, fmaf(df, fmaf(df, t4.w, t4.z), t4.y), t4.x);
+                const double v = fma(dl, fma(dl, fma(dl, fma(dl, (double)t, hi[3 * W + c]), hi[2 * W + c]),
+                                             hi[W + c]),
+                                     hi[c]);
+                const int j = (int)first + c, g = nu_fold(j, m);
+                const double vi = j == g ? v : -v;  // folded cells hold the conjugate
+                const NuCell u = row[g];
+                gr = fma(v, u.gr, gr);
+                gi = fma(vi, u.gi, gi);
+                dr = fma(v, u.hr, dr);
+                di = fma(vi, u.hi, di);
+            }
+            if (neg) {
+                gi = -gi;
+                di = -di;
+            }
+            hg = mk<double>(gr, gi);
+            hd = mk<double>(dr, di);
+            if (t0 != 0.0) {
+                double sn, cs;
+                const double q = nu * t0;
+                sincospi(2.0 * ((q - rint(q)) + fma(nu, t0, -q)), &sn, &cs);
+                const cx<double> w = mk<double>(cs, sn);
+                hg = cmul(w, hg);
+                hd = cmul(w, hd);
+            }
+        }
+        const cx<double> d2 = mk<double>(-twopi * hd.im, twopi * hd.re);
+        const size_t base = (size_t)s * n * n;
+        Gh[base + (size_t)a * n + b] = hg;
+        Gd[base + (size_t)a * n + b] = d2;
+        if (a != b) {
+            Gh[base + (size_t)b * n + a] = conj(hg);
+            Gd[base + (size_t)b * n + a] = mk<double>(-d2.re, d2.im);
+        }
+    }
+}
+
 }  // namespace
 
 cudaError_t launch_nufft_spread(const PhaseArgs &a, const NufftShape &s, int precision, char *ws,
@@ -701,6 +867,71 @@ cudaError_t launch_nufft_rows(const PhaseArgs &a, const NufftShape &s, int preci
                             (size_t)(2 * s.n2 + s.n2 / 2 + 1) * 8, st>>>(na);
     msp_nufft_dft2_kernel<<<dim3((s.tt + NU_OUT_K - 1) / NU_OUT_K, s.tiles, a.num_slots),
                             NU_OUT_K * NU_OUT_PARTS, 0, st>>>(a, na, out);
+    return cudaGetLastError();
+}
+
+// Shape of the adjoint transform: `points` frequencies against `slots` rows of
+// T uniform samples.  False when the direct sums are cheaper: they run 35
+// samples per ns (14 FP64 operations each, 72,000 x 1000 in 1.97 ms), the
+// transform costs 25 us of launches, 8 T n1 FMAs per row and 140 per frequency.
+bool nufft_adjoint_shape(long long points, int slots, int T, NufftShape *out) {
+    if (T < 64 || T > (1 << 22) || points < 1 || slots < 1) return false;
+    NufftShape s;
+    memset(&s, 0, sizeof(s));
+    s.tiles = 1;
+    s.tt = T;
+    s.n2 = 2 * (int)ceil(sqrt((double)T));
+    s.n1 = (4 * T + s.n2 - 1) / s.n2;
+    s.m = s.n1 * s.n2 / 2;
+    const double direct = (double)points * T / 35.0;
+    const double dft = (double)slots * (8.0 * s.m * s.n1 + 1.0 * T * s.n2) / 400.0;
+    if (25000.0 + dft + (double)points * 140.0 / 400.0 > direct) return false;
+    size_t off = 0;
+    s.off_root = off;
+    off += al256((size_t)2 * s.m * 16);
+    s.off_win = off;
+    off += al256((size_t)T * 8);
+    s.off_tab = off;
+    off += al256(NU_TAB_BYTES);
+    s.off_spec = off;
+    off += al256((size_t)slots * 2 * s.n1 * (s.n2 / 2 + 1) * 16);
+    s.off_rows = off;
+    off += al256((size_t)slots * (s.m + 1) * 32);
+    s.bytes = off;
+    *out = s;
+    return true;
+}
+
+// Fills the adjoint's tables G(l_b - l_a) and G'(l_b - l_a) of every snapshot.
+cudaError_t launch_nufft_adjoint(const NufftShape &s, char *ws, const double *evals, int n, int S,
+                                 const int *slot, const double *g, int slots, double t0, double dt,
+                                 cx<double> *Gh, cx<double> *Gd, cudaStream_t st) {
+    const NuArgs na = nu_args(s, MSP_PREC_FP64, ws);
+    NuCell *grid = reinterpret_cast<NuCell *>(ws + s.off_rows);
+    const int tabs = NU_ENTRIES * NU_DEG / 32;
+    msp_nufft_tables_kernel<<<tabs + (2 * s.m + 31) / 32, 32, 0, st>>>(na, NU_W64, tabs);
+    const int depth = (s.tt + s.n1 - 1) / s.n1;
+    const size_t smem = (size_t)(2 * s.n2 + depth) * 8;
+    cudaError_t e = cudaFuncSetAttribute(msp_nufft_adj_dft1_kernel,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    for (int r0 = 0; r0 < slots; r0 += 65535) {
+        const int rn = slots - r0 < 65535 ? slots - r0 : 65535;
+        NuArgs nr = na;
+        nr.spec += (size_t)r0 * 2 * s.n1 * (s.n2 / 2 + 1);
+        msp_nufft_adj_dft1_kernel<<<dim3(s.n1, 2, rn), 64, smem, st>>>(nr, g + (size_t)r0 * s.tt, s.tt,
+                                                                       t0, dt);
+        msp_nufft_adj_dft2_kernel<<<dim3((s.m + 32) / 32, rn), 256, 0, st>>>(
+            nr, grid + (size_t)r0 * (s.m + 1));
+    }
+    e = cudaFuncSetAttribute(msp_nufft_adj_eval_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             NU_TAB_BYTES);
+    if (e != cudaSuccess) return e;
+    const long long items = (long long)S * (n * (n + 1) / 2);
+    long long blocks = (items + 127) / 128;
+    if (blocks > 152 * 8) blocks = 152 * 8;
+    msp_nufft_adj_eval_kernel<<<(int)blocks, 128, NU_TAB_BYTES, st>>>(na, grid, evals, n, S, slot, t0,
+                                                                     dt, Gh, Gd);
     return cudaGetLastError();
 }
 

@@ -80,3 +80,29 @@ def test_non_finite_inputs_stay_non_finite():
     times = np.linspace(0.0, 19.0, 777)
     a, _ = _curves(8, 700, times, 2, _lib.MODE_FAST, _lib.PREC_FP64, np.nan)
     assert np.isnan(a).all()
+
+
+# the adjoint's transform against the direct sums (a grid that is not uniform,
+# its moved last sample without weight); the gradients are sums over 1e5 terms
+# with phases rounded to 1e-11: 1e-9 of their norm
+@pytest.mark.parametrize("dim,orient,nt,slots,t0", [(8, 300, 777, 1, 0.0), (8, 300, 777, 3, 0.4),
+                                                    (4, 2000, 64, 1, 0.0), (24, 40, 4097, 2, -1.0)])
+def test_adjoint_matches_direct_sum(dim, orient, nt, slots, t0):
+    times = np.linspace(t0, t0 + 12.0, nt)
+    moved = times.copy()
+    moved[-1] *= 1.0 + 1e-9
+    assert kernels.uniform_grid(times)[0] and not kernels.uniform_grid(moved)[0]
+    rng = np.random.default_rng(nt)
+    wl = workloads.random_system_workload(rng, dim, zcw_gen(orient), times, (0.0, 0.0, 0.02))
+    sy = wl.system()
+    qs, _ = orientation_rows_to_quats(wl.orientations)
+    B, p = Q.rotate(qs, wl.fields[0]), Q.rotate(qs, wl.polarization)
+    slot = np.sort(np.arange(orient) % slots).astype(np.int32)
+    g = rng.normal(size=(slots, nt))
+    g[:, -1] = 0.0
+    got = [kernels.adjoint_fast(dim, sy.hamiltonian_matrix(), sy.zeeman_operators(), B, p,
+                                np.full(orient, 1 / orient), slot, slots, t, g)
+           for t in (times, moved)]
+    for a, b in zip(got[0][:2], got[1][:2]):
+        a, b = a.cpu().numpy(), b.cpu().numpy()
+        assert np.linalg.norm(a - b) <= 1e-9 * np.linalg.norm(b)
