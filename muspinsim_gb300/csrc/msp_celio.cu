@@ -84,6 +84,7 @@ struct CeArgs {
     double2 *state;        // global path: [S*A][V] (double2, or float4 hi/lo pairs when dw)
     double *partial;       // global path: [S*A][chunks][2 nops]
     int chunks;
+    const int *done;       // shared-memory paths: states already evolved (NULL: none)
     void *dwmats;          // global double-word path: factor entries in lane patterns
     float *rnorms;         // global double-word path: [blocks][nf] row 2-norm bounds
 };
@@ -278,6 +279,7 @@ __global__ void __launch_bounds__(CE_THREADS) msp_celio_smem_kernel(CeArgs a) {
     const int V32 = (int)a.V;
     int loaded = -1;
     for (int st = blockIdx.x; st < a.S * a.A; st += gridDim.x) {
+        if (a.done && a.done[st]) continue;
         const int s = st / a.A;
         const int blk = a.mats_per_snap ? s : 0;
         if (blk != loaded) {
@@ -517,6 +519,7 @@ __global__ void __launch_bounds__(CE_DW_THREADS) msp_celio_smem_dw_kernel(CeArgs
     const int msk = (V32 & 7) == 0 ? 7 : 0;
     int loaded = -1;
     for (int st = blockIdx.x; st < a.S * a.A; st += gridDim.x) {
+        if (a.done && a.done[st]) continue;
         const int s = st / a.A;
         const int blk = a.mats_per_snap ? s : 0;
         if (blk != loaded) {
@@ -589,6 +592,372 @@ __global__ void __launch_bounds__(CE_DW_THREADS) msp_celio_smem_dw_kernel(CeArgs
                 }
             }
         }
+        __syncthreads();
+    }
+}
+
+// ----------------------------------------------------------- fixed-point tensor path
+// States in shared memory as 64-bit fixed-point numbers, group products on the
+// tensor cores with exact integer arithmetic -- both precisions, whenever every
+// factor is unitary with D <= 16 (checked on the device; a state that is not
+// taken here runs in the kernels above instead).
+//
+// What bounds the FP64 form is the FP64 pipe (1/74 of the FP32 rate): 4 D FMAs
+// per element and factor.  A unitary factor keeps the state's norm, so x = v
+// 2^-F with |v| <= 2^58 never overflows, and its absolute resolution (2^-58 of
+// the norm) is finer than an FP64 element's (2^-53 of elements of size
+// V^(-1/2)).  u and x are split into six balanced digits of ten bits, |d| <=
+// 512, exact in FP16; u_s x_t digit products summed over a group (K = 16) are
+// integers of at most 2^22, exact in FP32 accumulators, so
+//   y = sum_{s + t >= 4} 2^(10 (s + t) - 58) (u_s . x_t)
+// has an error of 2^-4 units (the dropped levels) before its rounding.  A group
+// is one column of an m16n8k16 MMA (U the 16 x 16 operand; smaller D: 16 / D
+// groups per column, U block-diagonal), 26 digit pairs x 4 real products per 8
+// columns.  The largest accumulator is tracked: one that reached 2^24, where
+// FP32 stops being exact, disqualifies the state.
+//
+// Single-spin factors are first multiplied into a two-spin factor on the same
+// digit where only factors on other digits lie between (they commute), so
+// mu + n V takes n products per pass instead of 2 n.
+constexpr int FX_DIGITS = 6, FX_THREADS = 256;
+constexpr int FX_LOW = 4, FX_LEVELS = 2 * FX_DIGITS - 1 - FX_LOW;  // levels s + t >= 4
+constexpr int FX_FRAG = FX_DIGITS * 2 * 32;  // uint4 per factor: [digit][re, im][lane]
+
+struct FxOp {
+    long long mat;  // source matrix
+    int D, where;   // acts on the factor's first digit (0), second (1) or both (2)
+    int right, pad; // multiplied from the right (an earlier factor) or the left
+};
+
+struct FxFactor {
+    CeFactor f;     // digits, strides, D (f.mat unused)
+    int D0, D1;     // dims in the factor's own order
+    int op0, ops;   // its products, base matrix first
+    int p, groups;  // groups per MMA column, V / D
+    int base0;      // first of its group bases
+    int pad;
+};
+
+struct FxArgs {
+    CeArgs c;
+    const FxFactor *fac;
+    const FxOp *ops;
+    int nf, nbase;
+    uint4 *frag;  // [block][nf][FX_FRAG]
+    int *good;    // [block]: every factor unitary
+    int *done;    // [state]
+};
+
+// A state entry's place: the low three bits XORed with the next nine in threes,
+// so that a fragment's 8 x 16 bytes at strides 1, 8, 64 and 512 entries fall in
+// distinct banks.  A permutation inside every aligned block of 8 entries.
+__device__ __forceinline__ int fx_swz(int x) { return x ^ (((x >> 3) ^ (x >> 6) ^ (x >> 9)) & 7); }
+
+// v + FX_BIAS has the digits plus 512 as its ten-bit fields.
+#define FX_BIAS 0x0802008020080200ull  // sum_s 512 2^(10 s), s < 6
+
+__device__ __forceinline__ unsigned fx_field(unsigned long long v, int s) {
+    return (unsigned)(v >> (10 * s)) & 1023u;
+}
+
+// FP16 pair of digit s of two biased values (1024 + field is exact, minus 1536).
+__device__ __forceinline__ unsigned fx_pair(unsigned long long a, unsigned long long b, int s) {
+    const unsigned w = fx_field(a, s) | fx_field(b, s) << 16 | 0x64006400u;
+    unsigned r;
+    asm("add.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(w), "r"(0xE600E600u));
+    return r;
+}
+
+__device__ __forceinline__ void fx_mma(float (&c)[4], const uint4 &a, unsigned b0, unsigned b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+        "{%0,%1,%2,%3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b0), "r"(b1));
+}
+
+// sum_l a_l 2^(10 (l + FX_LOW) - 58), rounded to the unit (levels 4 and 5 lie
+// below or across it).
+__device__ __forceinline__ long long fx_join(const float (&a)[FX_LEVELS]) {
+    long long y = (long long)__float2int_rn(a[1]) * 1024 + (__float2int_rn(a[0]) + (1 << 17));
+    y >>= 18;
+    y += (long long)__float2int_rn(a[2]) * (1 << 2);
+    y += (long long)__float2int_rn(a[3]) * (1 << 12);
+    y += (long long)__float2int_rn(a[4]) * (1 << 22);
+    y += (long long)((unsigned long long)(unsigned)__float2int_rn(a[5]) << 32);
+    y += (long long)((unsigned long long)((unsigned)__float2int_rn(a[6]) << 10) << 32);
+    return y;
+}
+
+// hi + lo += a b (the product's and the sum's rounding errors into lo).
+__device__ __forceinline__ void fx_acc(double &hi, double &lo, double a, double b) {
+    const double p = __dmul_rn(a, b), e = fma(a, b, -p);
+    const double t = __dadd_rn(hi, p), bb = __dsub_rn(t, hi);
+    lo += e + (__dadd_rn(__dsub_rn(hi, __dsub_rn(t, bb)), __dsub_rn(p, bb)));
+    hi = t;
+}
+
+// 2^58 (hi + lo), rounded.
+__device__ __forceinline__ long long fx_round(double hi, double lo) {
+    const double h = hi * 0x1p58;
+    const long long r = __double2ll_rn(h);
+    return r + __double2ll_rn((h - (double)r) + lo * 0x1p58);
+}
+
+// Products of the merged factors, their unitarity and their digit fragments;
+// one CTA of 256 threads per (factor, matrix block).  The products are
+// double-double: a merged factor acts thousands of times, so its rounding
+// would add up where that of separate factors averages out.
+__global__ void __launch_bounds__(256) msp_celio_fx_prep_kernel(FxArgs a) {
+    __shared__ double2 M[256], E[256];  // the product: hi and lo parts
+    __shared__ int bad;
+    const FxFactor &ff = a.fac[blockIdx.x];
+    const int D = ff.f.D, tid = threadIdx.x, i = tid / 16, j = tid % 16;
+    const double2 *src = a.c.mats + (size_t)blockIdx.y * a.c.mats_len;
+    const bool in = i < D && j < D;
+    if (tid == 0) bad = 0;
+    E[tid] = make_double2(0.0, 0.0);
+    M[tid] = in ? src[a.ops[ff.op0].mat + i * D + j] : make_double2(0.0, 0.0);
+    __syncthreads();
+    for (int o = 1; o < ff.ops; ++o) {
+        const FxOp op = a.ops[ff.op0 + o];
+        // the operand acts on one digit of i (left) or of j (right)
+        const int stride = op.where == 0 ? ff.D1 : 1;
+        const int x = op.right ? j : i, q = x / stride % op.D;
+        double rh = 0.0, rl = 0.0, ih = 0.0, il = 0.0;
+        if (in)
+            for (int l = 0; l < op.D; ++l) {
+                const int k = x + (l - q) * stride;
+                const double2 u = src[op.mat + (op.right ? l * op.D + q : q * op.D + l)];
+                const int at = op.right ? i * 16 + k : k * 16 + j;
+                const double2 h = M[at], e = E[at];
+                fx_acc(rh, rl, u.x, h.x);
+                fx_acc(rh, rl, -u.y, h.y);
+                fx_acc(ih, il, u.x, h.y);
+                fx_acc(ih, il, u.y, h.x);
+                rl += u.x * e.x - u.y * e.y;
+                il += u.x * e.y + u.y * e.x;
+            }
+        __syncthreads();
+        M[tid] = make_double2(rh, ih);
+        E[tid] = make_double2(rl, il);
+        __syncthreads();
+    }
+    if (in) {
+        double re = i == j ? -1.0 : 0.0, im = 0.0;
+        for (int k = 0; k < D; ++k) {
+            const double2 x = M[i * 16 + k], y = M[j * 16 + k];
+            re += x.x * y.x + x.y * y.y;
+            im += x.y * y.x - x.x * y.y;
+        }
+        if (!(fabs(re) + fabs(im) < 1e-9)) bad = 1;
+    }
+    __syncthreads();
+    if (bad) {
+        if (tid == 0) atomicAnd(&a.good[blockIdx.y], 0);
+        return;
+    }
+    // fragment registers: rows lane / 4 (+ 8), columns 2 (lane % 4) + {0, 1} (+ 8)
+    uint4 *out = a.frag + ((size_t)blockIdx.y * a.nf + blockIdx.x) * FX_FRAG;
+    for (int e = tid; e < FX_FRAG; e += 256) {
+        const int lane = e & 31, im = (e >> 5) & 1, s = e >> 6, g = lane >> 2, t = lane & 3;
+        unsigned r[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int row = g + 8 * (q & 1), c0 = 2 * t + 8 * (q >> 1);
+            unsigned long long v[2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int col = c0 + h;
+                v[h] = FX_BIAS;
+                if (row < ff.p * D && col < ff.p * D && row / D == col / D) {
+                    const int at = (row % D) * 16 + col % D;
+                    v[h] += (unsigned long long)(im ? fx_round(M[at].y, E[at].y)
+                                                    : fx_round(M[at].x, E[at].x));
+                }
+            }
+            r[q] = fx_pair(v[0], v[1], s);
+        }
+        out[e] = make_uint4(r[0], r[1], r[2], r[3]);
+    }
+}
+
+// One tile: 8 columns of factor ff's groups, by one warp.  xmax: the largest
+// accumulator so far.
+__device__ __forceinline__ void fx_tile(longlong2 *V, const uint4 *__restrict__ U,
+                                        const FxFactor &ff, const int *__restrict__ base,
+                                        const int *__restrict__ offs, int tile, int lane,
+                                        float &xmax) {
+    const int D = ff.f.D, p = ff.p, g = lane >> 2, t = lane & 3;
+    // entry of row r (group r / D of the column) and column n; -1: padding
+    auto entry = [&](int r, int n) {
+        const int sub = p == 1 ? 0 : r / D, j = r - sub * D;
+        const int grp = (tile * 8 + n) * p + sub;
+        return (sub < p && j < D && grp < ff.groups) ? fx_swz(base[grp] + offs[j]) : -1;
+    };
+    unsigned xr[FX_DIGITS][2], xi[FX_DIGITS][2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        unsigned long long vr[2], vi[2];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int x = entry(2 * t + 8 * h + q, g);
+            const longlong2 v = x >= 0 ? V[x] : make_longlong2(0, 0);
+            vr[q] = (unsigned long long)v.x + FX_BIAS;
+            vi[q] = (unsigned long long)v.y + FX_BIAS;
+        }
+#pragma unroll
+        for (int s = 0; s < FX_DIGITS; ++s) {
+            xr[s][h] = fx_pair(vr[0], vr[1], s);
+            xi[s][h] = fx_pair(vi[0], vi[1], s);
+        }
+    }
+    // one accumulator set per level: U's fragments are read once, and
+    // consecutive MMAs are independent
+    float cr[FX_LEVELS][4], ci[FX_LEVELS][4];
+#pragma unroll
+    for (int l = 0; l < FX_LEVELS; ++l)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) cr[l][e] = ci[l][e] = 0.f;
+#pragma unroll
+    for (int s = 0; s < FX_DIGITS; ++s) {
+        const uint4 ur = U[(2 * s) * 32 + lane], ui = U[(2 * s + 1) * 32 + lane];
+#pragma unroll
+        for (int q = 0; q < FX_DIGITS; ++q) {
+            if (s + q < FX_LOW) continue;
+            fx_mma(cr[s + q - FX_LOW], ur, xr[q][0], xr[q][1]);
+            fx_mma(ci[s + q - FX_LOW], ur, xi[q][0], xi[q][1]);
+        }
+#pragma unroll
+        for (int q = 0; q < FX_DIGITS; ++q) {
+            if (s + q < FX_LOW) continue;
+            // minus u_i x_i: FP16 sign bits
+            fx_mma(cr[s + q - FX_LOW], ui, xi[q][0] ^ 0x80008000u, xi[q][1] ^ 0x80008000u);
+            fx_mma(ci[s + q - FX_LOW], ui, xr[q][0], xr[q][1]);
+        }
+    }
+    float m = 0.f;
+    long long yr[4], yi[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        float ar[FX_LEVELS], ai[FX_LEVELS];
+#pragma unroll
+        for (int l = 0; l < FX_LEVELS; ++l) {
+            ar[l] = cr[l][e];
+            ai[l] = ci[l][e];
+            m = fmaxf(m, fmaxf(fabsf(ar[l]), fabsf(ai[l])));
+        }
+        yr[e] = fx_join(ar);
+        yi[e] = fx_join(ai);
+    }
+    xmax = fmaxf(xmax, m);
+    __syncwarp();  // the tile's entries have all been read
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const int x = entry(g + 8 * (e >> 1), 2 * t + (e & 1));
+        if (x >= 0) V[x] = make_longlong2(yr[e], yi[e]);
+    }
+}
+
+__global__ void __launch_bounds__(FX_THREADS, 1) msp_celio_fx_kernel(FxArgs a) {
+    extern __shared__ __align__(16) unsigned char ce_smem[];
+    const CeArgs &c = a.c;
+    longlong2 *V = reinterpret_cast<longlong2 *>(ce_smem);
+    uint4 *U = reinterpret_cast<uint4 *>(V + ((c.V + 7) & ~7ll));  // fx_swz stays inside blocks of 8
+    FxFactor *fac = reinterpret_cast<FxFactor *>(U + (size_t)a.nf * FX_FRAG);
+    int *base = reinterpret_cast<int *>(fac + a.nf);
+    int *offs = base + a.nbase;
+    __shared__ double red[64];
+    __shared__ int s_bad;
+    const int tid = threadIdx.x, nt = FX_THREADS, lane = tid & 31, warp = tid >> 5;
+    const int V32 = (int)c.V;
+    for (int i = tid; i < a.nf; i += nt) fac[i] = a.fac[i];
+    for (int i = tid; i < c.noffs; i += nt) offs[i] = (int)c.offs[i];
+    __syncthreads();
+    for (int f = 0; f < a.nf; ++f)
+        for (int g = tid; g < fac[f].groups; g += nt) base[fac[f].base0 + g] = ce_base<int>(fac[f].f, g);
+    int loaded = -1;
+    for (int st = blockIdx.x; st < c.S * c.A; st += gridDim.x) {
+        const int s = st / c.A, blk = c.mats_per_snap ? s : 0;
+        __syncthreads();
+        if (blk != loaded) {
+            const uint4 *src = a.frag + (size_t)blk * a.nf * FX_FRAG;
+            for (int i = tid; i < a.nf * FX_FRAG; i += nt) U[i] = src[i];
+            loaded = blk;
+        }
+        if (tid == 0) s_bad = a.good[blk] ? 0 : 1;
+        // norm of the initial state, then its fixed-point form
+        double n2 = 0.0, z = 0.0;
+        for (int x = tid; x < V32; x += nt) {
+            const double2 v = c.mode == MSP_CELIO_PURE ? ce_init_pure(c, st, x)
+                                                       : c.rho0[(size_t)s * c.V + x];
+            n2 += v.x * v.x + v.y * v.y;
+        }
+        block_sum2(n2, z, red);
+        if (s_bad || !(n2 > 1e-200 && n2 < 1e200)) continue;
+        // sqrt(n2) 2^F <= 2^58
+        const int F = 58 - (int)ceil(0.5 * (ilogb(n2) + 1));
+        const double up = scalbn(1.0, F), down = scalbn(1.0, -F);
+        for (int x = tid; x < V32; x += nt) {
+            const double2 v = c.mode == MSP_CELIO_PURE ? ce_init_pure(c, st, x)
+                                                       : c.rho0[(size_t)s * c.V + x];
+            V[fx_swz(x)] = make_longlong2(__double2ll_rn(v.x * up), __double2ll_rn(v.y * up));
+        }
+        __syncthreads();
+        float xmax = 0.f;
+        for (int t = 0; t < c.T; ++t) {
+            if (c.mode == MSP_CELIO_PURE) {
+                // |u|^2, |d|^2 and conj(u) d over the muon's two halves
+                double uu = 0.0, dd = 0.0, ur = 0.0, ui = 0.0;
+                for (int kk = tid; kk < (int)c.half; kk += nt) {
+                    const longlong2 a0 = V[fx_swz(kk)], a1 = V[fx_swz(kk + (int)c.half)];
+                    const double ux = (double)a0.x, uy = (double)a0.y, dx = (double)a1.x,
+                                 dy = (double)a1.y;
+                    uu = fma(ux, ux, fma(uy, uy, uu));
+                    dd = fma(dx, dx, fma(dy, dy, dd));
+                    ur = fma(ux, dx, fma(uy, dy, ur));
+                    ui = fma(ux, dy, fma(-uy, dx, ui));
+                }
+                block_sum2(uu, dd, red);
+                block_sum2(ur, ui, red);
+                if (tid == 0) {
+                    const double2 *sg = c.sigma + 4 * s;
+                    c.series_pure[(size_t)st * c.T + t] =
+                        (sg[0].x * uu + sg[3].x * dd + 2.0 * (sg[1].x * ur - sg[1].y * ui)) * down *
+                        down;
+                }
+            } else {
+                const double2 *W0 = c.meas + (size_t)(c.meas_per_snap ? s : 0) * c.nops * c.V;
+                for (int j = 0; j < c.nops; ++j) {
+                    const double2 *W = W0 + (size_t)j * c.V;
+                    double re = 0.0, im = 0.0;
+                    for (int x = tid; x < V32; x += nt) {
+                        const longlong2 v = V[fx_swz(x)];
+                        const double rx = (double)v.x, ry = (double)v.y;
+                        const double2 w = W[x];
+                        re = fma(rx, w.x, fma(-ry, w.y, re));
+                        im = fma(rx, w.y, fma(ry, w.x, im));
+                    }
+                    block_sum2(re, im, red);
+                    if (tid == 0)
+                        c.series_rho[((size_t)s * c.T + t) * c.nops + j] =
+                            make_double2(re * down, im * down);
+                }
+            }
+            if (t + 1 == c.T) break;  // the evolution after the last sample is never read
+            __syncthreads();
+            for (int r = 0; r < c.k; ++r)
+                for (int f = 0; f < a.nf; ++f) {
+                    const FxFactor &ff = fac[f];
+                    const int tiles = (ff.groups + 8 * ff.p - 1) / (8 * ff.p);
+                    for (int tile = warp; tile < tiles; tile += FX_THREADS / 32)
+                        fx_tile(V, U + (size_t)f * FX_FRAG, ff, base + ff.base0, offs + ff.f.off, tile,
+                                lane, xmax);
+                    __syncthreads();
+                }
+        }
+        if (xmax >= 16777216.f) s_bad = 1;  // an accumulator left the exact range
+        __syncthreads();
+        if (tid == 0) a.done[st] = s_bad ? 0 : 1;
         __syncthreads();
     }
 }
@@ -930,7 +1299,96 @@ struct CePlan {
     size_t smem = 0;
     bool use_smem = false;
     bool dw = false;  // double-word FP32 shared-memory kernel
+    // fixed-point tensor path
+    bool fx = false;
+    std::vector<FxFactor> fxf;
+    std::vector<FxOp> fxo;
+    int nbase = 0;
+    size_t fx_smem = 0;
 };
+
+// Merges single-digit factors into factors that act on their digit with only
+// factors on other digits between, and lists each product's operands.  False
+// when a product is larger than 16.
+static bool fx_plan(const msp_celio_args *a, CePlan &p) {
+    const int nf = (int)p.fac.size();
+    struct Item {
+        int d0, d1, src;
+        std::vector<FxOp> before, after;  // right (earlier) and left (later) operands
+        bool gone;
+    };
+    std::vector<Item> it(nf);
+    for (int i = 0; i < nf; ++i) {
+        it[i].d0 = a->factor_digits[2 * i];
+        it[i].d1 = a->factor_digits[2 * i + 1];
+        if (it[i].d1 < 0) it[i].d1 = -1;
+        it[i].src = i;
+        it[i].gone = false;
+    }
+    auto on = [&](const Item &x, int d) { return x.d0 == d || x.d1 == d; };
+    for (int i = 0; i < nf; ++i) {
+        if (it[i].d1 >= 0) continue;
+        const int d = it[i].d0;
+        int j = i - 1;
+        while (j >= 0 && (it[j].gone || !on(it[j], d))) --j;
+        const bool back = j >= 0;
+        if (!back) {
+            j = i + 1;
+            while (j < nf && !on(it[j], d)) ++j;
+            if (j >= nf) continue;
+        }
+        FxOp op;
+        memset(&op, 0, sizeof(op));
+        op.mat = p.fac[i].mat;
+        op.D = p.fac[i].D;
+        op.where = it[j].d1 < 0 ? 2 : (it[j].d0 == d ? 0 : 1);
+        op.right = back ? 0 : 1;
+        // a single factor keeps its own merged operands in order
+        std::vector<FxOp> seq(it[i].before.rbegin(), it[i].before.rend());
+        seq.push_back(op);
+        seq.insert(seq.end(), it[i].after.begin(), it[i].after.end());
+        for (FxOp &q : seq) q.where = op.where;
+        if (back) {
+            for (FxOp &q : seq) {
+                q.right = 0;
+                it[j].after.push_back(q);
+            }
+        } else {
+            for (auto q = seq.rbegin(); q != seq.rend(); ++q) {
+                q->right = 1;
+                it[j].before.push_back(*q);
+            }
+        }
+        it[i].gone = true;
+    }
+    for (int i = 0; i < nf; ++i) {
+        if (it[i].gone) continue;
+        FxFactor f;
+        memset(&f, 0, sizeof(f));
+        f.f = p.fac[i];
+        if (f.f.D > 16) return false;
+        f.D0 = a->digit_dims[it[i].d0];
+        f.D1 = it[i].d1 >= 0 ? a->digit_dims[it[i].d1] : 1;
+        f.op0 = (int)p.fxo.size();
+        FxOp op;
+        memset(&op, 0, sizeof(op));
+        op.mat = f.f.mat;
+        op.D = f.f.D;
+        op.where = 2;
+        p.fxo.push_back(op);
+        p.fxo.insert(p.fxo.end(), it[i].before.begin(), it[i].before.end());
+        p.fxo.insert(p.fxo.end(), it[i].after.begin(), it[i].after.end());
+        f.ops = (int)p.fxo.size() - f.op0;
+        f.p = 16 / f.f.D;
+        f.groups = (int)(p.V / f.f.D);
+        f.base0 = p.nbase;
+        p.nbase += f.groups;
+        p.fxf.push_back(f);
+    }
+    p.fx_smem = (size_t)((p.V + 7) & ~7ll) * 16 + p.fxf.size() * (FX_FRAG * 16 + sizeof(FxFactor)) +
+                ((size_t)p.nbase + p.offs.size()) * 4;
+    return !p.fxf.empty();
+}
 
 static int ce_plan(const msp_celio_args *a, CePlan &p) {
     if (a == NULL) return ce_fail(MSP_ERR_ARG, "msp_celio: args is NULL");
@@ -1027,7 +1485,18 @@ static int ce_plan(const msp_celio_args *a, CePlan &p) {
     if (p.use_smem && !fits)
         return ce_fail(MSP_ERR_UNSUPPORTED, "msp_celio: state does not fit in shared memory");
     p.dw = a->precision == MSP_PREC_MIXED;
+    // the kernel's static arrays take under 1 KB
+    p.fx = p.use_smem && fx_plan(a, p) && p.fx_smem + 1024 <= (size_t)optin;
     return MSP_OK;
+}
+
+// Workspace of the fixed-point path.
+static size_t fx_workspace(const msp_celio_args *a, const CePlan &p) {
+    if (!p.fx) return 0;
+    const size_t blocks = a->mats_per_snapshot ? (size_t)a->num_snapshots : 1;
+    return ce_align(p.fxf.size() * sizeof(FxFactor) + 16) + ce_align(p.fxo.size() * sizeof(FxOp) + 16) +
+           ce_align(blocks * p.fxf.size() * FX_FRAG * 16) + ce_align(blocks * 4) +
+           ce_align((size_t)p.states * 4);
 }
 
 static size_t ce_workspace(const msp_celio_args *a, const CePlan &p) {
@@ -1068,7 +1537,7 @@ int msp_celio_workspace(const msp_celio_args *args, size_t *bytes) {
     const int rc = ce_plan(args, p);
     if (rc != MSP_OK) return rc;
     if (bytes == NULL) return ce_fail(MSP_ERR_ARG, "msp_celio_workspace: bytes is NULL");
-    *bytes = ce_workspace(args, p);
+    *bytes = ce_workspace(args, p) + fx_workspace(args, p);
     return MSP_OK;
 }
 
@@ -1134,6 +1603,59 @@ int msp_celio_run(const msp_celio_args *a, void *workspace, size_t workspace_byt
     k.chunks = p.chunks;
     const int sms = ce_sms();
     if (p.use_smem) {
+        // a workspace without room for the fixed-point path leaves it out
+        if (p.fx && workspace_bytes >= ce_workspace(a, p) + fx_workspace(a, p)) {
+            const size_t blocks = a->mats_per_snapshot ? (size_t)a->num_snapshots : 1;
+            FxArgs fx;
+            fx.c = k;
+            FxFactor *ff = (FxFactor *)w;
+            w += ce_align(p.fxf.size() * sizeof(FxFactor) + 16);
+            FxOp *fo = (FxOp *)w;
+            w += ce_align(p.fxo.size() * sizeof(FxOp) + 16);
+            fx.frag = (uint4 *)w;
+            w += ce_align(blocks * p.fxf.size() * FX_FRAG * 16);
+            fx.good = (int *)w;
+            w += ce_align(blocks * 4);
+            fx.done = (int *)w;
+            w += ce_align((size_t)p.states * 4);
+            fx.fac = ff;
+            fx.ops = fo;
+            fx.nf = (int)p.fxf.size();
+            fx.nbase = p.nbase;
+            rc = ce_cuda(cudaMemcpyAsync(ff, p.fxf.data(), p.fxf.size() * sizeof(FxFactor),
+                                         cudaMemcpyHostToDevice, st));
+            if (rc == MSP_OK)
+                rc = ce_cuda(cudaMemcpyAsync(fo, p.fxo.data(), p.fxo.size() * sizeof(FxOp),
+                                             cudaMemcpyHostToDevice, st));
+            if (rc == MSP_OK) rc = ce_cuda(cudaMemsetAsync(fx.good, 0xff, blocks * 4, st));
+            if (rc == MSP_OK) rc = ce_cuda(cudaMemsetAsync(fx.done, 0, (size_t)p.states * 4, st));
+            if (rc == MSP_OK)
+                rc = ce_cuda(cudaFuncSetAttribute(msp_celio_fx_kernel,
+                                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                  (int)p.fx_smem));
+            if (rc != MSP_OK) return rc;
+            for (size_t b0 = 0; b0 < blocks; b0 += 65535) {
+                FxArgs q = fx;
+                q.c.mats += b0 * (size_t)k.mats_len;
+                q.frag += b0 * p.fxf.size() * FX_FRAG;
+                q.good += b0;
+                const unsigned bn = (unsigned)(blocks - b0 < 65535 ? blocks - b0 : 65535);
+                msp_celio_fx_prep_kernel<<<dim3((unsigned)p.fxf.size(), bn), 256, 0, st>>>(q);
+            }
+            int occ = 1;
+            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, msp_celio_fx_kernel, FX_THREADS,
+                                                              p.fx_smem) != cudaSuccess ||
+                occ < 1) {
+                cudaGetLastError();
+                occ = 1;
+            }
+            const long long cap = (long long)sms * occ;
+            const int grid = (int)(p.states < cap ? p.states : cap);
+            msp_celio_fx_kernel<<<grid, FX_THREADS, p.fx_smem, st>>>(fx);
+            rc = ce_cuda(cudaGetLastError());
+            if (rc != MSP_OK) return rc;
+            k.done = fx.done;
+        }
         void (*kern)(CeArgs) = p.dw ? msp_celio_smem_dw_kernel : msp_celio_smem_kernel;
         rc = ce_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)p.smem));
