@@ -18,7 +18,7 @@ CSRC = os.path.join(HERE, "csrc")
 BUILD_DIR = os.path.join(HERE, "_build")
 LIB_NAME = "libmspgpu.so"
 SOURCES = ["msp_snap.cu", "msp_snap64.cu", "msp_jacobi_warp.cu", "msp_ql_warp.cu", "msp_phase.cu", "msp_nufft.cu", "msp_api.cu", "msp_static.cu", "msp_adjoint.cu", "msp_large.cu",
-           "msp_large_mixed.cu",
+           "msp_large_solve.cu", "msp_large_refine.cu",
            "msp_multi.cu", "msp_orient.cu", "msp_assemble.cu",
            "msp_lindblad.cu", "msp_celio.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]

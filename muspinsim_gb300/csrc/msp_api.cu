@@ -335,8 +335,8 @@ static int check_powder(const msp_powder_args *a) {
 }
 
 // Workspace of a run.  `lean` leaves out what only buys speed (the Fourier
-// form of the phase sum, and in FP64 the two-stage snapshots): for callers
-// with a fixed scratch.
+// form of the phase sum, in FP64 the two-stage snapshots, and for n > 64 room to
+// have every snapshot in flight): for callers with a fixed scratch.
 static Layout powder_layout(const msp_powder_args *a, bool lean = false) {
     Layout L;
     const bool mixed = a->precision == MSP_PREC_MIXED;
@@ -381,11 +381,11 @@ static Layout powder_layout(const msp_powder_args *a, bool lean = false) {
     L.large = off;
     if (a->n > MSP_MAX_DIM) {
         if (a->mode == MSP_MODE_FAST)
-            off += align256(large_scratch_bytes(
-                a->n, large_grid(a->num_snap, a->n, a->precision), a->precision));
+            off += align256(large_fast_bytes(a->n, large_grid(a->num_snap, a->n, a->precision),
+                                             a->precision, lean));
         else
             off += align256(large_rho_scratch_bytes(
-                a->n, large_rho_grid(a->num_snap, a->n, powder_fac_len(a))));
+                a->n, large_rho_grid(a->num_snap, a->n, powder_fac_len(a)), lean));
     }
     L.total = off;
     return L;
@@ -503,12 +503,12 @@ int msp_powder_run(const msp_powder_args *a) {
     if (L.two_stage)
         rc = cuda_check(launch_snapshots_refine(sa, a->mode, a->precision, st), "msp_snap");
     else if (large && a->num_snap > 0 && a->mode == MSP_MODE_FAST)
-        rc = cuda_check(launch_large_fast(sa, reinterpret_cast<double *>(ws + L.large),
+        rc = cuda_check(launch_large_fast(sa, ws + L.large, L.total - L.large,
                                           large_grid(a->num_snap, a->n, a->precision), st, 0,
                                           a->precision),
                         "msp_large_fast");
     else if (large && a->num_snap > 0)
-        rc = cuda_check(launch_large_rho(sa, reinterpret_cast<double *>(ws + L.large),
+        rc = cuda_check(launch_large_rho(sa, ws + L.large, L.total - L.large,
                                          large_rho_grid(a->num_snap, a->n, sa.fac_len), st,
                                          a->mode == MSP_MODE_INTEGRAL),
                         "msp_large_rho");

@@ -61,26 +61,11 @@ __device__ __forceinline__ bool oa_in_cluster(const int *cstart, int n, int r) {
     return (r > 0 && cstart[r - 1] == cstart[r]) || (r + 1 < n && cstart[r + 1] == cstart[r]);
 }
 
-// Clusters of the refinement step: amax, the sort, the cluster starts and
-// the off-diagonal entries of T.  SR holds S_ij (i < j) at [i][j] and R_ij
-// at [j][i] (row stride ld); lam / lamf are the Rayleigh quotients (lam as
-// double-words, msp_dw.cuh; lamf their high words).
-// c.scal[0] must be zero on entry (made visible by a barrier).  All threads
-// of the CTA call it; it ends with a barrier.
-static __device__ void oa_clusters(const cx<float> *SR, int ld, const float2 *lam,
-                                   const float *lamf, int n, const OaCluster &c) {
+// The sort of the Rayleigh quotients lam (double-words, msp_dw.cuh) and the
+// cluster starts, once c.scal[0] holds amax (made visible by the barrier
+// inside).  All threads of the CTA call it; it ends with a barrier.
+static __device__ void oa_cluster_starts(const float2 *lam, int n, const OaCluster &c) {
     const int tid = threadIdx.x, nt = blockDim.x;
-    const int nup = n * (n - 1) / 2;
-    float amax = 0.f;
-    for (int e = tid; e < nup; e += nt) {
-        int i, j;
-        oa_pair_of(e, i, j);
-        const cx<float> S = SR[(size_t)i * ld + j], R = SR[(size_t)j * ld + i];
-        const float ar = S.re + lamf[i] * R.re, ai = S.im + lamf[i] * R.im;
-        const float br = S.re + lamf[j] * R.re, bi = S.im + lamf[j] * R.im;
-        amax = fmaxf(amax, fmaxf(fmaxf(fabsf(ar), fabsf(ai)), fmaxf(fabsf(br), fabsf(bi))));
-    }
-    atomicMax(&c.scal[0], __float_as_int(amax));  // non-negative: int order = float order
     // ascending order, ties by index
     for (int i = tid; i < n; i += nt) {
         const float2 li = lam[i];
@@ -117,6 +102,29 @@ static __device__ void oa_clusters(const cx<float> *SR, int ld, const float2 *la
             if (c.cstart[q] < 0) c.cstart[q] = before;
     }
     __syncthreads();
+}
+
+// Clusters of the refinement step: amax, the sort, the cluster starts and
+// the off-diagonal entries of T.  SR holds S_ij (i < j) at [i][j] and R_ij
+// at [j][i] (row stride ld); lam / lamf are the Rayleigh quotients (lam as
+// double-words, msp_dw.cuh; lamf their high words).
+// c.scal[0] must be zero on entry (made visible by a barrier).  All threads
+// of the CTA call it; it ends with a barrier.
+static __device__ void oa_clusters(const cx<float> *SR, int ld, const float2 *lam,
+                                   const float *lamf, int n, const OaCluster &c) {
+    const int tid = threadIdx.x, nt = blockDim.x;
+    const int nup = n * (n - 1) / 2;
+    float amax = 0.f;
+    for (int e = tid; e < nup; e += nt) {
+        int i, j;
+        oa_pair_of(e, i, j);
+        const cx<float> S = SR[(size_t)i * ld + j], R = SR[(size_t)j * ld + i];
+        const float ar = S.re + lamf[i] * R.re, ai = S.im + lamf[i] * R.im;
+        const float br = S.re + lamf[j] * R.re, bi = S.im + lamf[j] * R.im;
+        amax = fmaxf(amax, fmaxf(fmaxf(fabsf(ar), fabsf(ai)), fmaxf(fabsf(br), fabsf(bi))));
+    }
+    atomicMax(&c.scal[0], __float_as_int(amax));  // non-negative: int order = float order
+    oa_cluster_starts(lam, n, c);
     for (int e = tid; e < nup; e += nt) {
         int i, j;
         oa_pair_of(e, i, j);
@@ -172,16 +180,21 @@ static __device__ void oa_cluster_diagonal(const float2 *lam, const float *corr,
     __syncthreads();
 }
 
-// Resolves every cluster of two or more levels (one warp per cluster) on
-// the corrected eigenvector matrix X (nrows x n, row stride ldx), and sets
+// Resolves every cluster of two or more levels (one warp per cluster: the
+// starts are dealt out to `nwarps` warps, of which this is number `warp`; by
+// default the CTA's) on the corrected eigenvector matrix X (nrows x n, row stride ldx), and sets
 // the clusters' eigenvalues; the other levels get l_i + corr_i.  Returns
 // this thread's share of the step size.  Ends with a barrier.
 // Xl (optional, laid out like X): low words of X, zeroed in rotated columns.
 static __device__ float oa_resolve_clusters(cx<float> *X, int ldx, int nrows, float2 *lam,
                                      const float *corr, int n, const OaCluster &c,
-                                     float lscale, cx<float> *Xl = nullptr) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int nwarps = (blockDim.x + 31) >> 5;
+                                     float lscale, cx<float> *Xl = nullptr, int warp = -1,
+                                     int nwarps = 0) {
+    const int lane = threadIdx.x & 31;
+    if (warp < 0) {
+        warp = threadIdx.x >> 5;
+        nwarps = (blockDim.x + 31) >> 5;
+    }
     const float noise = 4.0f * (float)n * 5.684341886080802e-14f * lscale;  // 4 n 2^-44 max|l|
     const float big2 = 256.0f * noise * noise;
     float emax = 0.f;
@@ -247,6 +260,72 @@ static __device__ float oa_resolve_clusters(cx<float> *X, int ldx, int nrows, fl
             lam[c.order[r]] = dw_add_f(lam[c.order[r]], corr[c.order[r]]);
     __syncthreads();
     return emax;
+}
+
+// The clusters of the FP64 step (msp_snap64.cu, msp_large_refine.cu), one warp
+// per cluster, the starts dealt out to `nwarps` warps: a Jacobi on its couplings
+// T (off-diagonal FP32, sorted coordinates, row stride n; diagonal relative to
+// the cluster's first level in tdiag, FP64), each rotation applied to the FP64 vectors X with its cosine recomputed so
+// that it is unitary to FP64.
+__device__ __forceinline__ void oa_resolve64(const int *cst, const int *ord, double *lam,
+                                             double *tdiag, cx<float> *T, cx<double> *X, int n,
+                                             int ld, float noise, int warp, int nwarps) {
+    const int lane = threadIdx.x & 31;
+    for (int q0 = warp; q0 < n; q0 += nwarps) {
+        if (cst[q0] != q0 || q0 + 1 >= n || cst[q0 + 1] != q0) continue;
+        int k = 2;
+        while (q0 + k < n && cst[q0 + k] == q0) ++k;
+        cx<float> *Tc = T + (size_t)q0 * n + q0;
+        double *td = tdiag + q0;
+        for (int sweep = 0; sweep < 16; ++sweep) {
+            int nrot = 0;
+            for (int p = 0; p < k - 1; ++p) {
+                for (int q = p + 1; q < k; ++q) {
+                    const cx<float> apq = Tc[(size_t)p * n + q];
+                    const float mag = sqrtf(cabs2(apq));
+                    if (!(mag > noise)) continue;
+                    const double tp = td[p], tq = td[q];
+                    JRot<float> R;
+                    float na, nb;
+                    jacobi_rotation<float>(0.f, (float)(tq - tp), apq, noise, p, q, R, na, nb);
+                    ++nrot;
+                    const double sr = R.sr, si = R.si;
+                    const double c = sqrt(fma(-sr, sr, fma(-si, si, 1.0)));
+                    const cx<float> sf = mk<float>(R.sr, R.si);
+                    for (int col = lane; col < k; col += 32) {
+                        if (col == p || col == q) continue;
+                        const cx<float> a = Tc[(size_t)p * n + col], b = Tc[(size_t)q * n + col];
+                        const cx<float> np = cadd(cscale(R.c, a), cscale(-1.0f, cmul(sf, b)));
+                        const cx<float> nq = cadd(cmulc(sf, a), cscale(R.c, b));
+                        Tc[(size_t)p * n + col] = np;
+                        Tc[(size_t)q * n + col] = nq;
+                        Tc[(size_t)col * n + p] = conj(np);
+                        Tc[(size_t)col * n + q] = conj(nq);
+                    }
+                    const int i = ord[q0 + p], j = ord[q0 + q];
+                    const cx<double> sd = mk<double>(sr, si);
+                    for (int r = lane; r < n; r += 32) {
+                        const cx<double> x = X[(size_t)r * ld + i], y = X[(size_t)r * ld + j];
+                        X[(size_t)r * ld + i] = cadd(cscale(c, x), cscale(-1.0, cmulc(sd, y)));
+                        X[(size_t)r * ld + j] = cadd(cmul(sd, x), cscale(c, y));
+                    }
+                    __syncwarp();
+                    if (lane == 0) {
+                        td[p] = tp + (double)na;  // na = -t |a|: the shift alone
+                        td[q] = tq - (double)na;
+                        Tc[(size_t)p * n + q] = mk<float>(0.f, 0.f);
+                        Tc[(size_t)q * n + p] = mk<float>(0.f, 0.f);
+                    }
+                    __syncwarp();
+                }
+            }
+            if (nrot == 0) break;
+        }
+        const double lref = lam[ord[q0]];
+        __syncwarp();
+        for (int p = lane; p < k; p += 32) lam[ord[q0 + p]] = lref + td[p];
+        __syncwarp();
+    }
 }
 
 }  // namespace msp

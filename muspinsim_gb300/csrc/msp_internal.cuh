@@ -250,27 +250,23 @@ cudaError_t launch_evolve_phases(const double *evals, const double *rho, int n,
 cudaError_t launch_integrate(const double *evals, const double *rho, const double *ops, int n,
                              int num_ops, double tau, double *out, cudaStream_t st);
 
-// n > 64 (msp_large.cu): Householder + QL eigensolver, one CTA per matrix
-// with `grid` CTAs, each owning large_scratch_bytes(n, 1, precision) of
-// scratch.  The eigensolver API (launch_eigh_large) is FP64; the fast path
-// runs FP64 or MIXED (FP32 solve, double-word refinement).
+// n > 64.  The eigensolver API (FP64 Householder + QL, one CTA per matrix with
+// `grid` CTAs, each owning large_scratch_bytes(n, 1) of scratch).
 cudaError_t launch_eigh_large(const double *H, int n, int batch, double *evals, double *evecs,
                               int *status, double *scratch, int grid, cudaStream_t st);
-cudaError_t launch_large_fast(const SnapArgs &a, double *scratch, int grid, cudaStream_t st,
-                              int threads = 0, int precision = MSP_PREC_FP64);
+size_t large_scratch_bytes(int n, int grid);
+// The fast path, FP64 or MIXED, with up to `slots` snapshots in flight, and the
+// general path (EVOLVE / INTEGRAL, FP64 in both precisions).  FP64 takes less
+// scratch than slots need (lean): fewer are then in flight.
+cudaError_t launch_large_fast(const SnapArgs &a, void *scratch, size_t bytes, int slots,
+                              cudaStream_t st, int threads, int precision);
 int large_threads(int n);
-size_t large_scratch_bytes(int n, int grid, int precision = MSP_PREC_FP64);
+size_t large_fast_bytes(int n, int slots, int precision, bool lean = false);
 int large_ctas_per_sm(int n, int precision = MSP_PREC_FP64);
 int large_grid(int batch, int n, int precision = MSP_PREC_FP64);
-// The MIXED fast path's kernel (msp_large_mixed.cu).
-cudaError_t launch_large_fast_mixed(const SnapArgs &a, double *scratch, int grid,
-                                    cudaStream_t st, int threads);
-size_t large_mixed_scratch_per_cta(int n);
-int large_mixed_occupancy(int n, int threads);
-// General path for n > 64 (EVOLVE / INTEGRAL, FP64 in both precisions).
-cudaError_t launch_large_rho(const SnapArgs &a, double *scratch, int grid, cudaStream_t st,
-                             int integral);
-size_t large_rho_scratch_bytes(int n, int grid);
+cudaError_t launch_large_rho(const SnapArgs &a, void *scratch, size_t bytes, int slots,
+                             cudaStream_t st, int integral);
+size_t large_rho_scratch_bytes(int n, int slots, bool lean = false);
 int large_rho_grid(int batch, int n, int fac_len);
 
 // Work decomposition of the phase sum (host side).  A work item sums at

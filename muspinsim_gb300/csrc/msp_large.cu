@@ -1,11 +1,23 @@
 // The large-n kernels (64 < n <= MSP_MAX_DIM_LARGE) on the FP64 solver of
-// msp_large.cuh -- the eigensolver API, the fast path and the general path
-// (EVOLVE / INTEGRAL) -- and the host side of every large-n launch (the
-// MIXED fast path's kernel is in msp_large_mixed.cu).
+// msp_large.cuh: the eigensolver API, and the fast and general path (EVOLVE /
+// INTEGRAL) of the snapshots that the refinement of FP32 eigenvectors
+// (msp_large_solve.cu, msp_large_refine.cu) leaves over; and the scratch sizes
+// of every large-n launch.
 #include "msp_large.cuh"
+#include "msp_large_slots.cuh"
 #include "msp_rho.cuh"
 
 namespace msp {
+
+int large_sms() {
+    int dev = 0, sms = 152;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+        cudaGetLastError();
+        sms = 152;
+    }
+    return sms;
+}
 
 __global__ void msp_eigh_large_kernel(const cx<double> *__restrict__ Hin, int n, int batch,
                                       double *__restrict__ evals, cx<double> *__restrict__ evecs,
@@ -31,14 +43,16 @@ __global__ void msp_eigh_large_kernel(const cx<double> *__restrict__ Hin, int n,
 // Fast path per snapshot for n > 64 (muspinsim/hamiltonian.py:166-217), the
 // large-n counterpart of msp_snap_fast_kernel: H = Hsys + b . Z, eigenpairs,
 // M = U^H (sigma_p (x) 1_d) U, pair records and the constant part.
-__global__ void msp_large_fast_kernel(SnapArgs a, double *__restrict__ scratch) {
+__global__ void msp_large_fast_kernel(SnapArgs a, double *__restrict__ scratch, int first, int count,
+                                      const int *redo) {
     extern __shared__ __align__(16) char smem[];
     const int n = a.n, d = n / 2, P = n * (n - 1) / 2;
     LargeScratch s = large_carve(scratch + (size_t)blockIdx.x * large_scratch_doubles(n), n);
     const int tid = threadIdx.x, nt = blockDim.x;
     __shared__ double red[32];
     const size_t nn = (size_t)n * n;
-    for (int sn = blockIdx.x; sn < a.num_snap; sn += gridDim.x) {
+    for (int sn = first + blockIdx.x; sn < first + count; sn += gridDim.x) {
+        if (redo && !redo[sn - first]) continue;
         const SnapSource src = snap_source(a, sn);
         const size_t g = (size_t)src.g;
         const double bx = a.field[3 * g], by = a.field[3 * g + 1], bz = a.field[3 * g + 2];
@@ -138,7 +152,8 @@ __device__ void large_apply_digit(const cx<double> *F, int dim, int stride,
 }
 
 template <bool INTEGRAL>
-__global__ void msp_large_rho_kernel(SnapArgs a, double *__restrict__ scratch) {
+__global__ void msp_large_rho_kernel(SnapArgs a, double *__restrict__ scratch, int first, int count,
+                                     const int *redo) {
     extern __shared__ __align__(16) char smem[];
     const int n = a.n, P = n * (n - 1) / 2;
     const size_t nn = (size_t)n * n;
@@ -151,7 +166,8 @@ __global__ void msp_large_rho_kernel(SnapArgs a, double *__restrict__ scratch) {
     __shared__ double red[32];
     const double twopi = 6.283185307179586476925;
     const size_t ntri = (size_t)n * (n + 1) / 2;
-    for (int sn = blockIdx.x; sn < a.num_snap; sn += gridDim.x) {
+    for (int sn = first + blockIdx.x; sn < first + count; sn += gridDim.x) {
+        if (redo && !redo[sn - first]) continue;
         if (a.rho_fac) {
             for (int e = tid; e < a.fac_len; e += nt)
                 fac[e] = a.rho_fac[(size_t)sn * a.fac_len + e];
@@ -262,8 +278,9 @@ size_t large_rho_smem_bytes(int n, int threads, int fac_len) {
     return large_rho_fac_offset(n, threads) + (size_t)fac_len * sizeof(cx<double>);
 }
 
-size_t large_rho_scratch_bytes(int n, int grid) {
-    return large_rho_scratch_doubles(n) * 8 * (size_t)grid;
+size_t large_rho_scratch_bytes(int n, int grid, bool lean) {
+    return lean ? large_rho_scratch_doubles(n) * 8 * (size_t)grid
+                : (large_rho_slot_bytes(n) + sizeof(int)) * (size_t)grid;
 }
 
 // Persistent grid of the general path: resident CTAs per SM by occupancy,
@@ -278,20 +295,15 @@ int large_rho_grid(int batch, int n, int fac_len) {
         cudaGetLastError();
         occ = 1;
     }
-    int dev = 0, sms = 152;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
-        cudaGetLastError();
-        sms = 152;
-    }
+    const int sms = large_sms();
     const size_t per = large_rho_scratch_doubles(n) * 8, budget = (size_t)2 << 30;
     while (occ > 1 && (size_t)occ * sms * per > budget) --occ;
     const int g = sms * occ;
     return batch < g ? (batch > 0 ? batch : 1) : g;
 }
 
-cudaError_t launch_large_rho(const SnapArgs &a, double *scratch, int grid, cudaStream_t st,
-                             int integral) {
+cudaError_t launch_large_rho64(const SnapArgs &a, double *scratch, int grid, cudaStream_t st,
+                               int integral, int first, int count, const int *redo) {
     const int threads = large_threads(a.n);
     const size_t smem = large_rho_smem_bytes(a.n, threads, a.fac_len);
     const void *fn = integral ? reinterpret_cast<const void *>(msp_large_rho_kernel<true>)
@@ -300,9 +312,9 @@ cudaError_t launch_large_rho(const SnapArgs &a, double *scratch, int grid, cudaS
         cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     if (integral)
-        msp_large_rho_kernel<true><<<grid, threads, smem, st>>>(a, scratch);
+        msp_large_rho_kernel<true><<<grid, threads, smem, st>>>(a, scratch, first, count, redo);
     else
-        msp_large_rho_kernel<false><<<grid, threads, smem, st>>>(a, scratch);
+        msp_large_rho_kernel<false><<<grid, threads, smem, st>>>(a, scratch, first, count, redo);
     return cudaGetLastError();
 }
 
@@ -321,63 +333,50 @@ cudaError_t launch_eigh_large(const double *H, int n, int batch, double *evals, 
     return cudaGetLastError();
 }
 
-cudaError_t launch_large_fast(const SnapArgs &a, double *scratch, int grid, cudaStream_t st,
-                              int threads, int precision) {
-    if (threads <= 0) threads = large_threads(a.n);
-    if (threads & 31) return cudaErrorInvalidValue;
-    if (precision == MSP_PREC_MIXED) return launch_large_fast_mixed(a, scratch, grid, st, threads);
+cudaError_t launch_large_fast64(const SnapArgs &a, double *scratch, int grid, cudaStream_t st,
+                                int threads, int first, int count, const int *redo) {
     const size_t smem = large_smem_bytes(a.n, threads);
     cudaError_t e = cudaFuncSetAttribute(msp_large_fast_kernel,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    msp_large_fast_kernel<<<grid, threads, smem, st>>>(a, scratch);
+    msp_large_fast_kernel<<<grid, threads, smem, st>>>(a, scratch, first, count, redo);
     return cudaGetLastError();
 }
 
-size_t large_scratch_bytes(int n, int grid, int precision) {
-    const size_t per = precision == MSP_PREC_MIXED ? large_mixed_scratch_per_cta(n)
-                                                   : large_scratch_doubles(n) * 8;
-    return per * (size_t)grid;
+size_t large_scratch_bytes(int n, int grid) { return large_scratch_doubles(n) * 8 * (size_t)grid; }
+
+// Scratch of the fast path with `slots` snapshots in flight; lean: what FP64
+// takes at least, its solver's scratch, which holds fewer slots.
+size_t large_fast_bytes(int n, int slots, int precision, bool lean) {
+    if (precision == MSP_PREC_MIXED) return large_slot_bytes(n, precision) * (size_t)slots;
+    return lean ? large_scratch_bytes(n, slots)
+                : (large_slot_bytes(n, precision) + sizeof(int)) * (size_t)slots;
 }
 
-// Resident CTAs of the large-n kernels per SM with large_threads(n)
-// threads, cut so that all CTAs' scratch stays within about 2 GB (large n
-// keeps one CTA per SM).
+// Matrices in flight per SM: MIXED five; FP64 the resident CTAs of its solver
+// with large_threads(n) threads; cut so that the solver's scratch (MIXED: the
+// slots) stays within about 2 GB (large n keeps one per SM).
 int large_ctas_per_sm(int n, int precision) {
     const int threads = large_threads(n);
-    int occ = 1;
-    if (precision == MSP_PREC_MIXED) {
-        occ = large_mixed_occupancy(n, threads);
-    } else if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, msp_large_fast_kernel, threads,
-                                                             large_smem_bytes(n, threads)) !=
-                   cudaSuccess ||
-               occ < 1) {
+    int occ = 5;
+    if (precision != MSP_PREC_MIXED &&
+        (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, msp_large_fast_kernel, threads,
+                                                       large_smem_bytes(n, threads)) != cudaSuccess ||
+         occ < 1)) {
         cudaGetLastError();
         occ = 1;
     }
-    int dev = 0, sms = 152;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
-        cudaGetLastError();
-        sms = 152;
-    }
-    const size_t per = large_scratch_bytes(n, 1, precision), budget = (size_t)2 << 30;
+    const int sms = large_sms();
+    const size_t per = precision == MSP_PREC_MIXED ? large_slot_bytes(n, precision)
+                                                   : large_scratch_bytes(n, 1);
+    const size_t budget = (size_t)2 << 30;
     while (occ > 1 && (size_t)occ * sms * per > budget) --occ;
     return occ;
 }
 
-// A persistent grid of SMs x large_ctas_per_sm(n, precision) CTAs, at most
-// one per matrix.  (Spreading the matrices evenly over fewer CTAs to avoid
-// a short last round was measured slower: a snapshot's time is set by
-// latency, not by how many CTAs share the SM, so more resident matrices
-// win.)
+// SMs x large_ctas_per_sm(n, precision) matrices in flight, at most the batch.
 int large_grid(int batch, int n, int precision) {
-    int dev = 0, sms = 152;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
-        cudaGetLastError();
-        sms = 152;
-    }
+    const int sms = large_sms();
     const int g = sms * large_ctas_per_sm(n, precision);
     return batch < g ? (batch > 0 ? batch : 1) : g;
 }

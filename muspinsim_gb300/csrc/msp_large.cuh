@@ -1,7 +1,7 @@
-// Householder + QL Hermitian eigensolver for 64 < n <= MSP_MAX_DIM_LARGE,
-// shared by the large-n kernels (msp_large.cu: FP64 fast path, eigensolver
-// API and the general path; msp_large_mixed.cu: the solver in FP32 followed
-// by double-word refinement).  One CTA per matrix, working matrices in
+// Householder + QL Hermitian eigensolver for 64 < n <= MSP_MAX_DIM_LARGE in
+// FP64 (msp_large.cu: the eigensolver API, the general path, and what the fast
+// path's refinement leaves over), and parts of it that its FP32 form
+// (msp_large_solve.cu) shares.  One CTA per matrix, working matrices in
 // global memory.  Replaces numpy.linalg.eigh in Hermitian.diag
 // (muspinsim/spinop.py:51-82) where the shared-memory Jacobi does not fit:
 //   1. Householder tridiagonalisation of the lower triangle (H = Q T Q^H,
@@ -154,12 +154,8 @@ __device__ __forceinline__ float rsqrt_newton<float>(float x) {
 
 // Eigenpairs of the Hermitian matrix already in s.A (full, row-major):
 // eigenvalues into s.lam, eigenvectors (columns) into s.U.  Returns
-// MSP_ITEM_OK or MSP_ITEM_NOT_CONVERGED (QL iteration cap).  BACK = false
-// stops after the QL step (s.Zt holds Z, s.A the reflectors, s.tau their
-// scalars) for a caller that back-transforms by itself; TRI = false starts
-// at the QL step (the caller left d and e in this layout's shared memory,
-// the reflectors in s.A and s.tau).
-template <typename T, bool BACK = true, bool TRI = true>
+// MSP_ITEM_OK or MSP_ITEM_NOT_CONVERGED (QL iteration cap).
+template <typename T>
 __device__ int large_eigh(LargeScratchT<T> s, int n, char *smem) {
     const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5;
     const int nw = nt >> 5;
@@ -170,7 +166,7 @@ __device__ int large_eigh(LargeScratchT<T> s, int n, char *smem) {
     cx<T> *A = s.A;
 
     // ---- 1. tridiagonalisation
-    for (int k = 0; TRI && k + 1 < n; ++k) {
+    for (int k = 0; k + 1 < n; ++k) {
         const int m = n - k - 1;  // length of x = A[k+1.., k]
         T xn2 = T(0);
         for (int i = 1 + tid; i < m; i += nt) xn2 += cabs2(A[(size_t)(k + 1 + i) * n + k]);
@@ -260,7 +256,7 @@ __device__ int large_eigh(LargeScratchT<T> s, int n, char *smem) {
         for (int i = 1 + tid; i < m; i += nt) A[(size_t)(k + 1 + i) * n + k] = v[i];
         __syncthreads();
     }
-    if (TRI && tid == 0) {
+    if (tid == 0) {
         dsm[n - 1] = A[(size_t)(n - 1) * n + (n - 1)].re;
         esm[n - 1] = T(0);
     }
@@ -400,66 +396,64 @@ __device__ int large_eigh(LargeScratchT<T> s, int n, char *smem) {
 
 
     // ---- 3. U = Q Z (complex), reflectors applied last to first
-    if (BACK) {
-        for (size_t x = tid; x < (size_t)n * n; x += nt) {
-            const int i = (int)(x / n), j = (int)(x - (size_t)i * n);
-            s.U[x] = mk<T>(s.Zt[(size_t)j * n + i], T(0));
+    for (size_t x = tid; x < (size_t)n * n; x += nt) {
+        const int i = (int)(x / n), j = (int)(x - (size_t)i * n);
+        s.U[x] = mk<T>(s.Zt[(size_t)j * n + i], T(0));
+    }
+    __syncthreads();
+    for (int k = n - 2; k >= 0; --k) {
+        const cx<T> tau = s.tau[k];
+        if (tau.re == T(0) && tau.im == T(0)) continue;  // the same in every thread
+        const int m = n - k - 1;
+        for (int i = tid; i < m; i += nt)
+            v[i] = i == 0 ? mk<T>(T(1), T(0)) : A[(size_t)(k + 1 + i) * n + k];
+        __syncthreads();
+        // s_j = v^H U[k+1.., j]: thread (pr, pg) takes columns j = pr, pr + RW,
+        // ... and the pg-th of G parts of the rows
+        if (pg < G) {
+            const int ib = (int)((long long)m * pg / G), ie = (int)((long long)m * (pg + 1) / G);
+            for (int j = pr; j < n; j += RW) {
+                const cx<T> *col = s.U + (size_t)(k + 1) * n + j;
+                T r0 = T(0), i0 = T(0), r1 = T(0), i1 = T(0);
+                int i = ib;
+#pragma unroll 4
+                for (; i + 1 < ie; i += 2) {
+                    const cx<T> u0 = col[(size_t)i * n], u1 = col[(size_t)(i + 1) * n];
+                    const cx<T> v0 = v[i], v1 = v[i + 1];
+                    r0 += v0.re * u0.re + v0.im * u0.im;
+                    i0 += v0.re * u0.im - v0.im * u0.re;
+                    r1 += v1.re * u1.re + v1.im * u1.im;
+                    i1 += v1.re * u1.im - v1.im * u1.re;
+                }
+                if (i < ie) {
+                    const cx<T> u0 = col[(size_t)i * n], v0 = v[i];
+                    r0 += v0.re * u0.re + v0.im * u0.im;
+                    i0 += v0.re * u0.im - v0.im * u0.re;
+                }
+                part[(size_t)pg * (n + 32) + j] = mk<T>(r0 + r1, i0 + i1);
+            }
         }
         __syncthreads();
-        for (int k = n - 2; k >= 0; --k) {
-            const cx<T> tau = s.tau[k];
-            if (tau.re == T(0) && tau.im == T(0)) continue;  // the same in every thread
-            const int m = n - k - 1;
-            for (int i = tid; i < m; i += nt)
-                v[i] = i == 0 ? mk<T>(T(1), T(0)) : A[(size_t)(k + 1 + i) * n + k];
-            __syncthreads();
-            // s_j = v^H U[k+1.., j]: thread (pr, pg) takes columns j = pr, pr + RW,
-            // ... and the pg-th of G parts of the rows
-            if (pg < G) {
-                const int ib = (int)((long long)m * pg / G), ie = (int)((long long)m * (pg + 1) / G);
-                for (int j = pr; j < n; j += RW) {
-                    const cx<T> *col = s.U + (size_t)(k + 1) * n + j;
-                    T r0 = T(0), i0 = T(0), r1 = T(0), i1 = T(0);
-                    int i = ib;
-#pragma unroll 4
-                    for (; i + 1 < ie; i += 2) {
-                        const cx<T> u0 = col[(size_t)i * n], u1 = col[(size_t)(i + 1) * n];
-                        const cx<T> v0 = v[i], v1 = v[i + 1];
-                        r0 += v0.re * u0.re + v0.im * u0.im;
-                        i0 += v0.re * u0.im - v0.im * u0.re;
-                        r1 += v1.re * u1.re + v1.im * u1.im;
-                        i1 += v1.re * u1.im - v1.im * u1.re;
-                    }
-                    if (i < ie) {
-                        const cx<T> u0 = col[(size_t)i * n], v0 = v[i];
-                        r0 += v0.re * u0.re + v0.im * u0.im;
-                        i0 += v0.re * u0.im - v0.im * u0.re;
-                    }
-                    part[(size_t)pg * (n + 32) + j] = mk<T>(r0 + r1, i0 + i1);
-                }
+        for (int j = tid; j < n; j += nt) {
+            T sr = T(0), si = T(0);
+            for (int g = 0; g < G; ++g) {
+                sr += part[(size_t)g * (n + 32) + j].re;
+                si += part[(size_t)g * (n + 32) + j].im;
             }
-            __syncthreads();
-            for (int j = tid; j < n; j += nt) {
-                T sr = T(0), si = T(0);
-                for (int g = 0; g < G; ++g) {
-                    sr += part[(size_t)g * (n + 32) + j].re;
-                    si += part[(size_t)g * (n + 32) + j].im;
-                }
-                p[j] = cmul(tau, mk<T>(sr, si));  // tau s_j
-            }
-            __syncthreads();
-            // U[k+1.., j] -= v tau s_j: warps over rows, lanes over columns
-            for (int i = warp; i < m; i += nw) {
-                const cx<T> vi = v[i];
-                cx<T> *row = s.U + (size_t)(k + 1 + i) * n;
-#pragma unroll 4
-                for (int j = lane; j < n; j += 32) {
-                    const cx<T> t = cmul(vi, p[j]), u = row[j];
-                    row[j] = mk<T>(u.re - t.re, u.im - t.im);
-                }
-            }
-            __syncthreads();
+            p[j] = cmul(tau, mk<T>(sr, si));  // tau s_j
         }
+        __syncthreads();
+        // U[k+1.., j] -= v tau s_j: warps over rows, lanes over columns
+        for (int i = warp; i < m; i += nw) {
+            const cx<T> vi = v[i];
+            cx<T> *row = s.U + (size_t)(k + 1 + i) * n;
+#pragma unroll 4
+            for (int j = lane; j < n; j += 32) {
+                const cx<T> t = cmul(vi, p[j]), u = row[j];
+                row[j] = mk<T>(u.re - t.re, u.im - t.im);
+            }
+        }
+        __syncthreads();
     }
     for (int i = tid; i < n; i += nt) s.lam[i] = d[i];
     __syncthreads();

@@ -262,7 +262,7 @@ static int plan_layout(msp_multi_plan *p, const msp_multi_desc *d) {
             if (g > b.cap_snap) g = b.cap_snap;
             if (g < 1) g = 1;
             b.grid = g;
-            off += al256(large_scratch_bytes(b.n, g, p->precision));
+            off += al256(large_fast_bytes(b.n, g, p->precision));
         }
         b.bytes = off - start;
     }
@@ -402,7 +402,8 @@ static int plan_enqueue(msp_multi_plan *p, const msp_multi_io *io, cudaStream_t 
             sa.seg_hoff = reinterpret_cast<const long long *>(ws + c.seg_hoff);
             if (cs > 0) {
                 if (b.large)
-                    rc = mcuda(launch_large_fast(sa, reinterpret_cast<double *>(ws + b.off_large),
+                    rc = mcuda(launch_large_fast(sa, ws + b.off_large,
+                                                 large_fast_bytes(b.n, b.grid, p->precision),
                                                  std::min(b.grid, cs), b.stream, b.threads,
                                                  p->precision),
                                "msp_multi_run: large-n snapshots");

@@ -152,71 +152,6 @@ __device__ void load_h64(const HSource &h, int n, int m, int ld, cx<double> *dst
 
 // ------------------------------------------------------------------ 3. FP64 step
 
-// Resolves every cluster of two or more levels, one warp per cluster: a
-// Jacobi on its couplings T (off-diagonal FP32, sorted coordinates, row
-// stride n; diagonal relative to the cluster's first level in tdiag, FP64),
-// each rotation applied to the FP64 vectors X with its cosine recomputed so
-// that it is unitary to FP64.
-__device__ void resolve64(S64 &s, cx<float> *T, cx<double> *X, int n, int ld, float noise) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int nwarps = (blockDim.x + 31) >> 5;
-    for (int q0 = warp; q0 < n; q0 += nwarps) {
-        if (s.cst[q0] != q0 || q0 + 1 >= n || s.cst[q0 + 1] != q0) continue;
-        int k = 2;
-        while (q0 + k < n && s.cst[q0 + k] == q0) ++k;
-        cx<float> *Tc = T + (size_t)q0 * n + q0;
-        double *td = s.tdiag + q0;
-        for (int sweep = 0; sweep < 16; ++sweep) {
-            int nrot = 0;
-            for (int p = 0; p < k - 1; ++p) {
-                for (int q = p + 1; q < k; ++q) {
-                    const cx<float> apq = Tc[(size_t)p * n + q];
-                    const float mag = sqrtf(cabs2(apq));
-                    if (!(mag > noise)) continue;
-                    const double tp = td[p], tq = td[q];
-                    JRot<float> R;
-                    float na, nb;
-                    jacobi_rotation<float>(0.f, (float)(tq - tp), apq, noise, p, q, R, na, nb);
-                    ++nrot;
-                    const double sr = R.sr, si = R.si;
-                    const double c = sqrt(fma(-sr, sr, fma(-si, si, 1.0)));
-                    const cx<float> sf = mk<float>(R.sr, R.si);
-                    for (int col = lane; col < k; col += 32) {
-                        if (col == p || col == q) continue;
-                        const cx<float> a = Tc[(size_t)p * n + col], b = Tc[(size_t)q * n + col];
-                        const cx<float> np = cadd(cscale(R.c, a), cscale(-1.0f, cmul(sf, b)));
-                        const cx<float> nq = cadd(cmulc(sf, a), cscale(R.c, b));
-                        Tc[(size_t)p * n + col] = np;
-                        Tc[(size_t)q * n + col] = nq;
-                        Tc[(size_t)col * n + p] = conj(np);
-                        Tc[(size_t)col * n + q] = conj(nq);
-                    }
-                    const int i = s.ord[q0 + p], j = s.ord[q0 + q];
-                    const cx<double> sd = mk<double>(sr, si);
-                    for (int r = lane; r < n; r += 32) {
-                        const cx<double> x = X[r * ld + i], y = X[r * ld + j];
-                        X[r * ld + i] = cadd(cscale(c, x), cscale(-1.0, cmulc(sd, y)));
-                        X[r * ld + j] = cadd(cmul(sd, x), cscale(c, y));
-                    }
-                    __syncwarp();
-                    if (lane == 0) {
-                        td[p] = tp + (double)na;  // na = -t |a|: the shift alone
-                        td[q] = tq - (double)na;
-                        Tc[(size_t)p * n + q] = mk<float>(0.f, 0.f);
-                        Tc[(size_t)q * n + p] = mk<float>(0.f, 0.f);
-                    }
-                    __syncwarp();
-                }
-            }
-            if (nrot == 0) break;
-        }
-        const double lref = s.lam[s.ord[q0]];
-        __syncwarp();
-        for (int p = lane; p < k; p += 32) s.lam[s.ord[q0 + p]] = lref + td[p];
-        __syncwarp();
-    }
-}
-
 // One FP64 step on X = s.D0 (row stride ld) and the levels s.lam0: s.lam and X
 // corrected.  Returns the largest |E| (NaN or infinite when the input is
 // unusable).
@@ -396,7 +331,8 @@ __device__ float step64(S64 &s, const HSource &h, int n, int m) {
     // level, which only their warp writes)
     for (int r = tid; r < n; r += nt)
         if (!oa_in_cluster(s.cst, n, r)) s.lam[s.ord[r]] += (double)s.corr[s.ord[r]];
-    resolve64(s, T, X, n, ld, 1e-15f * __int_as_float(s.scal[1]));
+    oa_resolve64(s.cst, s.ord, s.lam, s.tdiag, T, X, n, ld, 1e-15f * __int_as_float(s.scal[1]),
+                 tid >> 5, (nt + 31) >> 5);
     __syncthreads();
     const float step = __int_as_float(s.scal[2]);
     __syncthreads();
