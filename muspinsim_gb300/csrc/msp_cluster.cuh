@@ -61,6 +61,14 @@ __device__ __forceinline__ bool oa_in_cluster(const int *cstart, int n, int r) {
     return (r > 0 && cstart[r - 1] == cstart[r]) || (r + 1 < n && cstart[r + 1] == cstart[r]);
 }
 
+// A double-word as an integer in the same order (NaN at either end), so that a
+// sort by (key, index) is a permutation whatever the input.
+__device__ __forceinline__ long long oa_sort_key(float2 l) {
+    const int h = __float_as_int(l.x), e = __float_as_int(l.y);
+    const int hk = h < 0 ? h ^ 0x7fffffff : h, ek = e < 0 ? e ^ 0x7fffffff : e;
+    return ((long long)hk << 32) | ((unsigned)ek ^ 0x80000000u);
+}
+
 // The sort of the Rayleigh quotients lam (double-words, msp_dw.cuh) and the
 // cluster starts, once c.scal[0] holds amax (made visible by the barrier
 // inside).  All threads of the CTA call it; it ends with a barrier.
@@ -68,11 +76,11 @@ static __device__ void oa_cluster_starts(const float2 *lam, int n, const OaClust
     const int tid = threadIdx.x, nt = blockDim.x;
     // ascending order, ties by index
     for (int i = tid; i < n; i += nt) {
-        const float2 li = lam[i];
+        const long long li = oa_sort_key(lam[i]);
         int r = 0;
         for (int k = 0; k < n; ++k) {
-            const float2 lk = lam[k];
-            r += dw_less(lk, li) || (dw_equal(lk, li) && k < i);
+            const long long lk = oa_sort_key(lam[k]);
+            r += lk < li || (lk == li && k < i);
         }
         c.rank[i] = r;
         c.order[r] = i;

@@ -125,3 +125,21 @@ def test_general_path(dims):
         assert np.abs(got[k] - _signal(H, p[k])).max() <= TOL[_lib.PREC_FP64]
         w = 2 * np.pi * (lam[:, None] - lam)
         assert abs(mean[k].item() - (A / (1 + (w * tau) ** 2)).sum()) <= TOL[_lib.PREC_FP64]
+
+
+# a Hamiltonian that is not a number: reported or carried through, and the next
+# snapshot is not touched
+@pytest.mark.parametrize("prec", [_lib.PREC_FP64, _lib.PREC_MIXED])
+@pytest.mark.parametrize("n", [24, 32, 66, 96])
+def test_nan_field(n, prec):
+    rng = np.random.default_rng(n)
+    Hsys = _herm(rng, n)
+    Z = np.array([_herm(rng, n) for _ in range(3)])
+    B, p = 0.3 * rng.normal(size=(3, 3)), _unit(rng, 3)
+    B[1] = np.nan
+    out, _ = kernels.powder_run(n, Hsys, Z, B, p, np.ones(3), np.arange(3, dtype=np.int32), 3, TIMES,
+                                precision=prec)
+    got = out.cpu().numpy()
+    for k in (0, 2):
+        ref = _signal(Hsys + np.tensordot(B[k], Z, 1), p[k])
+        assert np.abs(got[k] - ref).max() <= TOL[prec]
