@@ -180,6 +180,24 @@ __device__ __forceinline__ float2 dw_add_f(float2 a, float b) {
     return dw_two_sum(t.x, __fadd_rn(t.y, a.y));
 }
 
+// One term of Re(conj(x) y) summed lane by lane from an anchor (lm_step's
+// scheme): x FP32, y = yh + yl.
+__device__ __forceinline__ void dw_dot(u64 &s, u64 &c, u64 x, u64 yh, u64 yl) {
+    const u64 t = fma_f32x2(x, yh, s);
+    c = add2(c, fma_f32x2(x, yh, sub2(s, t)));
+    c = fma_f32x2(x, yl, c);
+    s = t;
+}
+
+// The double-word sum of both lanes, anchor K removed.
+__device__ __forceinline__ float2 dw_dot_value(u64 s, u64 c, u64 K) {
+    float a, b, ca, cb;
+    split_f32x2(sub2(s, K), a, b);  // exact
+    split_f32x2(c, ca, cb);
+    float2 t = dw_two_sum(a, b);
+    return dw_two_sum(t.x, __fadd_rn(t.y, __fadd_rn(ca, cb)));
+}
+
 // a - b as a double-word
 __device__ __forceinline__ float2 dw_sub(float2 a, float2 b) {
     const float2 t = dw_two_sum(a.x, -b.x);

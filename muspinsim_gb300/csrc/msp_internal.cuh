@@ -49,6 +49,7 @@ struct SnapArgs {
     double gammas[MSP_MAX_SPINS];
     int fac_len;
     double tau;
+    float tau_f, itau_f;  // tau and 1 / tau rounded (0 without a decay time)
     // time grid (uniform grids: t_k = t0 + k dt); c_dt, c_t0 = 2 pi dt and
     // 2 pi t0 as double-words (hi, lo) for the mixed path's phase records,
     // and t0_zero = (t0 == 0)
@@ -80,8 +81,10 @@ struct SnapArgs {
     const long long *seg_hoff;
 };
 
-// Sets c_dt, c_t0 and t0_zero from t0 and dt.
+// Sets c_dt, c_t0 and t0_zero from t0 and dt, tau_f and itau_f from tau.
 inline void snap_time_constants(SnapArgs &a) {
+    a.tau_f = (float)a.tau;
+    a.itau_f = a.tau > 0.0 ? (float)(1.0 / a.tau) : 0.f;
     a.c_dt = dw_of(6.283185307179586476925 * a.dt);
     a.c_t0 = dw_of(6.283185307179586476925 * a.t0);
     a.t0_zero = a.t0 == 0.0;
@@ -194,7 +197,7 @@ cudaError_t launch_snapshots64(const SnapArgs &a, int mode, bool pre, cudaStream
 cudaError_t launch_eigh64(const double *H, int n, int batch, int max_sweeps, double *evals,
                           double *evecs, int *status, cudaStream_t st);
 // Threads per CTA of the snapshot kernels when the caller gives none.
-int snap_default_threads(int n);
+int snap_default_threads(int n, int precision);
 // CTAs of one snapshot kernel that fit on one SM with `threads` threads.
 int snap_occupancy(int n, int mode, int precision, int threads);
 cudaError_t launch_eigh(const double *H, int n, int batch, int precision, int max_sweeps,

@@ -144,24 +144,6 @@ __device__ void lm_colnorms(const float2 *X, int n, float *out, const LmVec &v, 
 
 // ------------------------------------------------------------------ double-word step
 
-// One term of Re(conj(x) y) summed lane by lane from an anchor (lm_step's
-// scheme): x FP32, y = yh + yl.
-__device__ __forceinline__ void lm_dot(u64 &s, u64 &c, u64 x, u64 yh, u64 yl) {
-    const u64 t = fma_f32x2(x, yh, s);
-    c = add2(c, fma_f32x2(x, yh, sub2(s, t)));
-    c = fma_f32x2(x, yl, c);
-    s = t;
-}
-
-// The double-word sum of both lanes, anchor K removed.
-__device__ __forceinline__ float2 lm_dot_value(u64 s, u64 c, u64 K) {
-    float a, b, ca, cb;
-    split_f32x2(sub2(s, K), a, b);  // exact
-    split_f32x2(c, ca, cb);
-    float2 t = dw_two_sum(a, b);
-    return dw_two_sum(t.x, __fadd_rn(t.y, __fadd_rn(ca, cb)));
-}
-
 // Rayleigh quotients and residuals from Y = H X: v.lam, v.gf = x_j^H x_j - 1
 // (in every CTA) and R = Y - X diag(l), 32 columns per CTA and turn, rows over
 // the warps.
@@ -191,11 +173,11 @@ __device__ void lm_residuals(const LargeSlot &s, const cx<float> *X, const LmVec
             const u64 x = Xp[(size_t)k * n + jc];
             u64 yh, yl;
             lm_pairs(&s.Y[(size_t)k * n + jc], yh, yl);
-            lm_dot(sy, cy, x, yh, yl);
-            lm_dot(sx, cc, x, x, 0ull);
+            dw_dot(sy, cy, x, yh, yl);
+            dw_dot(sx, cc, x, x, 0ull);
         }
-        dots[64 * warp + lane] = lm_dot_value(sy, cy, Ky);
-        dots[64 * warp + 32 + lane] = lm_dot_value(sx, cc, Kx);
+        dots[64 * warp + lane] = dw_dot_value(sy, cy, Ky);
+        dots[64 * warp + 32 + lane] = dw_dot_value(sx, cc, Kx);
         __syncthreads();
         float2 xy = dots[lane], xx = dots[32 + lane];
         for (int w = 1; w < nw; ++w) {

@@ -147,7 +147,8 @@ static int plan_layout(msp_multi_plan *p, const msp_multi_desc *d) {
             }
         const msp_multi_tuning *t = find_tuning(d, n);
         b.threads = t && t->snap_threads > 0 ? t->snap_threads
-                                             : (b.large ? large_threads(n) : snap_default_threads(n));
+                                             : (b.large ? large_threads(n)
+                                                        : snap_default_threads(n, d->precision));
         b.ctas_per_sm = t && t->ctas_per_sm > 0 ? t->ctas_per_sm
                                                 : (b.large ? large_ctas_per_sm(n, d->precision) : 0);
         long long cap = max_pairs / (b.P > 0 ? b.P : 1);

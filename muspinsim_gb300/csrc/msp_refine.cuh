@@ -103,6 +103,7 @@ struct SnapSmem {
     cx<double> *fac;
     cx<float> *facf;    // MIXED: FP32 copy of fac
     cx<T> *B2;
+    float4 *H4, *part;  // refinement by rows: H as double-words, a slot per thread
 };
 
 template <typename T, bool REFINE>
@@ -531,6 +532,390 @@ static __device__ int eigenpairs(SnapSmem<float> &s, int n, int m, int max_refin
         const float step = n == 24   ? oa_refine<24>(s, n, m)
                            : n == 32 ? oa_refine<32>(s, n, m)
                                      : oa_refine<0>(s, n, m);
+        if (step <= 2e-4f) return MSP_ITEM_OK;
+    }
+    return MSP_ITEM_REFINE_LIMIT;
+}
+
+// ------------------------------------------------------------------ refinement by rows
+
+// The refinement of the two-stage kernels (n <= 32), in residual form:
+//   l_j = x_j^H H x_j / x_j^H x_j,  r_j = H x_j - l_j x_j,  B = X^H R,
+//   E_ij = B_ij / (l_j - l_i),  E_jj = (1 - x_j^H x_j) / 2,  X <- X + X E
+// (B_ij is the S_ij + l_j R_ij of oa_refine).  r_j is small, so only H X and the
+// Rayleigh quotients need double-words, where oa_refine forms X^H H X and X^H X
+// in them too.  A thread owns a column j and four rows of every product: H X's
+// stay in its registers until the residuals are formed, B's until they have
+// become E, and an element of the row operand is a broadcast that serves four
+// elements (oa_refine loads three operands for each).  n = 32: FP32 pipe 10
+// + 2 + 2 packed FMAs per complex product against 22, 42 KB of shared memory
+// against 59.  Scan of n = 32: 21.5 ms against 28.6; powder of n =
+// 24: 0.41 ms against 0.47.
+
+// Groups of rows, rows per group and rows the matrices are padded to.
+constexpr int ROW_MAX = 4;  // largest number of rows per thread
+
+struct RowShape {
+    int groups, rows, padded;
+};
+
+__host__ __device__ inline RowShape row_shape(int n, int threads) {
+    RowShape s;
+    s.groups = threads / n < n ? threads / n : n;
+    s.rows = (n + s.groups - 1) / s.groups;
+    s.padded = (s.groups - 1) * s.rows + ROW_MAX;
+    if (s.padded < n) s.padded = n;
+    return s;
+}
+
+// At most four rows per thread.  (Eight, in half the threads, spill at 96
+// registers and leave too few warps at 128: scan of n = 32, 27 ms against 22.)
+inline int row_threads(int n) { return n <= 8 ? 32 : n <= 16 ? 64 : n <= 24 ? 160 : 256; }
+
+// Row stride of H4: odd, for the transposed stores
+__host__ __device__ inline int row_ldh(int n) { return n | 1; }
+
+struct RowLayout {
+    size_t H4, U, R, SR, part, red, lw, corr, rk, ord, cst, scal, rn, fac, facf, total;
+};
+
+__host__ __device__ inline RowLayout row_layout(int n, bool rho, int fac_len, int threads) {
+    RowLayout L;
+    const size_t m = (size_t)(n + (n & 1)), mm = (size_t)row_shape(n, threads).padded * (m + 1) * 8;
+    size_t off = 0;
+    L.H4 = lay_take(off, (size_t)row_shape(n, threads).padded * row_ldh(n) * 16);
+    L.U = lay_take(off, mm);
+    L.R = lay_take(off, mm);
+    L.SR = lay_take(off, mm);
+    L.part = lay_take(off, (size_t)threads * 16);
+    L.red = lay_take(off, (size_t)(threads / 32) * 8);
+    L.lw = lay_take(off, m * 8);
+    L.corr = lay_take(off, m * 4);
+    L.rk = lay_take(off, m * 4);
+    L.ord = lay_take(off, m * 4);
+    L.cst = lay_take(off, m * 4);
+    L.scal = lay_take(off, 4 * 4);
+    L.rn = lay_take(off, (size_t)row_shape(n, threads).padded * 4);
+    L.fac = L.facf = 0;
+    if (rho) {
+        L.fac = lay_take(off, (size_t)fac_len * 16);
+        L.facf = lay_take(off, (size_t)fac_len * 8);
+    }
+    L.total = (off + 15) & ~size_t(15);
+    return L;
+}
+
+__device__ __forceinline__ SnapSmem<float> row_carve(char *base, int n, bool rho, int fac_len) {
+    const RowLayout L = row_layout(n, rho, fac_len, blockDim.x);
+    SnapSmem<float> s = {};
+    s.H4 = reinterpret_cast<float4 *>(base + L.H4);
+    s.w.U = reinterpret_cast<cx<float> *>(base + L.U);
+    s.w.H = reinterpret_cast<cx<float> *>(base + L.R);
+    s.SR = s.B2 = reinterpret_cast<cx<float> *>(base + L.SR);
+    s.part = reinterpret_cast<float4 *>(base + L.part);
+    s.w.red = reinterpret_cast<float *>(base + L.red);
+    s.lw = reinterpret_cast<float2 *>(base + L.lw);
+    s.corr = reinterpret_cast<float *>(base + L.corr);
+    s.rk = reinterpret_cast<int *>(base + L.rk);
+    s.ord = reinterpret_cast<int *>(base + L.ord);
+    s.cst = reinterpret_cast<int *>(base + L.cst);
+    s.scal = reinterpret_cast<int *>(base + L.scal);
+    s.rn = reinterpret_cast<float *>(base + L.rn);
+    if (rho) {
+        s.fac = reinterpret_cast<cx<double> *>(base + L.fac);
+        s.facf = reinterpret_cast<cx<float> *>(base + L.facf);
+    }
+    return s;
+}
+
+// H = Hsys + b . Z as double-words into s.H4 (row stride n, the upper triangle
+// mirrored), in double-word FP32 from pre-split matrices or in FP64, and the
+// row norms of its high words.
+__device__ __forceinline__ void load_hamiltonian_rows(const SnapSource &src, const double *b, int n,
+                                                      SnapSmem<float> &s) {
+    const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, ldh = row_ldh(n);
+    const size_t nn = (size_t)n * n;
+    float2 bx, by, bz;
+    field_dw(b, bx, by, bz);
+#pragma unroll 3
+    for (int e = tid; e < n * (n + 1) / 2; e += nt) {
+        int i, j;
+        tri_index(e, j, i);  // i <= j
+        const size_t o = (size_t)i * n + j;
+        float4 h;
+        if (src.Hdw != nullptr) {
+            const float4 hs = src.Hdw[o], z0 = src.Zdw[o], z1 = src.Zdw[nn + o], z2 = src.Zdw[2 * nn + o];
+            float sr = hs.x, cr = hs.z, si = hs.y, ci = hs.w;
+            dw_acc_prod(sr, cr, bx, z0.x, z0.z);
+            dw_acc_prod(si, ci, bx, z0.y, z0.w);
+            dw_acc_prod(sr, cr, by, z1.x, z1.z);
+            dw_acc_prod(si, ci, by, z1.y, z1.w);
+            dw_acc_prod(sr, cr, bz, z2.x, z2.z);
+            dw_acc_prod(si, ci, bz, z2.y, z2.w);
+            const float2 hr = dw_two_sum(sr, cr), hi = dw_two_sum(si, ci);
+            h = make_float4(hr.x, hi.x, hr.y, hi.y);
+        } else {
+            const cx<double> hs = src.Hsys[o], z0 = src.Z[o], z1 = src.Z[nn + o], z2 = src.Z[2 * nn + o];
+            h = dw_split(make_double2(hs.re + b[0] * z0.re + b[1] * z1.re + b[2] * z2.re,
+                                      hs.im + b[0] * z0.im + b[1] * z1.im + b[2] * z2.im));
+        }
+        if (i == j) h.y = h.w = 0.f;
+        s.H4[i * ldh + j] = h;
+        if (i != j) s.H4[j * ldh + i] = make_float4(h.x, -h.y, h.z, -h.w);
+    }
+    __syncthreads();
+    for (int i = tid >> 5; i < n; i += nt >> 5) {
+        const float4 h = lane < n ? s.H4[i * ldh + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
+        float acc = fmaf(h.x, h.x, h.y * h.y);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        if (lane == 0) s.rn[i] = sqrtf(acc);
+    }
+    __syncthreads();
+}
+
+// (X^H X)_ij, i != j, to FP32 rounding of its terms' sum
+__device__ __forceinline__ cx<float> row_gram(const cx<float> *X, int n, int ld, int i, int j, u64 K) {
+    u64 s1 = K, c1 = 0ull, s2 = K, c2 = 0ull;
+    for (int k = 0; k < n; ++k) {
+        const cx<float> y = X[k * ld + j];
+        lm_step<false, false>(s1, c1, s2, c2, *reinterpret_cast<const u64 *>(X + k * ld + i), 0ull,
+                              f32x2(y.re, y.re), f32x2(y.im, y.im), 0ull, 0ull);
+    }
+    const float4 r = lm_dw<true>(s1, c1, s2, c2, K);
+    return mk<float>(r.x + r.z, r.y + r.w);
+}
+
+// This thread's rows of column j of X^H W: b[r] = sum_k conj(X_k,i1+r) W_kj
+template <int NN, int RB>
+__device__ __forceinline__ void row_products(const cx<float> *X, const cx<float> *W, int n_rt, int i1,
+                                             int j, cx<float> (&b)[RB]) {
+    const int n = NN > 0 ? NN : n_rt, ld = n + (n & 1) + 1;
+    u64 s1[RB], s2[RB];
+#pragma unroll
+    for (int r = 0; r < RB; ++r) s1[r] = s2[r] = 0ull;
+#pragma unroll 8
+    for (int k = 0; k < n; ++k) {
+        const cx<float> q = W[k * ld + j];
+        const u64 bx = f32x2(q.re, q.re), by = f32x2(q.im, q.im);
+        const u64 *x = reinterpret_cast<const u64 *>(X + k * ld + i1);
+#pragma unroll
+        for (int r = 0; r < RB; ++r) {
+            s1[r] = fma_f32x2(x[r], bx, s1[r]);
+            s2[r] = fma_f32x2(x[r], by, s2[r]);
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < RB; ++r) b[r] = lm_plain<true>(s1[r], s2[r]);
+}
+
+// One refinement step by rows: the vectors in s.w.U, the levels in s.lw.
+// Returns its largest correction.  NN > 0: n = NN at compile time.
+template <int NN, int RB>
+__device__ __forceinline__ float oa_refine_rows(SnapSmem<float> &s, int n_rt) {
+    const int n = NN > 0 ? NN : n_rt, ld = n + (n & 1) + 1, tid = threadIdx.x;
+    const RowShape sh = row_shape(n, blockDim.x);
+    const int rg = tid / n, j = tid - rg * n, i0 = rg * sh.rows;
+    // threads past the last group follow along on the first rows and store nothing
+    const bool active = rg < sh.groups;
+    const int i1 = active ? i0 : 0;
+    auto mine = [&](int r) { return active && r < sh.rows && i0 + r < n; };
+    cx<float> *X = s.w.U, *R = s.w.H, *T = s.w.H;
+    if (tid < 4) s.scal[tid] = 0;  // [0]: amax, [1]: max|l|, [2]: step (float bits), [3]: clusters
+    float sx = 0.f;
+#pragma unroll
+    for (int r = 0; r < RB; ++r)
+        if (mine(r)) sx += cabs2(X[(i0 + r) * ld + j]);
+    if (active) s.part[tid].x = sx;
+    __syncthreads();
+    float cn = 0.f;
+    for (int g = 0; g < sh.groups; ++g) cn += s.part[g * n + j].x;
+    cn = sqrtf(cn);
+    // H X
+    float4 y[RB];
+    {
+        u64 s1[RB], c1[RB], s2[RB], c2[RB];
+#pragma unroll
+        for (int r = 0; r < RB; ++r) {
+            s1[r] = s2[r] = lm_anchor(s.rn[i1 + r] * cn);
+            c1[r] = c2[r] = 0ull;
+        }
+        const int ldh = row_ldh(n);
+        const float4 *H = s.H4 + i1 * ldh;
+#pragma unroll 4
+        for (int k = 0; k < n; ++k) {
+            const cx<float> x = X[k * ld + j];
+            const u64 bx = f32x2(x.re, x.re), by = f32x2(x.im, x.im);
+#pragma unroll
+            for (int r = 0; r < RB; ++r) {
+                const ulonglong2 h = *reinterpret_cast<const ulonglong2 *>(H + r * ldh + k);
+                lm_step<true, false>(s1[r], c1[r], s2[r], c2[r], h.x, h.y, bx, by, 0ull, 0ull);
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < RB; ++r)
+            y[r] = lm_dw<false>(s1[r], c1[r], s2[r], c2[r], lm_anchor(s.rn[i1 + r] * cn));
+    }
+    // Rayleigh quotients from this thread's rows, then every group's
+    {
+        float sy = 0.f;
+#pragma unroll
+        for (int r = 0; r < RB; ++r)
+            if (mine(r)) sy = fmaf(y[r].x, y[r].x, fmaf(y[r].y, y[r].y, sy));
+        const u64 Ky = lm_anchor(sqrtf(sx * sy)), Kx = lm_anchor(sx);
+        u64 dy = Ky, cy = 0ull, dx = Kx, cc = 0ull;
+#pragma unroll
+        for (int r = 0; r < RB; ++r) {
+            if (!mine(r)) continue;
+            const u64 x = *reinterpret_cast<const u64 *>(X + (i0 + r) * ld + j);
+            dw_dot(dy, cy, x, f32x2(y[r].x, y[r].y), f32x2(y[r].z, y[r].w));
+            dw_dot(dx, cc, x, x, 0ull);
+        }
+        const float2 a = dw_dot_value(dy, cy, Ky), b = dw_dot_value(dx, cc, Kx);
+        __syncthreads();  // the norms have been read
+        if (active) s.part[tid] = make_float4(a.x, a.y, b.x, b.y);
+    }
+    __syncthreads();
+    float4 d = s.part[j];
+    for (int g = 1; g < sh.groups; ++g) {
+        const float4 e = s.part[g * n + j];
+        dw_add(d.x, d.y, e.x, e.y);
+        dw_add(d.z, d.w, e.z, e.w);
+    }
+    const float2 gj = dw_add_f(dw_two_sum(d.z, d.w), -1.0f);
+    const float2 lj = dw_rayleigh(dw_two_sum(d.x, d.y), gj);
+    if (rg == 0) {
+        s.lw[j] = lj;
+        atomicMax(&s.scal[1], __float_as_int(fabsf(lj.x)));  // non-negative: int order = float order
+    }
+#pragma unroll
+    for (int r = 0; r < RB; ++r) {
+        if (!mine(r)) continue;
+        const cx<float> x = X[(i0 + r) * ld + j];
+        R[(i0 + r) * ld + j] = mk<float>(fmaf(-lj.x, x.re, y[r].x) + fmaf(-lj.y, x.re, y[r].z),
+                                         fmaf(-lj.x, x.im, y[r].y) + fmaf(-lj.y, x.im, y[r].w));
+    }
+    __syncthreads();
+    // B = X^H R
+    cx<float> b[RB];
+    row_products<NN, RB>(X, R, n, i1, j, b);
+    {
+        float amax = 0.f;
+#pragma unroll
+        for (int r = 0; r < RB; ++r) {
+            if (mine(r) && i0 + r != j) amax = fmaxf(amax, fmaxf(fabsf(b[r].re), fabsf(b[r].im)));
+        }
+        const int am = __reduce_max_sync(0xffffffffu, __float_as_int(amax));
+        if ((tid & 31) == 0) atomicMax(&s.scal[0], am);
+    }
+    __syncthreads();
+    OaCluster cl;
+    cl.rank = s.rk;
+    cl.order = s.ord;
+    cl.cstart = s.cst;
+    cl.scal = s.scal;
+    cl.T = T;
+    cl.ldt = ld;
+    oa_cluster_starts(s.lw, n, cl);
+    // E; the couplings inside clusters go to T
+    float emax = 0.f, corr = 0.f;
+    const int rj = s.rk[j], cj = s.cst[rj];
+    bool any = false;
+#pragma unroll
+    for (int r = 0; r < RB; ++r) {
+        const int i = i0 + r;
+        if (!mine(r)) continue;
+        cx<float> E;
+        if (i == j) {
+            E = mk<float>(-0.5f * (gj.x + gj.y), 0.f);
+        } else if (s.cst[s.rk[i]] == cj) {
+            any = true;
+            T[s.rk[i] * ld + rj] = b[r];
+            const cx<float> G = row_gram(X, n, ld, i, j, lm_anchor(1.1f * cn * cn));
+            E = mk<float>(-0.5f * G.re, -0.5f * G.im);
+        } else {
+            const float inv = 1.0f / dw_sub_f(lj, s.lw[i]);
+            E = mk<float>(b[r].re * inv, b[r].im * inv);
+            corr = fmaf(b[r].re * b[r].re + b[r].im * b[r].im, inv, corr);
+            emax = fmaxf(emax, fmaxf(fabsf(E.re), fabsf(E.im)));
+        }
+        s.SR[i * ld + j] = E;
+    }
+    if (active) s.part[tid].x = corr;
+    if (any) s.scal[3] = 1;
+    {
+        const int em = __reduce_max_sync(0xffffffffu, __float_as_int(emax));
+        if ((tid & 31) == 0) atomicMax(&s.scal[2], em);  // non-negative: int order = float order
+    }
+    __syncthreads();
+    const bool clusters = s.scal[3] != 0;  // the same in every thread
+    if (rg == 0) {
+        float c = 0.f;
+        for (int g = 0; g < sh.groups; ++g) c += s.part[g * n + j].x;
+        s.corr[j] = c;
+    }
+    if (clusters) {
+        // T Hermitian
+        for (int r = 0; r < sh.rows; ++r) {
+            const int i = i0 + r;
+            if (!mine(r) || i >= j || s.cst[s.rk[i]] != cj) continue;
+            const int ri = s.rk[i];
+            const cx<float> u = T[ri * ld + rj], l = T[rj * ld + ri];
+            const cx<float> t = mk<float>(0.5f * (u.re + l.re), 0.5f * (u.im - l.im));
+            T[ri * ld + rj] = t;
+            T[rj * ld + ri] = conj(t);
+        }
+        __syncthreads();
+        oa_cluster_diagonal(s.lw, s.corr, n, cl);
+    }
+    // X + X E
+    {
+        u64 s1[RB], s2[RB];
+#pragma unroll
+        for (int r = 0; r < RB; ++r) {
+            s1[r] = *reinterpret_cast<const u64 *>(X + (i1 + r) * ld + j);
+            s2[r] = 0ull;
+        }
+#pragma unroll 8
+        for (int i = 0; i < n; ++i) {
+            const cx<float> e = s.SR[i * ld + j];
+            const u64 bx = f32x2(e.re, e.re), by = f32x2(e.im, e.im);
+#pragma unroll
+            for (int r = 0; r < RB; ++r) {
+                const u64 x = *reinterpret_cast<const u64 *>(X + (i1 + r) * ld + i);
+                s1[r] = fma_f32x2(x, bx, s1[r]);
+                s2[r] = fma_f32x2(x, by, s2[r]);
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < RB; ++r)
+            if (mine(r)) X[(i0 + r) * ld + j] = lm_plain<false>(s1[r], s2[r]);
+    }
+    __syncthreads();
+    if (clusters) {
+        const float em = oa_resolve_clusters(X, ld, n, s.lw, s.corr, n, cl, __int_as_float(s.scal[1]));
+        atomicMax(&s.scal[2], __float_as_int(em));
+    } else if (rg == 0) {
+        s.lw[j] = dw_add_f(s.lw[j], s.corr[j]);
+    }
+    __syncthreads();
+    const float step = __int_as_float(s.scal[2]);
+    __syncthreads();
+    return step;
+}
+
+// Refined eigenpairs (see eigenpairs above) of a two-stage kernel.  One copy for
+// all kernels; it carves shared memory itself so that its accesses stay
+// shared-memory accesses.
+static __noinline__ __device__ int eigenpairs_rows(int n, bool rho, int fac_len, int max_refine) {
+    extern __shared__ __align__(16) char smem[];
+    SnapSmem<float> s = row_carve(smem, n, rho, fac_len);
+    if (max_refine <= 0) max_refine = 4;
+    for (int it = 0; it < max_refine; ++it) {
+        const float step = n == 24   ? oa_refine_rows<24, ROW_MAX>(s, n)
+                           : n == 32 ? oa_refine_rows<32, ROW_MAX>(s, n)
+                                     : oa_refine_rows<0, ROW_MAX>(s, n);
         if (step <= 2e-4f) return MSP_ITEM_OK;
     }
     return MSP_ITEM_REFINE_LIMIT;

@@ -69,12 +69,11 @@ __global__ void msp_eigh_kernel(const cx<double> *__restrict__ Hin, int n, int b
 
 // Mixed fast path: A_jk = |(U^H M)_jk|^2 over the lower triangle j >= k
 // (FP32), pair records for j > k, and this thread's share of sum_j A_jj as
-// a double-word.  NN > 0: n = NN at compile time.
-template <int NN>
+// a double-word.
 __device__ __forceinline__ float2 amplitudes_mixed(const SnapArgs &a, const SnapSmem<float> &s,
-                                                   const cx<float> *U, const cx<float> *M,
-                                                   int n_rt, int sn, float scale) {
-    const int n = NN > 0 ? NN : n_rt, ld = n + (n & 1) + 1;
+                                                   const cx<float> *U, const cx<float> *M, int n,
+                                                   int sn, float scale) {
+    const int ld = n + (n & 1) + 1;
     const int P = n * (n - 1) / 2, ntri = n * (n + 1) / 2;
     float2 diag = make_float2(0.f, 0.f);
     for (int e = threadIdx.x; e < ntri; e += blockDim.x) {
@@ -99,27 +98,61 @@ __device__ __forceinline__ float2 amplitudes_mixed(const SnapArgs &a, const Snap
     return diag;
 }
 
+// The same in the two-stage kernels: a thread's rows k <= j of column j of the
+// Hermitian U^H M (see oa_refine_rows).
+template <int NN>
+__device__ __forceinline__ float2 amplitudes_rows(const SnapArgs &a, const SnapSmem<float> &s,
+                                                  const cx<float> *U, const cx<float> *M, int n_rt,
+                                                  int sn, float scale) {
+    const int n = NN > 0 ? NN : n_rt;
+    const size_t rec = (size_t)sn * (n * (n - 1) / 2);
+    const RowShape sh = row_shape(n, blockDim.x);
+    const int rg = threadIdx.x / n, j = threadIdx.x - rg * n, i0 = rg * sh.rows;
+    float2 diag = make_float2(0.f, 0.f);
+    if (rg >= sh.groups || i0 > j) return diag;
+    cx<float> b[ROW_MAX];
+    row_products<NN, ROW_MAX>(U, M, n, i0, j, b);
+#pragma unroll
+    for (int r = 0; r < ROW_MAX; ++r) {
+        const int k = i0 + r;
+        if (r >= sh.rows || k > j) continue;
+        const float A = cabs2(b[r]);
+        if (j == k) {
+            diag = dw_add_f(diag, A);
+        } else {
+            const size_t o = rec + pair_index(j, k);
+            reinterpret_cast<float2 *>(a.pair_coef)[o] = make_float2(scale * A, 0.f);
+            store_frequency_dw(a, o, dw_sub(s.lw[j], s.lw[k]));
+        }
+    }
+    return diag;
+}
+
 // One snapshot of the muon-first T = inf shortcut (muspinsim/hamiltonian.py:
 // 166-217): A = |U^dag (sigma_p (x) 1_d) U|^2 and omega_jk = 2 pi (l_j - l_k)
 // for j > k, scaled by 0.5 * w / (d * N_avg), plus the constant
 // 0.5 * sum_j A_jj part.
-// At most 64 registers (no spills; ptxas would take ~88 and fit 5 instead of
-// 7-8 CTAs of 128 threads per SM).
+// PRE: the FP32 eigenvectors come from the first stage (n <= 32), refined by
+// rows; else (n > 32) Jacobi and oa_refine in this CTA.  At most 64 registers,
+// which leaves as many CTAs per SM as shared memory does.
 template <bool PRE>
 __global__ void __maxnreg__(64) msp_snap_fast_kernel(SnapArgs a) {
     typedef float T;
     extern __shared__ __align__(16) char smem[];
     const int n = a.n, m = n + (n & 1), ld = m + 1, d = n / 2;
-    SnapSmem<T> s = snap_carve<T, true>(smem, n, false, 0);
+    SnapSmem<T> s = PRE ? row_carve(smem, n, false, 0) : snap_carve<T, true>(smem, n, false, 0);
     const int tid = threadIdx.x, nt = blockDim.x;
 
     for (int sn = blockIdx.x; sn < a.num_snap; sn += gridDim.x) {
         const SnapSource src = snap_source(a, sn);
         const size_t g = (size_t)src.g;
-        load_hamiltonian<T, true, PRE>(src.Hsys, src.Z, src.Hdw, src.Zdw, a.field + 3 * g, n, m,
-                                       s);
+        if (PRE)
+            load_hamiltonian_rows(src, a.field + 3 * g, n, s);
+        else
+            load_hamiltonian<T, true, PRE>(src.Hsys, src.Z, src.Hdw, src.Zdw, a.field + 3 * g, n, m,
+                                           s);
         int st = snap_eigvecs<T, PRE>(a, sn, (int)g, n, m, s);
-        st |= eigenpairs(s, n, m, a.max_refine);
+        st |= PRE ? eigenpairs_rows(n, false, 0, a.max_refine) : eigenpairs(s, n, m, a.max_refine);
 
         // sigma_p = p . sigma (Pauli), applied on the muon (slowest) digit
         T px, py, pz;
@@ -140,9 +173,10 @@ __global__ void __maxnreg__(64) msp_snap_fast_kernel(SnapArgs a) {
         __syncthreads();
         // FP32 amplitudes, double-word level gaps and diagonal sum
         const float scale = (float)a.wscale[g] * (0.5f / (float)d);
-        const float2 diag = n == 24   ? amplitudes_mixed<24>(a, s, U, M, n, sn, scale)
-                            : n == 32 ? amplitudes_mixed<32>(a, s, U, M, n, sn, scale)
-                                      : amplitudes_mixed<0>(a, s, U, M, n, sn, scale);
+        const float2 diag = !PRE      ? amplitudes_mixed(a, s, U, M, n, sn, scale)
+                            : n == 24 ? amplitudes_rows<24>(a, s, U, M, n, sn, scale)
+                            : n == 32 ? amplitudes_rows<32>(a, s, U, M, n, sn, scale)
+                                      : amplitudes_rows<0>(a, s, U, M, n, sn, scale);
         const double dsum = dw_block_sum(diag, reinterpret_cast<float2 *>(s.w.red));
         if (tid == 0) {
             a.snap_const[sn] = 0.25 * a.wscale[g] * dsum / (double)d;
@@ -154,55 +188,82 @@ __global__ void __maxnreg__(64) msp_snap_fast_kernel(SnapArgs a) {
 
 // ------------------------------------------------------------------ general path
 
-// Mixed general path: every term C_jk = rho'_jk O'_kj (j >= k, O'_kj =
-// sum_i conj(U_ik) (O U)_ij): pair records (EVOLVE) or the decaying-integral
-// terms (INTEGRAL); returns this thread's share of the constant / integral
-// as a double-word.  rho' comes from Y, or (hot) from O' itself: (delta_jk +
-// hot_scale O'_jk n) / n.  NN > 0: n = NN at compile time.
-template <bool INTEGRAL, int NN>
+// The term C_jk = rho'_jk O'_kj of a pair j >= k: its pair record (EVOLVE) or
+// decaying-integral term (INTEGRAL); `local` collects the constant / integral.
+template <bool INTEGRAL>
+__device__ __forceinline__ void rho_term(const SnapArgs &a, const SnapSmem<float> &s, size_t rec, int j,
+                                         int k, cx<float> r, cx<float> o, float scale2, float tau_f,
+                                         float itau_f, float2 &local) {
+    const float cr = r.re * o.re - r.im * o.im;
+    const float ci = r.re * o.im + r.im * o.re;
+    if (INTEGRAL) {
+        // term = C_jk (-1) / (2 pi i (l_k - l_j) - 1/tau); pairs count twice
+        if (j == k) {
+            local = dw_add_f(local, cr * tau_f);
+        } else {
+            const float gap = dw_sub_f(s.lw[k], s.lw[j]);
+            const float x = fmaf(gap, MSP_TWOPI_HI, gap * MSP_TWOPI_LO);
+            const float den = fmaf(x, x, itau_f * itau_f);
+            local = dw_add_f(local, 2.0f * (cr * itau_f - ci * x) / den);
+        }
+    } else {
+        if (j == k) {
+            local = dw_add_f(local, cr);
+        } else {
+            const size_t at = rec + pair_index(j, k);
+            reinterpret_cast<float2 *>(a.pair_coef)[at] = make_float2(scale2 * cr, scale2 * ci);
+            store_frequency_dw(a, at, dw_sub(s.lw[j], s.lw[k]));
+        }
+    }
+}
+
+// Every term j >= k with O'_kj = sum_i conj(U_ik) (O U)_ij; returns this thread's
+// share of the constant / integral as a double-word.  rho' comes from rho0 U in
+// X, or (hot) from O' itself: rho'_jk = (delta_jk + hot_scale O'_jk n) / n.
+// !ROWS: rho'_jk in X already.
+template <bool INTEGRAL, bool ROWS, int NN>
 __device__ __forceinline__ float2 rho_terms_mixed(const SnapArgs &a, const SnapSmem<float> &s,
                                                   const cx<float> *U, const cx<float> *OU,
-                                                  const cx<float> *Y, int n_rt, int sn,
-                                                  float tau_f, float itau_f, bool hot,
-                                                  float hot_scale) {
+                                                  const cx<float> *X, int n_rt, int sn, float tau_f,
+                                                  float itau_f, bool hot, float hot_scale) {
     const int n = NN > 0 ? NN : n_rt, ld = n + (n & 1) + 1;
-    const int P = n * (n - 1) / 2, ntri = n * (n + 1) / 2;
+    const size_t rec = (size_t)sn * (n * (n - 1) / 2);
     const float scale2 = 2.0f * (float)a.wscale[sn];
     float2 local = make_float2(0.f, 0.f);
+    auto rho_hot = [&](cx<float> o, bool diagonal) {
+        return mk<float>(fmaf(hot_scale, o.re, diagonal ? 1.0f / (float)n : 0.f), -hot_scale * o.im);
+    };
+    if (ROWS) {
+        // a thread's rows k <= j of column j (see oa_refine_rows)
+        const RowShape sh = row_shape(n, blockDim.x);
+        const int rg = threadIdx.x / n, j = threadIdx.x - rg * n, i0 = rg * sh.rows;
+        if (rg >= sh.groups || i0 > j) return local;
+        cx<float> o[ROW_MAX], r[ROW_MAX];
+        row_products<NN, ROW_MAX>(U, OU, n, i0, j, o);
+        if (!hot) row_products<NN, ROW_MAX>(U, X, n, i0, j, r);  // rho'_kj
+#pragma unroll
+        for (int q = 0; q < ROW_MAX; ++q) {
+            const int k = i0 + q;
+            if (q >= sh.rows || k > j) continue;
+            rho_term<INTEGRAL>(a, s, rec, j, k, hot ? rho_hot(o[q], j == k) : conj(r[q]), o[q], scale2,
+                               tau_f, itau_f, local);
+        }
+        return local;
+    }
+    const int ntri = n * (n + 1) / 2;
     for (int e = threadIdx.x; e < ntri; e += blockDim.x) {
         int j, k;
         tri_index(e, j, k);
         float orr = 0.f, oii = 0.f;
-#pragma unroll
+#pragma unroll 4
         for (int i = 0; i < n; ++i) {
             const cx<float> u = U[i * ld + k], x = OU[i * ld + j];
             orr += u.re * x.re + u.im * x.im;
             oii += u.re * x.im - u.im * x.re;
         }
-        const cx<float> r =
-            hot ? mk<float>(fmaf(hot_scale, orr, j == k ? 1.0f / (float)n : 0.f), -hot_scale * oii)
-                : Y[j * ld + k];
-        const float cr = r.re * orr - r.im * oii;
-        const float ci = r.re * oii + r.im * orr;
-        if (INTEGRAL) {
-            // term = C_jk (-1) / (2 pi i (l_k - l_j) - 1/tau); pairs count twice
-            if (j == k) {
-                local = dw_add_f(local, cr * tau_f);
-            } else {
-                const float gap = dw_sub_f(s.lw[k], s.lw[j]);
-                const float x = fmaf(gap, MSP_TWOPI_HI, gap * MSP_TWOPI_LO);
-                const float den = fmaf(x, x, itau_f * itau_f);
-                local = dw_add_f(local, 2.0f * (cr * itau_f - ci * x) / den);
-            }
-        } else {
-            if (j == k) {
-                local = dw_add_f(local, cr);
-            } else {
-                const size_t o = (size_t)sn * P + pair_index(j, k);
-                reinterpret_cast<float2 *>(a.pair_coef)[o] = make_float2(scale2 * cr, scale2 * ci);
-                store_frequency_dw(a, o, dw_sub(s.lw[j], s.lw[k]));
-            }
-        }
+        const cx<float> o = mk<float>(orr, oii);
+        rho_term<INTEGRAL>(a, s, rec, j, k, hot ? rho_hot(o, j == k) : X[j * ld + k], o, scale2, tau_f,
+                           itau_f, local);
     }
     return local;
 }
@@ -214,34 +275,41 @@ __device__ __forceinline__ float2 rho_terms_mixed(const SnapArgs &a, const SnapS
 // divided by tau (muspinsim/hamiltonian.py:150-164, experiment.py:492-496).
 // At T = inf rho' follows from O' (rho_is_hot), which leaves one eigenbasis
 // product instead of two and the digit products.
-// At most 96 registers (shared memory limits these CTAs to ~4 per SM at n =
-// 32 anyway).
+// PRE: as in msp_snap_fast_kernel, 64 registers (four CTAs of 256 threads per SM
+// at n = 32; 22.6 ms with 80, 25.5 with 96 where 64 take 22.1).
 template <bool INTEGRAL, bool PRE>
-__global__ void __maxnreg__(96) msp_snap_rho_kernel(SnapArgs a) {
+__global__ void __maxnreg__(PRE ? 64 : 96) msp_snap_rho_kernel(SnapArgs a) {
     typedef float T;
     extern __shared__ __align__(16) char smem[];
     const int n = a.n, m = n + (n & 1), ld = m + 1;
-    SnapSmem<T> s = snap_carve<T, true>(smem, n, true, a.fac_len);
+    SnapSmem<T> s =
+        PRE ? row_carve(smem, n, true, a.fac_len) : snap_carve<T, true>(smem, n, true, a.fac_len);
     const int tid = threadIdx.x, nt = blockDim.x;
-    const float tau_f = INTEGRAL ? (float)a.tau : 0.f;
-    const float itau_f = INTEGRAL ? (float)(1.0 / a.tau) : 0.f;
+    const float tau_f = a.tau_f, itau_f = a.itau_f;
+    __shared__ float hot_scale[1];
 
     for (int sn = blockIdx.x; sn < a.num_snap; sn += gridDim.x) {
         const bool hot = rho_is_hot(a, sn);
+        // some forty FP64 operations: one thread's, read many barriers later
+        if (hot && tid == nt - 1) *hot_scale = (float)rho_hot_scale(a, sn);
         if (a.rho_fac) {
             for (int e = tid; e < a.fac_len; e += nt)
                 s.fac[e] = a.rho_fac[(size_t)sn * a.fac_len + e];
         } else if (!hot) {
             build_rho_factors(a, sn, s.fac);
         }
-        load_hamiltonian<T, true, PRE>(a.Hsys, a.Z, a.Hsys_dw, a.Z_dw, a.field + 3 * (size_t)sn,
-                                       n, m, s);
+        if (PRE)
+            load_hamiltonian_rows(snap_source(a, sn), a.field + 3 * (size_t)sn, n, s);
+        else
+            load_hamiltonian<T, true, PRE>(a.Hsys, a.Z, a.Hsys_dw, a.Z_dw,
+                                           a.field + 3 * (size_t)sn, n, m, s);
         // made visible by the eigensolve's barriers
         if (!hot)
             for (int e = tid; e < a.fac_len; e += nt)
                 s.facf[e] = mk<float>((float)s.fac[e].re, (float)s.fac[e].im);
         int st = snap_eigvecs<T, PRE>(a, sn, sn, n, m, s);
-        st |= eigenpairs(s, n, m, a.max_refine);
+        st |= PRE ? eigenpairs_rows(n, true, a.fac_len, a.max_refine)
+                  : eigenpairs(s, n, m, a.max_refine);
         const cx<T> *U = s.w.U;
 
         const cx<T> *X = s.w.H;
@@ -258,17 +326,17 @@ __global__ void __maxnreg__(96) msp_snap_rho_kernel(SnapArgs a) {
                 X = Y;
                 Y = (Y == s.w.H) ? s.B2 : s.w.H;
             }
-            // X holds rho0 U.  rho'_jk (j >= k) -> Y (the other buffer).
-            if (n == 24)
-                tri_conj_products<T, 24>(U, X, Y, n);
-            else if (n == 32)
-                tri_conj_products<T, 32>(U, X, Y, n);
-            else
+            if (!PRE) {
+                // X holds rho0 U.  rho'_jk (j >= k) -> Y (the other buffer).
                 tri_conj_products<T, 0>(U, X, Y, n);
-            __syncthreads();
+                __syncthreads();
+                cx<T> *t = Y;
+                Y = const_cast<cx<T> *>(X);
+                X = t;
+            }
         }
-        // O U into the buffer X (free now): O = sum_a p_a S^a on the muon digit
-        cx<T> *OU = const_cast<cx<T> *>(X);
+        // O U into the buffer Y (free now): O = sum_a p_a S^a on the muon digit
+        cx<T> *OU = Y;
         {
             T px, py, pz;
             load_vec3<T>(a.pol + 3 * (size_t)sn, px, py, pz);
@@ -289,11 +357,13 @@ __global__ void __maxnreg__(96) msp_snap_rho_kernel(SnapArgs a) {
         }
         __syncthreads();
         // FP32 terms, double-word level gaps and sums
-        const float hs = hot ? (float)rho_hot_scale(a, sn) : 0.f;
+        const float hs = hot ? *hot_scale : 0.f;
         const float2 local =
-            n == 24   ? rho_terms_mixed<INTEGRAL, 24>(a, s, U, OU, Y, n, sn, tau_f, itau_f, hot, hs)
-            : n == 32 ? rho_terms_mixed<INTEGRAL, 32>(a, s, U, OU, Y, n, sn, tau_f, itau_f, hot, hs)
-                      : rho_terms_mixed<INTEGRAL, 0>(a, s, U, OU, Y, n, sn, tau_f, itau_f, hot, hs);
+            PRE && n == 24
+                ? rho_terms_mixed<INTEGRAL, PRE, PRE ? 24 : 0>(a, s, U, OU, X, n, sn, tau_f, itau_f, hot, hs)
+            : PRE && n == 32
+                ? rho_terms_mixed<INTEGRAL, PRE, PRE ? 32 : 0>(a, s, U, OU, X, n, sn, tau_f, itau_f, hot, hs)
+                : rho_terms_mixed<INTEGRAL, PRE, 0>(a, s, U, OU, X, n, sn, tau_f, itau_f, hot, hs);
         const double sum = dw_block_sum(local, reinterpret_cast<float2 *>(s.w.red));
         if (tid == 0) {
             a.snap_const[sn] = INTEGRAL ? a.wscale[sn] * sum / a.tau : a.wscale[sn] * sum;
@@ -305,18 +375,22 @@ __global__ void __maxnreg__(96) msp_snap_rho_kernel(SnapArgs a) {
 
 // ------------------------------------------------------------------ launchers
 
-int snap_default_threads(int n) { return jacobi_threads(n + (n & 1)); }
+int snap_default_threads(int n, int precision) {
+    if (precision == MSP_PREC_MIXED && jacobi_warp_supported(n)) return row_threads(n);
+    return jacobi_threads(n + (n & 1));
+}
 
-// Shared memory of a snapshot kernel launched with `threads` threads (the
-// reduction scratch grows with the warp count).
-static size_t snap_smem_threads(int n, int mode, int precision, int fac_len, int threads) {
-    if (precision != MSP_PREC_MIXED)
-        return snap64_smem_bytes(n, mode != MSP_MODE_FAST ? fac_len : 0, threads);
-    return snap_layout(n, 4, true, mode != MSP_MODE_FAST, fac_len, threads / 32).total;
+// Shared memory of a snapshot kernel launched with `threads` threads.  rows: the
+// second stage of the two-stage MIXED form.
+static size_t snap_smem_threads(int n, int mode, int precision, int fac_len, int threads, bool rows) {
+    const bool rho = mode != MSP_MODE_FAST;
+    if (precision != MSP_PREC_MIXED) return snap64_smem_bytes(n, rho ? fac_len : 0, threads);
+    if (rows) return row_layout(n, rho, fac_len, threads).total;
+    return snap_layout(n, 4, true, rho, fac_len, threads / 32).total;
 }
 
 size_t snap_smem_bytes(int n, int mode, int precision, int fac_len) {
-    return snap_smem_threads(n, mode, precision, fac_len, snap_default_threads(n));
+    return snap_smem_threads(n, mode, precision, fac_len, jacobi_threads(n + (n & 1)), false);
 }
 
 template <typename K>
@@ -342,11 +416,20 @@ static int occupancy_of(K kernel, int threads, size_t smem) {
     return blocks > 0 ? blocks : 1;
 }
 
+// Threads of a snapshot kernel asked for `threads` (0: the default): the second
+// stage of the two-stage MIXED form takes at least what its eight rows per
+// thread need.
+static int stage2_threads(int n, int precision, int threads, bool rows) {
+    const int least = rows && precision == MSP_PREC_MIXED ? row_threads(n) : 0;
+    if (threads <= 0) threads = rows ? snap_default_threads(n, precision) : jacobi_threads(n + (n & 1));
+    return threads < least ? least : threads;
+}
+
 int snap_occupancy(int n, int mode, int precision, int threads) {
-    if (threads <= 0) threads = snap_default_threads(n);
-    const size_t smem = snap_smem_threads(n, mode, precision, 0, threads);
-    if (mode != MSP_MODE_FAST) return 1;
     const bool pre = jacobi_warp_supported(n);
+    threads = stage2_threads(n, precision, threads, pre);
+    const size_t smem = snap_smem_threads(n, mode, precision, 0, threads, pre);
+    if (mode != MSP_MODE_FAST) return 1;
     if (precision != MSP_PREC_MIXED) return snap64_occupancy(n, threads, pre);
     return pre ? occupancy_of(msp_snap_fast_kernel<true>, threads, smem)
                : occupancy_of(msp_snap_fast_kernel<false>, threads, smem);
@@ -362,10 +445,10 @@ size_t snap_evec_bytes(int n, long long num_snap) {
 cudaError_t launch_snapshots_refine(const SnapArgs &a, int mode, int precision, cudaStream_t st,
                                     int threads, int grid) {
     if (a.num_snap <= 0) return cudaSuccess;
-    if (threads <= 0) threads = snap_default_threads(a.n);
+    threads = stage2_threads(a.n, precision, threads, true);
     if (grid <= 0 || grid > a.num_snap) grid = a.num_snap;
     if (precision != MSP_PREC_MIXED) return launch_snapshots64(a, mode, true, st, threads, grid);
-    const size_t smem = snap_smem_threads(a.n, mode, precision, a.fac_len, threads);
+    const size_t smem = snap_smem_threads(a.n, mode, precision, a.fac_len, threads, true);
     if (mode == MSP_MODE_FAST)
         return launch_snap(msp_snap_fast_kernel<true>, a, grid, threads, smem, st);
     if (mode == MSP_MODE_EVOLVE)
@@ -378,7 +461,6 @@ cudaError_t launch_snapshots_refine(const SnapArgs &a, int mode, int precision, 
 cudaError_t launch_snapshots(const SnapArgs &a, int mode, int precision, cudaStream_t st,
                              int threads, int grid) {
     if (a.num_snap <= 0) return cudaSuccess;
-    if (threads <= 0) threads = snap_default_threads(a.n);
     if (grid <= 0 || grid > a.num_snap) grid = a.num_snap;
     if (a.evec != nullptr && jacobi_warp_supported(a.n)) {
         // two stages: FP32 eigenvectors, then refinement and eigenbasis products
@@ -386,8 +468,9 @@ cudaError_t launch_snapshots(const SnapArgs &a, int mode, int precision, cudaStr
         if (e != cudaSuccess) return e;
         return launch_snapshots_refine(a, mode, precision, st, threads, grid);
     }
+    threads = stage2_threads(a.n, precision, threads, false);
     if (precision != MSP_PREC_MIXED) return launch_snapshots64(a, mode, false, st, threads, grid);
-    const size_t smem = snap_smem_threads(a.n, mode, precision, a.fac_len, threads);
+    const size_t smem = snap_smem_threads(a.n, mode, precision, a.fac_len, threads, false);
     if (mode == MSP_MODE_FAST)
         return launch_snap(msp_snap_fast_kernel<false>, a, grid, threads, smem, st);
     if (mode == MSP_MODE_EVOLVE)
@@ -421,7 +504,7 @@ cudaError_t launch_eigh(const double *H, int n, int batch, int precision, int ma
                         double *evals, double *evecs, int *status, cudaStream_t st) {
     if (precision != MSP_PREC_MIXED)
         return launch_eigh64(H, n, batch, max_sweeps, evals, evecs, status, st);
-    const int threads = snap_default_threads(n);
+    const int threads = jacobi_threads(n + (n & 1));
     const size_t smem = snap_smem_bytes(n, MSP_MODE_FAST, precision, 0);
     const cudaError_t e = cudaFuncSetAttribute(
         msp_eigh_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
