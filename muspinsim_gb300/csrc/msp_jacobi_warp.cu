@@ -410,18 +410,21 @@ bool jacobi_warp_supported(int n) {
     return m >= 4 && m <= 32;
 }
 
-// First stage of the two-stage MIXED snapshots.  Batches of 4,096 snapshots
-// or more take the Householder + QL form (msp_ql_warp.cu: at 10,000
-// snapshots of dimension 24 it takes 0.55 ms against the Jacobi's 0.86 ms,
-// and 20% less at dimension 32); smaller batches fill the GPU with too few
-// of its four-matrix warp tasks and keep the Jacobi (at 4,000 snapshots the
-// two tie).  MSP_EIGH_WARP = 0 or 2 pins one form.
+// First stage of the two-stage snapshots.  Large batches take the Householder +
+// QL form (msp_ql_warp.cu), whose time is flat until its CTAs, of 16 or 32
+// matrices, fill the SMs; smaller ones would leave most of them idle and keep the
+// Jacobi, a warp or less per matrix.  Measured, Jacobi against QL in us: n = 32,
+// 500 snapshots 185 / 211, 1,000 254 / 216; n = 24, 1,000 149 / 159, 1,500 172 /
+// 161; n = 16, 2,000 75 / 79, 3,000 88 / 79; n = 8, 3,000 30 / 30, 10,000 83 / 54;
+// n = 6, 4,000 23 / 23, 10,000 49 / 44; n = 4, 10,000 25 / 27.  MSP_EIGH_WARP =
+// 0 or 2 pins one form.
 #ifndef MSP_EIGH_WARP
 #define MSP_EIGH_WARP 1
 #endif
 cudaError_t launch_jacobi_warp(const SnapArgs &a, cudaStream_t st) {
     if (MSP_EIGH_WARP == 2 && ql_warp_supported(a.n)) return launch_ql_warp(a, st);
-    if (MSP_EIGH_WARP == 1 && ql_warp_supported(a.n) && a.num_snap >= 4096)
+    if (MSP_EIGH_WARP == 1 && ql_warp_supported(a.n) && a.n > 4 &&
+        (a.num_snap >= 4096 || (long long)a.num_snap * a.n >= 32768))
         return launch_ql_warp(a, st);
     if (a.num_snap <= 0) return cudaSuccess;
     switch (a.n + (a.n & 1)) {

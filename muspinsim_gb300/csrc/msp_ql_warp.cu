@@ -1,533 +1,479 @@
 // FP32 Householder + implicit-shift QL eigensolver for batches of n <= 32
-// Hamiltonians: the first stage of the MIXED snapshot pipeline (the
-// alternative to msp_jacobi_warp.cu's cyclic Jacobi), replacing the FP32
-// part of Hermitian.diag's eigensolve (muspinsim/spinop.py:51-82) for the
+// Hamiltonians: the first stage of the two-stage snapshot pipeline for large
+// batches (the alternative to msp_jacobi_warp.cu's cyclic Jacobi), replacing the
+// FP32 part of Hermitian.diag's eigensolve (muspinsim/spinop.py:51-82) for the
 // batched snapshots of ExperimentRunner (muspinsim/experiment.py:332-341,
-// 434-498).  The second stage (msp_snap.cu, PRE variants) refines the
-// eigenvectors this kernel leaves in scratch, exactly as it refines the
-// Jacobi's.
+// 434-498).  The second stage (msp_snap.cu, msp_snap64.cu) refines the
+// eigenvectors this one leaves in scratch, exactly as it refines the Jacobi's;
+// they only have to be orthonormal to FP32 rounding.
 //
-// The algorithm is msp_large.cuh's (LAPACK zhetd2 tridiagonalisation of the
-// lower triangle, EISPACK tql2 QL with the rotations accumulated into a real
-// Z, back-transformation U = Q Z).  A warp takes G matrices at a time:
-//   1. two matrices at a time, one warp, their steps interleaved
-//      instruction by instruction (each step is a chain of warp reductions
-//      and shared-memory round trips; two independent chains fill each
-//      other's latency: 0.54 -> 0.52 ms on the headline): A (full
-//      Hermitian, row-major, row stride NM + 1 float2 so that column and
-//      row walks are both free of bank conflicts) in shared memory, both
-//      matrices side by side in the region the Z matrices later take.
-//      Step k: lane i holds x_i = A[k+1+i][k]; the reflector v_k (v_0 = 1)
-//      replaces column k of A, zero outside rows k+1 .. n-1, and is parked
-//      as row k of the snapshot's eigenvector scratch; p = tau A22 v and the
-//      rank-2 update A22 -= v w^H + w v^H are column-parallel (lane i owns
-//      column k+1+i; v_j, w_j are warp broadcasts).  d, e and tau stay in
-//      shared memory.
-//   2. the G QL runs side by side, 32 / G lanes per matrix: a QL step's
-//      shift and rotation chain are serial, so each lane group computes its
-//      own matrix's chain (its lanes redundantly) and applies every rotation
-//      to its rows of Z (column-major in shared memory, aliasing A).  The
-//      groups advance one QL step per round; a round waits for the longest
-//      chain, which on the 24 x 24 powder Hamiltonians (513 .. 613 rotations
-//      in 45 .. 49 steps) costs under 10% over the groups' own work.  The
-//      reciprocal square root of each rotation is the hardware
-//      approximation plus one Newton step.
-//   3. per matrix, one warp: lane j holds column j of U = Q Z in registers
-//      and applies the parked reflectors last to first, s = v^H u,
-//      u -= v (tau s), skipping the four-row groups where v is zero; U
-//      overwrites the reflectors in the scratch.
-// The FP32 eigenvectors only have to be orthonormal to FP32 rounding; the
-// refinement stage restores full accuracy and resolves clusters.
+// Two kernels, so that each has the registers and shared memory it wants (as
+// one kernel per four matrices and warp, ten warps fitted an SM and every stage
+// waited for its own latency: 20.2 ms for 201,000 matrices of n = 32, 0.52 ms for
+// 10,000 of n = 24; now 10.7 and 0.40 ms):
+//   1. msp_tri_warp_kernel, tridiagonalisation (LAPACK zhetd2), a warp per
+//      matrix, the matrix in registers (a lane holds a row);
+//   2. msp_ql_kernel, QL with the rotations accumulated into Z and the
+//      back-transformation U = Q Z, a CTA per QlShape::GM matrices: one warp runs
+//      the serial recurrences of all of them, a lane per matrix, one QL step
+//      ahead of eight warps that apply the rotations to Z in shared memory.
+// Between them the reflectors and the tridiagonal matrix lie in the snapshot's
+// eigenvector scratch, which U overwrites: row k holds reflector v_k in columns
+// k + 1 .. n - 1, (d_k, e_k) in column 0 and tau_k in column 1 (tau_0 in row
+// n - 1, column 1).
 #include "msp_internal.cuh"
-#include "msp_large.cuh"
 
 namespace msp {
 
 namespace {
 
-constexpr int QW_WARPS = 2;  // warps per CTA
+constexpr unsigned FULL = 0xffffffffu;
 
-// Per-warp shared memory for a batch of G matrices up to NM x NM (NM a
-// multiple of 8): region R holds the two working matrices A (NM x (NM + 1)
-// float2 each) while matrices are tridiagonalised and the G matrices Z_g
-// (NM x (NM + 1) floats each) from the QL on; then per matrix d, e (NM
-// floats each) and tau (NM float2); then the two v/w pair buffers (NM
-// float4 each).
-template <int NM, int G>
-struct QwShape {
-    static constexpr int LDA = NM + 1;  // float2
-    static constexpr int LDZ = NM + 1;  // float
-    static constexpr int A_BYTES = 8 * NM * LDA;
-    static constexpr int Z_FLOATS = NM * LDZ;  // one matrix
-    static constexpr int A_F2 = NM * LDA;  // float2 of one working matrix
-    static constexpr int R_BYTES =
-        (2 * A_BYTES > 4 * G * Z_FLOATS ? 2 * A_BYTES : 4 * G * Z_FLOATS + 15) / 16 * 16;
-    static constexpr int DEV_BYTES = 16 * NM;  // d, e, tau of one matrix
-    static constexpr int BYTES = R_BYTES + G * DEV_BYTES + 32 * NM;
-    static constexpr int LPM = 32 / G;              // lanes per matrix in the QL
-    static constexpr int RPL = (NM + LPM - 1) / LPM;  // rows of Z per lane
-    // CTAs per SM that the shared memory allows (1 KB reserved per CTA),
-    // capped where registers would fall below ~96 a thread
-    static constexpr int CTAS = (227 * 1024) / (QW_WARPS * BYTES + 1024);
-    static constexpr int REG_CTAS = 65536 / (QW_WARPS * 32 * 96);
-    static constexpr int MINB = CTAS < 1 ? 1 : (CTAS > REG_CTAS ? REG_CTAS : CTAS);
-    static_assert(NM % 8 == 0 && NM <= 32, "NM: a multiple of 8 up to 32");
-    static_assert(G == 1 || G == 2 || G == 4 || G == 8, "G divides 32");
-    static_assert(A_BYTES % 16 == 0 && BYTES % 16 == 0, "alignment");
+// ------------------------------------------------------------------ 1. tridiagonalisation
+
+constexpr int TRI_WARPS = 4;
+
+// Lanes per matrix: small ones share a warp.
+template <int NM>
+struct TriShape {
+    static constexpr int LN = NM <= 8 ? 8 : NM <= 16 ? 16 : 32;
+    static constexpr int PER_CTA = TRI_WARPS * 32 / LN;
 };
 
-}  // namespace
+__device__ __forceinline__ float fast_rsqrt(float x) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y * fmaf(-0.5f * x * y, y, 1.5f);
+}
 
-template <int NM, int G>
-__global__ void __launch_bounds__(QW_WARPS * 32, QwShape<NM, G>::MINB)
-    msp_ql_warp_kernel(SnapArgs a) {
-    using S = QwShape<NM, G>;
-    constexpr int LDA = S::LDA, LDZ = S::LDZ, LPM = S::LPM, RPL = S::RPL;
-    extern __shared__ __align__(16) char smem[];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    char *mine = smem + (size_t)warp * S::BYTES;
-    float2 *const A = reinterpret_cast<float2 *>(mine);  // phase 1
-    float *const Zb = reinterpret_cast<float *>(mine);   // phases 2, 3
-    char *const devb = mine + S::R_BYTES;
-    float4 *const vw = reinterpret_cast<float4 *>(devb + G * S::DEV_BYTES);
-    auto dptr = [&](int q) { return reinterpret_cast<float *>(devb + q * S::DEV_BYTES); };
+template <int LN>
+__device__ __forceinline__ float lanes_sum(float v) {
+#pragma unroll
+    for (int o = LN / 2; o > 0; o >>= 1) v += __shfl_xor_sync(FULL, v, o, LN);
+    return v;
+}
 
-    const int n = a.n;
-    const int nn = n * n;
-    float2 *evec = reinterpret_cast<float2 *>(a.evec);
-    const int ntask = (a.num_snap + G - 1) / G;
-    for (int task = blockIdx.x * QW_WARPS + warp; task < ntask; task += gridDim.x * QW_WARPS) {
-        const int sn0 = task * G;
-        const int cnt = min(G, a.num_snap - sn0);
-
-        // ---- 1. two matrices at a time (their steps interleaved instruction
-        // by instruction): H, tridiagonalisation.  A missing second matrix
-        // (odd count) is zero: no reflections, nothing stored for it.
-        for (int q0 = 0; q0 < cnt; q0 += 2) {
-            const bool has1 = q0 + 1 < cnt;
-            float2 *Ap[2] = {A, A + S::A_F2};
-            float4 *vwp[2] = {vw, vw + NM};
-            float *dsp[2], *esp[2];
-            float2 *tp[2], *Vtp[2];
-            SnapSource src[2];
-            double bx[2], by[2], bz[2];
+// Lane i holds row i.  Step k finds the column it eliminates in register 0: the
+// rank-2 update moves every entry one register down, so that no index depends on
+// k.  v and w reach the other lanes through shared memory, (v_j, w_j) by row
+// relative to k + 1, zero beyond the last.  p^H v = conj(tau) v^H A v with a real
+// v^H A v, so one real sum over the lanes does.  Bound by issue: 14 instructions
+// per trailing entry and row, some 110 per column.  201,000 matrices of n = 32:
+// 3.5 ms, 61% of the issue slots.
+template <int NM>
+__global__ void __launch_bounds__(TRI_WARPS * 32) msp_tri_warp_kernel(SnapArgs a) {
+    constexpr int LN = TriShape<NM>::LN, PER = 32 / LN;
+    __shared__ __align__(16) float4 sh_all[TRI_WARPS * PER][LN + 4];
+    const int n = a.n, lane = threadIdx.x & (LN - 1), grp = threadIdx.x / LN;
+    const int sn = blockIdx.x * TriShape<NM>::PER_CTA + grp;
+    const bool live = sn < a.num_snap;
+    float4 *sh = sh_all[grp];  // (v_j, w_j)
+    const int at = live ? sn : a.num_snap - 1;
+    const SnapSource src = snap_source(a, at);
+    float2 *out = reinterpret_cast<float2 *>(a.evec) + (size_t)at * n * n;
+    cx<float> r[NM];
+    {
+        const double *b = a.field + 3 * (size_t)src.g;
+        const size_t nn = (size_t)n * n;
+        const bool on = lane < n;
+        if (src.Hdw != nullptr) {
+            const float bx = (float)b[0], by = (float)b[1], bz = (float)b[2];
 #pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                const int q = q0 + u;
-                dsp[u] = dptr(q);
-                esp[u] = dsp[u] + NM;
-                tp[u] = reinterpret_cast<float2 *>(esp[u] + NM);
-                const int sn = (u == 0 || has1) ? sn0 + q : sn0 + q0;
-                Vtp[u] = evec + (size_t)sn * nn;
-                src[u] = snap_source(a, sn);
-                bx[u] = a.field[3 * (size_t)src[u].g];
-                by[u] = a.field[3 * (size_t)src[u].g + 1];
-                bz[u] = a.field[3 * (size_t)src[u].g + 2];
+            for (int j = 0; j < NM; ++j) {
+                r[j] = mk<float>(0.f, 0.f);
+                if (j >= n || !on) continue;
+                const size_t o = (size_t)j * n + lane;
+                auto hi = [](const float4 *p) { return *reinterpret_cast<const float2 *>(p); };
+                const float2 h = hi(src.Hdw + o), z0 = hi(src.Zdw + o), z1 = hi(src.Zdw + nn + o),
+                             z2 = hi(src.Zdw + 2 * nn + o);
+                // A[lane][j] = conj(A[j][lane])
+                r[j] = mk<float>(fmaf(bz, z2.x, fmaf(by, z1.x, fmaf(bx, z0.x, h.x))),
+                                 -fmaf(bz, z2.y, fmaf(by, z1.y, fmaf(bx, z0.y, h.y))));
             }
-            // H = Hsys + b . Z in FP32 (from the double-word high parts when
-            // the caller pre-split the matrices, else from FP64), upper
-            // triangle mirrored; rows and columns n .. NM-1 zero
-            for (int e = lane; e < NM * (NM + 1) / 2; e += 32) {
-                int i = (int)((sqrtf(8.0f * (float)e + 1.0f) - 1.0f) * 0.5f);  // e = i (i + 1) / 2 + j
-                while ((i + 1) * (i + 2) / 2 <= e) ++i;
-                while (i * (i + 1) / 2 > e) --i;
-                const int j = e - i * (i + 1) / 2;  // j <= i: element (j, i)
+        } else {
 #pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                    float hr = 0.f, hi = 0.f;
-                    if (i < n && (u == 0 || has1)) {
-                        const size_t o = (size_t)j * n + i;
-                        if (src[u].Hdw != nullptr) {
-                            const float bxf = (float)bx[u], byf = (float)by[u], bzf = (float)bz[u];
-                            const float4 hs = src[u].Hdw[o], z0 = src[u].Zdw[o],
-                                         z1 = src[u].Zdw[nn + o], z2 = src[u].Zdw[2 * (size_t)nn + o];
-                            hr = fmaf(bzf, z2.x, fmaf(byf, z1.x, fmaf(bxf, z0.x, hs.x)));
-                            hi = fmaf(bzf, z2.y, fmaf(byf, z1.y, fmaf(bxf, z0.y, hs.y)));
-                        } else {
-                            const cx<double> hs = src[u].Hsys[o], z0 = src[u].Z[o],
-                                             z1 = src[u].Z[nn + o], z2 = src[u].Z[2 * (size_t)nn + o];
-                            hr = (float)(hs.re + bx[u] * z0.re + by[u] * z1.re + bz[u] * z2.re);
-                            hi = (float)(hs.im + bx[u] * z0.im + by[u] * z1.im + bz[u] * z2.im);
-                        }
-                    }
-                    if (i == j) {
-                        Ap[u][i * LDA + i] = make_float2(hr, 0.f);
-                    } else {
-                        Ap[u][j * LDA + i] = make_float2(hr, hi);
-                        Ap[u][i * LDA + j] = make_float2(hr, -hi);
-                    }
-                }
+            for (int j = 0; j < NM; ++j) {
+                r[j] = mk<float>(0.f, 0.f);
+                if (j >= n || !on) continue;
+                const size_t o = (size_t)j * n + lane;
+                const cx<double> h = src.Hsys[o], z0 = src.Z[o], z1 = src.Z[nn + o], z2 = src.Z[2 * nn + o];
+                r[j] = mk<float>((float)(h.re + b[0] * z0.re + b[1] * z1.re + b[2] * z2.re),
+                                 -(float)(h.im + b[0] * z0.im + b[1] * z1.im + b[2] * z2.im));
             }
-            __syncwarp();
-
-            // d, e, tau; reflector k into column k of A and row k of the
-            // eigenvector scratch.  A step without a reflection (tau = 0)
-            // runs the updates too: they add exact zeros.
-            for (int k = 0; k + 1 < n; ++k) {
-                const int m = n - k - 1;  // length of x
-                float2 xi[2];
-                float dk[2], xn2[2];
-#pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                    xi[u] = lane < m ? Ap[u][(k + 1 + lane) * LDA + k] : make_float2(0.f, 0.f);
-                    dk[u] = Ap[u][k * LDA + k].x;
-                    xn2[u] = lane >= 1 ? xi[u].x * xi[u].x + xi[u].y * xi[u].y : 0.f;
-                }
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-                    for (int u = 0; u < 2; ++u) xn2[u] += __shfl_xor_sync(0xffffffffu, xn2[u], o);
-                }
-                float beta[2];
-                cx<float> tau[2], vi[2];
-#pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                    const float2 alpha = make_float2(__shfl_sync(0xffffffffu, xi[u].x, 0),
-                                                     __shfl_sync(0xffffffffu, xi[u].y, 0));
-                    const bool reflect = !(xn2[u] == 0.f && alpha.y == 0.f);
-                    const float br =
-                        -copysignf(sqrtf(alpha.x * alpha.x + alpha.y * alpha.y + xn2[u]), alpha.x);
-                    const cx<float> tr = mk<float>((br - alpha.x) / br, -alpha.y / br);
-                    // v = x / (alpha - beta), v_0 = 1
-                    const float dr = alpha.x - br, di = alpha.y;
-                    const float dd = 1.f / (dr * dr + di * di);
-                    const cx<float> vr = cmul(mk<float>(xi[u].x, xi[u].y), mk<float>(dr * dd, -di * dd));
-                    beta[u] = reflect ? br : alpha.x;
-                    tau[u] = reflect ? tr : mk<float>(0.f, 0.f);
-                    vi[u] = lane == 0 ? mk<float>(1.f, 0.f)
-                                      : (reflect ? vr : mk<float>(0.f, 0.f));
-                }
-                __syncwarp();  // column k (x, A[k][k]) read by every lane
-#pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                    // column k <- v, zero outside rows k+1 .. n-1
-                    const int src_lane = (lane - k - 1) & 31;
-                    const float vr = __shfl_sync(0xffffffffu, vi[u].re, src_lane);
-                    const float vim = __shfl_sync(0xffffffffu, vi[u].im, src_lane);
-                    const float2 vv =
-                        (lane > k && lane < n) ? make_float2(vr, vim) : make_float2(0.f, 0.f);
-                    if (lane < NM) Ap[u][lane * LDA + k] = vv;
-                    if (lane < n && (u == 0 || has1)) Vtp[u][(size_t)k * n + lane] = vv;
-                    if (lane == 0) {
-                        dsp[u][k] = dk[u];
-                        esp[u][k] = beta[u];
-                        tp[u][k] = make_float2(tau[u].re, tau[u].im);
-                    }
-                }
-                __syncwarp();
-                // p_i = tau sum_j conj(A22[j][i]) v_j (A22 Hermitian), lane i
-                // owns column k+1+i
-                cx<float> pi[2] = {mk<float>(0.f, 0.f), mk<float>(0.f, 0.f)};
-                if (lane < m) {
-                    float r0[2] = {0.f, 0.f}, i0[2] = {0.f, 0.f}, r1[2] = {0.f, 0.f},
-                          i1[2] = {0.f, 0.f};
-                    int j = 0;
-                    for (; j + 1 < m; j += 2) {
-#pragma unroll
-                        for (int u = 0; u < 2; ++u) {
-                            const float2 *col = Ap[u] + (k + 1) * LDA + (k + 1 + lane);
-                            const float2 *vk = Ap[u] + (k + 1) * LDA + k;
-                            const float2 a0 = col[j * LDA], a1 = col[(j + 1) * LDA];
-                            const float2 v0 = vk[j * LDA], v1 = vk[(j + 1) * LDA];
-                            r0[u] += a0.x * v0.x + a0.y * v0.y;
-                            i0[u] += a0.x * v0.y - a0.y * v0.x;
-                            r1[u] += a1.x * v1.x + a1.y * v1.y;
-                            i1[u] += a1.x * v1.y - a1.y * v1.x;
-                        }
-                    }
-                    if (j < m) {
-#pragma unroll
-                        for (int u = 0; u < 2; ++u) {
-                            const float2 a0 = Ap[u][(k + 1 + j) * LDA + (k + 1 + lane)];
-                            const float2 v0 = Ap[u][(k + 1 + j) * LDA + k];
-                            r0[u] += a0.x * v0.x + a0.y * v0.y;
-                            i0[u] += a0.x * v0.y - a0.y * v0.x;
-                        }
-                    }
-#pragma unroll
-                    for (int u = 0; u < 2; ++u)
-                        pi[u] = cmul(tau[u], mk<float>(r0[u] + r1[u], i0[u] + i1[u]));
-                }
-                // alpha2 = -1/2 tau (p^H v); w = p + alpha2 v
-                float hr[2], hi[2];
-#pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                    const cx<float> pv = lane < m ? cmulc(pi[u], vi[u]) : mk<float>(0.f, 0.f);
-                    hr[u] = pv.re;
-                    hi[u] = pv.im;
-                }
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-                    for (int u = 0; u < 2; ++u) {
-                        hr[u] += __shfl_xor_sync(0xffffffffu, hr[u], o);
-                        hi[u] += __shfl_xor_sync(0xffffffffu, hi[u], o);
-                    }
-                }
-                cx<float> wi[2];
-#pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                    const cx<float> a2 = cscale(-0.5f, cmul(tau[u], mk<float>(hr[u], hi[u])));
-                    wi[u] = cadd(pi[u], cmul(a2, vi[u]));
-                    if (lane < m) vwp[u][lane] = make_float4(vi[u].re, vi[u].im, wi[u].re, wi[u].im);
-                }
-                __syncwarp();
-                // A22[j][i] -= v_j conj(w_i) + w_j conj(v_i), lane i owns column i
-                if (lane < m) {
-                    for (int j = 0; j < m; ++j) {
-#pragma unroll
-                        for (int u = 0; u < 2; ++u) {
-                            float2 *cp = Ap[u] + (k + 1 + j) * LDA + (k + 1 + lane);
-                            const float4 qv = vwp[u][j];
-                            const float2 x = *cp;
-                            const float tr = qv.x * wi[u].re + qv.y * wi[u].im + qv.z * vi[u].re +
-                                             qv.w * vi[u].im;
-                            const float ti = qv.y * wi[u].re - qv.x * wi[u].im + qv.w * vi[u].re -
-                                             qv.z * vi[u].im;
-                            *cp = make_float2(x.x - tr, x.y - ti);
-                        }
-                    }
-                }
-                __syncwarp();
-            }
-            if (lane == 0) {
-#pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                    dsp[u][n - 1] = Ap[u][(n - 1) * LDA + (n - 1)].x;
-                    esp[u][n - 1] = 0.f;
-                }
-            }
-            __syncwarp();  // A is reused by the next pair, then by Z
         }
-
-        // ---- 2. QL with implicit shifts (tql2) on the G matrices side by
-        // side: lane group g (LPM lanes) runs matrix g; Z_g = I
-        for (int e = lane; e < G * S::Z_FLOATS; e += 32) Zb[e] = 0.f;
-        __syncwarp();
-        for (int e = lane; e < G * NM; e += 32) {
-            const int q = e / NM, i = e - q * NM;
-            if (i < n) Zb[q * S::Z_FLOATS + i * LDZ + i] = 1.f;
+    }
+    float2 tau0 = make_float2(0.f, 0.f);
+    for (int k = 0; k + 1 < n; ++k) {
+        const int m = n - k - 1;
+        const bool below = lane > k && lane < n;
+        const cx<float> x = below ? r[0] : mk<float>(0.f, 0.f);
+        const float dk = __shfl_sync(FULL, r[0].re, k, LN);
+        const float xn2 = lanes_sum<LN>(lane > k + 1 ? cabs2(x) : 0.f);
+        const cx<float> alpha =
+            mk<float>(__shfl_sync(FULL, x.re, k + 1, LN), __shfl_sync(FULL, x.im, k + 1, LN));
+        const float s2 = fmaf(alpha.re, alpha.re, fmaf(alpha.im, alpha.im, xn2));
+        float beta = alpha.re;
+        cx<float> tau = mk<float>(0.f, 0.f), sc = tau;
+        if (xn2 != 0.f || alpha.im != 0.f) {
+            float root, inv;  // |beta| and its reciprocal
+            if (s2 > 1e-36f && s2 < 1e36f) {
+                inv = fast_rsqrt(s2);
+                root = s2 * inv;
+            } else {
+                root = sqrtf(s2);
+                inv = 1.f / root;
+            }
+            beta = -copysignf(root, alpha.re);
+            inv = -copysignf(inv, alpha.re);
+            tau = mk<float>(1.f - alpha.re * inv, -alpha.im * inv);
+            const cx<float> den = mk<float>(alpha.re - beta, alpha.im);
+            const float dd = 1.f / cabs2(den);
+            sc = mk<float>(den.re * dd, -den.im * dd);
         }
-        __syncwarp();
-        const int g = lane / LPM, sub = lane - g * LPM;
-        const unsigned gmask = LPM == 32 ? 0xffffffffu : (((1u << (LPM & 31)) - 1u) << (g * LPM));
-        int status = MSP_ITEM_OK;
+        const cx<float> v = lane == k + 1 ? mk<float>(1.f, 0.f) : cmul(x, sc);
         {
-            float *const ds = dptr(g);
-            float *const es = ds + NM;
-            float *const Zg = Zb + g * S::Z_FLOATS;
-            const float eps = 1.1920928955078125e-7f;  // 2^-23
-            bool done = g >= cnt;
-            int l = 0, iter = 0;
-            float f = 0.f, tst = 0.f;
-            for (;;) {
-                // deflate converged levels; m: the first index >= l whose
-                // coupling is negligible (n - 1 at the latest)
-                int m = l;
-                if (!done) {
-                    for (;;) {
-                        if (iter == 0) tst = fmaxf(tst, fabsf(ds[l]) + fabsf(es[l]));
-                        m = l;
-                        while (m < n - 1 && fabsf(es[m]) > eps * tst) ++m;
-                        if (m != l && iter < 60) break;
-                        if (m != l) status = MSP_ITEM_NOT_CONVERGED;
-                        __syncwarp(gmask);
-                        if (sub == 0) {
-                            ds[l] += f;
-                            es[l] = 0.f;
-                        }
-                        __syncwarp(gmask);
-                        iter = 0;
-                        if (++l >= n) {
-                            done = true;
-                            break;
-                        }
-                    }
-                }
-                if (__all_sync(0xffffffffu, done)) break;
-                if (!done) {
-                    ++iter;
-                    const float g0 = ds[l], el = es[l], el1 = es[l + 1];
-                    const float qs = (ds[l + 1] - g0) / (2.f * el);
-                    const float r0 = hypotf(qs, 1.f);
-                    const float t1 = qs + copysignf(r0, qs);
-                    const float dl = el / t1, dl1 = el * t1;
-                    const float h = g0 - dl;
-                    f += h;
-                    __syncwarp(gmask);  // every lane of the group has read d and e
-                    if (sub == 0) {
-                        ds[l] = dl;
-                        ds[l + 1] = dl1;
-                    }
-                    for (int i = l + 2 + sub; i < n; i += LPM) ds[i] -= h;
-                    __syncwarp(gmask);
-                    float pp = ds[m];
-                    float c = 1.f, c2 = 1.f, c3 = 1.f, s = 0.f, s2 = 0.f;
-                    // this lane's rows of Z: r = sub + LPM t
-                    float hc[RPL], zi[RPL];
+            float2 o = make_float2(v.re, v.im);
+            if (lane == 0) o = make_float2(dk, beta);
+            if (lane == 1 && k > 0) o = make_float2(tau.re, tau.im);
+            if (k == 0) tau0 = make_float2(tau.re, tau.im);
+            if (live && lane < n && (lane > k || lane < 2)) out[(size_t)k * n + lane] = o;
+        }
+        // relative row of this lane; retired ones and padding fill the end with zeros
+        const int rel = below ? lane - k - 1 : (lane <= k ? m + lane : lane);
+        sh[rel] = make_float4(v.re, v.im, 0.f, 0.f);
+        __syncwarp();
+        // p = A v
+        float p0 = 0.f, p1 = 0.f, p2 = 0.f, p3 = 0.f;
 #pragma unroll
-                    for (int t = 0; t < RPL; ++t) {
-                        const int r = sub + LPM * t;
-                        hc[t] = r < n ? Zg[m * LDZ + r] : 0.f;
-                        zi[t] = r < n ? Zg[(m - 1) * LDZ + r] : 0.f;
-                    }
-                    float ei = es[m - 1], di = ds[m - 1];
-                    for (int i = m - 1; i >= l; --i) {
-                        // operands of the next rotation: written by this chain
-                        // only after they are read
-                        const int ip = max(i - 1, l);
-                        const float ein = es[ip], din = ds[ip];
-                        float zin[RPL];
+        for (int g = 0; g < NM / 4; ++g) {
+            if (4 * g >= m) continue;
 #pragma unroll
-                        for (int t = 0; t < RPL; ++t) {
-                            const int r = sub + LPM * t;
-                            zin[t] = r < n ? Zg[ip * LDZ + r] : 0.f;
-                        }
-                        c3 = c2;
-                        c2 = c;
-                        s2 = s;
-                        const float gq = c * ei, hh = c * pp;
-                        const float x2 = fmaf(pp, pp, ei * ei);
-                        float r, cn, sn;
-                        if (x2 > 1e-36f && x2 < 1e36f) {
-                            const float y = rsqrt_newton<float>(x2);
-                            r = x2 * y;
-                            sn = ei * y;
-                            cn = pp * y;
-                        } else {
-                            r = hypotf(pp, ei);
-                            sn = ei / r;
-                            cn = pp / r;
-                        }
-                        es[i + 1] = s * r;
-                        s = sn;
-                        c = cn;
-                        pp = c * di - s * gq;
-                        ds[i + 1] = hh + s * (c * gq + s * di);
-#pragma unroll
-                        for (int t = 0; t < RPL; ++t) {
-                            const int rr = sub + LPM * t;
-                            if (rr < n) Zg[(i + 1) * LDZ + rr] = s * zi[t] + c * hc[t];
-                            hc[t] = c * zi[t] - s * hc[t];
-                            zi[t] = zin[t];
-                        }
-                        ei = ein;
-                        di = din;
-                    }
-#pragma unroll
-                    for (int t = 0; t < RPL; ++t) {
-                        const int r = sub + LPM * t;
-                        if (r < n) Zg[l * LDZ + r] = hc[t];
-                    }
-                    pp = -s * s2 * c3 * el1 * el / dl1;
-                    __syncwarp(gmask);
-                    if (sub == 0) {
-                        es[l] = s * pp;
-                        ds[l] = c * pp;
-                    }
-                    __syncwarp(gmask);
-                }
-                __syncwarp();
+            for (int t = 0; t < 4; ++t) {
+                const int j = 4 * g + t;
+                if (j + 1 >= NM) continue;
+                const float2 q = *reinterpret_cast<const float2 *>(sh + j);
+                p0 = fmaf(r[j + 1].re, q.x, p0);
+                p1 = fmaf(-r[j + 1].im, q.y, p1);
+                p2 = fmaf(r[j + 1].re, q.y, p2);
+                p3 = fmaf(r[j + 1].im, q.x, p3);
             }
         }
+        const cx<float> p = mk<float>(p0 + p1, p2 + p3);
+        const float vav = lanes_sum<LN>(below ? fmaf(v.re, p.re, v.im * p.im) : 0.f);
+        const float half = -0.5f * cabs2(tau) * vav;
+        cx<float> w = cmul(tau, p);
+        w = below ? mk<float>(fmaf(half, v.re, w.re), fmaf(half, v.im, w.im)) : mk<float>(0.f, 0.f);
+        const cx<float> vi = below ? v : mk<float>(0.f, 0.f);
+        __syncwarp();
+        sh[rel] = make_float4(vi.re, vi.im, w.re, w.im);
+        __syncwarp();
+        // A -= v w^H + w v^H, one register down
+#pragma unroll
+        for (int g = 0; g < NM / 4; ++g) {
+            if (4 * g >= m) continue;
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                const int j = 4 * g + t;
+                if (j + 1 >= NM) continue;
+                const float4 q = sh[j];
+                cx<float> h = r[j + 1];
+                h.re = fmaf(-vi.re, q.z, fmaf(-vi.im, q.w, fmaf(-w.re, q.x, fmaf(-w.im, q.y, h.re))));
+                h.im = fmaf(-vi.im, q.z, fmaf(vi.re, q.w, fmaf(-w.im, q.x, fmaf(w.re, q.y, h.im))));
+                r[j] = h;
+            }
+        }
+        __syncwarp();
+    }
+    const float dl = __shfl_sync(FULL, r[0].re, n - 1, LN);
+    if (live && lane < 2) out[(size_t)(n - 1) * n + lane] = lane == 0 ? make_float2(dl, 0.f) : tau0;
+}
 
-        // ---- 3. per matrix: U = Q Z, lane j holds column j of U
-        for (int q = 0; q < cnt; ++q) {
-            const int sn = sn0 + q;
-            const int status_q = __shfl_sync(0xffffffffu, status, q * LPM);
-            const float *Zq = Zb + q * S::Z_FLOATS;
-            const float2 *taus = reinterpret_cast<const float2 *>(dptr(q) + 2 * NM);
-            float2 *const Vt = evec + (size_t)sn * nn;
-            cx<float> u[NM];
+// ------------------------------------------------------------------ 2. QL
+
+constexpr int QL_APPLY = 8;                         // warps that apply rotations
+constexpr int QL_THREADS = 32 * (QL_APPLY + 1);
+constexpr int QL_AHEAD = 2;  // reflectors fetched ahead of the one that acts
+
+// GM matrices of up to NM x NM per CTA, LN lanes per matrix in the application.
+template <int NM>
+struct QlShape {
+    static constexpr int GM = NM <= 24 ? 32 : 16;
+    static constexpr int LN = NM <= 8 ? 8 : NM <= 16 ? 16 : 32;
+    static constexpr int LDZ = NM + 1;
+    static constexpr int Z_FLOATS = NM * LDZ;
+    static constexpr size_t RING = (size_t)2 * NM * GM * 8;  // two steps' rotations
+    static constexpr size_t BYTES = (size_t)GM * Z_FLOATS * 4 + RING + (size_t)2 * NM * GM * 4;
+    static_assert(RING >= (size_t)(QL_APPLY + 1) * 2 * NM * 8, "reflectors alias the ring");
+};
+
+// What bounds it is the chain of one rotation (a product sum, a reciprocal square
+// root with one Newton step and a product), of which GM run side by side: a QL
+// step takes as long as its longest chain, some 1.4 times the average.  The
+// shift of a step is applied as the chain loads the diagonal, and a bit mask per
+// matrix, rebuilt as the chain passes, tells where its off-diagonal is
+// negligible.  The tridiagonal matrix is scaled to norm 1 .. 2 and split below
+// 2^-23, the error of the reduction to it, so the reciprocal square root's operand
+// stays in range.  201,000 matrices of n = 32: 7.2 ms, half of the issue
+// slots; more CTAs per SM (GM = 8 or 16, n = 24) took as long.
+template <int NM>
+__global__ void __launch_bounds__(QL_THREADS, 2) msp_ql_kernel(SnapArgs a) {
+    using S = QlShape<NM>;
+    constexpr int GM = S::GM, LN = S::LN, LDZ = S::LDZ;
+    extern __shared__ __align__(16) char smem[];
+    float2 *const ring = reinterpret_cast<float2 *>(smem);  // [2][NM][GM]
+    float *const d = reinterpret_cast<float *>(smem + S::RING), *const e = d + NM * GM;  // [NM][GM]
+    float *const Z = e + NM * GM;  // [GM][column][row]
+    __shared__ int head[2][GM], alive[2], status[GM];  // head: m | l << 8, -1: no step
+    const int n = a.n, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int sn0 = blockIdx.x * GM, cnt = min(GM, a.num_snap - sn0);
+    float2 *const evec = reinterpret_cast<float2 *>(a.evec);
+    for (int x = tid; x < n * GM; x += QL_THREADS) {
+        const int i = x / GM, g = x - i * GM;
+        const float2 v = g < cnt ? evec[((size_t)(sn0 + g) * n + i) * n] : make_float2(0.f, 0.f);
+        d[x] = v.x;
+        e[x] = v.y;
+    }
+    for (int x = tid; x < GM * S::Z_FLOATS; x += QL_THREADS) {
+        const int y = x % S::Z_FLOATS;
+        Z[x] = y / LDZ == y % LDZ ? 1.f : 0.f;
+    }
+    __syncthreads();
+    // the recurrences (warp 0), a lane per matrix
+    const bool mine = warp == 0 && lane < cnt;
+    const int g0 = warp == 0 ? lane & (GM - 1) : 0;
+    float *const dg = d + g0, *const eg = e + g0;  // entry i at [i * GM]
+    const float small = 1.1920928955078125e-7f;  // 2^-23
+    unsigned mask = 0;  // bit i: entry i of e is negligible
+    int l = 0, iter = 0, st = MSP_ITEM_OK;
+    if (mine) {
+        float norm = 0.f;
+        for (int i = 0; i < n; ++i) norm = fmaxf(norm, fabsf(dg[i * GM]) + fabsf(eg[i * GM]));
+        // 0 for an overflowed matrix: its entries become NaN and split everywhere
+        const float inv = norm < 1e37f ? 2.f / pow2_above(norm) : 0.f;
+        for (int i = 0; i < n; ++i) {
+            dg[i * GM] *= inv;
+            const float x = eg[i * GM] * inv;
+            eg[i * GM] = x;
+            if (!(fabsf(x) > small)) mask |= 1u << i;
+        }
+        mask |= 1u << (n - 1);
+    }
+    for (int step = 0;; ++step) {
+        const int slot = step & 1;
+        if (warp == 0) {
+            // one QL step of every matrix that is not finished
+            bool on = mine && l < n;
+            if (on) {
+                if (iter >= 60 && !((mask >> l) & 1u)) {
+                    st = MSP_ITEM_NOT_CONVERGED;
+                    mask |= 1u << l;
+                }
+                const unsigned rest = ~(mask >> l);
+                const int skip = rest ? __ffs(rest) - 1 : 32;  // levels that are done
+                if (skip > 0) {
+                    l += skip;
+                    iter = 0;
+                }
+                on = l < n;
+            }
+            const unsigned go = __ballot_sync(FULL, on);
+            if (lane == 0) alive[slot] = go != 0;
+            int m = 0, len = 0;
+            float h = 0.f, dl = 0.f, dl1 = 0.f, el1 = 0.f, e0 = 0.f;
+            if (on) {
+                ++iter;
+                m = l + __ffs(mask >> l) - 1;
+                len = m - l;
+                const float g = dg[l * GM];
+                e0 = eg[l * GM];
+                el1 = eg[(l + 1) * GM];
+                // the shift only has to be good, not exact
+                const float pp = __fdividef(dg[(l + 1) * GM] - g, 2.f * e0);
+                const float t1 = fmaf(pp, pp, 1.f), t = pp + copysignf(t1 * fast_rsqrt(t1), pp);
+                dl = __fdividef(e0, t);
+                dl1 = e0 * t;
+                h = g - dl;
+            }
+            if (lane < GM) head[slot][lane] = on ? m | l << 8 : -1;
+            const int longest = __reduce_max_sync(FULL, len);
+            float c = 1.f, c2 = 1.f, c3 = 1.f, s = 0.f, s2 = 0.f, pp = 0.f, di = 0.f, ei = 0.f;
+            unsigned seen = 0;
+            auto diagonal = [&](int i) {
+                const float x = dg[i * GM] - h;
+                return i == l ? dl : i == l + 1 ? dl1 : x;
+            };
+            if (on) {
+                pp = diagonal(m);
+                di = diagonal(m - 1);
+                ei = eg[(m - 1) * GM];
+            }
+            float2 *out = ring + slot * NM * GM + g0;
+            for (int t = 0; t < longest; ++t, out += GM) {
+                if (t >= len) continue;
+                const int i = m - 1 - t, nx = max(i - 1, l);
+                const float dn = diagonal(nx), en = eg[nx * GM];
+                c3 = c2;
+                c2 = c;
+                s2 = s;
+                const float g = c * ei, hh = c * pp;
+                const float x2 = fmaf(pp, pp, ei * ei), u = fmaf(pp, di, -ei * g);
+                const float y = fast_rsqrt(x2);
+                const float en1 = s * (x2 * y);
+                s = ei * y;
+                c = pp * y;
+                pp = u * y;  // c d_i - s g
+                eg[(i + 1) * GM] = en1;
+                dg[(i + 1) * GM] = fmaf(s, fmaf(c, g, s * di), hh);
+                *out = make_float2(c, s);
+                seen = seen << 1 | (fabsf(en1) > small ? 0u : 1u);
+                di = dn;
+                ei = en;
+            }
+            if (on) {
+                pp = __fdividef(-s * s2 * c3 * el1 * e0, dl1);
+                const float x = s * pp;
+                eg[l * GM] = x;
+                dg[l * GM] = c * pp;
+                seen = seen << 1 | (fabsf(x) > small ? 0u : 1u);
+                // bits l .. m
+                const unsigned span = (2u << len) - 1u;
+                mask = (mask & ~(span << l)) | (seen & span) << l;
+                mask |= 1u << m;  // e_m = 0 r: the block's end
+            }
+        } else if (step > 0) {
+            // the previous step's rotations, a lane per row of Z
+            const int old = slot ^ 1, sub = lane & (LN - 1);
+            for (int g = (warp - 1) * (32 / LN) + lane / LN; g < GM; g += QL_APPLY * (32 / LN)) {
+                const int hd = head[old][g];
+                if (hd < 0 || sub >= n) continue;
+                const int m = hd & 255, l = hd >> 8;
+                const float2 *rot = ring + old * NM * GM + g;
+                float *z = Z + g * S::Z_FLOATS + m * LDZ + sub;
+                float hc = *z;
+                int len = m - l;
+                for (; len >= 8; len -= 8) {
+                    float zi[8];
+                    float2 q[8];
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) {
+                        zi[u] = z[-(u + 1) * LDZ];
+                        q[u] = rot[u * GM];
+                    }
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) {
+                        z[-u * LDZ] = q[u].y * zi[u] + q[u].x * hc;
+                        hc = q[u].x * zi[u] - q[u].y * hc;
+                    }
+                    z -= 8 * LDZ;
+                    rot += 8 * GM;
+                }
+                for (; len > 0; --len) {
+                    const float zi = z[-LDZ];
+                    const float2 q = *rot;
+                    *z = q.y * zi + q.x * hc;
+                    hc = q.x * zi - q.y * hc;
+                    z -= LDZ;
+                    rot += GM;
+                }
+                *z = hc;
+            }
+        }
+        __syncthreads();
+        if (!alive[slot]) break;
+    }
+    if (mine) status[lane] = st;
+    __syncthreads();
+    // U = Q Z, a warp per matrix: lane j holds column j and applies the reflectors
+    // last to first, each staged in shared memory while the one before it acts
+    float2 *const vb = ring + warp * 2 * NM;
+    for (int g = warp; g < cnt; g += QL_APPLY + 1) {
+        float2 *const V = evec + (size_t)(sn0 + g) * n * n;
+        const float *z = Z + g * S::Z_FLOATS + min(lane, NM - 1) * LDZ;
+        cx<float> u[NM];
+#pragma unroll
+        for (int i = 0; i < NM; ++i) u[i] = mk<float>(i < n ? z[i] : 0.f, 0.f);
+        auto fetch = [&](int k) {
+            return k >= 0 && lane > k && lane < n ? V[(size_t)k * n + lane] : make_float2(0.f, 0.f);
+        };
+        auto scalar = [&](int k) { return V[(size_t)(k > 0 ? k : n - 1) * n + 1]; };
+        float2 next[QL_AHEAD], tn[QL_AHEAD];
+#pragma unroll
+        for (int q = 0; q < QL_AHEAD; ++q) {
+            next[q] = fetch(n - 2 - q);
+            tn[q] = scalar(n - 2 - q);
+        }
+        for (int k = n - 2; k >= 0; --k) {
+            float2 *const vk = vb + (k & 1) * NM;
+            const float2 tau = tn[0];
+            if (lane < NM) vk[lane] = next[0];
+#pragma unroll
+            for (int q = 0; q + 1 < QL_AHEAD; ++q) {
+                next[q] = next[q + 1];
+                tn[q] = tn[q + 1];
+            }
+            next[QL_AHEAD - 1] = fetch(k - QL_AHEAD);
+            tn[QL_AHEAD - 1] = scalar(k - QL_AHEAD);
+            __syncwarp();
+            float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
+#pragma unroll
+            for (int q = 0; q < NM / 4; ++q) {
+                if (4 * q + 3 <= k || 4 * q >= n) continue;
+#pragma unroll
+                for (int t = 0; t < 4; ++t) {
+                    const int i = 4 * q + t;
+                    const float2 v = vk[i];
+                    s0 = fmaf(v.x, u[i].re, s0);
+                    s1 = fmaf(v.y, u[i].im, s1);
+                    s2 = fmaf(v.x, u[i].im, s2);
+                    s3 = fmaf(-v.y, u[i].re, s3);
+                }
+            }
+            const cx<float> ts = cmul(mk<float>(tau.x, tau.y), mk<float>(s0 + s1, s2 + s3));
+#pragma unroll
+            for (int q = 0; q < NM / 4; ++q) {
+                if (4 * q + 3 <= k || 4 * q >= n) continue;
+#pragma unroll
+                for (int t = 0; t < 4; ++t) {
+                    const int i = 4 * q + t;
+                    const float2 v = vk[i];
+                    u[i].re = fmaf(-v.x, ts.re, fmaf(v.y, ts.im, u[i].re));
+                    u[i].im = fmaf(-v.x, ts.im, fmaf(-v.y, ts.re, u[i].im));
+                }
+            }
+        }
+        __syncwarp();  // every lane has read the reflectors
+        if (lane < n) {
 #pragma unroll
             for (int i = 0; i < NM; ++i)
-                u[i] = mk<float>(lane < n && i < n ? Zq[lane * LDZ + i] : 0.f, 0.f);
-            for (int k = n - 2; k >= 0; --k) {
-                const float2 tk = taus[k];
-                if (tk.x == 0.f && tk.y == 0.f) continue;  // the same in every lane
-                const float2 *vk = Vt + (size_t)k * n;
-                // s = v^H u over the four-row groups that hold part of v
-                // (rows k+1 .. n-1)
-                float sr0 = 0.f, si0 = 0.f, sr1 = 0.f, si1 = 0.f;
-#pragma unroll
-                for (int gq = 0; gq < NM / 4; ++gq) {
-                    if (4 * gq + 3 > k && 4 * gq < n) {
-#pragma unroll
-                        for (int t = 0; t < 4; t += 2) {
-                            const int i = 4 * gq + t;
-                            const float2 v0 = i < n ? vk[i] : make_float2(0.f, 0.f);
-                            const float2 v1 = i + 1 < n ? vk[i + 1] : make_float2(0.f, 0.f);
-                            sr0 += v0.x * u[i].re + v0.y * u[i].im;
-                            si0 += v0.x * u[i].im - v0.y * u[i].re;
-                            sr1 += v1.x * u[i + 1].re + v1.y * u[i + 1].im;
-                            si1 += v1.x * u[i + 1].im - v1.y * u[i + 1].re;
-                        }
-                    }
-                }
-                const cx<float> ts = cmul(mk<float>(tk.x, tk.y), mk<float>(sr0 + sr1, si0 + si1));
-#pragma unroll
-                for (int gq = 0; gq < NM / 4; ++gq) {
-                    if (4 * gq + 3 > k && 4 * gq < n) {
-#pragma unroll
-                        for (int t = 0; t < 4; ++t) {
-                            const int i = 4 * gq + t;
-                            const float2 v = i < n ? vk[i] : make_float2(0.f, 0.f);
-                            u[i].re -= v.x * ts.re - v.y * ts.im;
-                            u[i].im -= v.x * ts.im + v.y * ts.re;
-                        }
-                    }
-                }
-            }
-            __syncwarp();  // every lane has read the reflectors
-            // eigenvectors (columns of U) to scratch, row-major
-            if (lane < n) {
-#pragma unroll
-                for (int i = 0; i < NM; ++i)
-                    if (i < n) Vt[(size_t)i * n + lane] = make_float2(u[i].re, u[i].im);
-            }
-            if (lane == 0) a.status[snap_source(a, sn).g] = status_q;
+                if (i < n) V[(size_t)i * n + lane] = make_float2(u[i].re, u[i].im);
         }
-        __syncwarp();  // R and the per-matrix tables are reused by the next batch
+        if (lane == 0) a.status[snap_source(a, sn0 + g).g] = status[g];
     }
 }
 
-template <int NM, int G>
-static cudaError_t qw_launch(const SnapArgs &a, cudaStream_t st) {
-    using S = QwShape<NM, G>;
-    const size_t smem = (size_t)QW_WARPS * S::BYTES;
-    cudaError_t e = cudaFuncSetAttribute(msp_ql_warp_kernel<NM, G>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+template <int NM>
+cudaError_t launch(const SnapArgs &a, cudaStream_t st) {
+    using S = QlShape<NM>;
+    msp_tri_warp_kernel<NM><<<(a.num_snap + TriShape<NM>::PER_CTA - 1) / TriShape<NM>::PER_CTA,
+                              TRI_WARPS * 32, 0, st>>>(a);
+    cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    int occ = 0, sms = 0, dev = 0;
-    e = cudaGetDevice(&dev);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e == cudaSuccess)
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, msp_ql_warp_kernel<NM, G>,
-                                                          QW_WARPS * 32, smem);
+    e = cudaFuncSetAttribute(msp_ql_kernel<NM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::BYTES);
     if (e != cudaSuccess) return e;
-    const long long tasks = (a.num_snap + G - 1) / G;
-    long long grid = (tasks + QW_WARPS - 1) / QW_WARPS;
-    const long long cap = (long long)sms * (occ > 0 ? occ : 1);
-    if (grid > cap) grid = cap;
-    if (grid < 1) grid = 1;
-    msp_ql_warp_kernel<NM, G><<<(int)grid, QW_WARPS * 32, smem, st>>>(a);
+    msp_ql_kernel<NM><<<(a.num_snap + S::GM - 1) / S::GM, QL_THREADS, S::BYTES, st>>>(a);
     return cudaGetLastError();
 }
 
-bool ql_warp_supported(int n) { return n >= 2 && n <= 32; }
+}  // namespace
 
-#ifndef QW_G24
-#define QW_G24 4
-#endif
-#ifndef QW_G32
-#define QW_G32 4
-#endif
+bool ql_warp_supported(int n) { return n >= 3 && n <= 32; }
+
 cudaError_t launch_ql_warp(const SnapArgs &a, cudaStream_t st) {
     if (a.num_snap <= 0) return cudaSuccess;
-    if (a.n <= 8) return qw_launch<8, 8>(a, st);
-    if (a.n <= 16) return qw_launch<16, 8>(a, st);
-    if (a.n <= 24) return qw_launch<24, QW_G24>(a, st);
-    if (a.n <= 32) return qw_launch<32, QW_G32>(a, st);
+    if (a.n <= 8) return launch<8>(a, st);
+    if (a.n <= 16) return launch<16>(a, st);
+    if (a.n <= 24) return launch<24>(a, st);
+    if (a.n <= 32) return launch<32>(a, st);
     return cudaErrorInvalidValue;
 }
 
