@@ -13,8 +13,10 @@
 //   * a = S_ij + l_i R_ij, b = S_ij + l_j R_ij; amax = the largest
 //     component of any a or b;
 //   * levels sorted by l form clusters: runs whose consecutive gaps are at
-//     most gamma = 100 amax.  Two levels in different clusters are more
-//     than gamma apart, so their first-order |E| stays below 1e-2;
+//     most gamma = 30 amax.  Two levels in different clusters are more
+//     than gamma apart, so their first-order |E| stays below 0.05 (at 100 amax
+//     a scan of n = 32 took 22.7 ms for 21.4: four snapshots in ten had a
+//     cluster to resolve);
 //   * pairs in different clusters get the first-order E and the
 //     second-order eigenvalue term; pairs in one cluster are only
 //     orthonormalised (E_ij = R_ij / 2);
@@ -74,19 +76,38 @@ __device__ __forceinline__ long long oa_sort_key(float2 l) {
 // inside).  All threads of the CTA call it; it ends with a barrier.
 static __device__ void oa_cluster_starts(const float2 *lam, int n, const OaCluster &c) {
     const int tid = threadIdx.x, nt = blockDim.x;
-    // ascending order, ties by index
-    for (int i = tid; i < n; i += nt) {
-        const long long li = oa_sort_key(lam[i]);
-        int r = 0;
-        for (int k = 0; k < n; ++k) {
-            const long long lk = oa_sort_key(lam[k]);
-            r += lk < li || (lk == li && k < i);
+    // ascending order, ties by index: parts of the comparisons per thread where
+    // there are threads enough (n = 32, 256 threads: 4 instead of 32 in a row)
+    const int parts = nt / n;
+    if (parts > 1) {
+        for (int i = tid; i < n; i += nt) c.rank[i] = 0;
+        __syncthreads();
+        const int part = tid / n, i = tid - part * n;
+        if (part < parts) {
+            const long long li = oa_sort_key(lam[i]);
+            int r = 0;
+            for (int k = part; k < n; k += parts) {
+                const long long lk = oa_sort_key(lam[k]);
+                r += lk < li || (lk == li && k < i);
+            }
+            atomicAdd(&c.rank[i], r);
         }
-        c.rank[i] = r;
-        c.order[r] = i;
+        __syncthreads();
+        if (tid < n) c.order[c.rank[tid]] = tid;
+    } else {
+        for (int i = tid; i < n; i += nt) {
+            const long long li = oa_sort_key(lam[i]);
+            int r = 0;
+            for (int k = 0; k < n; ++k) {
+                const long long lk = oa_sort_key(lam[k]);
+                r += lk < li || (lk == li && k < i);
+            }
+            c.rank[i] = r;
+            c.order[r] = i;
+        }
     }
     __syncthreads();
-    const float gamma = 100.0f * __int_as_float(c.scal[0]);
+    const float gamma = 30.0f * __int_as_float(c.scal[0]);
     if (tid < 32) {
         // cluster start of every sorted position: an inclusive max-scan of
         // the break positions, in contiguous chunks of `per` positions

@@ -549,7 +549,7 @@ static __device__ int eigenpairs(SnapSmem<float> &s, int n, int m, int max_refin
 // become E, and an element of the row operand is a broadcast that serves four
 // elements (oa_refine loads three operands for each).  n = 32: FP32 pipe 10
 // + 2 + 2 packed FMAs per complex product against 22, 42 KB of shared memory
-// against 59.  Scan of n = 32: 21.5 ms against 28.6; powder of n =
+// against 59.  Scan of n = 32: 19.4 ms against 28.6; powder of n =
 // 24: 0.41 ms against 0.47.
 
 // Groups of rows, rows per group and rows the matrices are padded to.
@@ -848,11 +848,79 @@ __device__ __forceinline__ float oa_refine_rows(SnapSmem<float> &s, int n_rt) {
         if ((tid & 31) == 0) atomicMax(&s.scal[2], em);  // non-negative: int order = float order
     }
     __syncthreads();
-    const bool clusters = s.scal[3] != 0;  // the same in every thread
+    // the same in every thread
+    const bool clusters = s.scal[3] != 0;
+    const float first = __int_as_float(s.scal[2]);
+    const bool second = n > 24 && !clusters && first > 2e-4f && first <= 3e-3f;
     if (rg == 0) {
         float c = 0.f;
         for (int g = 0; g < sh.groups; ++g) c += s.part[g * n + j].x;
         s.corr[j] = c;
+    }
+    if (second) {
+        // The exact E solves E_ij (l'_j - l_i) = (B + B E)_ij, with l'_j - l_j =
+        // sum_i conj(B_ij) E_ij: one more pass with the first-order E on the right
+        // leaves errors of its third power (no gap is below 30 amax here), where
+        // another refinement step would cost a double-word product.  B comes back
+        // as E times the gap, so that no register holds it.  Scan of n = 32: 19.4 ms
+        // against 21.3.  Not at n <= 24, where nine first steps in ten suffice and
+        // the branch alone cost 6% (0.44 ms against 0.41).
+        auto coupling = [&](int r) {
+            const cx<float> e = s.SR[(i0 + r) * ld + j];
+            const float gap = dw_sub_f(lj, s.lw[i0 + r]);
+            return mk<float>(e.re * gap, e.im * gap);
+        };
+#pragma unroll
+        for (int r = 0; r < RB; ++r)
+            if (mine(r)) R[(i0 + r) * ld + j] = coupling(r);
+        __syncthreads();
+        const float dj = s.corr[j];
+        cx<float> q[RB];
+        {
+            u64 s1[RB], s2[RB];
+#pragma unroll
+            for (int r = 0; r < RB; ++r) s1[r] = s2[r] = 0ull;
+#pragma unroll 8
+            for (int k = 0; k < n; ++k) {
+                const cx<float> e = s.SR[k * ld + j];
+                const u64 bx = f32x2(e.re, e.re), by = f32x2(e.im, e.im);
+#pragma unroll
+                for (int r = 0; r < RB; ++r) {
+                    const u64 x = *reinterpret_cast<const u64 *>(R + (i1 + r) * ld + k);
+                    s1[r] = fma_f32x2(x, bx, s1[r]);
+                    s2[r] = fma_f32x2(x, by, s2[r]);
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < RB; ++r) q[r] = lm_plain<false>(s1[r], s2[r]);
+        }
+        float shift = 0.f, norm = 0.f;
+#pragma unroll
+        for (int r = 0; r < RB; ++r) {
+            if (!mine(r) || i0 + r == j) continue;
+            const cx<float> b1 = R[(i0 + r) * ld + j];
+            const float inv = 1.0f / (dw_sub_f(lj, s.lw[i0 + r]) + dj);
+            q[r] = mk<float>((b1.re + q[r].re) * inv, (b1.im + q[r].im) * inv);
+            shift = fmaf(b1.re, q[r].re, fmaf(b1.im, q[r].im, shift));
+            norm += cabs2(q[r]);
+        }
+        if (active) {
+            s.part[tid].x = shift;
+            s.part[tid].y = norm;
+        }
+        __syncthreads();
+        norm = 0.f;
+        for (int g = 0; g < sh.groups; ++g) norm += s.part[g * n + j].y;
+#pragma unroll
+        for (int r = 0; r < RB; ++r)
+            if (mine(r))
+                s.SR[(i0 + r) * ld + j] = i0 + r == j ? mk<float>(-0.5f * (gj.x + gj.y + norm), 0.f) : q[r];
+        if (rg == 0) {
+            float c = 0.f;
+            for (int g = 0; g < sh.groups; ++g) c += s.part[g * n + j].x;
+            s.corr[j] = c;
+        }
+        __syncthreads();
     }
     if (clusters) {
         // T Hermitian
@@ -900,7 +968,7 @@ __device__ __forceinline__ float oa_refine_rows(SnapSmem<float> &s, int n_rt) {
         s.lw[j] = dw_add_f(s.lw[j], s.corr[j]);
     }
     __syncthreads();
-    const float step = __int_as_float(s.scal[2]);
+    const float step = second ? first * first : __int_as_float(s.scal[2]);
     __syncthreads();
     return step;
 }
