@@ -354,8 +354,7 @@ class CelioBatch:
         d = kernels.device()
         order_s = np.argsort(np.asarray(rows), kind="stable")
         rows_sorted = np.asarray(rows)[order_s]
-        self.row_start = kernels.dev(
-            np.searchsorted(rows_sorted, np.arange(nrows + 1)).astype(np.int32), torch.int32)
+        row_start = np.searchsorted(rows_sorted, np.arange(nrows + 1)).astype(np.int32)
         if field:
             mats = kernels.dev(np.broadcast_to(block, (S, mats_len)), torch.complex128).clone()
             out_off = []
@@ -377,7 +376,7 @@ class CelioBatch:
         self.nrows = int(nrows)
         self.pure = pure
         self.averages = int(averages)
-        self.wscale = kernels.dev(np.asarray(wscale, dtype=float)[order_s], torch.float64)
+        wscale = np.asarray(wscale, dtype=float)[order_s]
         p_sorted = p_lab[order_s]
         if pure:
             half = N // 2
@@ -387,13 +386,14 @@ class CelioBatch:
             sig[:, 1, 0] = p_lab[:, 0] + 1j * p_lab[:, 1]
             sig[:, 1, 1] = -p_lab[:, 2]
             mu = _mu_psi(sig) if S else np.zeros((0, 2), dtype=complex)
-            self.sigma = kernels.dev(sig[order_s], torch.complex128)
-            self.mu_psi = kernels.dev(mu[order_s], torch.complex128)
             self.seed = int(seed)
-            self.phases = None
+            ph = None
             if not device_phases:
                 ph = np.random.rand(S * self.averages * half).reshape(S, self.averages, half)
-                self.phases = kernels.dev(ph[order_s], torch.float64)
+                ph = ph[order_s]
+            self.sigma, self.mu_psi, self.phases, self.row_start, self.wscale = kernels.upload(
+                (sig[order_s], torch.complex128), (mu[order_s], torch.complex128),
+                (ph, torch.float64), (row_start, torch.int32), (wscale, torch.float64))
             return
 
         from muspinsim_gb300.experiment import thermal_state
@@ -410,10 +410,11 @@ class CelioBatch:
             for m in fac[1:]:
                 M = np.kron(M, m)
             rho[s_i] = M
-        self.rho0 = kernels.dev(rho, torch.complex128)
-        self.meas = kernels.dev(np.stack([_dense(system.operator({system.muon_index: ax}).matrix).T
-                                          for ax in "xyz"])[None], torch.complex128)
-        self.pol = torch.as_tensor(p_sorted, dtype=torch.complex128, device=d)
+        meas = np.stack([_dense(system.operator({system.muon_index: ax}).matrix).T
+                         for ax in "xyz"])[None]
+        self.rho0, self.meas, self.pol, self.row_start, self.wscale = kernels.upload(
+            (rho, torch.complex128), (meas, torch.complex128), (p_sorted, torch.complex128),
+            (row_start, torch.int32), (wscale, torch.float64))
         self.rows_sorted = torch.as_tensor(rows_sorted, dtype=torch.int64, device=d)
 
     def run(self, path=0):

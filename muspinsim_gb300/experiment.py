@@ -22,7 +22,7 @@ from muspinsim_gb300.celio import CelioHamiltonian
 from muspinsim_gb300.lindbladian import Lindbladian
 from muspinsim_gb300.powder import run_snapshots, t_inf_speedup
 from muspinsim_gb300.simconfig import MuSpinConfig
-from muspinsim_gb300.spinop import DensityOperator, SpinOperator, spin_projectors
+from muspinsim_gb300.spinop import DensityOperator, SpinOperator, _dense, spin_projectors
 
 
 def get_xy(z):
@@ -259,28 +259,33 @@ class ExperimentRunner:
         idx = np.unravel_index(np.arange(S), dims) if dims else ()
         consts = cfg.constants
 
-        def gather(key):
-            if key in keys:
-                pos = keys.index(key)
-                rng = [g for g in groups if key in g][0][key]
-                return [rng[i] for i in idx[pos]] if key != "t" else None
-            return None
+        def gather(key, convert):
+            # the range's values as an array, then one row per snapshot
+            if key not in keys:
+                return None
+            rng = [g for g in groups if key in g][0][key]
+            return convert(rng)[idx[keys.index(key)]]
+
+        def floats(values):
+            return np.asarray([v for v in values], dtype=float)
 
         def vec3(key):
-            got = gather(key)
+            got = gather(key, floats)
             if got is None:
                 return np.broadcast_to(np.asarray(consts[key], dtype=float), (S, 3))
-            return np.asarray(got, dtype=float)
+            return got
 
         B = vec3("B")
         intr = vec3("intrinsic_B")
         mupol = vec3("mupol")
-        Tg = gather("T")
-        T = np.full(S, float(consts["T"])) if Tg is None else np.asarray(Tg, dtype=float)
-        og = gather("orient")
-        orients = [consts["orient"]] * S if og is None else og
-        qs = np.array([q.q for q, w in orients])
-        ws = np.array([w for q, w in orients], dtype=float)
+        T = gather("T", floats)
+        if T is None:
+            T = np.full(S, float(consts["T"]))
+        qs = gather("orient", lambda rng: np.array([q.q for q, w in rng]))
+        ws = gather("orient", lambda rng: np.array([w for q, w in rng], dtype=float))
+        if qs is None:
+            q, w = consts["orient"]
+            qs, ws = np.tile(q.q, (S, 1)), np.full(S, float(w))
 
         # result layout: file dims then x dims; the time axis (x or file) is
         # computed in full by every snapshot
@@ -310,8 +315,13 @@ class ExperimentRunner:
         sy = self._system
         order = _rows_sorted(np.asarray(rows))
         n = int(np.prod(sy.dimension))
-        S_ops = np.array([[sy.operator({i: ax}).matrix.toarray() for ax in "xyz"]
-                          for i in range(len(sy.spins))], dtype=complex)
+        # S^a of spin i: 1 (x) S^a (x) 1
+        S_ops = np.empty((len(sy.spins), 3, n, n), dtype=complex)
+        for i, D in enumerate(sy.dimension):
+            before = np.eye(int(np.prod(sy.dimension[:i])))
+            after = np.eye(int(np.prod(sy.dimension[i + 1:])))
+            for a, ax in enumerate("xyz"):
+                S_ops[i, a] = np.kron(np.kron(before, _dense(sy._operators[i][ax].matrix)), after)
         mode = _lib.MODE_INTEGRAL if self._config.y_axis == "integral" else _lib.MODE_EVOLVE
         out, st = kernels.lindblad_run(
             n, sy.hamiltonian_matrix(), sy.zeeman_operators(), S_ops, list(sy.dimension),

@@ -7,6 +7,7 @@ basis and the sums over eigenvalue pairs run in ``libmspgpu`` (FP64).
 """
 
 import numpy as np
+import torch
 
 from muspinsim_gb300 import kernels
 from muspinsim_gb300.spinop import DensityOperator, Hermitian, Operator, SpinOperator, _dense
@@ -27,12 +28,17 @@ class Hamiltonian(Operator, Hermitian):
     def from_spin_operator(cls, spinop):
         return cls(spinop.matrix, spinop.dimension)
 
-    def _eigenbasis(self, rho0, operators):
+    def _eigenbasis(self, rho0, operators, times=None):
+        # on the device, after one upload: eigenvalues, eigenvectors, rho0 and
+        # the operators in the eigenbasis, times
         evals, evecs = self.diag()
-        U = np.asarray(evecs)
         mats = [_dense(rho0.matrix)] + [_dense(o.matrix) for o in operators]
-        rot = kernels.basis_change(U, np.asarray(mats, dtype=complex))
-        return evals, U, rot[0], rot[1:]
+        ev, U, M, t = kernels.upload(
+            (evals, torch.float64), (evecs, torch.complex128),
+            (np.asarray(mats, dtype=complex), torch.complex128),
+            (None if times is None else times.astype(np.float64), torch.float64))
+        rot = kernels.basis_change(U, M)
+        return ev, U, rot[0], rot[1:], t
 
     def evolve(self, rho0, times, operators=None):
         """Expectation values <O>(t) as a complex (T, n_ops) array, or the list
@@ -45,12 +51,12 @@ class Hamiltonian(Operator, Hermitian):
             operators = [operators]
         validate_evolve_params(rho0, times, operators)
         dim = rho0.dimension
-        evals, U, rho_e, ops_e = self._eigenbasis(rho0, operators)
+        evals, U, rho_e, ops_e, t = self._eigenbasis(rho0, operators, times)
         if len(operators) > 0:
-            out = kernels.evolve_expect(evals, rho_e, ops_e, times.astype(np.float64))
+            out = kernels.evolve_expect(evals, rho_e, ops_e, t)
             return out.cpu().numpy()
         # density matrices: U (exp(-i w t) o rho') U^dag for every time
-        ph = kernels.evolve_phases(evals, rho_e, times.astype(np.float64))
+        ph = kernels.evolve_phases(evals, rho_e, t)
         back = kernels.basis_change(U, ph, adjoint=True).cpu().numpy()
         return [DensityOperator(back[i], dim).clone_sparse() for i in range(len(times))]
 
@@ -60,7 +66,7 @@ class Hamiltonian(Operator, Hermitian):
         if isinstance(operators, SpinOperator):
             operators = [operators]
         validate_integrate_decaying_params(rho0, tau, operators)
-        evals, U, rho_e, ops_e = self._eigenbasis(rho0, operators)
+        evals, U, rho_e, ops_e, _ = self._eigenbasis(rho0, operators)
         return kernels.integrate_decaying(evals, rho_e, ops_e, tau).cpu().numpy()
 
     def fast_evolve(self, sigma_mu, times, other_dimension):

@@ -49,22 +49,67 @@ def dev(a, dtype):
     return torch.as_tensor(arr, dtype=dtype).to(d)
 
 
+_NUMPY = {torch.complex128: np.complex128, torch.float64: np.float64, torch.int32: np.int32}
+_PACK_BYTES = 1 << 20  # larger arrays are copied by themselves
+
+
+def upload(*pairs):
+    """:func:`dev` of several (array, dtype) pairs, None staying None.  The
+    small host arrays among them cross the bus in one copy and share its
+    device allocation: a copy costs some 15 us of host time whatever its
+    size, and a call has half a dozen inputs."""
+    d = device()
+    out, host, size = [None] * len(pairs), [], 0
+    for k, (a, dtype) in enumerate(pairs):
+        if a is None:
+            continue
+        if isinstance(a, torch.Tensor):
+            fits = a.dtype is dtype and a.device == d and a.is_contiguous()
+            out[k] = a if fits else dev(a, dtype)
+            continue
+        a = np.ascontiguousarray(a, dtype=_NUMPY[dtype])
+        if a.nbytes > _PACK_BYTES:
+            out[k] = dev(a, dtype)
+            continue
+        host.append((k, a, dtype, size))
+        size += (a.nbytes + 255) // 256 * 256
+    if len(host) == 1:
+        k, a, dtype, _ = host[0]
+        out[k] = dev(a, dtype)
+    elif host:
+        staging = np.empty(size, dtype=np.uint8)
+        for _, a, _, o in host:
+            staging[o:o + a.nbytes] = a.reshape(-1).view(np.uint8)
+        buf = torch.from_numpy(staging).to(d)
+        for k, a, dtype, o in host:
+            out[k] = buf[o:o + a.nbytes].view(dtype).reshape(a.shape)
+    return out
+
+
 def eigh(H, precision=_lib.PREC_FP64, max_sweeps=0):
     """Batched Hermitian eigensolve of (batch, n, n) complex matrices.
 
     Returns (evals (batch, n) float64 ascending, evecs (batch, n, n)
     complex128 with eigenvectors as columns, status (batch,) int32)."""
+    return _eigh(H, precision, max_sweeps)[1:]
+
+
+def _eigh(H, precision, max_sweeps):
+    # (the bytes of all three results, evals, evecs, status)
     Hd = dev(H, torch.complex128)
     if Hd.dim() == 2:
         Hd = Hd[None]
     b, n, _ = Hd.shape
-    evals = torch.empty((b, n), dtype=torch.float64, device=Hd.device)
-    evecs = torch.empty((b, n, n), dtype=torch.complex128, device=Hd.device)
-    status = torch.empty((b,), dtype=torch.int32, device=Hd.device)
+    size = (16 * b * n * n, 8 * b * n, 4 * b)
+    buf = torch.empty(sum(size), dtype=torch.uint8, device=Hd.device)
+    evecs, evals, status = torch.split(buf, size)
+    evecs = evecs.view(torch.complex128).reshape(b, n, n)
+    evals = evals.view(torch.float64).reshape(b, n)
+    status = status.view(torch.int32)
     if n <= _lib.MAX_DIM:
         _lib.call("msp_eigh_batched", ptr(Hd), n, b, int(precision), int(max_sweeps), ptr(evals),
                   ptr(evecs), ptr(status), stream())
-        return evals, evecs, status
+        return buf, evals, evecs, status
     # n > 64: Householder + QL in FP64 with caller scratch
     nbytes = ctypes.c_size_t(0)
     _lib.call("msp_eigh_workspace", n, b, ctypes.byref(nbytes))
@@ -72,7 +117,17 @@ def eigh(H, precision=_lib.PREC_FP64, max_sweeps=0):
     wp = ws.data_ptr() + ((-ws.data_ptr()) % 256)
     _lib.call("msp_eigh_batched_ws", ptr(Hd), n, b, int(precision), int(max_sweeps), ptr(evals),
               ptr(evecs), ptr(status), ctypes.c_void_p(wp), int(nbytes.value), stream())
-    return evals, evecs, status
+    return buf, evals, evecs, status
+
+
+def eigh_host(H):
+    """:func:`eigh` of one (n, n) matrix in FP64 with the results on the host
+    after a single copy: (evals (n,), evecs (n, n), status) as numpy arrays
+    and an int."""
+    n = np.shape(H)[-1]
+    host = _eigh(H, _lib.PREC_FP64, 0)[0].cpu().numpy()
+    evecs = host[:16 * n * n].view(np.complex128).reshape(n, n)
+    return host[16 * n * n:-4].view(np.float64), evecs, int(host[-4:].view(np.int32)[0])
 
 
 def assemble(Hsys, Z, fields):
@@ -107,8 +162,7 @@ def assemble_rotated(system, rotations):
 
 def basis_change(U, M, adjoint=False):
     """U^dag M U (or U M U^dag when adjoint) for batched or single matrices."""
-    Ud = dev(U, torch.complex128)
-    Md = dev(M, torch.complex128)
+    Ud, Md = upload((U, torch.complex128), (M, torch.complex128))
     n = Ud.shape[-1]
     ub = Ud.reshape(-1, n, n).shape[0]
     mb = Md.reshape(-1, n, n).shape[0]
@@ -342,26 +396,25 @@ class PowderPlan:
         if gammas is not None:
             for i, g in enumerate(gammas):
                 a.gammas[i] = float(g)
-        self.Hs = dev(Hsys, torch.complex128)
-        self.Zd = dev(Z, torch.complex128)
-        self.F = dev(field, torch.float64).reshape(-1, 3)
-        self.Pl = dev(pol, torch.float64).reshape(-1, 3)
-        self.W = dev(wscale, torch.float64).reshape(-1)
-        self.Sl = dev(slot, torch.int32).reshape(-1)
-        S = self.F.shape[0]
+        S = int(np.prod(np.shape(field))) // 3
+        tarr = None
+        if temperature is not None:
+            tarr = np.broadcast_to(np.asarray(temperature, dtype=np.float64), (S,))
+        self.Hs, self.Zd, F, Pl, W, Sl, self.R, self.Tp, T = upload(
+            (Hsys, torch.complex128), (Z, torch.complex128), (field, torch.float64),
+            (pol, torch.float64), (wscale, torch.float64), (slot, torch.int32),
+            (rho_fac, torch.complex128), (tarr, torch.float64),
+            (None if mode == _lib.MODE_INTEGRAL else times, torch.float64))
+        self.F, self.Pl = F.reshape(-1, 3), Pl.reshape(-1, 3)
+        self.W, self.Sl = W.reshape(-1), Sl.reshape(-1)
         self.num_snap = S
         a.Hsys, a.Z = self.Hs.data_ptr(), self.Zd.data_ptr()
         a.num_snap = S
         a.field, a.pol = self.F.data_ptr(), self.Pl.data_ptr()
         a.wscale, a.slot = self.W.data_ptr(), self.Sl.data_ptr()
-        self.R = None
-        if rho_fac is not None:
-            self.R = dev(rho_fac, torch.complex128)
+        if self.R is not None:
             a.rho_fac = self.R.data_ptr()
-        self.Tp = None
-        if temperature is not None:
-            tarr = np.broadcast_to(np.asarray(temperature, dtype=np.float64), (S,))
-            self.Tp = dev(np.ascontiguousarray(tarr), torch.float64)
+        if self.Tp is not None:
             a.temperature = self.Tp.data_ptr()
         a.num_slots = int(num_slots)
         self.T = None
@@ -372,7 +425,7 @@ class PowderPlan:
         else:
             th = times.detach().cpu().numpy() if isinstance(times, torch.Tensor) else np.asarray(times)
             uni, t0, dt = uniform_grid(th)
-            self.T = dev(times, torch.float64).reshape(-1)
+            self.T = T.reshape(-1)
             a.times = self.T.data_ptr()
             a.num_times = self.T.shape[0]
             a.uniform = 1 if uni else 0
@@ -457,17 +510,15 @@ def adjoint_fast(n, Hsys, Z, field, pol, wscale, slot, num_slots, times, grad_ou
     d = device()
     a = _lib.AdjointArgs()
     a.n = int(n)
-    Hs = dev(Hsys, torch.complex128)
-    Zd = dev(Z, torch.complex128)
-    F = dev(field, torch.float64).reshape(-1, 3)
-    Pl = dev(pol, torch.float64).reshape(-1, 3)
-    W = dev(wscale, torch.float64).reshape(-1)
-    Sl = dev(slot, torch.int32).reshape(-1)
-    S = F.shape[0]
     th = times.detach().cpu().numpy() if isinstance(times, torch.Tensor) else np.asarray(times)
     uni, t0, dt = uniform_grid(th)
-    Td = dev(th, torch.float64).reshape(-1)
-    g = dev(grad_out, torch.float64).reshape(int(num_slots), -1)
+    Hs, Zd, F, Pl, W, Sl, Td, g = upload(
+        (Hsys, torch.complex128), (Z, torch.complex128), (field, torch.float64),
+        (pol, torch.float64), (wscale, torch.float64), (slot, torch.int32),
+        (times if isinstance(times, torch.Tensor) else th, torch.float64), (grad_out, torch.float64))
+    F, Pl, W, Sl, Td = F.reshape(-1, 3), Pl.reshape(-1, 3), W.reshape(-1), Sl.reshape(-1), Td.reshape(-1)
+    S = F.shape[0]
+    g = g.reshape(int(num_slots), -1)
     if g.shape[1] != Td.shape[0]:
         raise ValueError("grad_out must have one row of len(times) values per slot")
     gH = torch.empty((a.n, a.n), dtype=torch.complex128, device=d)
@@ -616,13 +667,12 @@ def _superop_ws(n, num_ops):
 def superop_evolve(L, n, rho0, ops, times):
     """rho(t) = exp(2 pi L t) rho0 (msp_superop_evolve): (T, n_ops) complex
     expectations Tr(O rho(t)), or (T, n*n) vec(rho(t)) when ``ops`` is empty."""
-    Ld = dev(L, torch.complex128)
-    r = dev(rho0, torch.complex128)
     th = np.asarray(times, dtype=float)
-    o = dev(ops, torch.complex128).reshape(-1, n, n) if len(ops) else None
+    Ld, r, o, Td = upload((L, torch.complex128), (rho0, torch.complex128),
+                          (ops if len(ops) else None, torch.complex128), (th, torch.float64))
+    o = None if o is None else o.reshape(-1, n, n)
     nops = 0 if o is None else int(o.shape[0])
     uni, t0, dt = uniform_grid(th)
-    Td = dev(th, torch.float64)
     out = torch.empty((th.size, nops if nops else n * n), dtype=torch.complex128, device=Ld.device)
     ws, wp, nb = _superop_ws(n, nops)
     _lib.call("msp_superop_evolve", ptr(Ld), int(n), ptr(r), ptr(o), nops, ptr(Td), int(th.size),
@@ -657,35 +707,29 @@ def lindblad_run(n, Hsys, Z, spin_ops, dims, mu_index, gammas, dissipation, fiel
     for i, x in enumerate(dims):
         a.dims[i] = int(x)
         a.gammas[i] = float(gammas[i])
-    keep = [dev(Hsys, torch.complex128), dev(Z, torch.complex128), dev(spin_ops, torch.complex128)]
-    a.Hsys, a.Z, a.spin_ops = (t.data_ptr() for t in keep)
     a.num_dissipative = len(dissipation)
     for k, (i, rate) in enumerate(sorted(dissipation.items())):
         a.dissipative_spin[k] = int(i)
         a.dissipative_rate[k] = float(rate)
-    F = dev(field, torch.float64).reshape(-1, 3)
-    S = int(F.shape[0])
-    vecs = [F, dev(pol, torch.float64).reshape(-1, 3), dev(wscale, torch.float64).reshape(-1),
-            dev(slot, torch.int32).reshape(-1)]
-    keep += vecs
-    a.num_snap = S
-    a.field, a.pol, a.wscale, a.slot = (t.data_ptr() for t in vecs)
+    S = int(np.prod(np.shape(field))) // 3
+    Tp = th = None
     if temperature is not None:
-        Tp = dev(np.ascontiguousarray(np.broadcast_to(np.asarray(temperature, float), (S,))),
-                 torch.float64)
-        keep.append(Tp)
-        a.temperature = Tp.data_ptr()
-    a.num_slots = int(num_slots)
+        Tp = np.broadcast_to(np.asarray(temperature, float), (S,))
     if mode == _lib.MODE_INTEGRAL:
         a.num_times, a.uniform = 1, 1
         shape = (int(num_slots),)
     else:
         th = np.asarray(times, dtype=float)
         uni, t0, dt = uniform_grid(th)
-        Td = dev(th, torch.float64)
-        keep.append(Td)
-        a.times, a.num_times, a.uniform, a.t0, a.dt = Td.data_ptr(), int(th.size), int(uni), t0, dt
+        a.num_times, a.uniform, a.t0, a.dt = int(th.size), int(uni), t0, dt
         shape = (int(num_slots), int(th.size))
+    keep = upload((Hsys, torch.complex128), (Z, torch.complex128), (spin_ops, torch.complex128),
+                  (field, torch.float64), (pol, torch.float64), (wscale, torch.float64),
+                  (slot, torch.int32), (Tp, torch.float64), (th, torch.float64))
+    (a.Hsys, a.Z, a.spin_ops, a.field, a.pol, a.wscale, a.slot, a.temperature, a.times) = (
+        None if x is None else x.data_ptr() for x in keep)
+    a.num_snap = S
+    a.num_slots = int(num_slots)
     a.tau, a.mode = float(tau), int(mode)
     a.precision = int(precision)
     out = torch.empty(shape, dtype=torch.float64, device=d)

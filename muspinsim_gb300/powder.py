@@ -68,17 +68,18 @@ def _cached_plan(system, Hs, Zd, n, F, Pl, W, slot, num_slots, times, mode, prec
     """A PowderPlan for the device-side powder_average path, reused across
     calls with the same system matrices and sizes (its output, status and
     workspace stay allocated; only the per-call inputs are re-pointed and
-    the time grid re-uploaded).  Plans with finite temperatures are not
-    cached."""
+    the time grid re-uploaded).  Only plans of the fast path are cached."""
     th = np.asarray(times, dtype=float)
+    keep = mode == _lib.MODE_FAST
     key = (Hs.data_ptr(), Zd.data_ptr(), int(F.shape[0]), th.size, int(num_slots), mode, prec,
            max_sweeps, Tarr is None)
-    plan = _PLANS.get(key) if Tarr is None else None
+    plan = _PLANS.get(key) if keep else None
     if plan is None:
         plan = kernels.PowderPlan(n, Hs, Zd, F, Pl, W, slot, num_slots, th, mode=mode,
                                   precision=prec, dims=dims, mu_index=mu, gammas=system.gammas,
-                                  temperature=Tarr, tau=MU_TAU, max_sweeps=max_sweeps)
-        if Tarr is None:
+                                  temperature=None if keep else Tarr, tau=MU_TAU,
+                                  max_sweeps=max_sweeps)
+        if keep:
             if len(_PLANS) >= 8:
                 _PLANS.clear()
             _PLANS[key] = plan
@@ -92,6 +93,11 @@ def _cached_plan(system, Hs, Zd, n, F, Pl, W, slot, num_slots, times, mode, prec
         a.uniform, a.t0, a.dt = (1 if uni else 0), t0, dt
         plan._times_host = th.copy()
     return plan
+
+
+def _all_inf(T):
+    """T = inf throughout, which the kernels assume when given no temperatures."""
+    return bool(np.all(np.asarray(T, dtype=float) == np.inf))
 
 
 def run_snapshots(system, B_lab, p_lab, T, wscale, slot, num_slots, times,
@@ -140,7 +146,8 @@ def run_snapshots(system, B_lab, p_lab, T, wscale, slot, num_slots, times,
         mode = _lib.MODE_INTEGRAL if y_axis == "integral" else (
             _lib.MODE_FAST if fast_mask else _lib.MODE_EVOLVE)
         plan = _cached_plan(system, Hs, Zd, n, B_lab, p_lab, wscale, slot, num_slots, times, mode,
-                            prec, dims, mu, None if mode == _lib.MODE_FAST else Tarr, max_sweeps)
+                            prec, dims, mu,
+                            None if mode == _lib.MODE_FAST or _all_inf(T) else Tarr, max_sweeps)
         out = plan.run()
         if host_out:
             return plan.fetch()
@@ -148,13 +155,12 @@ def run_snapshots(system, B_lab, p_lab, T, wscale, slot, num_slots, times,
 
     if y_axis == "integral":
         groups = [(_lib.MODE_INTEGRAL, np.ones(S, dtype=bool))]
-        out = torch.zeros((num_slots,), dtype=torch.float64, device=dev)
     else:
         fast = t_inf_speedup(B_lab, Tarr, mu)
         groups = [(_lib.MODE_FAST, fast), (_lib.MODE_EVOLVE, ~fast)]
-        out = torch.zeros((num_slots, len(times)), dtype=torch.float64, device=dev)
+    hot = _all_inf(T)
     status = np.zeros(S, dtype=np.int32)
-    first = True
+    out = None
     for mode, mask in groups:
         idx = np.nonzero(mask)[0]
         if idx.size == 0:
@@ -163,13 +169,16 @@ def run_snapshots(system, B_lab, p_lab, T, wscale, slot, num_slots, times,
         res, st = kernels.powder_run(
             n, Hs, Zd, B_lab[idx], p_lab[idx], wscale[idx], slot[idx].astype(np.int32),
             num_slots, times, mode=mode, precision=prec, dims=dims, mu_index=mu,
-            gammas=system.gammas, temperature=Tarr[idx], tau=MU_TAU, max_sweeps=max_sweeps)
-        if first:
+            gammas=system.gammas, temperature=None if hot else Tarr[idx], tau=MU_TAU,
+            max_sweeps=max_sweeps)
+        if out is None:
             out = res
-            first = False
         else:
             out += res
         status[idx] = st.cpu().numpy()
+    if out is None:  # no snapshots
+        shape = (num_slots,) if y_axis == "integral" else (num_slots, len(times))
+        out = torch.zeros(shape, dtype=torch.float64, device=dev)
     if host_out:
         return out.cpu().numpy(), status
     return out, status

@@ -81,10 +81,10 @@ class Hermitian:
         cached = getattr(self, "_eigh_cache", None)
         if cached is not None and cached[0].shape == M.shape and np.array_equal(cached[0], M):
             return cached[1]
-        evals, evecs, status = kernels.eigh(M[None])
-        if int(status[0].item()) != 0:
+        evals, evecs, status = kernels.eigh_host(M)
+        if status != 0:
             raise RuntimeError("Hermitian.diag: the Jacobi eigensolver did not converge")
-        eigh = (evals[0].cpu().numpy(), evecs[0].cpu().numpy())
+        eigh = (evals, evecs)
         self._eigh_cache = (M.copy(), eigh)
         return eigh
 
