@@ -72,6 +72,8 @@ struct MultiBucket {
     int ctas_per_sm;  // persistent CTAs per SM (0: occupancy limit, set at first run)
     int grid;         // persistent grid of the snapshot kernel (set at first run for n <= 64)
     int ip;           // pairs per phase-sum work item
+    bool fourier;     // the phase sum as a nonuniform Fourier transform
+    NufftShape nu;
     int cap_snap;     // snapshots per chunk
     long long num_snap;
     std::vector<int> systems;  // global system ids, ascending
@@ -163,6 +165,15 @@ static int plan_layout(msp_multi_plan *p, const msp_multi_desc *d) {
         if (ip > (1LL << 30)) ip = 1LL << 30;
         if (ip < 1) ip = 1;
         b.ip = (int)ip;
+        // on a uniform grid the transform, where it is the cheaper form (msp_nufft.cu);
+        // a tuned item size asks for the direct sum.  64 orientations of three n = 192
+        // systems, 2,048 samples, MIXED: the run takes 8.9 ms instead of 9.6; of three n =
+        // 24 systems in FP64: 0.46 ms instead of 1.69
+        b.fourier = p->uniform && !(t && t->snaps_per_item > 0) && b.num_snap > 0 &&
+                    b.systems.size() <= 65535 &&
+                    nufft_shape(b.cap_snap, b.P, (int)b.systems.size(), p->num_times, d->precision,
+                                d->t0 != 0.0, &b.nu);
+        if (b.fourier) b.ip = b.nu.ip;
         b.grid = 0;
         b.stream = NULL;
         b.done = NULL;
@@ -254,7 +265,7 @@ static int plan_layout(msp_multi_plan *p, const msp_multi_desc *d) {
         b.off_const = off;
         off += al256(S * 8);
         b.off_partial = off;
-        off += al256((size_t)b.max_items * T * (records ? 4 : 8));
+        off += al256(b.fourier ? b.nu.bytes : (size_t)b.max_items * T * (records ? 4 : 8));
         b.off_evec = off;
         off += al256(b.large ? 0 : snap_evec_bytes(b.n, (long long)S));
         b.off_large = off;
@@ -432,6 +443,16 @@ static int plan_enqueue(msp_multi_plan *p, const msp_multi_io *io, cudaStream_t 
             pa.partial_f32 = records ? reinterpret_cast<float *>(ws + b.off_partial) : NULL;
             pa.slot_row = reinterpret_cast<const int *>(ws + c.slot_row);
             pa.accumulate = 1;
+            if (b.fourier && c.num_items > 0) {
+                rc = mcuda(launch_nufft_spread(pa, b.nu, p->precision, ws + b.off_partial, b.stream),
+                           "msp_multi_run: phase sum");
+                if (rc == MSP_OK)
+                    rc = mcuda(launch_nufft_rows(pa, b.nu, p->precision, ws + b.off_partial,
+                                                 sa.snap_const, io->out, b.stream),
+                               "msp_multi_run: reduction");
+                if (rc != MSP_OK) return rc;
+                continue;
+            }
             if (c.num_items > 0) {
                 rc = mcuda(launch_phase(pa, p->precision, c.num_items, p->uniform, b.stream),
                            "msp_multi_run: phase sum");
