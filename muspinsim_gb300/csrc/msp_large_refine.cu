@@ -15,7 +15,7 @@
 // Eigenvalues come out FP64-accurate, eigenvectors to FP32 rounding: the MIXED
 // result.  FP64 keeps the last correction's low words and
 // goes on with the FP64 step of the n <= 64 kernels (msp_snap64.cu):
-//   r_j = H x_j - l_j x_j in FP64 (4 n^3 FMAs), everything after it except
+//   r_j = H x_j - l_j x_j in FP64 (4 n FMAs per entry of H that is not zero), everything after it except
 //   norms in FP32, because r_j is small,
 // until its correction is below 2e-8, and forms M in FP64 (2 n^3
 // FMAs).  A snapshot that does not get there is left to the FP64 solver
@@ -81,7 +81,8 @@ struct LmVec {
     float2 *lam;                        // eigenvalues as double-words
     int *rank, *order, *cstart;         // clusters of levels (msp_cluster.cuh)
     float *corr, *corr_part, *norm, *norm_part, *rn, *cn, *gf;
-    int *scal;     // [0]: largest correction, [1]: largest |l_i|, [2]: largest coupling (float bits)
+    int *scal;     // [0]: largest correction, [1]: largest |l_i|, [2]: largest coupling (float
+                   // bits), [3]: nonzeros of H's fullest row
     double *dsum;  // one per CTA of the team
     char *slab;    // two stages of GEMM slabs
 };
@@ -142,7 +143,103 @@ __device__ void lm_colnorms(const float2 *X, int n, float *out, const LmVec &v, 
     }
 }
 
+// ------------------------------------------------------------------ rows of H
+
+// A spin Hamiltonian in the product basis is sparse: a term reaches the states
+// that differ in one or two spins (19 of 96 entries a row for five nuclei and
+// spins with an electron and a muon, 22 of 192 for six).  H X skips the zeros of H: its
+// rows are compacted in place, the nonzero entries first, the column of entry q in
+// the 4-byte word 2 + q from the row's end and their number in the last word.
+// Only where no row has more than n / 2 of them, so that both fit (fuller ones stay
+// dense for the tiled product): 192 snapshots of n = 192 in 8.05 ms at n / 2 - 1
+// entries a row against 8.13 for the tiled product at n / 2 + 1, 96 of n = 96 in
+// 1.51 against 1.64 (all stages, MIXED).  Batch of 21 systems up to n = 192: 9.6 -> 8.0
+// ms; n = 96 in FP64, where the FP64 pipe is the bound: 2.45 -> 2.07 ms.
+
+__device__ __forceinline__ bool lm_nonzero(const float4 &h) {
+    return !(h.x == 0.f && h.y == 0.f && h.z == 0.f && h.w == 0.f);  // true for a NaN
+}
+__device__ __forceinline__ bool lm_nonzero(const cx<double> &h) { return !(h.re == 0.0 && h.im == 0.0); }
+
+// Compacts H (n x n, seen by the team) where it is sparse and says whether it was;
+// *most is zero in every CTA.  A warp per row; n <= 1024, so lane c can keep the
+// nonzeros of columns 32 c .. 32 c + 31.
+template <typename T>
+__device__ bool lm_compact(T *H, int n, int *most, const Team &team) {
+    static_assert(sizeof(T) == 16, "room for the columns");
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int me = team.rank * nw + warp, all = team.size * nw;
+    int fullest = 0;
+    for (int i = me; i < n; i += all) {
+        int cnt = 0;
+#pragma unroll 4
+        for (int k0 = 0; k0 < n; k0 += 32)
+            cnt += __popc(__ballot_sync(0xffffffffu, k0 + lane < n && lm_nonzero(H[(size_t)i * n + min(k0 + lane, n - 1)])));
+        fullest = max(fullest, cnt);
+    }
+    if (lane == 0)
+        for (int r = 0; r < team.size; ++r) atomicMax(team.of(most, r), fullest);
+    team.sync();
+    if (2 * *most > n) return false;  // the same in every CTA
+    for (int i = me; i < n; i += all) {
+        T *row = H + (size_t)i * n;
+        unsigned mine = 0;
+        int cnt = 0;
+        for (int k0 = 0; k0 < n; k0 += 32) {
+            const T h = row[min(k0 + lane, n - 1)];
+            const bool nz = k0 + lane < n && lm_nonzero(h);
+            const unsigned b = __ballot_sync(0xffffffffu, nz);  // everyone has read
+            if (lane == k0 >> 5) mine = b;
+            if (nz) row[cnt + __popc(b & ((1u << lane) - 1))] = h;
+            cnt += __popc(b);
+            __syncwarp();
+        }
+        int *tail = reinterpret_cast<int *>(row + n);
+        int q = 0;
+        for (int k0 = 0; k0 < n; k0 += 32) {
+            const unsigned b = __shfl_sync(0xffffffffu, mine, k0 >> 5);
+            if (b >> lane & 1) tail[-2 - (q + __popc(b & ((1u << lane) - 1)))] = k0 + lane;
+            q += __popc(b);
+        }
+        if (lane == 0) tail[-1] = cnt;
+    }
+    team.sync();
+    return true;
+}
+
+// H X by compacted rows: a warp makes 64 columns of a row, two per lane, so that an
+// entry of H serves both; X comes through L1 / L2 in whole rows.  init(i, j) starts a
+// sum, step(sum, h, x) adds a product, epi(i, j, sum) consumes it.
+template <typename T, typename X, typename Init, typename Step, typename Epi>
+__device__ __forceinline__ void lm_sparse_rows(const T *H, const X *x, int n, const Team &team,
+                                               Init init, Step step, Epi epi) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int groups = (n + 63) >> 6;
+    for (int u = team.rank * nw + warp; u < n * groups; u += team.size * nw) {
+        const int i = u / groups, j = (u - i * groups) * 64 + lane;
+        const bool two = j - lane + 32 < n;  // the same in the whole warp
+        const int ja = min(j, n - 1), jb = min(j + 32, n - 1);
+        const T *row = H + (size_t)i * n;
+        const int *tail = reinterpret_cast<const int *>(row + n);
+        const int cnt = tail[-1];
+        auto a = init(i, ja), b = init(i, jb);
+#pragma unroll 4
+        for (int q = 0; q < cnt; ++q) {
+            const T h = row[q];
+            const X *xk = x + (size_t)tail[-2 - q] * n;
+            step(a, h, xk[ja]);
+            if (two) step(b, h, xk[jb]);
+        }
+        if (j < n) epi(i, j, a);
+        if (j + 32 < n) epi(i, j + 32, b);
+    }
+}
+
 // ------------------------------------------------------------------ double-word step
+
+struct LmSum {
+    u64 s1, c1, s2, c2;
+};
 
 // Rayleigh quotients and residuals from Y = H X: v.lam, v.gf = x_j^H x_j - 1
 // (in every CTA) and R = Y - X diag(l), 32 columns per CTA and turn, rows over
@@ -291,9 +388,10 @@ __device__ __forceinline__ int lm_owner(int q0, const Team &team) {
 // into Xl) and of the eigenvalues v.lam, clusters resolved as in the n <= 64
 // refinement (msp_cluster.cuh).  Y holds the couplings B, then E in their
 // place, and T behind them.  Returns the step's largest correction.
+// sparse: H is compacted.
 template <bool LO>
 __device__ float lm_refine(const LargeSlot &s, const cx<float> *X, cx<float> *X2, const LmVec &v,
-                           int n, const Team &team) {
+                           int n, bool sparse, const Team &team) {
     const int tid = threadIdx.x, nt = blockDim.x, nw = nt >> 5, warp = tid >> 5;
     const float2 *Xf = reinterpret_cast<const float2 *>(X);
     if (tid < 3) v.scal[tid] = 0;
@@ -301,12 +399,27 @@ __device__ float lm_refine(const LargeSlot &s, const cx<float> *X, cx<float> *X2
     team.sync();
     // Y = H X
     auto bound = [&](int i, int j) { return v.rn[min(i, n - 1)] * v.cn[min(j, n - 1)]; };
-    lm_tiles<LM_DW_ALO, false>(
-        n, n, n, s.H, n, Xf, n, v.slab, team.rank, team.size, [](int, int) { return false; },
-        [&](int i, int j, u64 &s1, u64 &, u64 &s2, u64 &) { s1 = s2 = lm_anchor(bound(i, j)); },
-        [&](int i, int j, u64 s1, u64 c1, u64 s2, u64 c2) {
-            s.Y[(size_t)i * n + j] = lm_dw<false>(s1, c1, s2, c2, lm_anchor(bound(i, j)));
-        });
+    if (sparse)
+        lm_sparse_rows(
+            s.H, Xf, n, team,
+            [&](int i, int j) {
+                const u64 K = lm_anchor(bound(i, j));
+                return LmSum{K, 0ull, K, 0ull};
+            },
+            [](LmSum &t, const float4 &h, const float2 &x) {
+                lm_step<true, false>(t.s1, t.c1, t.s2, t.c2, f32x2(h.x, h.y), f32x2(h.z, h.w),
+                                     f32x2(x.x, x.x), f32x2(x.y, x.y), 0ull, 0ull);
+            },
+            [&](int i, int j, const LmSum &t) {
+                s.Y[(size_t)i * n + j] = lm_dw<false>(t.s1, t.c1, t.s2, t.c2, lm_anchor(bound(i, j)));
+            });
+    else
+        lm_tiles<LM_DW_ALO, false>(
+            n, n, n, s.H, n, Xf, n, v.slab, team.rank, team.size, [](int, int) { return false; },
+            [&](int i, int j, u64 &s1, u64 &, u64 &s2, u64 &) { s1 = s2 = lm_anchor(bound(i, j)); },
+            [&](int i, int j, u64 s1, u64 c1, u64 s2, u64 c2) {
+                s.Y[(size_t)i * n + j] = lm_dw<false>(s1, c1, s2, c2, lm_anchor(bound(i, j)));
+            });
     team.sync();
     lm_residuals(s, X, v, n, team);
     team.sync();
@@ -468,23 +581,37 @@ __device__ __forceinline__ void fp64_blocks(int n, const cx<double> *const (&B)[
 // the levels v.lam0: v.lam64 and X64 corrected.  H in FP64; XF the vectors in
 // FP32; R, B and Bt n x n scratch (the couplings, which the corrections replace, and
 // their transpose; T, the couplings inside clusters, takes R's place).  Returns the largest column norm of E (NaN or infinite when the input is
-// unusable): the step leaves an error of that order squared.
+// unusable): the step leaves an error of that order squared.  sparse: H is compacted.
 __device__ float lm_step64(const cx<double> *H, cx<double> *X64, const cx<float> *XF, cx<float> *R,
-                           cx<float> *B, cx<float> *Bt, const LmVec &v, int n, const Team &team) {
+                           cx<float> *B, cx<float> *Bt, const LmVec &v, int n, bool sparse,
+                           const Team &team) {
     const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
     const int me = team.rank * nt + tid, all = team.size * nt;
     if (tid < 3) v.scal[tid] = 0;
     // r = H x - l x
-    const cx<double> *const x64[1] = {X64};
-    fp64_blocks<1>(
-        n, x64, team, [](int, int) { return false; },
-        [&](int i, int k) { return H[(size_t)i * n + k]; },
-        [&](int i, int j, const double *re, const double *im) {
-            const size_t o = (size_t)i * n + j;
-            const cx<double> x = X64[o];
-            const double l = v.lam0[j];
-            R[o] = mk<float>((float)fma(-l, x.re, re[0]), (float)fma(-l, x.im, im[0]));
-        });
+    auto residual = [&](int i, int j, double re, double im) {
+        const size_t o = (size_t)i * n + j;
+        const cx<double> x = X64[o];
+        const double l = v.lam0[j];
+        R[o] = mk<float>((float)fma(-l, x.re, re), (float)fma(-l, x.im, im));
+    };
+    if (sparse) {
+        lm_sparse_rows(
+            H, X64, n, team, [](int, int) { return mk<double>(0.0, 0.0); },
+            [](cx<double> &t, const cx<double> &h, const cx<double> &x) {
+                t.re = fma(h.re, x.re, t.re);
+                t.im = fma(h.re, x.im, t.im);
+                t.re = fma(-h.im, x.im, t.re);
+                t.im = fma(h.im, x.re, t.im);
+            },
+            [&](int i, int j, const cx<double> &t) { residual(i, j, t.re, t.im); });
+    } else {
+        const cx<double> *const x64[1] = {X64};
+        fp64_blocks<1>(
+            n, x64, team, [](int, int) { return false; },
+            [&](int i, int k) { return H[(size_t)i * n + k]; },
+            [&](int i, int j, const double *re, const double *im) { residual(i, j, re[0], im[0]); });
+    }
     team.sync();
     // column norms (FP64) and level corrections, a thread per column and part
     // of the rows
@@ -690,10 +817,8 @@ __device__ double team_sum(double x, double *dsum, const Team &team) {
 // 6e-5 (four at most), then FP64 steps until 2e-8 (three at most); the vectors
 // stay in the slot's Y, the levels in its R, for the pair kernels, and
 // redo[slot] asks for the FP64 solver.
-// Bound by the FP32 pipe in H X (ten packed FMAs per complex product), by issue
-// in the plain products; FP64 by r = H x - l x.  192 snapshots of n = 192 MIXED:
-// 4.1 ms, some 12 ms as the tail of one kernel per snapshot; 49 of n = 96 FP64:
-// 0.8 ms.
+// Bound by issue in the plain products; H X skips the zeros of H (4.1 ms for 192
+// snapshots of n = 192 MIXED where it did not, 2.4 ms now).
 template <bool FP64>
 __global__ void __maxnreg__(128)
     msp_large_refine_kernel(SnapArgs a, char *scratch, size_t per, int first, int *redo) {
@@ -708,6 +833,7 @@ __global__ void __maxnreg__(128)
     const SnapSource src = snap_source(a, sn);
     const size_t g = (size_t)src.g;
     int st = s.ql->status;
+    if (tid == 0) v.scal[3] = 0;
     team.sync();  // every CTA of the team runs before its shared memory is written
     // row norms of H
     for (int i = team.rank * nw + warp; i < n; i += team.size * nw) {
@@ -720,7 +846,7 @@ __global__ void __maxnreg__(128)
         for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
         if (lane == 0) team.put(v.rn + i, sqrtf(acc));
     }
-    team.sync();
+    bool sparse = lm_compact(s.H, n, v.scal + 3, team);  // behind a team barrier
     cx<float> *X = s.X, *X2 = s.X2;
     const int max_refine = FP64 || a.max_refine <= 0 ? 4 : a.max_refine;
     bool ok = true;
@@ -735,7 +861,7 @@ __global__ void __maxnreg__(128)
     }
     st |= MSP_ITEM_REFINE_LIMIT;
     for (int it = 0; ok && it < max_refine; ++it) {
-        const float step = lm_refine<FP64>(s, X, X2, v, n, team);
+        const float step = lm_refine<FP64>(s, X, X2, v, n, sparse, team);
         cx<float> *t = X;
         X = X2;
         X2 = t;
@@ -747,6 +873,7 @@ __global__ void __maxnreg__(128)
     if (FP64) {
         cx<double> *H = reinterpret_cast<cx<double> *>(s.H), *X64 = reinterpret_cast<cx<double> *>(s.Y);
         if (ok) {
+            if (tid == 0) v.scal[3] = 0;  // read before the first step
             for (int j = tid; j < n; j += nt) v.lam0[j] = dw_to_double(v.lam[j]);
             const double bx = a.field[3 * g], by = a.field[3 * g + 1], bz = a.field[3 * g + 2];
             for (int x = me; x < nn; x += all) {
@@ -763,9 +890,10 @@ __global__ void __maxnreg__(128)
                 H[(size_t)j * n + i] = conj(h);
             }
             team.sync();
+            sparse = lm_compact(H, n, v.scal + 3, team);
             ok = false;
             for (int it = 0; it < 3; ++it) {
-                const float step = lm_step64(H, X64, X, s.R, X2, s.Xl, v, n, team);
+                const float step = lm_step64(H, X64, X, s.R, X2, s.Xl, v, n, sparse, team);
                 if (!(step < 1e-2f)) break;
                 if (step <= 2e-8f) {
                     ok = true;
