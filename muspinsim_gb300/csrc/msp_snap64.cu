@@ -12,7 +12,7 @@
 //   2. their double-word refinement (oa_refine): eigenvalues to ~2^-48,
 //      vectors to ~1e-12, kept as hi + lo FP32;
 //   3. one FP64 step.  With x_j the vectors and l_j the levels from 2:
-//        r_j = H x_j - l_j x_j                (FP64, 4 n^3 FMAs),
+//        r_j = H x_j - l_j x_j                (FP64, 4 n FMAs per nonzero entry of H),
 //        d_j = x_j^H r_j / x_j^H x_j          (level correction),
 //        E_ij = x_i^H r_j / (l_j - l_i),  E_jj = (1 - x_j^H x_j) / 2,
 //        x_j += sum_i x_i E_ij.
@@ -25,8 +25,10 @@
 //   The step is repeated while its largest E exceeds 4e-9 (its error is of
 //   order E^2).  A snapshot that does not get there (entries outside the FP32
 //   range, no convergence in stage 1) takes the FP64 Jacobi (msp_jacobi.cuh).
-// 4 n^3 + the eigenbasis products (2 n^3) are all the FP64 pipe sees: 83 k
-// FMAs at n = 24.
+// That and the eigenbasis product (n^3 FMAs) are nearly all that the FP64 pipe sees:
+// 44 k FMAs for a molecule of n = 24, 83 k with the zeros of H and with the
+// product over all n rows.  Powder of n = 24 (10,000): 3.91 -> 3.43 ms in all; scan of
+// n = 12 (14,544): 1.63 -> 1.54 ms.
 #include "msp_refine.cuh"
 
 namespace msp {
@@ -41,7 +43,7 @@ namespace {
 // entries after: D1 over the FP32 matrix and vectors, D0 next, D2 last, so
 // that D0 can be filled from the FP32 vectors in place.
 struct Snap64Layout {
-    size_t lam0, lam, gn, tdiag, red, acc, dl, corr, rk, ord, cst, scal, fac;
+    size_t lam0, lam, gn, tdiag, nz, red, acc, dl, corr, rk, ord, cst, scal, fac;
     size_t region, xl, total;
 };
 
@@ -55,6 +57,7 @@ __host__ __device__ inline Snap64Layout snap64_layout(int n, int fac_len, int nw
     L.lam = lay_take(off, m * 8);
     L.gn = lay_take(off, m * 8);
     L.tdiag = lay_take(off, m * 8);
+    L.nz = lay_take(off, m * 8);
     L.red = lay_take(off, 2 * (size_t)nwarps * 8);
     L.acc = lay_take(off, 16);
     L.dl = lay_take(off, m * 4);
@@ -86,6 +89,7 @@ __host__ __device__ inline Snap64Layout snap64_layout(int n, int fac_len, int nw
 struct S64 {
     cx<double> *D0, *D1, *D2;
     double *lam0, *lam, *gn, *tdiag, *red, *acc;
+    unsigned long long *nz;  // bit k of row i: H_ik is not zero
     float *dl, *corr;
     int *rk, *ord, *cst, *scal;
     cx<double> *fac;
@@ -101,6 +105,7 @@ __device__ __forceinline__ S64 carve64(char *base, int n, int fac_len) {
     s.lam = reinterpret_cast<double *>(base + L.lam);
     s.gn = reinterpret_cast<double *>(base + L.gn);
     s.tdiag = reinterpret_cast<double *>(base + L.tdiag);
+    s.nz = reinterpret_cast<unsigned long long *>(base + L.nz);
     s.red = reinterpret_cast<double *>(base + L.red);
     s.acc = reinterpret_cast<double *>(base + L.acc);
     s.dl = reinterpret_cast<float *>(base + L.dl);
@@ -167,13 +172,27 @@ __device__ float step64(S64 &s, const HSource &h, int n, int m) {
         XF[e] = mk<float>((float)x.re, (float)x.im);
     }
     __syncthreads();
-    // r = H x - l x
+    for (int i = tid >> 5; i < n; i += nt >> 5) {
+        const int lane = tid & 31;
+        unsigned w[2];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int k = 32 * q + lane;
+            const cx<double> a = H[i * ld + (k < n ? k : 0)];
+            w[q] = __ballot_sync(0xffffffffu, k < n && !(a.re == 0.0 && a.im == 0.0));  // a NaN counts
+        }
+        if (lane == 0) s.nz[i] = (unsigned long long)w[1] << 32 | w[0];
+    }
+    __syncthreads();
+    // r = H x - l x over the nonzero entries of H: a spin Hamiltonian in the product
+    // basis is sparse (13 of 24 entries a row with two nuclei, an electron and a
+    // muon), and the FP64 pipe is the bound
     for (int e = tid; e < n * n; e += nt) {
         const int i = FastDiv(n).div(e), j = e - i * n;
         const cx<double> *row = H + i * ld, *col = X + j;
         double r0 = 0.0, r1 = 0.0, i0 = 0.0, i1 = 0.0;
-#pragma unroll 4
-        for (int k = 0; k < n; ++k) {
+        for (unsigned long long w = s.nz[i]; w != 0; w &= w - 1) {
+            const int k = __ffsll((long long)w) - 1;
             const cx<double> a = row[k], x = col[k * ld];
             r0 = fma(a.re, x.re, r0);
             r1 = fma(-a.im, x.im, r1);
@@ -492,6 +511,53 @@ __device__ __forceinline__ int snapshot64(const SnapArgs &a, const SnapSource &s
     return eigenpairs64(n, fac_len, h, st, a.max_sweeps, !PRE);
 }
 
+// sigma_p = p . sigma = 2 w w^H / |w|^2 |p| - |p| with w its eigenvector of +|p|,
+// (|p| + p_z, p_x + i p_y) or, p_z < 0, (p_x - i p_y, |p| - p_z); |w|^2 = 2 |p| (|p| +
+// |p_z|).  With V = w^H on the muon digit of U, the d = n / 2 rows of the other
+// digits, U^dag (sigma_p (x) 1) U is V^H V / (|p| + |p_z|) - |p| 1, because U is
+// unitary to FP64: half the FP64 FMAs of the product with U.
+struct MuonAxis {
+    double norm, inv;  // |p|, 1 / (|p| + |p_z|) (0 for p = 0, where sigma_p is too)
+};
+
+// One thread's work (a square root and a division in FP64).
+__device__ __forceinline__ MuonAxis muon_axis(const double *p) {
+    MuonAxis x;
+    x.norm = sqrt(p[0] * p[0] + p[1] * p[1] + p[2] * p[2]);
+    x.inv = x.norm == 0.0 ? 0.0 : 1.0 / (x.norm + fabs(p[2]));
+    return x;
+}
+
+// V (d x n, row stride ld) from U; `stride` is the muon digit's.  The caller
+// follows with a barrier.
+__device__ __forceinline__ void muon_project(const double *p, double norm, const cx<double> *U,
+                                             cx<double> *V, int n, int ld, int stride) {
+    const double px = p[0], py = p[1], pz = p[2];
+    const bool up = pz >= 0.0;
+    const double c = norm + fabs(pz);
+    for (int e = threadIdx.x; e < n / 2 * n; e += blockDim.x) {
+        const int i = FastDiv(n).div(e), k = e - i * n;
+        const int hi = i / stride, base = (i + hi * stride) * ld + k;  // muon digit 0
+        const cx<double> u0 = U[base], u1 = U[base + stride * ld];
+        V[i * ld + k] = up ? cadd(cscale(c, u0), cmul(mk<double>(px, -py), u1))
+                           : cadd(cmul(mk<double>(px, py), u0), cscale(c, u1));
+    }
+}
+
+// (V^H V)_jk
+__device__ __forceinline__ cx<double> muon_product(const cx<double> *V, int n, int ld, int j, int k) {
+    double g0 = 0.0, g1 = 0.0, h0 = 0.0, h1 = 0.0;
+#pragma unroll 4
+    for (int i = 0; i < n / 2; ++i) {
+        const cx<double> a = V[i * ld + j], b = V[i * ld + k];
+        g0 = fma(a.re, b.re, g0);
+        g1 = fma(a.im, b.im, g1);
+        h0 = fma(a.re, b.im, h0);
+        h1 = fma(-a.im, b.re, h1);
+    }
+    return mk<double>(g0 + g1, h0 + h1);
+}
+
 // Sum of every thread's v (all threads get it); begins with a barrier.
 __device__ __forceinline__ double block_sum64(double v, double *red) {
     double z = 0.0;
@@ -512,37 +578,23 @@ __global__ void __maxnreg__(80) msp_snap64_fast_kernel(SnapArgs a) {
     const int tid = threadIdx.x, nt = blockDim.x;
     const int P = n * (n - 1) / 2, ntri = n * (n + 1) / 2;
     double2 *coef = reinterpret_cast<double2 *>(a.pair_coef);
+    __shared__ MuonAxis axis;
     for (int sn = blockIdx.x; sn < a.num_snap; sn += gridDim.x) {
         const SnapSource src = snap_source(a, sn);
         const size_t g = (size_t)src.g;
+        if (tid == nt - 1) axis = muon_axis(a.pol + 3 * g);  // read many barriers later
         const int st = snapshot64<PRE>(a, src, sn, s, n, m, 0);
-        // sigma_p = p . sigma (Pauli), applied on the muon (slowest) digit
-        const double px = a.pol[3 * g], py = a.pol[3 * g + 1], pz = a.pol[3 * g + 2];
-        const cx<double> s01 = mk<double>(px, -py), s10 = mk<double>(px, py);
-        const cx<double> *U = s.D0;
-        cx<double> *M = s.D1;
-        for (int e = tid; e < d * n; e += nt) {
-            const int i = FastDiv(n).div(e), k = e - i * n;
-            const cx<double> u0 = U[i * ld + k], u1 = U[(i + d) * ld + k];
-            M[i * ld + k] = cadd(cscale(pz, u0), cmul(s01, u1));
-            M[(i + d) * ld + k] = cadd(cmul(s10, u0), cscale(-pz, u1));
-        }
+        // sigma_p = p . sigma (Pauli) on the muon (slowest) digit
+        cx<double> *V = s.D1;
+        muon_project(a.pol + 3 * g, axis.norm, s.D0, V, n, ld, d);
         __syncthreads();
-        const double scale = 0.5 * a.wscale[g] / (double)d;
+        const double scale = 0.5 * a.wscale[g] / (double)d, inv = axis.inv, norm = axis.norm;
         double diag = 0.0;
         for (int e = tid; e < ntri; e += nt) {
             int j, k;
             tri_index(e, j, k);
-            double g0 = 0.0, g1 = 0.0, h0 = 0.0, h1 = 0.0;
-#pragma unroll 4
-            for (int i = 0; i < n; ++i) {
-                const cx<double> u = U[i * ld + j], mm = M[i * ld + k];
-                g0 = fma(u.re, mm.re, g0);
-                g1 = fma(u.im, mm.im, g1);
-                h0 = fma(u.re, mm.im, h0);
-                h1 = fma(-u.im, mm.re, h1);
-            }
-            const double gr = g0 + g1, gi = h0 + h1;
+            const cx<double> G = muon_product(V, n, ld, j, k);
+            const double gr = fma(inv, G.re, j == k ? -norm : 0.0), gi = inv * G.im;
             const double A = gr * gr + gi * gi;
             if (j == k) {
                 diag += A;
@@ -575,9 +627,15 @@ __global__ void __maxnreg__(96) msp_snap64_rho_kernel(SnapArgs a) {
     const int tid = threadIdx.x, nt = blockDim.x;
     const int P = n * (n - 1) / 2, ntri = n * (n + 1) / 2;
     double2 *coef = reinterpret_cast<double2 *>(a.pair_coef);
-    const double twopi = 6.283185307179586476925;
+    const double twopi = 6.283185307179586476925, inv_tau = INTEGRAL ? 1.0 / a.tau : 0.0;
+    __shared__ MuonAxis axis;
+    __shared__ double axis_hot;
     for (int sn = blockIdx.x; sn < a.num_snap; sn += gridDim.x) {
         const bool hot = rho_is_hot(a, sn);
+        if (tid == nt - 1) {  // read many barriers later
+            axis = muon_axis(a.pol + 3 * (size_t)sn);
+            axis_hot = axis.norm > 0.0 ? 2.0 / (axis.norm * n) : 0.0;  // rho_hot_scale
+        }
         if (a.rho_fac) {
             for (int e = tid; e < a.fac_len; e += nt)
                 s.fac[e] = a.rho_fac[(size_t)sn * a.fac_len + e];
@@ -610,39 +668,18 @@ __global__ void __maxnreg__(96) msp_snap64_rho_kernel(SnapArgs a) {
             tri_conj_products<double, 0>(U, X, Y, n);
             __syncthreads();
         }
-        // O U into the buffer X (free now): O = sum_a p_a S^a on the muon digit
-        cx<double> *OU = const_cast<cx<double> *>(X);
-        {
-            const double px = a.pol[3 * (size_t)sn], py = a.pol[3 * (size_t)sn + 1],
-                         pz = a.pol[3 * (size_t)sn + 2];
-            const int stride = a.strides[a.mu_index];
-            const cx<double> o01 = mk<double>(0.5 * px, -0.5 * py), o10 = mk<double>(0.5 * px, 0.5 * py);
-            for (int e = tid; e < n * n; e += nt) {
-                const int i = FastDiv(n).div(e), k = e - i * n;
-                const int di = (i / stride) & 1;
-                const int base = i - di * stride;
-                const cx<double> x0 = U[base * ld + k], x1 = U[(base + stride) * ld + k];
-                OU[i * ld + k] = di == 0 ? cadd(cscale(0.5 * pz, x0), cmul(o01, x1))
-                                        : cadd(cmul(o10, x0), cscale(-0.5 * pz, x1));
-            }
-        }
+        // O = p . S on the muon digit: half of sigma_p.  V into the buffer X (free now)
+        cx<double> *V = const_cast<cx<double> *>(X);
+        muon_project(a.pol + 3 * (size_t)sn, axis.norm, U, V, n, ld, a.strides[a.mu_index]);
         __syncthreads();
-        const double scale = a.wscale[sn], hs = hot ? rho_hot_scale(a, sn) : 0.0;
+        const double scale = a.wscale[sn], hs = axis_hot, inv = 0.5 * axis.inv, norm = 0.5 * axis.norm;
         double local = 0.0;
         for (int e = tid; e < ntri; e += nt) {
             int j, k;
             tri_index(e, j, k);
-            // O'_kj = sum_i conj(U_ik) (O U)_ij
-            double g0 = 0.0, g1 = 0.0, h0 = 0.0, h1 = 0.0;
-#pragma unroll 4
-            for (int i = 0; i < n; ++i) {
-                const cx<double> u = U[i * ld + k], x = OU[i * ld + j];
-                g0 = fma(u.re, x.re, g0);
-                g1 = fma(u.im, x.im, g1);
-                h0 = fma(u.re, x.im, h0);
-                h1 = fma(-u.im, x.re, h1);
-            }
-            const double orr = g0 + g1, oii = h0 + h1;
+            // O'_kj
+            const cx<double> G = muon_product(V, n, ld, k, j);
+            const double orr = fma(inv, G.re, j == k ? -norm : 0.0), oii = inv * G.im;
             // rho'_jk, at T = inf from O'_jk
             const cx<double> r = hot ? mk<double>(fma(hs, orr, j == k ? 1.0 / n : 0.0), -hs * oii)
                                      : Y[j * ld + k];
@@ -650,7 +687,6 @@ __global__ void __maxnreg__(96) msp_snap64_rho_kernel(SnapArgs a) {
             const double cr = r.re * orr - r.im * oii, ci = r.re * oii + r.im * orr;
             if (INTEGRAL) {
                 // term = C_jk (-1) / (2 pi i (l_k - l_j) - 1/tau); pairs count twice
-                const double inv_tau = 1.0 / a.tau;
                 if (j == k) {
                     local += cr * a.tau;
                 } else {
