@@ -6,6 +6,13 @@
 
 namespace msp {
 
+// The FP32 reductions form a column's reflector from the squares of its entries.
+// Where their sum is below REFLECT_TINY (a decoupled block leaves columns that are
+// rounding errors of rounding errors) some have underflowed: the column is
+// scaled by REFLECT_UP (exactly) first, and one that is still below is taken as
+// zero.
+constexpr float REFLECT_TINY = 1e-28f, REFLECT_UP = 1152921504606846976.f;  // 2^60
+
 template <typename T>
 struct PairCoef;
 template <>

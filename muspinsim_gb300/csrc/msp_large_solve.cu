@@ -122,15 +122,27 @@ __global__ void __launch_bounds__(512)
         }
         if (k + 1 >= n) break;
         xn2 = warp_sum(xn2);
+        float up = 1.f;
+        if (alpha.re * alpha.re + alpha.im * alpha.im + xn2 < REFLECT_TINY) {
+            up = REFLECT_UP;
+            alpha = cscale(up, alpha);
+            xn2 = 0.f;
+#pragma unroll
+            for (int q = 0; q < Q; ++q)
+                if (32 * q + lane > k + 1) xn2 += cabs2(cscale(up, vn[q]));
+            xn2 = warp_sum(xn2);
+            if (cabs2(alpha) + xn2 < REFLECT_TINY) xn2 = alpha.im = 0.f;
+        }
         float beta = alpha.re;
         cx<float> tau = zero, sc = zero;
         if (!(xn2 == 0.f && alpha.im == 0.f)) {
             beta = -copysignf(sqrtf(alpha.re * alpha.re + alpha.im * alpha.im + xn2), alpha.re);
             tau = mk<float>((beta - alpha.re) / beta, -alpha.im / beta);
             const cx<float> den = mk<float>(alpha.re - beta, alpha.im);
-            const float dd = 1.f / cabs2(den);
+            const float dd = up / cabs2(den);
             sc = mk<float>(den.re * dd, -den.im * dd);
         }
+        if (up != 1.f) beta *= 1.f / REFLECT_UP;
 #pragma unroll
         for (int q = 0; q < Q; ++q) {
             const int i = 32 * q + lane;
@@ -282,7 +294,18 @@ __global__ void __maxnreg__(96)
             float xn2 = 0.f;
             for (int i = 1 + tid; i < m; i += nt) xn2 += cabs2(A[(size_t)(k + 1 + i) * n + k]);
             xn2 = block_sum(xn2, sm.red);
-            const cx<float> alpha = A[(size_t)(k + 1) * n + k];
+            cx<float> alpha = A[(size_t)(k + 1) * n + k];
+            float up = 1.f;
+            if (alpha.re * alpha.re + alpha.im * alpha.im + xn2 < REFLECT_TINY) {
+                up = REFLECT_UP;
+                alpha = cscale(up, alpha);
+                xn2 = 0.f;
+                for (int i = 1 + tid; i < m; i += nt)
+                    xn2 += cabs2(cscale(up, A[(size_t)(k + 1 + i) * n + k]));
+                __syncthreads();  // sm.red again
+                xn2 = block_sum(xn2, sm.red);
+                if (cabs2(alpha) + xn2 < REFLECT_TINY) xn2 = alpha.im = 0.f;
+            }
             cx<float> tau = mk<float>(0.f, 0.f);
             float beta = alpha.re;
             const bool reflect = !(xn2 == 0.f && alpha.im == 0.f);
@@ -290,13 +313,14 @@ __global__ void __maxnreg__(96)
                 beta = -copysignf(sqrtf(alpha.re * alpha.re + alpha.im * alpha.im + xn2), alpha.re);
                 tau = mk<float>((beta - alpha.re) / beta, -alpha.im / beta);
                 const cx<float> den = mk<float>(alpha.re - beta, alpha.im);
-                const float dd = 1.f / cabs2(den);
+                const float dd = up / cabs2(den);
                 const cx<float> sc = mk<float>(den.re * dd, -den.im * dd);
                 for (int i = tid; i < m; i += nt)
                     v[i] = i == 0 ? mk<float>(1.f, 0.f) : cmul(A[(size_t)(k + 1 + i) * n + k], sc);
             } else {
                 for (int i = tid; i < m; i += nt) v[i] = mk<float>(0.f, 0.f);  // V and W columns stay 0
             }
+            if (up != 1.f) beta *= 1.f / REFLECT_UP;
             if (tid == 0) {
                 s.d[k] = A[(size_t)k * n + k].re;
                 s.e[k] = beta;

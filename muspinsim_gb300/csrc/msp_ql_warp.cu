@@ -108,10 +108,20 @@ __global__ void __launch_bounds__(TRI_WARPS * 32) msp_tri_warp_kernel(SnapArgs a
         const bool below = lane > k && lane < n;
         const cx<float> x = below ? r[0] : mk<float>(0.f, 0.f);
         const float dk = __shfl_sync(FULL, r[0].re, k, LN);
-        const float xn2 = lanes_sum<LN>(lane > k + 1 ? cabs2(x) : 0.f);
-        const cx<float> alpha =
+        float xn2 = lanes_sum<LN>(lane > k + 1 ? cabs2(x) : 0.f);
+        cx<float> alpha =
             mk<float>(__shfl_sync(FULL, x.re, k + 1, LN), __shfl_sync(FULL, x.im, k + 1, LN));
-        const float s2 = fmaf(alpha.re, alpha.re, fmaf(alpha.im, alpha.im, xn2));
+        float s2 = fmaf(alpha.re, alpha.re, fmaf(alpha.im, alpha.im, xn2)), up = 1.f;
+        if (__any_sync(FULL, s2 < REFLECT_TINY)) {
+            const float u2 = lanes_sum<LN>(lane > k + 1 ? cabs2(cscale(REFLECT_UP, x)) : 0.f);
+            if (s2 < REFLECT_TINY) {
+                up = REFLECT_UP;
+                alpha = cscale(up, alpha);
+                xn2 = u2;
+                s2 = cabs2(alpha) + xn2;
+                if (s2 < REFLECT_TINY) xn2 = alpha.im = 0.f;
+            }
+        }
         float beta = alpha.re;
         cx<float> tau = mk<float>(0.f, 0.f), sc = tau;
         if (xn2 != 0.f || alpha.im != 0.f) {
@@ -127,9 +137,10 @@ __global__ void __launch_bounds__(TRI_WARPS * 32) msp_tri_warp_kernel(SnapArgs a
             inv = -copysignf(inv, alpha.re);
             tau = mk<float>(1.f - alpha.re * inv, -alpha.im * inv);
             const cx<float> den = mk<float>(alpha.re - beta, alpha.im);
-            const float dd = 1.f / cabs2(den);
+            const float dd = up / cabs2(den);
             sc = mk<float>(den.re * dd, -den.im * dd);
         }
+        if (up != 1.f) beta *= 1.f / REFLECT_UP;
         const cx<float> v = lane == k + 1 ? mk<float>(1.f, 0.f) : cmul(x, sc);
         {
             float2 o = make_float2(v.re, v.im);
