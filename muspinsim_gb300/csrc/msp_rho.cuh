@@ -113,6 +113,23 @@ __device__ __forceinline__ double rho_hot_scale(const SnapArgs &a, int s) {
     return pn > 0.0 ? 2.0 / (pn * a.n) : 0.0;
 }
 
+// sigma_p = p . sigma = 2 w w^H / |w|^2 |p| - |p| with w its eigenvector of +|p|,
+// (|p| + p_z, p_x + i p_y) or, p_z < 0, (p_x - i p_y, |p| - p_z); |w|^2 = 2 |p| (|p| +
+// |p_z|).  With V = w^H on the muon digit of U, the d = n / 2 rows of the other
+// digits, U^dag (sigma_p (x) 1) U is V^H V / (|p| + |p_z|) - |p| 1, because U is
+// unitary to FP64: half the FP64 FMAs of the product with U.
+struct MuonAxis {
+    double norm, inv;  // |p|, 1 / (|p| + |p_z|) (0 for p = 0, where sigma_p is too)
+};
+
+// One thread's work (a square root and a division in FP64).
+__device__ __forceinline__ MuonAxis muon_axis(const double *p) {
+    MuonAxis x;
+    x.norm = sqrt(p[0] * p[0] + p[1] * p[1] + p[2] * p[2]);
+    x.inv = x.norm == 0.0 ? 0.0 : 1.0 / (x.norm + fabs(p[2]));
+    return x;
+}
+
 // Kronecker factors of rho0 for snapshot s (muspinsim/experiment.py:170-236):
 // the muon in the pure +1/2 state along its polarisation, every other spin
 // thermal in its own Zeeman field gamma_i B (uniform at T = inf, ground
