@@ -298,13 +298,12 @@ __device__ void load_hamiltonian(const cx<double> *Hsys, const cx<double> *Z, co
 
 // The eigensolve of a snapshot: FP64 or FP32 Jacobi in this CTA, or (PRE)
 // the FP32 eigenvectors the warp Jacobi stage left in a.evec, with the
-// status it wrote.  Leaves the eigenvectors in s.w.U (row stride m + 1).
+// status it wrote.  Leaves the eigenvectors in s.w.U (row stride ld; m + 1 after Jacobi).
 template <typename T, bool PRE>
-__device__ __forceinline__ int snap_eigvecs(const SnapArgs &a, int sn, int g, int n, int m,
+__device__ __forceinline__ int snap_eigvecs(const SnapArgs &a, int sn, int g, int n, int m, int ld,
                                             SnapSmem<T> &s) {
     if (!PRE) return jacobi_sweeps<T>(s.w, m, a.max_sweeps);
     const float2 *X = reinterpret_cast<const float2 *>(a.evec) + (size_t)sn * n * n;
-    const int ld = m + 1;
     for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
         const int i = FastDiv(n).div(e), j = e - i * n;
         const float2 x = X[e];
@@ -478,12 +477,11 @@ __device__ float oa_refine(SnapSmem<float> &s, int n_rt, int m_rt, cx<float> *Xl
 }
 
 // Applies the single-spin matrix F (dim x dim, complex FP64 or FP32) on
-// digit `stride` of the row index of X (n x n, leading dim m) into Y:
+// digit `stride` of the row index of X (n x n, row stride ld) into Y:
 // Y = (1 (x) F (x) 1) X.
 template <typename T, typename TF>
 __device__ void apply_digit(const cx<TF> *F, int dim, int stride, const cx<T> *X, cx<T> *Y, int n,
-                            int m) {
-    const int ld = m + 1;
+                            int ld) {
     for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
         const int i = FastDiv(n).div(e), k = e - i * n;
         const int di = (i / stride) % dim;
@@ -563,6 +561,8 @@ __host__ __device__ inline RowShape row_shape(int n, int threads) {
     RowShape s;
     s.groups = threads / n < n ? threads / n : n;
     s.rows = (n + s.groups - 1) / s.groups;
+    s.rows += s.rows & 1;  // pairs of rows start on 16 bytes
+    s.groups = (n + s.rows - 1) / s.rows;
     s.padded = (s.groups - 1) * s.rows + ROW_MAX;
     if (s.padded < n) s.padded = n;
     return s;
@@ -571,6 +571,11 @@ __host__ __device__ inline RowShape row_shape(int n, int threads) {
 // At most four rows per thread.  (Eight, in half the threads, spill at 96
 // registers and leave too few warps at 128: scan of n = 32, 27 ms against 22.)
 inline int row_threads(int n) { return n <= 8 ? 32 : n <= 16 ? 64 : n <= 24 ? 160 : 256; }
+
+// Row stride of the FP32 matrices: even, so that two elements of a row operand are
+// one 16-byte load (the plain products are bound by shared-memory loads: scan of n = 32
+// 29.9 -> 29.5 ms in all, powder of n = 24 1.17 -> 1.15).
+__host__ __device__ constexpr int row_ld(int n) { return n + (n & 1) + 2; }
 
 // Row stride of H4: odd, for the transposed stores
 __host__ __device__ inline int row_ldh(int n) { return n | 1; }
@@ -581,7 +586,7 @@ struct RowLayout {
 
 __host__ __device__ inline RowLayout row_layout(int n, bool rho, int fac_len, int threads) {
     RowLayout L;
-    const size_t m = (size_t)(n + (n & 1)), mm = (size_t)row_shape(n, threads).padded * (m + 1) * 8;
+    const size_t m = (size_t)(n + (n & 1)), mm = (size_t)row_shape(n, threads).padded * row_ld(n) * 8;
     size_t off = 0;
     L.H4 = lay_take(off, (size_t)row_shape(n, threads).padded * row_ldh(n) * 16);
     L.U = lay_take(off, mm);
@@ -690,7 +695,8 @@ __device__ __forceinline__ cx<float> row_gram(const cx<float> *X, int n, int ld,
 template <int NN, int RB>
 __device__ __forceinline__ void row_products(const cx<float> *X, const cx<float> *W, int n_rt, int i1,
                                              int j, cx<float> (&b)[RB]) {
-    const int n = NN > 0 ? NN : n_rt, ld = n + (n & 1) + 1;
+    static_assert(RB == 4, "two pairs of rows");
+    const int n = NN > 0 ? NN : n_rt, ld = row_ld(n);
     u64 s1[RB], s2[RB];
 #pragma unroll
     for (int r = 0; r < RB; ++r) s1[r] = s2[r] = 0ull;
@@ -698,7 +704,9 @@ __device__ __forceinline__ void row_products(const cx<float> *X, const cx<float>
     for (int k = 0; k < n; ++k) {
         const cx<float> q = W[k * ld + j];
         const u64 bx = f32x2(q.re, q.re), by = f32x2(q.im, q.im);
-        const u64 *x = reinterpret_cast<const u64 *>(X + k * ld + i1);
+        const ulonglong2 xa = *reinterpret_cast<const ulonglong2 *>(X + k * ld + i1),
+                         xb = *reinterpret_cast<const ulonglong2 *>(X + k * ld + i1 + 2);
+        const u64 x[RB] = {xa.x, xa.y, xb.x, xb.y};
 #pragma unroll
         for (int r = 0; r < RB; ++r) {
             s1[r] = fma_f32x2(x[r], bx, s1[r]);
@@ -709,11 +717,44 @@ __device__ __forceinline__ void row_products(const cx<float> *X, const cx<float>
     for (int r = 0; r < RB; ++r) b[r] = lm_plain<true>(s1[r], s2[r]);
 }
 
+// s1, s2 += this thread's rows of A E, column j
+template <int NN, int RB>
+__device__ __forceinline__ void row_times(const cx<float> *A, const cx<float> *E, int n_rt, int i1, int j,
+                                          u64 (&s1)[RB], u64 (&s2)[RB]) {
+    const int n = NN > 0 ? NN : n_rt, ld = row_ld(n);
+    if constexpr (NN > 0 && NN % 2 == 0) {
+#pragma unroll 4
+        for (int i = 0; i < n; i += 2) {
+            const cx<float> e = E[i * ld + j], f = E[(i + 1) * ld + j];
+            const u64 ex = f32x2(e.re, e.re), ey = f32x2(e.im, e.im);
+            const u64 fx = f32x2(f.re, f.re), fy = f32x2(f.im, f.im);
+#pragma unroll
+            for (int r = 0; r < RB; ++r) {
+                const ulonglong2 x = *reinterpret_cast<const ulonglong2 *>(A + (i1 + r) * ld + i);
+                s1[r] = fma_f32x2(x.y, fx, fma_f32x2(x.x, ex, s1[r]));
+                s2[r] = fma_f32x2(x.y, fy, fma_f32x2(x.x, ey, s2[r]));
+            }
+        }
+    } else {
+#pragma unroll 8
+        for (int i = 0; i < n; ++i) {
+            const cx<float> e = E[i * ld + j];
+            const u64 bx = f32x2(e.re, e.re), by = f32x2(e.im, e.im);
+#pragma unroll
+            for (int r = 0; r < RB; ++r) {
+                const u64 x = *reinterpret_cast<const u64 *>(A + (i1 + r) * ld + i);
+                s1[r] = fma_f32x2(x, bx, s1[r]);
+                s2[r] = fma_f32x2(x, by, s2[r]);
+            }
+        }
+    }
+}
+
 // One refinement step by rows: the vectors in s.w.U, the levels in s.lw.
 // Returns its largest correction.  NN > 0: n = NN at compile time.
 template <int NN, int RB>
 __device__ __forceinline__ float oa_refine_rows(SnapSmem<float> &s, int n_rt) {
-    const int n = NN > 0 ? NN : n_rt, ld = n + (n & 1) + 1, tid = threadIdx.x;
+    const int n = NN > 0 ? NN : n_rt, ld = row_ld(n), tid = threadIdx.x;
     const RowShape sh = row_shape(n, blockDim.x);
     const int rg = tid / n, j = tid - rg * n, i0 = rg * sh.rows;
     // threads past the last group follow along on the first rows and store nothing
@@ -880,17 +921,7 @@ __device__ __forceinline__ float oa_refine_rows(SnapSmem<float> &s, int n_rt) {
             u64 s1[RB], s2[RB];
 #pragma unroll
             for (int r = 0; r < RB; ++r) s1[r] = s2[r] = 0ull;
-#pragma unroll 8
-            for (int k = 0; k < n; ++k) {
-                const cx<float> e = s.SR[k * ld + j];
-                const u64 bx = f32x2(e.re, e.re), by = f32x2(e.im, e.im);
-#pragma unroll
-                for (int r = 0; r < RB; ++r) {
-                    const u64 x = *reinterpret_cast<const u64 *>(R + (i1 + r) * ld + k);
-                    s1[r] = fma_f32x2(x, bx, s1[r]);
-                    s2[r] = fma_f32x2(x, by, s2[r]);
-                }
-            }
+            row_times<NN, RB>(R, s.SR, n, i1, j, s1, s2);
 #pragma unroll
             for (int r = 0; r < RB; ++r) q[r] = lm_plain<false>(s1[r], s2[r]);
         }
@@ -944,17 +975,7 @@ __device__ __forceinline__ float oa_refine_rows(SnapSmem<float> &s, int n_rt) {
             s1[r] = *reinterpret_cast<const u64 *>(X + (i1 + r) * ld + j);
             s2[r] = 0ull;
         }
-#pragma unroll 8
-        for (int i = 0; i < n; ++i) {
-            const cx<float> e = s.SR[i * ld + j];
-            const u64 bx = f32x2(e.re, e.re), by = f32x2(e.im, e.im);
-#pragma unroll
-            for (int r = 0; r < RB; ++r) {
-                const u64 x = *reinterpret_cast<const u64 *>(X + (i1 + r) * ld + i);
-                s1[r] = fma_f32x2(x, bx, s1[r]);
-                s2[r] = fma_f32x2(x, by, s2[r]);
-            }
-        }
+        row_times<NN, RB>(X, s.SR, n, i1, j, s1, s2);
         __syncthreads();
 #pragma unroll
         for (int r = 0; r < RB; ++r)

@@ -139,7 +139,7 @@ template <bool PRE>
 __global__ void __maxnreg__(64) msp_snap_fast_kernel(SnapArgs a) {
     typedef float T;
     extern __shared__ __align__(16) char smem[];
-    const int n = a.n, m = n + (n & 1), ld = m + 1, d = n / 2;
+    const int n = a.n, m = n + (n & 1), ld = PRE ? row_ld(n) : m + 1, d = n / 2;
     SnapSmem<T> s = PRE ? row_carve(smem, n, false, 0) : snap_carve<T, true>(smem, n, false, 0);
     const int tid = threadIdx.x, nt = blockDim.x;
 
@@ -151,7 +151,7 @@ __global__ void __maxnreg__(64) msp_snap_fast_kernel(SnapArgs a) {
         else
             load_hamiltonian<T, true, PRE>(src.Hsys, src.Z, src.Hdw, src.Zdw, a.field + 3 * g, n, m,
                                            s);
-        int st = snap_eigvecs<T, PRE>(a, sn, (int)g, n, m, s);
+        int st = snap_eigvecs<T, PRE>(a, sn, (int)g, n, m, ld, s);
         st |= PRE ? eigenpairs_rows(n, false, 0, a.max_refine) : eigenpairs(s, n, m, a.max_refine);
 
         // sigma_p = p . sigma (Pauli), applied on the muon (slowest) digit
@@ -226,7 +226,7 @@ __device__ __forceinline__ float2 rho_terms_mixed(const SnapArgs &a, const SnapS
                                                   const cx<float> *U, const cx<float> *OU,
                                                   const cx<float> *X, int n_rt, int sn, float tau_f,
                                                   float itau_f, bool hot, float hot_scale) {
-    const int n = NN > 0 ? NN : n_rt, ld = n + (n & 1) + 1;
+    const int n = NN > 0 ? NN : n_rt, ld = n + (n & 1) + 1;  // !ROWS
     const size_t rec = (size_t)sn * (n * (n - 1) / 2);
     const float scale2 = 2.0f * (float)a.wscale[sn];
     float2 local = make_float2(0.f, 0.f);
@@ -281,7 +281,7 @@ template <bool INTEGRAL, bool PRE>
 __global__ void __maxnreg__(PRE ? 64 : 96) msp_snap_rho_kernel(SnapArgs a) {
     typedef float T;
     extern __shared__ __align__(16) char smem[];
-    const int n = a.n, m = n + (n & 1), ld = m + 1;
+    const int n = a.n, m = n + (n & 1), ld = PRE ? row_ld(n) : m + 1;
     SnapSmem<T> s =
         PRE ? row_carve(smem, n, true, a.fac_len) : snap_carve<T, true>(smem, n, true, a.fac_len);
     const int tid = threadIdx.x, nt = blockDim.x;
@@ -307,7 +307,7 @@ __global__ void __maxnreg__(PRE ? 64 : 96) msp_snap_rho_kernel(SnapArgs a) {
         if (!hot)
             for (int e = tid; e < a.fac_len; e += nt)
                 s.facf[e] = mk<float>((float)s.fac[e].re, (float)s.fac[e].im);
-        int st = snap_eigvecs<T, PRE>(a, sn, sn, n, m, s);
+        int st = snap_eigvecs<T, PRE>(a, sn, sn, n, m, ld, s);
         st |= PRE ? eigenpairs_rows(n, true, a.fac_len, a.max_refine)
                   : eigenpairs(s, n, m, a.max_refine);
         const cx<T> *U = s.w.U;
@@ -321,7 +321,7 @@ __global__ void __maxnreg__(PRE ? 64 : 96) msp_snap_rho_kernel(SnapArgs a) {
             int off = 0;
             for (int sp = 0; sp < a.num_spins; ++sp) {
                 const int dim = a.dims[sp];
-                apply_digit<T>(s.facf + off, dim, a.strides[sp], X, Y, n, m);
+                apply_digit<T>(s.facf + off, dim, a.strides[sp], X, Y, n, ld);
                 off += dim * dim;
                 X = Y;
                 Y = (Y == s.w.H) ? s.B2 : s.w.H;

@@ -507,7 +507,7 @@ __device__ __forceinline__ int snapshot64(const SnapArgs &a, const SnapSource &s
     const HSource h = {src.Hsys, src.Z, a.field + 3 * (size_t)src.g};
     SnapSmem<float> f = snap_carve<float, true>(s.region, n, false, 0);
     load_hamiltonian<float, true, PRE>(src.Hsys, src.Z, src.Hdw, src.Zdw, h.b, n, m, f);
-    const int st = snap_eigvecs<float, PRE>(a, sn, src.g, n, m, f);
+    const int st = snap_eigvecs<float, PRE>(a, sn, src.g, n, m, m + 1, f);
     return eigenpairs64(n, fac_len, h, st, a.max_sweeps, !PRE);
 }
 
@@ -642,7 +642,7 @@ __global__ void __maxnreg__(96) msp_snap64_rho_kernel(SnapArgs a) {
             int off = 0;
             for (int sp = 0; sp < a.num_spins; ++sp) {
                 const int dim = a.dims[sp];
-                apply_digit<double>(s.fac + off, dim, a.strides[sp], X, Y, n, m);
+                apply_digit<double>(s.fac + off, dim, a.strides[sp], X, Y, n, ld);
                 off += dim * dim;
                 X = Y;
                 Y = (Y == s.D1) ? s.D2 : s.D1;
