@@ -481,38 +481,27 @@ def run_gb300(args, world, rank, local):
     samples = S * T
     value = world * samples / (t_mixed_max * 1e-3)
 
-    # roofline per stage (live CUDA-event stage times; each stage is one
-    # kernel on this path) and of the dominant one
+    # roofline per stage (live CUDA-event stage times) and of the dominant one
     per_run = {k: v / max(runs, 1) for k, v in stages.items()}
-    peaks = {}
-    try:
-        with open(os.path.join(ROOT, "MEASURED_PEAKS.json")) as f:
-            peaks = json.load(f)
-    except OSError:
-        pass
     fp32_peak = SMS * FP32_FMA_PER_SM * 2 * 2070e6 / 1e12
-    bf16 = peaks.get("bf16_tflops")
-    tf32_peak = (bf16 if bf16 else 1900.0) / 2.0  # dense TF32 runs at half the bf16 rate
-    tf32_src = ("measured bf16 burst / 2 (MEASURED_PEAKS.json)" if bf16
-                else "fallback 1.9 PF/s bf16 / 2")
     # algorithmic work per snapshot: eigensolve 36 n^3 (six Jacobi sweeps) or
     # 19 n^3 (Householder 16/3 n^3, QL rotations 6 n^3 at ~n^2 rotations,
-    # back-transformation 8 n^3), eigenbasis products 32 n^3; per time
-    # sample 4 n^2 + 2 (phase sum + accumulation)
+    # back-transformation 8 n^3), eigenbasis products 32 n^3.  The phase sum is a
+    # nonuniform Fourier transform: per pair ten grid cells of 15 operations; its
+    # transform (the "reduce" stage) 5 T log2 T for the one output row
     ql = S >= QL_MIN_SNAPSHOTS
     kernels_rl = {
-        "eigensolve": (("msp_ql_warp_kernel<24,4> (Householder + QL, four matrices a warp)"
+        "eigensolve": (("msp_tri_warp_kernel<24> + msp_ql_kernel<24> (Householder + QL)"
                         if ql else "msp_jacobi_warp_kernel<24>"),
                        (19.0 if ql else 36.0) * n**3 * S, "fp32-pipe", fp32_peak,
                        "nominal FP32 FMA pipe (152 x 128 x 2 x 2070 MHz)"),
-        "snapshots": ("msp_snap_fast_kernel<float,true,true> (refinement + amplitudes)",
+        "snapshots": ("msp_snap_fast_kernel<true> (refinement + amplitudes)",
                       32.0 * n**3 * S, "fp32-pipe", fp32_peak,
                       "nominal FP32 FMA pipe (152 x 128 x 2 x 2070 MHz)"),
-        "phase": ("msp_phase_tcw_kernel<32> (tcgen05 kind::tf32, 3xTF32, A in tensor memory, "
-                  "warp-specialised)",
-                  (4.0 * n * n) * samples, "tensor", tf32_peak, tf32_src),
-        "reduce": ("msp_reduce_kernel", 2.0 * samples, "fp32-pipe", fp32_peak,
-                   "nominal FP32 FMA pipe"),
+        "phase": ("msp_nufft_spread_kernel", 150.0 * S * n * (n - 1) / 2, "fp32-pipe", fp32_peak,
+                  "nominal FP32 FMA pipe; bound by shared-memory atomics"),
+        "reduce": ("msp_nufft_reduce_kernel + msp_nufft_dft1_kernel + msp_nufft_dft2_kernel",
+                   5.0 * T * float(np.log2(max(T, 2))), "latency", fp32_peak, "nominal FP32 FMA pipe"),
     }
     rl_all = {}
     for k, (kn, fl, bound, pk, src) in kernels_rl.items():
@@ -528,9 +517,9 @@ def run_gb300(args, world, rank, local):
         "metric": METRIC, "value": value, "unit": "samples/s", "n_gpus": world,
         "steps": args.steps, "warmup": args.warmup, "ms_per_step": t_mixed_max,
         "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-        "dtype": "f32 (Householder + QL eigensolve, 3xTF32 phase sum) + double-word f32 "
-                 "(refinement, eigenvalues, phase records, item reduction); f64 only in the "
-                 "final per-time sums",
+        "dtype": "f32 (Householder + QL eigensolve, amplitudes, window of the phase sum) + "
+                 "double-word f32 (refinement, eigenvalues, phase records); phase grid in 64-bit "
+                 "fixed point, its transform in f64",
         "data": "synthetic (seeded couplings, ZCW-style grid)",
         "config": {"workload": WORKLOAD, "orientations": S, "times": T, "dim": n,
                    "precision": "mixed", "l2": "flushed between timed steps (258 MB write)",
@@ -554,14 +543,14 @@ def run_gb300(args, world, rank, local):
                               "scaled per snapshot",
             "algorithmic": {"eigensolve": ("19 n^3" if ql else "36 n^3") + " per snapshot",
                             "snapshots": "32 n^3 per snapshot",
-                            "phase": "4 n^2 per sample", "reduce": "2 per sample"}[dom],
+                            "phase": "150 per pair", "reduce": "5 T log2 T"}[dom],
             "peak_source": src,
             "stages": rl_all,
         },
         "clocks": clk,
-        # double-word split of the system matrices, eigensolve, refinement,
-        # schedule, phase sum, reduction
-        "gpu_launches": 6 * args.steps,
+        # double-word split of the system matrices, reduction and QL, refinement,
+        # schedule, and the phase sum's tables, spread, reduction and two transforms
+        "gpu_launches": (10 if ql else 9) * args.steps,
     }
     if rank == 0 and world == 1 and not args.no_cpu_baseline:
         threads = os.cpu_count() or 1
