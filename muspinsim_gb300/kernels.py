@@ -440,15 +440,36 @@ class PowderPlan:
         self.status = torch.zeros((max(S, 1),), dtype=torch.int32, device=d)
         a.out = self.out.data_ptr()
         a.status = self.status.data_ptr()
+        self.args = a
+        self.ws = None
+        self._fit_workspace()
+
+    def _fit_workspace(self):
+        """Scratch for the arguments as they are now, reallocated when what is
+        there is too small."""
+        a = self.args
         nbytes = ctypes.c_size_t(0)
         _lib.check(_lib.load().msp_powder_workspace(ctypes.byref(a), ctypes.byref(nbytes)),
                    "msp_powder_workspace")
-        self.ws = torch.empty(int(nbytes.value) + 256, dtype=torch.uint8, device=d)
-        off = (-self.ws.data_ptr()) % 256
-        a.workspace = self.ws.data_ptr() + off
-        a.workspace_bytes = int(nbytes.value)
-        self.workspace_bytes = int(nbytes.value)
-        self.args = a
+        if self.ws is None or nbytes.value > self.workspace_bytes:
+            # freed before its successor is allocated; a run that comes after a
+            # failed allocation is refused
+            self.ws, self.workspace_bytes = None, 0
+            a.workspace, a.workspace_bytes = None, 0
+            self.ws = torch.empty(int(nbytes.value) + 256, dtype=torch.uint8, device=device())
+            self.workspace_bytes = int(nbytes.value)
+        a.workspace = self.ws.data_ptr() + (-self.ws.data_ptr()) % 256
+        a.workspace_bytes = self.workspace_bytes
+
+    def set_times(self, times):
+        """Move the plan to another time grid (host array) of the same length.
+        The scratch grows with it where the new grid's form of the phase sum
+        takes more (uniform, or not starting at 0)."""
+        a = self.args
+        uni, t0, dt = uniform_grid(times)
+        self.T.copy_(torch.as_tensor(times), non_blocking=False)
+        a.uniform, a.t0, a.dt = (1 if uni else 0), t0, dt
+        self._fit_workspace()
 
     def rebind(self, field, pol, wscale, slot):
         """Point the plan at new per-snapshot inputs of the same sizes (device

@@ -67,8 +67,9 @@ def _cached_plan(system, Hs, Zd, n, F, Pl, W, slot, num_slots, times, mode, prec
                  max_sweeps):
     """A PowderPlan for the device-side powder_average path, reused across
     calls with the same system matrices and sizes (its output, status and
-    workspace stay allocated; only the per-call inputs are re-pointed and
-    the time grid re-uploaded).  Only plans of the fast path are cached."""
+    workspace stay allocated, the workspace growing where a new grid needs
+    more; only the per-call inputs are re-pointed and the time grid
+    re-uploaded).  Only plans of the fast path are cached."""
     th = np.asarray(times, dtype=float)
     keep = mode == _lib.MODE_FAST
     key = (Hs.data_ptr(), Zd.data_ptr(), int(F.shape[0]), th.size, int(num_slots), mode, prec,
@@ -87,10 +88,8 @@ def _cached_plan(system, Hs, Zd, n, F, Pl, W, slot, num_slots, times, mode, prec
     plan.rebind(F, Pl, W, slot)
     last = getattr(plan, "_times_host", None)
     if last is None or not np.array_equal(last, th):  # the grid only moves when it changed
-        uni, t0, dt = kernels.uniform_grid(th)
-        plan.T.copy_(torch.as_tensor(th), non_blocking=False)
-        a = plan.args
-        a.uniform, a.t0, a.dt = (1 if uni else 0), t0, dt
+        plan._times_host = None
+        plan.set_times(th)
         plan._times_host = th.copy()
     return plan
 
