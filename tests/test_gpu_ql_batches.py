@@ -131,3 +131,21 @@ def test_ql_batch_alc_near_degenerate():
                                   _lib.MODE_INTEGRAL, tau=constants.MU_TAU)
     print("near-degenerate ALC slots |mixed - fp64|:", np.abs(mixed - fp64))
     assert np.abs(mixed - fp64).max() <= MIXED_TOL
+
+
+@pytest.mark.parametrize("n,S", [(8, 4000), (10, 3300), (24, 1400), (32, 1100)])
+def test_field_that_is_not_a_number_is_reported(n, S):
+    """Batches under 4,096 snapshots report it, whichever first stage they take."""
+    from muspinsim_gb300 import _lib, kernels
+    from tests.helpers import random_hermitian
+
+    rng = np.random.default_rng(n)
+    H, Z = random_hermitian(rng, n), np.array([random_hermitian(rng, n) for _ in range(3)])
+    B, p = 0.1 * rng.normal(size=(S, 3)), np.tile([0.0, 0.0, 1.0], (S, 1))
+    bad = [0, S // 2, S - 1]
+    B[bad] = np.nan
+    for prec in (_lib.PREC_MIXED, _lib.PREC_FP64):
+        _, st = kernels.powder_run(n, H, Z, B, p, np.ones(S), np.zeros(S, np.int32), 1,
+                                   np.linspace(0, 1, 8), precision=prec)
+        flagged = np.nonzero(st.cpu().numpy() & _lib.MSP_ITEM_NOT_CONVERGED)[0]
+        assert flagged.tolist() == bad
