@@ -613,8 +613,14 @@ __global__ void __launch_bounds__(CE_DW_THREADS) msp_celio_smem_dw_kernel(CeArgs
 // has an error of 2^-4 units (the dropped levels) before its rounding.  A group
 // is one column of an m16n8k16 MMA (U the 16 x 16 operand; smaller D: 16 / D
 // groups per column, U block-diagonal), 26 digit pairs x 4 real products per 8
-// columns.  The largest accumulator is tracked: one that reached 2^24, where
-// FP32 stops being exact, disqualifies the state.
+// columns.  A level sums up to twelve such products, more than FP32 holds exactly
+// if all their digits are large and aligned.  Top digits are not: a row of U and a
+// group of the state have norm 1, so their squares sum to 2^16 and a product with
+// them stays below 2^20 (Cauchy-Schwarz).  So levels 8 to 10 stay below 2^24
+// throughout, and level 7 does where it ends below FX_EXACT, for only products with a
+// top digit follow its others.  Levels 4 to 6 could round on the way up and come back:
+// 2^-53 of the norm at most.  A state with an accumulator that ends at FX_EXACT or
+// above is disqualified.
 //
 // Single-spin factors are first multiplied into a two-spin factor on the same
 // digit where only factors on other digits lie between (they commute), so
@@ -622,6 +628,7 @@ __global__ void __launch_bounds__(CE_DW_THREADS) msp_celio_smem_dw_kernel(CeArgs
 constexpr int FX_DIGITS = 6, FX_THREADS = 256;
 constexpr int FX_LOW = 4, FX_LEVELS = 2 * FX_DIGITS - 1 - FX_LOW;  // levels s + t >= 4
 constexpr int FX_FRAG = FX_DIGITS * 2 * 32;  // uint4 per factor: [digit][re, im][lane]
+constexpr float FX_EXACT = 16777216.f - 1048576.f;  // 2^24 - 2^20
 
 struct FxOp {
     long long mat;  // source matrix
@@ -955,7 +962,7 @@ __global__ void __launch_bounds__(FX_THREADS, 1) msp_celio_fx_kernel(FxArgs a) {
                     __syncthreads();
                 }
         }
-        if (xmax >= 16777216.f) s_bad = 1;  // an accumulator left the exact range
+        if (!(xmax < FX_EXACT)) s_bad = 1;  // an accumulator may have left the exact range
         __syncthreads();
         if (tid == 0) a.done[st] = s_bad ? 0 : 1;
         __syncthreads();

@@ -112,3 +112,62 @@ def test_density_form():
         for _ in range(3):
             for u in full:
                 rho = u.conj().T @ rho @ u
+
+
+def _digits_sum(d2, d3, d4, d5):
+    """Integers with the given balanced ten-bit digits, lowest two zero."""
+    return [sum(int(v) << 10 * s if v >= 0 else -(int(-v) << 10 * s)
+                for s, v in ((2, a), (3, b), (4, c), (5, d)))
+            for a, b, c, d in zip(d2, d3, d4, d5)]
+
+
+def _aligned_row_and_state():
+    """A unit row u and a state x (16 complex entries as 32 integers of 2^-58, real
+    parts first) whose digits 3 and 4 are all +-511 with the signs aligned: Re u . x
+    sums them to 1.04 x 2^24 before the products with the top digits take it back
+    below 2^24."""
+    rng = np.random.default_rng(0)
+    im = np.arange(32) >= 16
+    sx = rng.choice([-1, 1], 32)
+    x5 = sx * rng.integers(34, 42, 32)
+    u2 = 511 * sx * np.where(im, -1, 1)
+    u3 = np.full(32, -511)
+    u3[31] = -510  # an odd total
+    u4 = np.full(32, -511)
+    frac = u4 / 2**10 + u3 / 2**20 + u2 / 2**30
+    while True:
+        u5 = rng.choice([-1, 1], 32) * rng.integers(38, 52, 32)
+        # the last two entries give the sum and the sum of squares a unit row needs
+        A, B = 16 - u5[:30].sum(), 65544 - (u5[:30] ** 2).sum()
+        root = int(round(max(2 * B - A * A, 0) ** 0.5))
+        if root * root != 2 * B - A * A or (A + root) % 2:
+            continue
+        u5[30], u5[31] = (A + root) // 2, (A - root) // 2
+        if np.abs(((u5 + frac) ** 2).sum() / 65536 - 1) < 7e-10:
+            break
+    x2 = 511 * np.sign(u5) * np.where(im, 1, -1)
+    x3 = np.where(im, 511, -511)
+    return _digits_sum(u2, u3, u4, u5), _digits_sum(x2, x3, x3, x5)
+
+
+def test_aligned_digits():
+    """Digits that align beyond what an FP32 accumulator holds exactly: the state
+    goes to the FP64 kernel (an entry is a sum of 32 products of a unit row and a
+    state of norm below 1: 2^-48), it does not lose the 2^-46 that a rounded sum
+    would."""
+    u, x = _aligned_row_and_state()
+    rng = np.random.default_rng(1)
+    row = (np.array(u[:16], float) + 1j * np.array(u[16:], float)) * 2.0**-58
+    q = np.linalg.qr(np.concatenate([row[None], rng.normal(size=(15, 16)) + 0j]).conj().T)[0]
+    M = q.conj().T
+    M[0] = row
+    psi = (np.array(x[:16], float) + 1j * np.array(x[16:], float)) * 2.0**-58
+    pick = np.zeros((1, 16))
+    pick[0, 0] = 1.0
+    got, _ = kernels.celio_run(_lib.CELIO_DENSITY, [4, 4], [(0, 1)], [0], M.reshape(1, -1), False, 1,
+                               1, 1, 2, rho0=psi[None], meas=pick[None], path=1)
+    got = got.cpu().numpy()[0, 1, 0]
+    exact = (sum(a * b for a, b in zip(u[:16], x[:16])) - sum(a * b for a, b in zip(u[16:], x[16:])),
+             sum(a * b for a, b in zip(u[:16], x[16:])) + sum(a * b for a, b in zip(u[16:], x[:16])))
+    assert abs(got.real - exact[0] / 2**116) <= 2.0**-47.5
+    assert abs(got.imag - exact[1] / 2**116) <= 2.0**-47.5
