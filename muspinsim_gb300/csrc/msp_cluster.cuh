@@ -36,6 +36,8 @@
 // the clusters are disjoint diagonal blocks of one n x n buffer.
 #pragma once
 
+#include <string.h>
+
 #include "msp_dw.cuh"
 #include "msp_jacobi.cuh"
 
@@ -69,6 +71,27 @@ __device__ __forceinline__ long long oa_sort_key(float2 l) {
     const int h = __float_as_int(l.x), e = __float_as_int(l.y);
     const int hk = h < 0 ? h ^ 0x7fffffff : h, ek = e < 0 ? e ^ 0x7fffffff : e;
     return ((long long)hk << 32) | ((unsigned)ek ^ 0x80000000u);
+}
+
+// The larger of a largest value so far and w >= 0; a NaN among them stays.
+__host__ __device__ __forceinline__ float max_or_nan(float a, float w) { return w > a || w != w ? w : a; }
+
+// Position of level i in ascending order, ties by index: counted on integer keys in
+// the order of the numbers (NaN at either end), so that the positions are a
+// permutation whatever the levels.
+__host__ __device__ __forceinline__ long long level_key(double l) {
+    long long b;
+    memcpy(&b, &l, sizeof(b));
+    return b < 0 ? b ^ 0x7fffffffffffffffLL : b;
+}
+__host__ __device__ __forceinline__ int level_rank(const double *lam, int n, int i) {
+    const long long li = level_key(lam[i]);
+    int r = 0;
+    for (int k = 0; k < n; ++k) {
+        const long long lk = level_key(lam[k]);
+        r += lk < li || (lk == li && k < i);
+    }
+    return r;
 }
 
 // The sort of the Rayleigh quotients lam (double-words, msp_dw.cuh) and the

@@ -655,7 +655,7 @@ __device__ float lm_step64(const cx<double> *H, cx<double> *X64, const cx<float>
             B[(size_t)i * n + j] = b;
             Bt[(size_t)j * n + i] = b;
             const float w = fabsf(b.re) + fabsf(b.im);
-            if (i != j) amax = w <= amax ? amax : w;  // a NaN survives
+            if (i != j) amax = max_or_nan(amax, w);
         });
     team.put_max(&v.scal[2], amax);
     team.sync();
@@ -664,7 +664,7 @@ __device__ float lm_step64(const cx<double> *H, cx<double> *X64, const cx<float>
     // ascending order, ties by index; runs of gaps up to 100 couplings
     float lmax = 0.f;
     for (int i = tid; i < n; i += nt) {
-        const int r = large_rank(v.lam64, n, i);
+        const int r = level_rank(v.lam64, n, i);
         v.rank[i] = r;
         v.order[r] = i;
         v.corr_part[i] = v.norm_part[i] = 0.f;
@@ -735,7 +735,7 @@ __device__ float lm_step64(const cx<double> *H, cx<double> *X64, const cx<float>
     lm_sum(v.norm, v.norm_part, n, team);
     __syncthreads();
     float emax = 0.f;
-    for (int j = tid; j < n; j += nt) emax = v.norm[j] <= emax ? emax : v.norm[j];  // a NaN survives
+    for (int j = tid; j < n; j += nt) emax = max_or_nan(emax, v.norm[j]);
     atomicMax(&v.scal[0], __float_as_int(emax));  // the same in every CTA
     for (int r = tid; r < n; r += nt) {
         const int i = v.order[r];

@@ -243,7 +243,7 @@ __device__ float step64(S64 &s, const HSource &h, int n, int m) {
         }
         B[e] = v;
         const float w = fabsf(v.re) + fabsf(v.im);
-        if (i != j) amax = w <= amax ? amax : w;  // a NaN survives
+        if (i != j) amax = max_or_nan(amax, w);
     }
     atomicMax(&s.scal[0], __float_as_int(amax));  // NaN: above every number
     __syncthreads();
@@ -251,12 +251,7 @@ __device__ float step64(S64 &s, const HSource &h, int n, int m) {
     if (!(big < CUDART_INF_F)) return CUDART_INF_F;
     // ascending order, ties by index; runs of gaps up to 100 couplings
     for (int i = tid; i < n; i += nt) {
-        const double li = s.lam[i];
-        int r = 0;
-        for (int k = 0; k < n; ++k) {
-            const double lk = s.lam[k];
-            r += lk < li || (lk == li && k < i);
-        }
+        const int r = level_rank(s.lam, n, i);
         s.rk[i] = r;
         s.ord[r] = i;
     }
@@ -318,7 +313,7 @@ __device__ float step64(S64 &s, const HSource &h, int n, int m) {
                     }
                 }
                 const float w = fabsf(E.re) + fabsf(E.im);
-                emax = w <= emax ? emax : w;
+                emax = max_or_nan(emax, w);
                 EX[i * n + j] = E;
             }
         }
