@@ -154,7 +154,7 @@ struct PhaseArgs {
 // Pair range [begin, end) of work item `item`; begin = -1 when the item does
 // not exist.  item_first / slot_first are num_slots + 1 prefix arrays; the
 // items of a slot cover its pairs in runs of IP.
-__device__ __forceinline__ void phase_item_range(const PhaseArgs &a, int item, int *b, int *e) {
+__host__ __device__ __forceinline__ void phase_item_range(const PhaseArgs &a, int item, int *b, int *e) {
     const int total = a.item_first[a.num_slots];
     if (item >= total) {
         *b = -1;
@@ -171,9 +171,8 @@ __device__ __forceinline__ void phase_item_range(const PhaseArgs &a, int item, i
     }
     const int pb = a.slot_first[lo] * a.P + (item - a.item_first[lo]) * a.IP;
     const int slot_end = a.slot_first[lo + 1] * a.P;
-    const int pe = pb + a.IP;
     *b = pb;
-    *e = pe < slot_end ? pe : slot_end;
+    *e = slot_end - pb > a.IP ? pb + a.IP : slot_end;  // pb + IP may pass 2^31
 }
 
 size_t snap_smem_bytes(int n, int mode, int precision, int fac_len);
