@@ -191,11 +191,10 @@ static __device__ void oa_clusters(const cx<float> *SR, int ld, const float2 *la
     __syncthreads();
 }
 
-// E for the pair (i < j) in place of S_ij / R_ij, with the second-order
-// eigenvalue terms (cross-cluster pairs) and the step size.
+// E for the pair (i < j) in place of S_ij / R_ij, and the step size.
 __device__ __forceinline__ void oa_pair_correction(cx<float> *SR, int ld, const float2 *lam,
-                                                   const float *lamf, const OaCluster &c,
-                                                   float *corr, int i, int j, float &emax) {
+                                                   const float *lamf, const OaCluster &c, int i,
+                                                   int j, float &emax) {
     const cx<float> S = SR[(size_t)i * ld + j], R = SR[(size_t)j * ld + i];
     cx<float> Eij, Eji;
     if (c.cstart[c.rank[i]] == c.cstart[c.rank[j]]) {
@@ -210,13 +209,31 @@ __device__ __forceinline__ void oa_pair_correction(cx<float> *SR, int ld, const 
         const float inv = 1.0f / dl;
         Eij = mk<float>(br * inv, bi * inv);
         Eji = mk<float>(-ar * inv, ai * inv);
-        atomicAdd(&corr[i], -(ar * ar + ai * ai) * inv);
-        atomicAdd(&corr[j], (br * br + bi * bi) * inv);
         emax = fmaxf(emax, fmaxf(fmaxf(fabsf(Eij.re), fabsf(Eij.im)),
                                  fmaxf(fabsf(Eji.re), fabsf(Eji.im))));
     }
     SR[(size_t)i * ld + j] = Eij;
     SR[(size_t)j * ld + i] = Eji;
+}
+
+// Second-order terms of the levels, corr_j = sum_i |E_ij|^2 (l_j - l_i) over the
+// other clusters' levels, four threads per column: a sum in a fixed order, so that
+// results repeat bit for bit.  Between two barriers of the caller's.
+static __device__ void oa_second_order(const cx<float> *SR, int ld, const float2 *lam, int n,
+                                       const OaCluster &c, float *corr) {
+    for (int e = threadIdx.x; e < 4 * ((n + 7) & ~7); e += blockDim.x) {  // whole warps
+        const int j = e >> 2;
+        float t = 0.f;
+        if (j < n) {
+            const int cj = c.cstart[c.rank[j]];
+            for (int i = e & 3; i < n; i += 4)
+                if (c.cstart[c.rank[i]] != cj)
+                    t = fmaf(cabs2(SR[(size_t)i * ld + j]), dw_sub_f(lam[j], lam[i]), t);
+        }
+        t += __shfl_xor_sync(0xffffffffu, t, 1);
+        t += __shfl_xor_sync(0xffffffffu, t, 2);
+        if (j < n && (e & 3) == 0) corr[j] = t;
+    }
 }
 
 // Diagonal of T (after the pair corrections, so the second-order terms are

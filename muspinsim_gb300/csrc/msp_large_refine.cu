@@ -80,7 +80,7 @@ struct LmVec {
     double *lam64, *lam0, *gn, *tdiag;  // FP64 step
     float2 *lam;                        // eigenvalues as double-words
     int *rank, *order, *cstart;         // clusters of levels (msp_cluster.cuh)
-    float *corr, *corr_part, *norm, *norm_part, *rn, *cn, *gf;
+    float *corr, *rn, *cn, *gf;
     int *scal;     // [0]: largest correction, [1]: largest |l_i|, [2]: largest coupling (float
                    // bits), [3]: nonzeros of H's fullest row
     double *dsum;  // one per CTA of the team
@@ -88,7 +88,7 @@ struct LmVec {
 };
 
 __host__ __device__ inline size_t lm_vec_bytes(int n, bool fp64) {
-    return (((fp64 ? 32 : 0) + 48) * (size_t)n + 16 + 8 * 8 + 15) & ~size_t(15);
+    return (((fp64 ? 32 : 0) + 36) * (size_t)n + 16 + 8 * 8 + 15) & ~size_t(15);
 }
 
 __host__ __device__ inline size_t lm_smem_bytes(int n, int threads, bool fp64) {
@@ -107,10 +107,7 @@ __device__ __forceinline__ LmVec lm_vec(char *smem, int n, bool fp64) {
     v.order = v.rank + n;
     v.cstart = v.order + n;
     v.corr = reinterpret_cast<float *>(v.cstart + n);
-    v.corr_part = v.corr + n;
-    v.norm = v.corr_part + n;
-    v.norm_part = v.norm + n;
-    v.rn = v.norm_part + n;
+    v.rn = v.corr + n;
     v.cn = v.rn + n;
     v.gf = v.cn + n;
     v.scal = reinterpret_cast<int *>(v.gf + n);
@@ -336,18 +333,11 @@ __device__ cx<float> lm_gram64(const cx<double> *X, int n, int i, int j) {
     return mk<float>((float)re, (float)im);
 }
 
-__device__ __forceinline__ float lm_warp_sum(float x) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-    return x;
-}
-
 // visit(i, j, gram) for every pair i < j of levels, in this order: the warps of
 // the team take the j in turn, the lanes i (in whole groups of 32: on = i < j).
 // Where want(i, j) asks for it, gram(i, j), a warp-wide computation, comes first.
-template <typename Want, typename Gram, typename Visit, typename Done>
-__device__ __forceinline__ void lm_pairs_of(int n, const Team &team, Want want, Gram gram, Visit visit,
-                                            Done done) {
+template <typename Want, typename Gram, typename Visit>
+__device__ __forceinline__ void lm_pairs_of(int n, const Team &team, Want want, Gram gram, Visit visit) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     // the longest rows first
     for (int j = n - 1 - (team.rank * nw + warp); j > 0; j -= team.size * nw) {
@@ -364,16 +354,32 @@ __device__ __forceinline__ void lm_pairs_of(int n, const Team &team, Want want, 
             }
             if (on) visit(i, j, G);
         }
-        done(j);
     }
 }
 
-// out = the sum of every CTA's part (after a team barrier)
-__device__ __forceinline__ void lm_sum(float *out, float *part, int n, const Team &team) {
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        float t = 0.f;
-        for (int r = 0; r < team.size; ++r) t += team.of(part, r)[i];
-        out[i] = t;
+// out[0][j] = sum_i first(i, j), out[1][j] = sum_i second(i, j) (where given) into
+// every CTA: 32 columns per CTA and turn, rows over the warps.  The order of the sums
+// is fixed, so that results repeat bit for bit.
+template <int NS, typename Term>
+__device__ void lm_column_sums(int n, float *const (&out)[NS], const LmVec &v, const Team &team, Term term) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    float *part = reinterpret_cast<float *>(v.slab);
+    for (int g = team.rank; 32 * g < n; g += team.size) {
+        const int j = 32 * g + lane;
+        float acc[NS] = {};
+        if (j < n)
+            for (int i = warp; i < n; i += nw) term(i, j, acc);
+#pragma unroll
+        for (int q = 0; q < NS; ++q) part[(q * nw + warp) * 32 + lane] = acc[q];
+        __syncthreads();
+        if (warp == 0 && j < n) {
+#pragma unroll
+            for (int q = 0; q < NS; ++q) {
+                for (int w = 1; w < nw; ++w) acc[q] += part[(q * nw + w) * 32 + lane];
+                team.put(out[q] + j, acc[q]);
+            }
+        }
+        __syncthreads();
     }
 }
 
@@ -437,10 +443,7 @@ __device__ float lm_refine(const LargeSlot &s, const cx<float> *X, cx<float> *X2
         });
     team.put_max(&v.scal[2], amax);
     float lmax = 0.f;
-    for (int i = tid; i < n; i += nt) {
-        v.corr_part[i] = 0.f;
-        lmax = fmaxf(lmax, fabsf(v.lam[i].x));
-    }
+    for (int i = tid; i < n; i += nt) lmax = fmaxf(lmax, fabsf(v.lam[i].x));
     atomicMax(&v.scal[1], __float_as_int(lmax));  // the same in every CTA
     team.sync();
     OaCluster cl;
@@ -451,7 +454,7 @@ __device__ float lm_refine(const LargeSlot &s, const cx<float> *X, cx<float> *X2
     cl.T = B + (size_t)n * n;
     cl.ldt = n;
     oa_cluster_starts(v.lam, n, cl);
-    float emax = 0.f, cj = 0.f;
+    float emax = 0.f;
     auto same = [&](int i, int j) { return v.cstart[v.rank[i]] == v.cstart[v.rank[j]]; };
     lm_pairs_of(
         n, team, same, [&](int i, int j) { return lm_gram(X, n, i, j, v.cn[i] * v.cn[j]); },
@@ -470,24 +473,24 @@ __device__ float lm_refine(const LargeSlot &s, const cx<float> *X, cx<float> *X2
                 const float inv = 1.0f / dw_sub_f(v.lam[j], v.lam[i]);
                 Eij = mk<float>(b.re * inv, b.im * inv);
                 Eji = mk<float>(-c.re * inv, -c.im * inv);
-                atomicAdd(&v.corr_part[i], -(c.re * c.re + c.im * c.im) * inv);
-                cj += (b.re * b.re + b.im * b.im) * inv;
                 emax = fmaxf(emax, fmaxf(fmaxf(fabsf(Eij.re), fabsf(Eij.im)),
                                          fmaxf(fabsf(Eji.re), fabsf(Eji.im))));
             }
             B[up] = Eij;
             B[lo] = Eji;
-        },
-        [&](int j) {
-            const float t = lm_warp_sum(cj);
-            cj = 0.f;
-            if ((tid & 31) == 0) atomicAdd(&v.corr_part[j], t);
         });
     for (int j = team.rank * nt + tid; j < n; j += team.size * nt)
         B[(size_t)j * n + j] = mk<float>(-0.5f * v.gf[j], 0.f);
     team.sync();
-    lm_sum(v.corr, v.corr_part, n, team);
-    __syncthreads();
+    // second-order terms of the levels: |E_ij|^2 (l_j - l_i) over other clusters
+    {
+        float *const out[1] = {v.corr};
+        lm_column_sums<1>(n, out, v, team, [&](int i, int j, float (&acc)[1]) {
+            if (!same(i, j))
+                acc[0] = fmaf(cabs2(B[(size_t)i * n + j]), dw_sub_f(v.lam[j], v.lam[i]), acc[0]);
+        });
+    }
+    team.sync();
     // every CTA writes the same diagonal of T
     oa_cluster_diagonal(v.lam, v.corr, n, cl);
     // X2 = X + X E
@@ -667,7 +670,6 @@ __device__ float lm_step64(const cx<double> *H, cx<double> *X64, const cx<float>
         const int r = level_rank(v.lam64, n, i);
         v.rank[i] = r;
         v.order[r] = i;
-        v.corr_part[i] = v.norm_part[i] = 0.f;
         lmax = fmaxf(lmax, fabsf((float)v.lam64[i]));
     }
     atomicMax(&v.scal[1], __float_as_int(lmax));
@@ -685,7 +687,6 @@ __device__ float lm_step64(const cx<double> *H, cx<double> *X64, const cx<float>
     // levels take X^H X in FP64.
     cx<float> *T = R;
     const float close = __int_as_float(v.scal[1]) * (1.0f / 32.0f);
-    float cj = 0.f, ej = 0.f;
     auto same = [&](int i, int j) { return v.cstart[v.rank[i]] == v.cstart[v.rank[j]]; };
     auto gap_of = [&](int i, int j) { return (float)(v.lam64[j] - v.lam64[i]); };
     lm_pairs_of(
@@ -708,34 +709,26 @@ __device__ float lm_step64(const cx<double> *H, cx<double> *X64, const cx<float>
                 const cx<float> t = mk<float>(0.5f * (b.re + c.re), 0.5f * (b.im - c.im));
                 T[(size_t)ri * n + rj] = t;
                 T[(size_t)rj * n + ri] = conj(t);
-            } else {
-                cj += (b.re * b.re + b.im * b.im) * inv;
-                atomicAdd(&v.corr_part[i], -(c.re * c.re + c.im * c.im) * inv);
             }
-            ej += cabs2(Eij);
-            atomicAdd(&v.norm_part[i], cabs2(Eji));
             B[up] = Eij;
             B[lo] = Eji;
-        },
-        [&](int j) {
-            const float t = lm_warp_sum(cj), u = lm_warp_sum(ej);
-            cj = ej = 0.f;
-            if (lane == 0) {
-                atomicAdd(&v.corr_part[j], t);
-                atomicAdd(&v.norm_part[j], u);
-            }
         });
-    for (int j = me; j < n; j += all) {
-        const cx<float> d = mk<float>(-0.5f * (float)v.gn[j], 0.f);
-        atomicAdd(&v.norm_part[j], cabs2(d));
-        B[(size_t)j * n + j] = d;
+    for (int j = me; j < n; j += all) B[(size_t)j * n + j] = mk<float>(-0.5f * (float)v.gn[j], 0.f);
+    team.sync();
+    // second-order terms of the levels and squared column norms of E (over cn, which
+    // the double-word steps have used)
+    float *const norm = v.cn;
+    {
+        float *const out[2] = {v.corr, norm};
+        lm_column_sums<2>(n, out, v, team, [&](int i, int j, float (&acc)[2]) {
+            const float e2 = cabs2(B[(size_t)i * n + j]);
+            if (!same(i, j)) acc[0] = fmaf(e2, gap_of(i, j), acc[0]);
+            acc[1] += e2;
+        });
     }
     team.sync();
-    lm_sum(v.corr, v.corr_part, n, team);
-    lm_sum(v.norm, v.norm_part, n, team);
-    __syncthreads();
     float emax = 0.f;
-    for (int j = tid; j < n; j += nt) emax = max_or_nan(emax, v.norm[j]);
+    for (int j = tid; j < n; j += nt) emax = max_or_nan(emax, norm[j]);
     atomicMax(&v.scal[0], __float_as_int(emax));  // the same in every CTA
     for (int r = tid; r < n; r += nt) {
         const int i = v.order[r];

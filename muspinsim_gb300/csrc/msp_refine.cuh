@@ -415,7 +415,6 @@ __device__ float oa_refine(SnapSmem<float> &s, int n_rt, int m_rt, cx<float> *Xl
         const float l = lw.x;
         s.lw[i] = lw;
         s.lamf[i] = l;
-        s.corr[i] = 0.f;
         lmax = fmaxf(lmax, fabsf(l));
     }
     atomicMax(&s.scal[1], __float_as_int(lmax));  // non-negative: int order = float order
@@ -434,8 +433,10 @@ __device__ float oa_refine(SnapSmem<float> &s, int n_rt, int m_rt, cx<float> *Xl
     for (int e = tid; e < nup; e += nt) {
         int i, j;
         oa_pair_of(e, i, j);
-        oa_pair_correction(s.SR, ld, s.lw, s.lamf, cl, s.corr, i, j, emax);
+        oa_pair_correction(s.SR, ld, s.lw, s.lamf, cl, i, j, emax);
     }
+    __syncthreads();
+    oa_second_order(s.SR, ld, s.lw, n, cl, s.corr);
     __syncthreads();
     oa_cluster_diagonal(s.lw, s.corr, n, cl);
     // X' = X + X E  (into Yh), E_ii = R_ii / 2
