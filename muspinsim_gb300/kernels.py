@@ -747,6 +747,7 @@ def lindblad_run(n, Hsys, Z, spin_ops, dims, mu_index, gammas, dissipation, fiel
     keep = upload((Hsys, torch.complex128), (Z, torch.complex128), (spin_ops, torch.complex128),
                   (field, torch.float64), (pol, torch.float64), (wscale, torch.float64),
                   (slot, torch.int32), (Tp, torch.float64), (th, torch.float64))
+    keep[3], keep[4] = keep[3].reshape(-1, 3), keep[4].reshape(-1, 3)
     (a.Hsys, a.Z, a.spin_ops, a.field, a.pol, a.wscale, a.slot, a.temperature, a.times) = (
         None if x is None else x.data_ptr() for x in keep)
     a.num_snap = S

@@ -60,3 +60,15 @@ def test_sample_counts(nt, t0):
 @pytest.mark.parametrize("rate", [0.0, 50.0])
 def test_rates_and_temperatures(temperature, rate):
     assert _compare(["mu", "e", "H"], {1: rate}, np.linspace(0.0, 4.0, 120), temperature) <= 1e-10
+
+
+@pytest.mark.parametrize("bad", ["field", "pol"])
+def test_vectors_of_the_wrong_length_are_refused(bad):
+    sy = workloads.Workload("l", ["mu"], [], zcw_gen(1), np.zeros((1, 3)), np.array([0.0, 0.0, 1.0]),
+                            np.zeros(1), 5.0).system()
+    ops = np.array([[sy.operator({0: ax}).matrix.toarray() for ax in "xyz"]], dtype=complex)
+    vec = {"field": np.zeros((2, 3)), "pol": np.ones((2, 3)), bad: np.ones(7)}
+    with pytest.raises(RuntimeError):
+        kernels.lindblad_run(2, sy.hamiltonian_matrix(), sy.zeeman_operators(), ops, [2], 0, sy.gammas,
+                             {0: 0.1}, vec["field"], vec["pol"], np.ones(2), np.zeros(2, np.int32), 1,
+                             np.linspace(0, 1, 5))
