@@ -269,6 +269,11 @@ typedef struct msp_powder_args {
  * dereferenced). */
 int msp_powder_workspace(const msp_powder_args *args, size_t *bytes);
 
+/* The least scratch msp_powder_run takes: with less than msp_powder_workspace
+ * bytes it leaves out what only buys speed (the Fourier form of the phase sum,
+ * FP64 snapshots of n <= 32 in two stages, for n > 64 all snapshots in flight). */
+int msp_powder_min_workspace(const msp_powder_args *args, size_t *bytes);
+
 /* Runs the batch: Hamiltonian assembly, batched eigensolve, eigenbasis
  * amplitudes, phase sum over time, weighted reduction into args->out
  * (overwritten).  Kernels launched: msp_snap_* (one CTA per snapshot),
@@ -508,6 +513,9 @@ typedef struct msp_adjoint_args {
 /* Scratch bytes msp_adjoint_fast needs (no pointer is dereferenced). */
 int msp_adjoint_workspace(const msp_adjoint_args *args, size_t *bytes);
 
+/* The least scratch it takes: without the Fourier form of its sums. */
+int msp_adjoint_min_workspace(const msp_adjoint_args *args, size_t *bytes);
+
 /* Kernels: msp_assemble, msp_eigh (FP64), msp_adjoint_transform (per level
  * pair: sum_t g(t) e^{2 pi i nu t} and its t-weighted form, FP64),
  * msp_adjoint_snap (one CTA per snapshot: dL/dH_s, dL/db_s),
@@ -583,6 +591,8 @@ typedef struct msp_celio_args {
 } msp_celio_args;
 
 int msp_celio_workspace(const msp_celio_args *args, size_t *bytes);
+/* The least scratch msp_celio_run takes: without the fixed-point tensor form. */
+int msp_celio_min_workspace(const msp_celio_args *args, size_t *bytes);
 int msp_celio_run(const msp_celio_args *args, void *workspace, size_t workspace_bytes,
                   void *stream);
 

@@ -307,9 +307,17 @@ _SIGNATURES = {
         ctypes.c_int,
         [ctypes.POINTER(PowderArgs), ctypes.POINTER(ctypes.c_size_t)],
     ),
+    "msp_powder_min_workspace": (
+        ctypes.c_int,
+        [ctypes.POINTER(PowderArgs), ctypes.POINTER(ctypes.c_size_t)],
+    ),
     "msp_powder_run": (ctypes.c_int, [ctypes.POINTER(PowderArgs)]),
     "msp_powder_run_static": (ctypes.c_int, [ctypes.POINTER(PowderArgs)]),
     "msp_adjoint_workspace": (
+        ctypes.c_int,
+        [ctypes.POINTER(AdjointArgs), ctypes.POINTER(ctypes.c_size_t)],
+    ),
+    "msp_adjoint_min_workspace": (
         ctypes.c_int,
         [ctypes.POINTER(AdjointArgs), ctypes.POINTER(ctypes.c_size_t)],
     ),
@@ -342,6 +350,8 @@ _SIGNATURES = {
         ctypes.c_int, [ctypes.POINTER(LindbladArgs), ctypes.POINTER(ctypes.c_size_t)]),
     "msp_lindblad_run": (ctypes.c_int, [ctypes.POINTER(LindbladArgs)]),
     "msp_celio_workspace": (
+        ctypes.c_int, [ctypes.POINTER(CelioArgs), ctypes.POINTER(ctypes.c_size_t)]),
+    "msp_celio_min_workspace": (
         ctypes.c_int, [ctypes.POINTER(CelioArgs), ctypes.POINTER(ctypes.c_size_t)]),
     "msp_celio_run": (
         ctypes.c_int, [ctypes.POINTER(CelioArgs), _c_dp, ctypes.c_size_t, _c_dp]),

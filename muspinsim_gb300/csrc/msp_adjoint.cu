@@ -335,6 +335,14 @@ int msp_adjoint_workspace(const msp_adjoint_args *a, size_t *bytes) {
     return MSP_OK;
 }
 
+int msp_adjoint_min_workspace(const msp_adjoint_args *a, size_t *bytes) {
+    const int rc = adj_check(a);
+    if (rc != MSP_OK) return rc;
+    if (bytes == NULL) return adj_fail(MSP_ERR_ARG, "msp_adjoint_min_workspace: bytes is NULL");
+    *bytes = adjoint_layout(a, true).total;
+    return MSP_OK;
+}
+
 int msp_adjoint_fast(const msp_adjoint_args *a) {
     int rc = adj_check(a);
     if (rc != MSP_OK) return rc;

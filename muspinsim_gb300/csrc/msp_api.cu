@@ -399,11 +399,20 @@ int msp_powder_workspace(const msp_powder_args *args, size_t *bytes) {
     return MSP_OK;
 }
 
+int msp_powder_min_workspace(const msp_powder_args *args, size_t *bytes) {
+    const int rc = check_powder(args);
+    if (rc != MSP_OK) return rc;
+    MSP_CHECK_PTR(bytes);
+    const size_t full = powder_layout(args).total, lean = powder_layout(args, true).total;
+    *bytes = full < lean ? full : lean;
+    return MSP_OK;
+}
+
 }  // extern "C"
 
 namespace msp {
-// Smallest workspace msp_powder_run accepts (0 when the arguments are bad).
-size_t powder_min_workspace(const msp_powder_args *args) {
+// Workspace of the lean layout (0 when the arguments are bad).
+size_t powder_lean_workspace(const msp_powder_args *args) {
     return check_powder(args) == MSP_OK ? powder_layout(args, true).total : 0;
 }
 }  // namespace msp

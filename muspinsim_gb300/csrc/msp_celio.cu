@@ -1548,6 +1548,15 @@ int msp_celio_workspace(const msp_celio_args *args, size_t *bytes) {
     return MSP_OK;
 }
 
+int msp_celio_min_workspace(const msp_celio_args *args, size_t *bytes) {
+    CePlan p;
+    const int rc = ce_plan(args, p);
+    if (rc != MSP_OK) return rc;
+    if (bytes == NULL) return ce_fail(MSP_ERR_ARG, "msp_celio_min_workspace: bytes is NULL");
+    *bytes = ce_workspace(args, p);
+    return MSP_OK;
+}
+
 int msp_celio_run(const msp_celio_args *a, void *workspace, size_t workspace_bytes,
                   void *stream) {
     CePlan p;

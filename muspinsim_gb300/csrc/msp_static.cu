@@ -32,7 +32,7 @@
 
 namespace msp {
 int record_error(int code, const char *msg);
-size_t powder_min_workspace(const msp_powder_args *args);
+size_t powder_lean_workspace(const msp_powder_args *args);
 }
 
 static __device__ __align__(256) unsigned char g_msp_static_scratch[MSP_STATIC_SCRATCH_BYTES];
@@ -74,7 +74,7 @@ extern "C" int msp_powder_run_static(const msp_powder_args *args) {
     size_t need = 0;
     int rc = msp_powder_workspace(args, &need);
     if (rc != MSP_OK) return rc;
-    need = msp::powder_min_workspace(args);  // what msp_powder_run can do with
+    need = msp::powder_lean_workspace(args);  // what msp_powder_run can do with
     if (need > (size_t)MSP_STATIC_SCRATCH_BYTES) {
         char msg[256];
         snprintf(msg, sizeof(msg),

@@ -86,6 +86,21 @@ def upload(*pairs):
     return out
 
 
+def _scratch(name, args):
+    """Scratch of the entry point whose sizes ``<name>_workspace`` and
+    ``<name>_min_workspace`` give for ``args``: the first, or the second (slower
+    forms) where the device has no room for it.  Returns (tensor, 256-byte
+    aligned address, bytes)."""
+    nbytes = ctypes.c_size_t(0)
+    _lib.call(name + "_workspace", ctypes.byref(args), ctypes.byref(nbytes))
+    try:
+        buf = torch.empty(nbytes.value + 256, dtype=torch.uint8, device=device())
+    except torch.cuda.OutOfMemoryError:
+        _lib.call(name + "_min_workspace", ctypes.byref(args), ctypes.byref(nbytes))
+        buf = torch.empty(nbytes.value + 256, dtype=torch.uint8, device=device())
+    return buf, buf.data_ptr() + (-buf.data_ptr()) % 256, int(nbytes.value)
+
+
 def eigh(H, precision=_lib.PREC_FP64, max_sweeps=0):
     """Batched Hermitian eigensolve of (batch, n, n) complex matrices.
 
@@ -456,10 +471,8 @@ class PowderPlan:
             # failed allocation is refused
             self.ws, self.workspace_bytes = None, 0
             a.workspace, a.workspace_bytes = None, 0
-            self.ws = torch.empty(int(nbytes.value) + 256, dtype=torch.uint8, device=device())
-            self.workspace_bytes = int(nbytes.value)
-        a.workspace = self.ws.data_ptr() + (-self.ws.data_ptr()) % 256
-        a.workspace_bytes = self.workspace_bytes
+            self.ws, a.workspace, a.workspace_bytes = _scratch("msp_powder", a)
+            self.workspace_bytes = a.workspace_bytes
 
     def set_times(self, times):
         """Move the plan to another time grid (host array) of the same length.
@@ -556,15 +569,9 @@ def adjoint_fast(n, Hsys, Z, field, pol, wscale, slot, num_slots, times, grad_ou
     a.grad_field = gF.data_ptr() if gF is not None else None
     a.status = status.data_ptr()
     a.max_sweeps = int(max_sweeps)
-    nbytes = ctypes.c_size_t(0)
-    lib = _lib.load()
-    _lib.check(lib.msp_adjoint_workspace(ctypes.byref(a), ctypes.byref(nbytes)),
-               "msp_adjoint_workspace")
-    ws = torch.empty(int(nbytes.value) + 256, dtype=torch.uint8, device=d)
-    a.workspace = ws.data_ptr() + ((-ws.data_ptr()) % 256)
-    a.workspace_bytes = int(nbytes.value)
+    ws, a.workspace, a.workspace_bytes = _scratch("msp_adjoint", a)
     a.stream = torch.cuda.current_stream().cuda_stream
-    _lib.check(lib.msp_adjoint_fast(ctypes.byref(a)), "msp_adjoint_fast")
+    _lib.check(_lib.load().msp_adjoint_fast(ctypes.byref(a)), "msp_adjoint_fast")
     return gH, gF, status[:S]
 
 
@@ -601,22 +608,28 @@ class MultiPlan:
         desc.t0, desc.dt = t0, dt
         desc.precision = int(precision)
         desc.max_sweeps = int(max_sweeps)
-        desc.max_pairs_per_chunk = int(max_pairs_per_chunk)
-        self._tuning = None
-        if tuning:
-            arr = (_lib.MultiTuning * len(tuning))()
+
+        def create(tuning, max_pairs):
+            desc.max_pairs_per_chunk = int(max_pairs)
+            arr = (_lib.MultiTuning * max(len(tuning), 1))()
             for i, t in enumerate(tuning):
                 arr[i].n = int(t["n"])
                 arr[i].snap_threads = int(t.get("snap_threads", 0))
                 arr[i].ctas_per_sm = int(t.get("ctas_per_sm", 0))
                 arr[i].snaps_per_item = int(t.get("snaps_per_item", 0))
             self._tuning = arr
-            desc.tuning = ctypes.cast(arr, ctypes.POINTER(_lib.MultiTuning))
+            desc.tuning = ctypes.cast(arr, ctypes.POINTER(_lib.MultiTuning)) if tuning else None
             desc.num_tuning = len(tuning)
-        h = ctypes.c_void_p(0)
-        _lib.check(lib.msp_multi_plan_create(ctypes.byref(desc), ctypes.byref(h)),
-                   "msp_multi_plan_create")
-        self.handle = h
+            h = ctypes.c_void_p(0)
+            _lib.check(lib.msp_multi_plan_create(ctypes.byref(desc), ctypes.byref(h)),
+                       "msp_multi_plan_create")
+            self.handle = h
+            nbytes = ctypes.c_size_t(0)
+            _lib.check(lib.msp_multi_workspace(h, ctypes.byref(nbytes)), "msp_multi_workspace")
+            return int(nbytes.value)
+
+        tuning = list(tuning or [])
+        nbytes = create(tuning, max_pairs_per_chunk)
         self.dims = dims
         self.snap_first = first
         self.num_snap = int(first[-1])
@@ -631,18 +644,29 @@ class MultiPlan:
         self.T = dev(th, torch.float64).reshape(-1)
         self.out = torch.empty((ns, int(th.size)), dtype=torch.float64, device=d)
         self.status = torch.zeros((max(self.num_snap, 1),), dtype=torch.int32, device=d)
-        nbytes = ctypes.c_size_t(0)
-        _lib.check(lib.msp_multi_workspace(h, ctypes.byref(nbytes)), "msp_multi_workspace")
-        self.ws = torch.empty(int(nbytes.value) + 256, dtype=torch.uint8, device=d)
+        try:
+            self.ws = torch.empty(nbytes + 256, dtype=torch.uint8, device=d)
+        except torch.cuda.OutOfMemoryError:
+            # the least scratch: direct phase sums (an item size asks for them) and
+            # short chunks
+            self.close()
+            asked = {int(t["n"]): t for t in tuning}
+            short = []
+            for n in np.unique(dims):
+                t = asked.get(int(n), {})
+                snaps = int(np.diff(first)[dims == n].sum())
+                short.append(dict(t, n=n, snaps_per_item=t.get("snaps_per_item") or -(-snaps // 1500) or 1))
+            nbytes = create(short, min(max_pairs_per_chunk or 1 << 22, 1 << 22))
+            self.ws = torch.empty(nbytes + 256, dtype=torch.uint8, device=d)
         io = _lib.MultiIO()
         io.Hsys_all, io.Z_all = self.Hs.data_ptr(), self.Zd.data_ptr()
         io.field, io.pol, io.wscale = self.F.data_ptr(), self.Pl.data_ptr(), self.W.data_ptr()
         io.times = self.T.data_ptr()
         io.out, io.status = self.out.data_ptr(), self.status.data_ptr()
         io.workspace = self.ws.data_ptr() + ((-self.ws.data_ptr()) % 256)
-        io.workspace_bytes = int(nbytes.value)
+        io.workspace_bytes = nbytes
         self.io = io
-        self.workspace_bytes = int(nbytes.value)
+        self.workspace_bytes = nbytes
 
     def info(self):
         """Buckets in launch order: list of dicts (n, num_systems, num_snap,
@@ -840,13 +864,8 @@ def celio_run(mode, digit_dims, factor_digits, factor_mat, mats, mats_per_snapsh
             a.wscale = ptr(ws_)
     a.path = int(path)
     a.precision = int(precision)
-    nbytes = ctypes.c_size_t(0)
-    _lib.call("msp_celio_workspace", ctypes.byref(a), ctypes.byref(nbytes))
-    ws = torch.empty(int(nbytes.value) + 256, dtype=torch.uint8, device=d)
-    base = ws.data_ptr()
-    aligned = (base + 255) & ~255
-    _lib.call("msp_celio_run", ctypes.byref(a), ctypes.c_void_p(aligned),
-              ctypes.c_size_t(int(nbytes.value)), stream())
+    ws, base, nbytes = _scratch("msp_celio", a)
+    _lib.call("msp_celio_run", ctypes.byref(a), ctypes.c_void_p(base), ctypes.c_size_t(nbytes), stream())
     return series, rows
 
 
