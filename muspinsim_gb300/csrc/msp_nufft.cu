@@ -146,6 +146,7 @@ bool nufft_shape(long long S, int P, int slots, int T, int precision, bool two, 
     s.m = s.n1 * s.n2 / 2;
     const int grids = s.two ? 2 : 1;
     s.cols = grids * (s.m + 1);
+    if ((long long)s.tiles * grids > 65535) return false;  // the transform's launch grid
     // Times of both forms in ns, measured on GB300 (152 SMs) with 10,000 x 276
     // pairs x 4096 samples: the direct FP64 sum 44.3 ms (255 pair-samples per
     // ns), the tensor-core mixed sum 0.617 ms (18,300); spreading 0.80 ms

@@ -366,3 +366,17 @@ def test_capi_large_n_workspace_sizes():
     # the general path adds two complex n x n matrices per CTA
     assert evolve >= fast64 + 10 * 4 * n * n * 8 - 10 * 4096
     assert integ >= 10 * (9 * n * n * 8)
+
+
+def test_grids_beyond_the_transform():
+    """140 million uniform samples: more time tiles than the Fourier form's launch
+    grid holds, so the direct sum's scratch (1.1 GB of partial sums for one snapshot)
+    and not the transform's (22 GB) is asked for."""
+    from muspinsim_gb300 import _lib
+
+    a = _lib.PowderArgs()
+    a.n, a.num_snap, a.num_slots, a.num_times = 64, 1, 1, 140_000_000
+    a.mode, a.precision, a.uniform, a.t0, a.dt = _lib.MODE_FAST, _lib.PREC_FP64, 1, 0.0, 1e-7
+    nbytes = ctypes.c_size_t(0)
+    _lib.call("msp_powder_workspace", ctypes.byref(a), ctypes.byref(nbytes))
+    assert nbytes.value < 3 * 8 * a.num_times
