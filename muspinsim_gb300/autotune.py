@@ -18,8 +18,9 @@ import threading
 
 import numpy as np
 
-# bump when a kernel change invalidates cached choices
-TUNER_VERSION = 1
+# bump when a kernel change invalidates cached choices (2: the row refinement, the
+# staged n > 64 kernels and the Fourier phase sum)
+TUNER_VERSION = 2
 
 _lock = threading.Lock()
 

@@ -139,3 +139,13 @@ def test_cache_round_trip(tmp_path, monkeypatch):
     autotune.save_cache({key: {"params": {"snap_threads": 128}}})
     assert autotune.load_cache()[key]["params"]["snap_threads"] == 128
     assert key != autotune.cache_key("GB300", 24, 4096, True, 1, 10000)
+
+
+def test_choices_of_the_first_tuner_are_not_taken(tmp_path, monkeypatch):
+    """Those were timed on kernels that are no longer there."""
+    path = str(tmp_path / "tune.json")
+    monkeypatch.setenv("MSP_AUTOTUNE_CACHE", path)
+    key = autotune.cache_key("GB300", 24, 2048, True, 1, 10000)
+    old = key.rsplit("|", 1)[0] + "|tuner=1"
+    autotune.save_cache({old: {"params": {"snaps_per_item": 16}}})
+    assert key not in autotune.load_cache()
