@@ -106,25 +106,22 @@ def eigh(H, precision=_lib.PREC_FP64, max_sweeps=0):
 
     Returns (evals (batch, n) float64 ascending, evecs (batch, n, n)
     complex128 with eigenvectors as columns, status (batch,) int32)."""
-    return _eigh(H, precision, max_sweeps)[1:]
-
-
-def _eigh(H, precision, max_sweeps):
-    # (the bytes of all three results, evals, evecs, status)
     Hd = dev(H, torch.complex128)
     if Hd.dim() == 2:
         Hd = Hd[None]
     b, n, _ = Hd.shape
-    size = (16 * b * n * n, 8 * b * n, 4 * b)
-    buf = torch.empty(sum(size), dtype=torch.uint8, device=Hd.device)
-    evecs, evals, status = torch.split(buf, size)
-    evecs = evecs.view(torch.complex128).reshape(b, n, n)
-    evals = evals.view(torch.float64).reshape(b, n)
-    status = status.view(torch.int32)
+    evals = torch.empty((b, n), dtype=torch.float64, device=Hd.device)
+    evecs = torch.empty((b, n, n), dtype=torch.complex128, device=Hd.device)
+    status = torch.empty((b,), dtype=torch.int32, device=Hd.device)
+    _eigh(Hd, n, b, precision, max_sweeps, evals, evecs, status)
+    return evals, evecs, status
+
+
+def _eigh(Hd, n, b, precision, max_sweeps, evals, evecs, status):
     if n <= _lib.MAX_DIM:
         _lib.call("msp_eigh_batched", ptr(Hd), n, b, int(precision), int(max_sweeps), ptr(evals),
                   ptr(evecs), ptr(status), stream())
-        return buf, evals, evecs, status
+        return
     # n > 64: Householder + QL in FP64 with caller scratch
     nbytes = ctypes.c_size_t(0)
     _lib.call("msp_eigh_workspace", n, b, ctypes.byref(nbytes))
@@ -132,17 +129,21 @@ def _eigh(H, precision, max_sweeps):
     wp = ws.data_ptr() + ((-ws.data_ptr()) % 256)
     _lib.call("msp_eigh_batched_ws", ptr(Hd), n, b, int(precision), int(max_sweeps), ptr(evals),
               ptr(evecs), ptr(status), ctypes.c_void_p(wp), int(nbytes.value), stream())
-    return buf, evals, evecs, status
 
 
 def eigh_host(H):
     """:func:`eigh` of one (n, n) matrix in FP64 with the results on the host
     after a single copy: (evals (n,), evecs (n, n), status) as numpy arrays
     and an int."""
-    n = np.shape(H)[-1]
-    host = _eigh(H, _lib.PREC_FP64, 0)[0].cpu().numpy()
-    evecs = host[:16 * n * n].view(np.complex128).reshape(n, n)
-    return host[16 * n * n:-4].view(np.float64), evecs, int(host[-4:].view(np.int32)[0])
+    Hd = dev(H, torch.complex128)
+    n = Hd.shape[-1]
+    size = (16 * n * n, 8 * n, 4)
+    buf = torch.empty(sum(size), dtype=torch.uint8, device=Hd.device)
+    evecs, evals, status = torch.split(buf, size)
+    _eigh(Hd, n, 1, _lib.PREC_FP64, 0, evals, evecs, status)
+    host = buf.cpu().numpy()
+    evecs = host[:size[0]].view(np.complex128).reshape(n, n)
+    return host[size[0]:-4].view(np.float64), evecs, int(host[-4:].view(np.int32)[0])
 
 
 def assemble(Hsys, Z, fields):
