@@ -1445,7 +1445,8 @@ static int ce_plan(const msp_celio_args *a, CePlan &p) {
         f.D = D0 * D1;
         if (f.D > CE_MAX_D) return ce_fail(MSP_ERR_UNSUPPORTED, "msp_celio: factor dimension > 128");
         if (f.two) {
-            const int a_ = strides[d0] > strides[d1] ? d0 : d1, b_ = a_ == d0 ? d1 : d0;
+            // the slower digit first; a digit of dimension 1 shares its neighbour's stride
+            const int a_ = d0 < d1 ? d0 : d1, b_ = d0 < d1 ? d1 : d0;
             f.sA = strides[a_];
             f.DA = a->digit_dims[a_];
             f.sB = strides[b_];

@@ -171,3 +171,14 @@ def test_aligned_digits():
              sum(a * b for a, b in zip(u[:16], x[16:])) + sum(a * b for a, b in zip(u[16:], x[:16])))
     assert abs(got.real - exact[0] / 2**116) <= 2.0**-47.5
     assert abs(got.imag - exact[1] / 2**116) <= 2.0**-47.5
+
+
+# a spin of I = 0 has one state, and its digit the stride of the digit before it
+@pytest.mark.parametrize("prec", [_lib.PREC_FP64, _lib.PREC_MIXED])
+@pytest.mark.parametrize("dims", [[2, 1, 5], [2, 1, 1, 3], [2, 3, 1]])
+def test_digits_of_dimension_one(dims, prec):
+    last = len(dims) - 1
+    factors = [(0, 1), (1, 0), (0, last), (last, 1), (1, -1)] + [(1, 2)] * (last > 1)
+    # 36 products of 2^-40 each in double-words
+    tol = 1e-13 if prec == _lib.PREC_FP64 else 1e-10
+    assert _pure(dims, factors, 2, 4, prec=prec, seed=last) <= tol
