@@ -30,6 +30,7 @@
 #include <math_constants.h>
 #include <string.h>
 
+#include <algorithm>
 #include <vector>
 
 #include "msp_dw.cuh"
@@ -598,9 +599,9 @@ __global__ void __launch_bounds__(CE_DW_THREADS) msp_celio_smem_dw_kernel(CeArgs
 
 // ----------------------------------------------------------- fixed-point tensor path
 // States in shared memory as 64-bit fixed-point numbers, group products on the
-// tensor cores with exact integer arithmetic -- both precisions, whenever every
-// factor is unitary with D <= 16 (checked on the device; a state that is not
-// taken here runs in the kernels above instead).
+// tensor cores with exact integer arithmetic -- FP64 and, where it is the faster form
+// (fx_faster), MIXED, whenever every factor is unitary with D <= 16 (checked on the
+// device; a state that is not taken here runs in the kernels above instead).
 //
 // What bounds the FP64 form is the FP64 pipe (1/74 of the FP32 rate): 4 D FMAs
 // per element and factor.  A unitary factor keeps the state's norm, so x = v
@@ -630,6 +631,17 @@ constexpr int FX_LOW = 4, FX_LEVELS = 2 * FX_DIGITS - 1 - FX_LOW;  // levels s +
 constexpr int FX_FRAG = FX_DIGITS * 2 * 32;  // uint4 per factor: [digit][re, im][lane]
 constexpr float FX_EXACT = 16777216.f - 1048576.f;  // 2^24 - 2^20
 
+// Small factors (FX_SMALL) take their products on the integer pipe instead: u and x in
+// two limbs of 29 bits, u_1 x_1, u_1 x_0 + u_0 x_1 and u_0 x_0 summed apart in 64 bits,
+// exactly, and joined with one rounding.  A tile of MMAs costs a warp 2.3 to 2.6 us
+// whatever D is; a complex product here costs 16 multiply-adds, some 20 of which an SM
+// makes per clock, spread over a lane per row where there are threads to spare.  us per
+// factor, tiles / integers: D = 2, V = 64, 3.1 / 1.2; D = 4, V = 128, 2.5 / 1.0; D = 6, V
+// = 192, 2.6 / 1.2; D = 8, V = 64, 2.6 / 1.5; D = 4, V = 2048, 6.3 / 4.3; D = 8, V = 1024,
+// 3.4 / 3.6, but 13.9 / 12.2 for 1,000 states, of which an SM then holds two or more.
+constexpr int FX_SMALL = 8;
+constexpr int FX_LIMB = 29;
+
 struct FxOp {
     long long mat;  // source matrix
     int D, where;   // acts on the factor's first digit (0), second (1) or both (2)
@@ -642,6 +654,8 @@ struct FxFactor {
     int op0, ops;   // its products, base matrix first
     int p, groups;  // groups per MMA column, V / D
     int base0;      // first of its group bases
+    int lanes;      // integer form: lanes per group (0: MMA tiles)
+    int u0;         // its matrix, as an offset into a block's U
     int pad;
 };
 
@@ -649,8 +663,8 @@ struct FxArgs {
     CeArgs c;
     const FxFactor *fac;
     const FxOp *ops;
-    int nf, nbase;
-    uint4 *frag;  // [block][nf][FX_FRAG]
+    int nf, nbase, ulen;
+    uint4 *frag;  // [block][ulen]: MMA fragments, or limbs (re 1, re 0, im 1, im 0) per entry
     int *good;    // [block]: every factor unitary
     int *done;    // [state]
 };
@@ -710,6 +724,18 @@ __device__ __forceinline__ long long fx_round(double hi, double lo) {
     return r + __double2ll_rn((h - (double)r) + lo * 0x1p58);
 }
 
+// v = y 2^29 + x with |x| <= 2^28
+__device__ __forceinline__ int2 fx_limbs(long long v) {
+    const int hi = (int)((v + (1ll << (FX_LIMB - 1))) >> FX_LIMB);
+    return make_int2((int)(v - ((long long)hi << FX_LIMB)), hi);
+}
+
+// 2^-58 (a 2^58 + b 2^29 + c), rounded
+__device__ __forceinline__ long long fx_join(long long a, long long b, long long c) {
+    const long long half = 1ll << (FX_LIMB - 1);
+    return a + ((b + ((c + half) >> FX_LIMB) + half) >> FX_LIMB);
+}
+
 // Products of the merged factors, their unitarity and their digit fragments;
 // one CTA of 256 threads per (factor, matrix block).  The products are
 // double-double: a merged factor acts thousands of times, so its rounding
@@ -763,8 +789,15 @@ __global__ void __launch_bounds__(256) msp_celio_fx_prep_kernel(FxArgs a) {
         if (tid == 0) atomicAnd(&a.good[blockIdx.y], 0);
         return;
     }
+    uint4 *out = a.frag + (size_t)blockIdx.y * a.ulen + ff.u0;
+    if (ff.lanes) {
+        if (in) {
+            const int2 r = fx_limbs(fx_round(M[tid].x, E[tid].x)), c = fx_limbs(fx_round(M[tid].y, E[tid].y));
+            out[i * D + j] = make_uint4((unsigned)r.y, (unsigned)r.x, (unsigned)c.y, (unsigned)c.x);
+        }
+        return;
+    }
     // fragment registers: rows lane / 4 (+ 8), columns 2 (lane % 4) + {0, 1} (+ 8)
-    uint4 *out = a.frag + ((size_t)blockIdx.y * a.nf + blockIdx.x) * FX_FRAG;
     for (int e = tid; e < FX_FRAG; e += 256) {
         const int lane = e & 31, im = (e >> 5) & 1, s = e >> 6, g = lane >> 2, t = lane & 3;
         unsigned r[4];
@@ -865,12 +898,86 @@ __device__ __forceinline__ void fx_tile(longlong2 *V, const uint4 *__restrict__ 
     }
 }
 
-__global__ void __launch_bounds__(FX_THREADS, 1) msp_celio_fx_kernel(FxArgs a) {
+// Every group of a small factor: `lanes` lanes per group (a power of two) take its
+// rows in turn.
+template <int D>
+__device__ __forceinline__ void fx_groups(longlong2 *V, const uint4 *__restrict__ U, int groups, int lanes,
+                                          const int *__restrict__ base, const int *__restrict__ offs) {
+    const int tid = threadIdx.x, part = tid & (lanes - 1), per = FX_THREADS / lanes;
+#pragma unroll 1
+    for (int g0 = 0; g0 < groups; g0 += per) {  // the same count in every thread
+        const int g = g0 + tid / lanes;
+        const bool on = g < groups;
+        const int b = on ? base[g] : 0;
+        int2 xr[D], xi[D];
+        if (on) {
+#pragma unroll
+            for (int j = 0; j < D; ++j) {
+                const longlong2 v = V[fx_swz(b + offs[j])];
+                xr[j] = fx_limbs(v.x);
+                xi[j] = fx_limbs(v.y);
+            }
+        }
+        __syncwarp();  // the group's lanes have read
+        if (!on) continue;
+#pragma unroll 1
+        for (int i = part; i < D; i += lanes) {
+            long long r2 = 0, r1 = 0, r0 = 0, c2 = 0, c1 = 0, c0 = 0;
+#pragma unroll
+            for (int j = 0; j < D; ++j) {
+                const uint4 w = U[i * D + j];
+                const int ur1 = (int)w.x, ur0 = (int)w.y, ui1 = (int)w.z, ui0 = (int)w.w;
+                auto mac = [](long long &s, int x, int y) { s += (long long)x * y; };
+                mac(r2, ur1, xr[j].y);
+                mac(c2, ur1, xi[j].y);
+                mac(r1, ur1, xr[j].x);
+                mac(c1, ur1, xi[j].x);
+                mac(r0, ur0, xr[j].x);
+                mac(c0, ur0, xi[j].x);
+                mac(r2, -ui1, xi[j].y);
+                mac(c2, ui1, xr[j].y);
+                mac(r1, ur0, xr[j].y);
+                mac(c1, ur0, xi[j].y);
+                mac(r0, -ui0, xi[j].x);
+                mac(c0, ui0, xr[j].x);
+                mac(r1, -ui1, xi[j].x);
+                mac(c1, ui1, xr[j].x);
+                mac(r1, -ui0, xi[j].y);
+                mac(c1, ui0, xr[j].y);
+            }
+            V[fx_swz(b + offs[i])] = make_longlong2(fx_join(r2, r1, r0), fx_join(c2, c1, c0));
+        }
+    }
+}
+
+__device__ __forceinline__ void fx_small(longlong2 *V, const uint4 *U, const FxFactor &ff, const int *base,
+                                         const int *offs) {
+    switch (ff.f.D) {
+#define FX_CASE(DD)                                                                 \
+    case DD:                                                                        \
+        fx_groups<DD>(V, U, ff.groups, ff.lanes, base, offs);                       \
+        return;
+        FX_CASE(1)
+        FX_CASE(2)
+        FX_CASE(3)
+        FX_CASE(4)
+        FX_CASE(5)
+        FX_CASE(6)
+        FX_CASE(7)
+        FX_CASE(8)
+#undef FX_CASE
+    }
+}
+
+// TILES: some factor takes MMA tiles (255 registers; the integer form alone leaves
+// room for two CTAs per SM).
+template <bool TILES>
+__global__ void __launch_bounds__(FX_THREADS, TILES ? 1 : 2) msp_celio_fx_kernel(FxArgs a) {
     extern __shared__ __align__(16) unsigned char ce_smem[];
     const CeArgs &c = a.c;
     longlong2 *V = reinterpret_cast<longlong2 *>(ce_smem);
     uint4 *U = reinterpret_cast<uint4 *>(V + ((c.V + 7) & ~7ll));  // fx_swz stays inside blocks of 8
-    FxFactor *fac = reinterpret_cast<FxFactor *>(U + (size_t)a.nf * FX_FRAG);
+    FxFactor *fac = reinterpret_cast<FxFactor *>(U + a.ulen);
     int *base = reinterpret_cast<int *>(fac + a.nf);
     int *offs = base + a.nbase;
     __shared__ double red[64];
@@ -887,8 +994,8 @@ __global__ void __launch_bounds__(FX_THREADS, 1) msp_celio_fx_kernel(FxArgs a) {
         const int s = st / c.A, blk = c.mats_per_snap ? s : 0;
         __syncthreads();
         if (blk != loaded) {
-            const uint4 *src = a.frag + (size_t)blk * a.nf * FX_FRAG;
-            for (int i = tid; i < a.nf * FX_FRAG; i += nt) U[i] = src[i];
+            const uint4 *src = a.frag + (size_t)blk * a.ulen;
+            for (int i = tid; i < a.ulen; i += nt) U[i] = src[i];
             loaded = blk;
         }
         if (tid == 0) s_bad = a.good[blk] ? 0 : 1;
@@ -955,10 +1062,13 @@ __global__ void __launch_bounds__(FX_THREADS, 1) msp_celio_fx_kernel(FxArgs a) {
             for (int r = 0; r < c.k; ++r)
                 for (int f = 0; f < a.nf; ++f) {
                     const FxFactor &ff = fac[f];
-                    const int tiles = (ff.groups + 8 * ff.p - 1) / (8 * ff.p);
-                    for (int tile = warp; tile < tiles; tile += FX_THREADS / 32)
-                        fx_tile(V, U + (size_t)f * FX_FRAG, ff, base + ff.base0, offs + ff.f.off, tile,
-                                lane, xmax);
+                    if (ff.lanes) {
+                        fx_small(V, U + ff.u0, ff, base + ff.base0, offs + ff.f.off);
+                    } else if (TILES) {
+                        const int tiles = (ff.groups + 8 * ff.p - 1) / (8 * ff.p);
+                        for (int tile = warp; tile < tiles; tile += FX_THREADS / 32)
+                            fx_tile(V, U + ff.u0, ff, base + ff.base0, offs + ff.f.off, tile, lane, xmax);
+                    }
                     __syncthreads();
                 }
         }
@@ -1297,6 +1407,16 @@ static int ce_cuda(cudaError_t e) {
 
 static size_t ce_align(size_t x) { return (x + 255) & ~(size_t)255; }
 
+static int ce_sms() {
+    int dev = 0, sms = 152;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+        cudaGetLastError();
+        sms = 152;
+    }
+    return sms;
+}
+
 struct CePlan {
     std::vector<CeFactor> fac;
     std::vector<long long> offs;
@@ -1310,9 +1430,45 @@ struct CePlan {
     bool fx = false;
     std::vector<FxFactor> fxf;
     std::vector<FxOp> fxo;
-    int nbase = 0;
+    int nbase = 0, ulen = 0;
+    bool tiles = false;
     size_t fx_smem = 0;
 };
+
+// Time of one application of a factor to a state in each form, us, from the
+// measurements beside the kernels.
+static double fx_tiles_us(const FxFactor &f) {
+    const double tiles = (f.groups + 8 * f.p - 1) / (8 * f.p);
+    return f.p == 1 ? std::max(2.2, 0.6 + 0.27 * tiles) : std::max(2.6, 0.6 + 0.36 * tiles);
+}
+
+static double fx_integer_us(const CePlan &p, const FxFactor &f) {
+    const double alone = std::max(1.0, 0.6 + 3.7e-4 * (double)p.V * f.f.D);
+    return p.states > ce_sms() ? 0.85 * alone : alone;
+}
+
+// The double-word form (MIXED): a thread per group, D^2 products long, or a warp per
+// group in FP64 where D is not register-resident.
+static double dw_us(const CePlan &p, const CeFactor &f) {
+    const double G = (double)(p.V / f.D);
+    const bool resident = f.D <= 6 || (f.D >= 8 && f.D <= 10) || f.D == 12 || f.D == 16;
+    return resident ? 0.5 * std::max(1.0, G / 400.0) + 0.0225 * f.D * f.D * std::max(1.0, G / 165.0)
+                    : 3.0 + 0.58 * G;
+}
+
+// Whether the fixed-point form is the faster one in MIXED, its preparation (14 us)
+// counted in.  us per factor, fixed point / double words: D = 4, V = 128, 1.0 / 1.0, with
+// its two single-spin factors (merged in the one, apart in the other) 1.1 / 2.3, V = 512,
+// 1.5 / 1.05, V = 2048, 4.3 / 2.2; D = 6, V = 768, 2.4 / 1.5; D = 8, V = 256, 2.0 / 2.0, V =
+// 1024, 3.4 / 2.1; D = 10, V = 320, 2.1 / 2.7, V = 1280, 5.0 / 2.8; D = 16, V = 512, 2.1 /
+// 6.3, V = 8192, 19.1 / 19.6.  In FP64 the form on the FP64 pipe is nowhere faster.
+static bool fx_faster(const msp_celio_args *a, const CePlan &p) {
+    double fx = 0.0, dw = 0.0;
+    for (const FxFactor &f : p.fxf) fx += f.lanes ? fx_integer_us(p, f) : fx_tiles_us(f);
+    for (const CeFactor &f : p.fac) dw += dw_us(p, f);
+    const double rounds = std::max(1.0, (double)p.states / ce_sms());
+    return 14.0 < (dw - fx) * rounds * a->trotter_k * std::max(0, a->num_times - 1);
+}
 
 // Merges single-digit factors into factors that act on their digit with only
 // factors on other digits between, and lists each product's operands.  False
@@ -1390,9 +1546,17 @@ static bool fx_plan(const msp_celio_args *a, CePlan &p) {
         f.groups = (int)(p.V / f.f.D);
         f.base0 = p.nbase;
         p.nbase += f.groups;
+        if (f.f.D <= FX_SMALL && fx_integer_us(p, f) < fx_tiles_us(f)) {
+            f.lanes = 1;
+            while (f.lanes < f.f.D && (long long)f.groups * 2 * f.lanes <= FX_THREADS) f.lanes *= 2;
+        } else {
+            p.tiles = true;
+        }
+        f.u0 = p.ulen;
+        p.ulen += f.lanes ? f.f.D * f.f.D : FX_FRAG;
         p.fxf.push_back(f);
     }
-    p.fx_smem = (size_t)((p.V + 7) & ~7ll) * 16 + p.fxf.size() * (FX_FRAG * 16 + sizeof(FxFactor)) +
+    p.fx_smem = (size_t)((p.V + 7) & ~7ll) * 16 + (size_t)p.ulen * 16 + p.fxf.size() * sizeof(FxFactor) +
                 ((size_t)p.nbase + p.offs.size()) * 4;
     return !p.fxf.empty();
 }
@@ -1494,7 +1658,8 @@ static int ce_plan(const msp_celio_args *a, CePlan &p) {
         return ce_fail(MSP_ERR_UNSUPPORTED, "msp_celio: state does not fit in shared memory");
     p.dw = a->precision == MSP_PREC_MIXED;
     // the kernel's static arrays take under 1 KB
-    p.fx = p.use_smem && fx_plan(a, p) && p.fx_smem + 1024 <= (size_t)optin;
+    p.fx = p.use_smem && fx_plan(a, p) && p.fx_smem + 1024 <= (size_t)optin &&
+           (!p.dw || fx_faster(a, p));
     return MSP_OK;
 }
 
@@ -1503,7 +1668,7 @@ static size_t fx_workspace(const msp_celio_args *a, const CePlan &p) {
     if (!p.fx) return 0;
     const size_t blocks = a->mats_per_snapshot ? (size_t)a->num_snapshots : 1;
     return ce_align(p.fxf.size() * sizeof(FxFactor) + 16) + ce_align(p.fxo.size() * sizeof(FxOp) + 16) +
-           ce_align(blocks * p.fxf.size() * FX_FRAG * 16) + ce_align(blocks * 4) +
+           ce_align(blocks * (size_t)p.ulen * 16) + ce_align(blocks * 4) +
            ce_align((size_t)p.states * 4);
 }
 
@@ -1524,16 +1689,6 @@ static size_t ce_workspace(const msp_celio_args *a, const CePlan &p) {
         }
     }
     return b;
-}
-
-static int ce_sms() {
-    int dev = 0, sms = 152;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
-        cudaGetLastError();
-        sms = 152;
-    }
-    return sms;
 }
 
 }  // namespace
@@ -1630,7 +1785,7 @@ int msp_celio_run(const msp_celio_args *a, void *workspace, size_t workspace_byt
             FxOp *fo = (FxOp *)w;
             w += ce_align(p.fxo.size() * sizeof(FxOp) + 16);
             fx.frag = (uint4 *)w;
-            w += ce_align(blocks * p.fxf.size() * FX_FRAG * 16);
+            w += ce_align(blocks * (size_t)p.ulen * 16);
             fx.good = (int *)w;
             w += ce_align(blocks * 4);
             fx.done = (int *)w;
@@ -1639,6 +1794,7 @@ int msp_celio_run(const msp_celio_args *a, void *workspace, size_t workspace_byt
             fx.ops = fo;
             fx.nf = (int)p.fxf.size();
             fx.nbase = p.nbase;
+            fx.ulen = p.ulen;
             rc = ce_cuda(cudaMemcpyAsync(ff, p.fxf.data(), p.fxf.size() * sizeof(FxFactor),
                                          cudaMemcpyHostToDevice, st));
             if (rc == MSP_OK)
@@ -1646,29 +1802,28 @@ int msp_celio_run(const msp_celio_args *a, void *workspace, size_t workspace_byt
                                              cudaMemcpyHostToDevice, st));
             if (rc == MSP_OK) rc = ce_cuda(cudaMemsetAsync(fx.good, 0xff, blocks * 4, st));
             if (rc == MSP_OK) rc = ce_cuda(cudaMemsetAsync(fx.done, 0, (size_t)p.states * 4, st));
+            void (*const fxk)(FxArgs) = p.tiles ? msp_celio_fx_kernel<true> : msp_celio_fx_kernel<false>;
             if (rc == MSP_OK)
-                rc = ce_cuda(cudaFuncSetAttribute(msp_celio_fx_kernel,
-                                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
+                rc = ce_cuda(cudaFuncSetAttribute(fxk, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                   (int)p.fx_smem));
             if (rc != MSP_OK) return rc;
             for (size_t b0 = 0; b0 < blocks; b0 += 65535) {
                 FxArgs q = fx;
                 q.c.mats += b0 * (size_t)k.mats_len;
-                q.frag += b0 * p.fxf.size() * FX_FRAG;
+                q.frag += b0 * (size_t)p.ulen;
                 q.good += b0;
                 const unsigned bn = (unsigned)(blocks - b0 < 65535 ? blocks - b0 : 65535);
                 msp_celio_fx_prep_kernel<<<dim3((unsigned)p.fxf.size(), bn), 256, 0, st>>>(q);
             }
             int occ = 1;
-            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, msp_celio_fx_kernel, FX_THREADS,
-                                                              p.fx_smem) != cudaSuccess ||
+            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fxk, FX_THREADS, p.fx_smem) != cudaSuccess ||
                 occ < 1) {
                 cudaGetLastError();
                 occ = 1;
             }
             const long long cap = (long long)sms * occ;
             const int grid = (int)(p.states < cap ? p.states : cap);
-            msp_celio_fx_kernel<<<grid, FX_THREADS, p.fx_smem, st>>>(fx);
+            fxk<<<grid, FX_THREADS, p.fx_smem, st>>>(fx);
             rc = ce_cuda(cudaGetLastError());
             if (rc != MSP_OK) return rc;
             k.done = fx.done;

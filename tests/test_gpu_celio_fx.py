@@ -182,3 +182,12 @@ def test_digits_of_dimension_one(dims, prec):
     # 36 products of 2^-40 each in double-words
     tol = 1e-13 if prec == _lib.PREC_FP64 else 1e-10
     assert _pure(dims, factors, 2, 4, prec=prec, seed=last) <= tol
+
+
+# the integer form of small factors where its lanes per group and its rounds change:
+# one group, a lane per row, rows shared by fewer lanes, more groups than threads
+@pytest.mark.parametrize("d", [1, 2, 3, 4])
+@pytest.mark.parametrize("groups", [1, 7, 31, 32, 33, 64, 65, 128, 129, 255, 257])
+def test_small_factors(d, groups):
+    dims, factors = [2, d, groups], [(0, 1), (0, -1)] + ([(1, -1)] if d > 1 else [])
+    assert _pure(dims, factors, 2, 4, seed=groups + d) <= 1e-13
