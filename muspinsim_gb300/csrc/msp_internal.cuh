@@ -184,6 +184,7 @@ cudaError_t launch_split_dw(const double *Hsys, size_t nh, const double *Z, size
 // (msp_jacobi_warp.cu) writes eigenvectors to SnapArgs::evec; the snapshot
 // kernels refine them.  Bytes of that scratch for num_snap snapshots (0 when
 // the form does not apply).
+int large_sms();  // SMs of the current device
 bool jacobi_warp_supported(int n);
 size_t snap_evec_bytes(int n, long long num_snap);
 cudaError_t launch_jacobi_warp(const SnapArgs &a, cudaStream_t st);

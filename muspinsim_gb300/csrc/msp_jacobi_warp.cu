@@ -42,6 +42,8 @@
 // refinement stage restores full accuracy.  Convergence test and tolerances are those of
 // msp_jacobi.cuh (FP32: off-diagonal norm <= 4e-7 of the total, or a
 // rounding floor of 2e-5 that a sweep no longer shrinks).
+#include <algorithm>
+
 #include "msp_internal.cuh"
 #include "msp_jacobi.cuh"
 
@@ -413,18 +415,22 @@ bool jacobi_warp_supported(int n) {
 // First stage of the two-stage snapshots.  Large batches take the Householder +
 // QL form (msp_ql_warp.cu), whose time is flat until its CTAs, of 16 or 32
 // matrices, fill the SMs; smaller ones would leave most of them idle and keep the
-// Jacobi, a warp or less per matrix.  Measured, Jacobi against QL in us: n = 32,
-// 500 snapshots 185 / 211, 1,000 254 / 216; n = 24, 1,000 149 / 159, 1,500 172 /
-// 161; n = 16, 2,000 75 / 79, 3,000 88 / 79; n = 8, 3,000 30 / 30, 10,000 83 / 54;
-// n = 6, 4,000 23 / 23, 10,000 49 / 44; n = 4, 10,000 25 / 27.  MSP_EIGH_WARP =
-// 0 or 2 pins one form.
+// Jacobi, a warp or less per matrix, whose time steps up with every warp per
+// scheduler, 608 snapshots.  QL pays from the second of them at n = 32 on, from the
+// third at n = 24, ... , the sixth at n = 12.  Stage in us, Jacobi / QL: n = 32, 500
+// snapshots 192 / 205, 700 242 / 213; n = 28, 700 183 / 180; n = 24, 1,200 156 / 170,
+// 1,500 180 / 172; n = 20, 1,800 116 / 133, 2,200 138 / 135; n = 16, 2,200 82 / 86,
+// 2,700 95 / 88; n = 14, 2,700 70 / 76, 3,300 95 / 78; n = 12, 2,700 60 / 65, 4,000 86 /
+// 65; n = 10, 3,300 54 / 55, 4,000 70 / 55; n = 8, 3,300 41 / 40, 10,000 95 / 63; n = 6,
+// 4,000 30 / 30, 10,000 58 / 47; n = 4, 10,000 32 / 32.  MSP_EIGH_WARP = 0 or 2 pins
+// one form.
 #ifndef MSP_EIGH_WARP
 #define MSP_EIGH_WARP 1
 #endif
 cudaError_t launch_jacobi_warp(const SnapArgs &a, cudaStream_t st) {
     if (MSP_EIGH_WARP == 2 && ql_warp_supported(a.n)) return launch_ql_warp(a, st);
     if (MSP_EIGH_WARP == 1 && ql_warp_supported(a.n) && a.n > 4 &&
-        (a.num_snap >= 4096 || (long long)a.num_snap * a.n >= 32768))
+        (a.num_snap >= 4096 || a.num_snap > 4 * large_sms() * std::max(1, 8 - a.n / 4)))
         return launch_ql_warp(a, st);
     if (a.num_snap <= 0) return cudaSuccess;
     switch (a.n + (a.n & 1)) {

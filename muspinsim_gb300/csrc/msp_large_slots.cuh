@@ -38,7 +38,6 @@ cudaError_t launch_large_fast64(const SnapArgs &a, double *scratch, int grid, cu
                                 int threads, int first, int count, const int *redo);
 cudaError_t launch_large_rho64(const SnapArgs &a, double *scratch, int grid, cudaStream_t st,
                                int integral, int first, int count, const int *redo);
-int large_sms();
 
 // The QL recurrence between two rounds of its kernel.
 struct QlState {

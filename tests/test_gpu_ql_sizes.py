@@ -70,3 +70,16 @@ def test_spectra(n, prec):
                np.diag(rng.normal(size=n)).astype(complex), tri,
                np.kron(np.eye(2), _herm(rng, n // 2)), 0.5 * (H + H.conj().T)):
         _check(Hs, Z, np.zeros((S, 3)), prec, rng, [0, 1, S - 1])
+
+
+# both sides of the batch size from which the dispatch takes QL: 608 snapshots (a warp
+# per scheduler of 152 SMs) times 8 - n / 4, at least one
+@pytest.mark.parametrize("prec", [_lib.PREC_FP64, _lib.PREC_MIXED])
+@pytest.mark.parametrize("n,edge", [(10, 3648), (12, 3040), (16, 2432), (20, 1824), (22, 1824),
+                                    (24, 1216), (28, 608), (32, 608)])
+@pytest.mark.parametrize("over", [0, 1])
+def test_dispatch_edges(n, edge, over, prec):
+    rng = np.random.default_rng(100 + n)
+    S = edge + over
+    Z = np.array([_herm(rng, n) for _ in range(3)])
+    _check(_herm(rng, n), Z, 0.3 * rng.normal(size=(S, 3)), prec, rng, [0, 33, S // 2, S - 2, S - 1])
