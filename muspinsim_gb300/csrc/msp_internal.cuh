@@ -13,6 +13,12 @@ namespace msp {
 // zero.
 constexpr float REFLECT_TINY = 1e-28f, REFLECT_UP = 1152921504606846976.f;  // 2^60
 
+// The FP32 first stage of n <= 32 reports a matrix that is not a number as not
+// converged in batches below this size, in larger ones as converged, whichever of
+// its two forms takes the batch (launch_jacobi_warp): powder_scan and
+// MultiSystemBatch raise for the one and return NaN rows for the other.
+constexpr int STAGE1_REPORT_NAN = 4096;
+
 template <typename T>
 struct PairCoef;
 template <>

@@ -282,6 +282,10 @@ __global__ void __launch_bounds__(JW_WARPS * 32, M <= 24 ? 5 : 4) msp_jacobi_war
                 status = MSP_ITEM_OK;
                 break;
             }
+            if (off != off) {  // not a number
+                if (a.num_snap >= STAGE1_REPORT_NAN) status = MSP_ITEM_OK;
+                break;
+            }
             if (sweep >= a.max_sweeps) break;
             prev_off = off;
             for (int step = 0; step < M - 1; ++step) {

@@ -204,11 +204,6 @@ __global__ void __launch_bounds__(TRI_WARPS * 32) msp_tri_warp_kernel(SnapArgs a
 constexpr int QL_APPLY = 8;                         // warps that apply rotations
 constexpr int QL_THREADS = 32 * (QL_APPLY + 1);
 constexpr int QL_AHEAD = 2;  // reflectors fetched ahead of the one that acts
-// A matrix that is not a number splits everywhere and counts as converged, except in
-// batches below this size: the Jacobi reports it there (powder_scan and
-// MultiSystemBatch then raise), and which of the two a batch takes
-// (launch_jacobi_warp) is not the caller's concern.
-constexpr int QL_REPORT_NAN = 4096;
 
 // GM matrices of up to NM x NM per CTA, LN lanes per matrix in the application.
 template <int NM>
@@ -269,7 +264,8 @@ __global__ void __launch_bounds__(QL_THREADS, 2) msp_ql_kernel(SnapArgs a) {
             nan |= x != x;
             norm = fmaxf(norm, x);
         }
-        if (nan && a.num_snap < QL_REPORT_NAN) st = MSP_ITEM_NOT_CONVERGED;
+        // it splits everywhere and would count as converged
+        if (nan && a.num_snap < STAGE1_REPORT_NAN) st = MSP_ITEM_NOT_CONVERGED;
         // 0 for an overflowed matrix: its entries become NaN and split everywhere
         const float inv = norm < 1e37f ? 2.f / pow2_above(norm) : 0.f;
         for (int i = 0; i < n; ++i) {

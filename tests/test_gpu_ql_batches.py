@@ -149,3 +149,22 @@ def test_field_that_is_not_a_number_is_reported(n, S):
                                    np.linspace(0, 1, 8), precision=prec)
         flagged = np.nonzero(st.cpu().numpy() & _lib.MSP_ITEM_NOT_CONVERGED)[0]
         assert flagged.tolist() == bad
+
+
+@pytest.mark.parametrize("n", [4, 6, 24])
+def test_field_that_is_not_a_number_in_large_batches(n):
+    """MIXED batches of 4,096 snapshots and more carry it through; FP64 reports it."""
+    from muspinsim_gb300 import _lib, kernels
+    from tests.helpers import random_hermitian
+
+    rng = np.random.default_rng(n)
+    S = 4100
+    H, Z = random_hermitian(rng, n), np.array([random_hermitian(rng, n) for _ in range(3)])
+    B, p = 0.1 * rng.normal(size=(S, 3)), np.tile([0.0, 0.0, 1.0], (S, 1))
+    B[7] = np.nan
+    for prec, bad in ((_lib.PREC_MIXED, []), (_lib.PREC_FP64, [7])):
+        out, st = kernels.powder_run(n, H, Z, B, p, np.ones(S), np.arange(S, dtype=np.int32), S,
+                                     np.linspace(0, 1, 8), precision=prec)
+        assert np.nonzero(st.cpu().numpy() & _lib.MSP_ITEM_NOT_CONVERGED)[0].tolist() == bad
+        ok = np.isfinite(out.cpu().numpy()).all(axis=1)
+        assert not ok[7] and ok.sum() == S - 1
