@@ -571,7 +571,9 @@ __host__ __device__ inline RowShape row_shape(int n, int threads) {
 
 // At most four rows per thread.  (Eight, in half the threads, spill at 96
 // registers and leave too few warps at 128: scan of n = 32, 27 ms against 22.)
-inline int row_threads(int n) { return n <= 8 ? 32 : n <= 16 ? 64 : n <= 24 ? 160 : 256; }
+// Four rows per thread of n = 20 need 100 threads: 160 leave room for fewer CTAs (2,000
+// snapshots in three rounds of six per SM, 88 us; 75 in two of eight).
+inline int row_threads(int n) { return n <= 8 ? 32 : n <= 16 ? 64 : n <= 20 ? 128 : n <= 24 ? 160 : 256; }
 
 // Row stride of the FP32 matrices: even, so that two elements of a row operand are
 // one 16-byte load (the plain products are bound by shared-memory loads: scan of n = 32
