@@ -376,7 +376,7 @@ static Layout powder_layout(const msp_powder_args *a, bool lean = false) {
     off += align256(L.two_stage ? snap_evec_bytes(a->n, a->num_snap) : 0);
     // n <= MSP_MAX_DIM: Hsys and Z as double-words for the FP32 stages
     L.hdw = off;
-    L.split = a->n <= MSP_MAX_DIM && a->num_snap > 0 && (mixed || !lean);
+    L.split = a->n <= MSP_MAX_DIM && a->num_snap > 0 && (mixed || (!lean && a->n > S64_DIRECT_MAX));
     off += align256(L.split ? (size_t)4 * a->n * a->n * 16 : 0);
     L.large = off;
     if (a->n > MSP_MAX_DIM) {

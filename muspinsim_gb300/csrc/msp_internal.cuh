@@ -203,6 +203,9 @@ cudaError_t launch_snapshots_refine(const SnapArgs &a, int mode, int precision, 
 cudaError_t launch_snapshots(const SnapArgs &a, int mode, int precision, cudaStream_t st,
                              int threads = 0, int grid = 0);
 // FP64 snapshots and eigensolver, n <= 64 (msp_snap64.cu).
+// Up to S64_DIRECT_MAX an FP64 rotation diagonalises the matrix (powder of n = 2 and 16
+// orientations: 33 us in all; 55 through FP32 vectors, 39 by FP64 Jacobi sweeps).
+constexpr int S64_DIRECT_MAX = 2;
 size_t snap64_smem_bytes(int n, int fac_len, int threads);
 int snap64_occupancy(int n, int threads, bool pre);
 cudaError_t launch_snapshots64(const SnapArgs &a, int mode, bool pre, cudaStream_t st, int threads,

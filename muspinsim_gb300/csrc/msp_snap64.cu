@@ -432,6 +432,37 @@ __noinline__ __device__ int eigenpairs64(int n, int fac_len, const HSource h, in
     return st;
 }
 
+// The same for n <= S64_DIRECT_MAX: one FP64 rotation, by every warp.
+__noinline__ __device__ int eigenpair64(int n, int fac_len, const HSource h, int max_sweeps) {
+    extern __shared__ __align__(16) char smem[];
+    const S64 s = carve64(smem, n, fac_len);
+    const int tid = threadIdx.x, lane = tid & 31;
+    cx<double> v = mk<double>(0.0, 0.0);  // entries 00, 01, 11 of lanes 0, 1, 2
+    if (lane < n * (n + 1) / 2) v = h_entry(h, (size_t)n * n, lane < 2 ? lane : 3);
+    const double h0 = __shfl_sync(0xffffffffu, v.re, 0), h1 = __shfl_sync(0xffffffffu, v.re, 2);
+    const cx<double> b =
+        mk<double>(__shfl_sync(0xffffffffu, v.re, 1), __shfl_sync(0xffffffffu, v.im, 1));
+    const double tol = JacobiConst<double>::tol, off = 2.0 * cabs2(b), fro = h0 * h0 + h1 * h1 + off;
+    JRot<double> R;
+    double e0, e1;
+    jacobi_rotation<double>(h0, h1, b, off <= tol * tol * fro || max_sweeps < 1 ? CUDART_INF : 0.0, 0, 1, R,
+                            e0, e1);
+    const bool ok = (off <= tol * tol * fro || max_sweeps > 0) && fro >= 0.0;  // false for a NaN
+    if (tid == 0) {
+        const int ld = n + (n & 1) + 1;
+        s.lam[0] = e0;
+        s.D0[0] = mk<double>(R.c, 0.0);
+        if (n == 2) {
+            s.lam[1] = e1;
+            s.D0[1] = mk<double>(R.sr, R.si);
+            s.D0[ld] = mk<double>(-R.sr, R.si);
+            s.D0[ld + 1] = mk<double>(R.c, 0.0);
+        }
+    }
+    __syncthreads();
+    return ok ? MSP_ITEM_OK : MSP_ITEM_NOT_CONVERGED;
+}
+
 }  // namespace
 
 // ------------------------------------------------------------------ eigh
@@ -446,28 +477,33 @@ __global__ void __maxnreg__(128)
     const int tid = threadIdx.x, nt = blockDim.x;
     for (int bidx = blockIdx.x; bidx < batch; bidx += gridDim.x) {
         const HSource h = {Hin + (size_t)bidx * n * n, nullptr, nullptr};
-        SnapSmem<float> f = snap_carve<float, true>(s.region, n, false, 0);
-        for (int e = tid; e < m * (m + 1) / 2; e += nt) {
-            int i, j;
-            tri_index(e, j, i);  // j >= i
-            cx<double> v = mk<double>(0.0, 0.0);
-            if (j < n) v = h.Hsys[(size_t)i * n + j];
-            if (i == j) v.im = 0.0;
-            const cx<float> hi = mk<float>((float)v.re, (float)v.im);
-            const cx<float> lo = mk<float>((float)(v.re - (double)hi.re), (float)(v.im - (double)hi.im));
-            f.w.H[i * ldh + j] = hi;
-            f.w.H[j * ldh + i] = conj(hi);
-            f.Hh[i * ld + j] = hi;
-            f.Hl[i * ld + j] = lo;
-            if (i != j) {
-                f.Hh[j * ld + i] = conj(hi);
-                f.Hl[j * ld + i] = conj(lo);
+        int st;
+        if (n <= S64_DIRECT_MAX) {
+            st = eigenpair64(n, 0, h, max_sweeps);
+        } else {
+            SnapSmem<float> f = snap_carve<float, true>(s.region, n, false, 0);
+            for (int e = tid; e < m * (m + 1) / 2; e += nt) {
+                int i, j;
+                tri_index(e, j, i);  // j >= i
+                cx<double> v = mk<double>(0.0, 0.0);
+                if (j < n) v = h.Hsys[(size_t)i * n + j];
+                if (i == j) v.im = 0.0;
+                const cx<float> hi = mk<float>((float)v.re, (float)v.im);
+                const cx<float> lo = mk<float>((float)(v.re - (double)hi.re), (float)(v.im - (double)hi.im));
+                f.w.H[i * ldh + j] = hi;
+                f.w.H[j * ldh + i] = conj(hi);
+                f.Hh[i * ld + j] = hi;
+                f.Hl[i * ld + j] = lo;
+                if (i != j) {
+                    f.Hh[j * ld + i] = conj(hi);
+                    f.Hl[j * ld + i] = conj(lo);
+                }
             }
+            __syncthreads();
+            hamiltonian_row_norms(f, n, m);
+            st = jacobi_sweeps<float>(f.w, m, max_sweeps);
+            st = eigenpairs64(n, 0, h, st, max_sweeps, true);
         }
-        __syncthreads();
-        hamiltonian_row_norms(f, n, m);
-        int st = jacobi_sweeps<float>(f.w, m, max_sweeps);
-        st = eigenpairs64(n, 0, h, st, max_sweeps, true);
         // ascending order, ties by index (stable)
         for (int j = tid; j < n; j += nt) {
             const double lj = s.lam[j];
@@ -500,6 +536,7 @@ template <bool PRE>
 __device__ __forceinline__ int snapshot64(const SnapArgs &a, const SnapSource &src, int sn, S64 &s,
                                           int n, int m, int fac_len) {
     const HSource h = {src.Hsys, src.Z, a.field + 3 * (size_t)src.g};
+    if (!PRE && n <= S64_DIRECT_MAX) return eigenpair64(n, fac_len, h, a.max_sweeps);
     SnapSmem<float> f = snap_carve<float, true>(s.region, n, false, 0);
     load_hamiltonian<float, true, PRE>(src.Hsys, src.Z, src.Hdw, src.Zdw, h.b, n, m, f);
     const int st = snap_eigvecs<float, PRE>(a, sn, src.g, n, m, m + 1, f);

@@ -47,6 +47,22 @@ def test_scales(n, scale):
     _check(scale * np.array([random_hermitian(rng, n) for _ in range(3)]))
 
 
+# one rotation: any scale, diagonal and degenerate matrices, one snapshot and many
+@pytest.mark.parametrize("scale", [1e-100, 1e-20, 1.0, 1e20, 1e100])
+@pytest.mark.parametrize("n", [1, 2])
+def test_two_levels(n, scale):
+    rng = np.random.default_rng(n)
+    H = np.array([random_hermitian(rng, n) for _ in range(300)])
+    H[0] = np.diag(np.arange(n))
+    H[1] = np.eye(n)
+    H[2, -1, 0] *= 1e-9
+    H[2, 0, -1] = np.conj(H[2, -1, 0])
+    _check(scale * H)
+    H[3, 0, -1] = H[3, -1, 0] = np.nan
+    st = kernels.eigh(scale * H)[2].cpu().numpy()
+    assert st[3] == 1 and st.sum() == 1
+
+
 @pytest.mark.parametrize("n", [4, 8, 24, 32, 64])
 def test_degenerate_and_clustered(n):
     rng = np.random.default_rng(n)
