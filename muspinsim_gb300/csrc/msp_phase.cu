@@ -1438,7 +1438,7 @@ cudaError_t launch_fast_amplitudes(const double *evals, const double *evecs,
 // sum_i conj(z_i) sum_j C_ij z_j, C_ij = rho_ij op_ji: n sines and cosines per
 // time instead of n^2, and 4 n^2 FMAs.  l t is reduced to its fraction
 // exactly (product and its rounding error by FMA), so z is good to 1e-16 at
-// any l t.  One CTA takes TT times of one operator, 16 rows at a time; C in
+// any l t.  One CTA takes TT times of one operator, 256 / TT rows at a time; C in
 // slabs of EV_COLS columns.  n = 24, 2 operators, 2000 times: 1.43 ms (one
 // thread per time, a sincos per pair) -> 0.038 ms.
 #define MSP_EV_THREADS 256
@@ -1508,9 +1508,11 @@ static cudaError_t evolve_expect(const double *evals, const double *rho, const d
     size_t tail = (size_t)rb * (nc + 1);
     if (tail < MSP_EV_THREADS) tail = MSP_EV_THREADS;  // the final reduction
     const size_t smem = ((size_t)n * TT + tail) * sizeof(cx<double>);
-    const cudaError_t e = cudaFuncSetAttribute(
-        msp_evolve_expect_kernel<TT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
+    if (smem > 48 * 1024) {  // the call costs as much as a small launch
+        const cudaError_t e = cudaFuncSetAttribute(
+            msp_evolve_expect_kernel<TT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+    }
     // operators in slices of the grid's y limit
     for (int o = 0; o < num_ops; o += 65535) {
         // the output rows interleave the operators: the kernel indexes from o
@@ -1528,7 +1530,9 @@ cudaError_t launch_evolve_expect(const double *evals, const double *rho, const d
                                  double *out, cudaStream_t st) {
     if (num_times <= 0 || num_ops <= 0) return cudaSuccess;
     // 16 times per CTA while their n z values leave room for several CTAs per
-    // SM (64 KB at n = 256), else 4
+    // SM (64 KB at n = 256), else 4; a few levels keep a CTA's threads busy only with
+    // many times (n = 2, 50,000 times, 3 operators: 80 us with 16, 31 with 128)
+    if (n <= 4) return evolve_expect<128>(evals, rho, ops, n, num_ops, times, num_times, out, st);
     return n <= 256 ? evolve_expect<16>(evals, rho, ops, n, num_ops, times, num_times, out, st)
                     : evolve_expect<4>(evals, rho, ops, n, num_ops, times, num_times, out, st);
 }
