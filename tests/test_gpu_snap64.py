@@ -140,3 +140,32 @@ def test_temperatures_of_one_launch(prec, tol, mode, length):
         ref = (port.evolve(H, rho, times, [op])[:, 0].real if mode == _lib.MODE_EVOLVE
                else port.integrate_decaying(H, rho, 2.197, [op])[:1].real / 2.197)
         assert np.abs(out[k].cpu().numpy() - ref).max() <= tol
+
+
+# thermal states of one larger spin per launch, a warp's work: I = 1 ... 9/2
+@pytest.mark.parametrize("prec,tol", [(_lib.PREC_FP64, 1e-10), (_lib.PREC_MIXED, 1e-6)])
+@pytest.mark.parametrize("nucleus", ["N", "Cu", "Al", "V", "Nb"])
+def test_thermal_states_of_large_spins(prec, tol, nucleus):
+    from oracle import port
+    from tests.helpers import oracle_system
+
+    rng = np.random.default_rng(7)
+    spins, coup = ["mu", nucleus], [("dipolar", {"i": 1, "j": 2}, workloads.random_vector(rng, 1.0, 2.0))]
+    temps = np.array([2e-5, 1e-4, 0.0, 3.0, 1e-6, np.inf])
+    S, times = len(temps), np.linspace(0.0, 10.0, 30)
+    B = rng.normal(size=(S, 3)) * 0.05
+    B[3] = 0.0
+    p = rng.normal(size=(S, 3))
+    p /= np.linalg.norm(p, axis=1)[:, None]
+    sy = workloads.Workload("s", spins, coup, np.zeros((1, 3)), B[:1], p[0], times).system()
+    out, st = kernels.powder_run(
+        int(np.prod(sy.dimension)), sy.hamiltonian_matrix(), sy.zeeman_operators(), B, p, np.ones(S),
+        np.arange(S, dtype=np.int32), S, times, mode=_lib.MODE_EVOLVE, precision=prec,
+        dims=list(sy.dimension), mu_index=0, gammas=sy.gammas, temperature=temps)
+    assert int(st.max().item()) == 0
+    osy = oracle_system(spins, coup)
+    Z = osy.zeeman_operators()
+    for k in range(S):
+        H = osy.hamiltonian() + np.einsum("a,aij->ij", B[k], Z)
+        ref = port.evolve(H, port.rho0(osy, B[k], p[k], temps[k]), times, [osy.muon_operator(p[k])])
+        assert np.abs(out[k].cpu().numpy() - ref[:, 0].real).max() <= tol
