@@ -15,7 +15,7 @@ import pytest
 from muspinsim_gb300 import _lib, kernels, workloads
 from muspinsim_gb300 import quaternion as Q
 from muspinsim_gb300.orientations import orientation_rows_to_quats, zcw_gen
-from tests.helpers import oracle_powder
+from tests.helpers import oracle_powder, random_hermitian
 
 pytestmark = pytest.mark.gpu
 
@@ -106,3 +106,21 @@ def test_adjoint_matches_direct_sum(dim, orient, nt, slots, t0):
     for a, b in zip(got[0][:2], got[1][:2]):
         a, b = a.cpu().numpy(), b.cpu().numpy()
         assert np.linalg.norm(a - b) <= 1e-9 * np.linalg.norm(b)
+
+
+# a frequency that is not finite: its row is not either, the others are untouched
+@pytest.mark.parametrize("prec", [_lib.PREC_FP64, _lib.PREC_MIXED])
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_non_finite_field(prec, bad):
+    rng = np.random.default_rng(3)
+    n, S = 24, 3000 if prec == _lib.PREC_MIXED else 300
+    H, Z = random_hermitian(rng, n), np.array([random_hermitian(rng, n) for _ in range(3)])
+    B, p = 0.1 * rng.normal(size=(S, 3)), np.tile([0.0, 0.0, 1.0], (S, 1))
+    slot = (np.arange(S) * 3 // S).astype(np.int32)
+    times = np.linspace(0.0, 3.0, 2000)
+    good = kernels.powder_run(n, H, Z, B, p, np.full(S, 1 / S), slot, 3, times, precision=prec)[0]
+    B[S // 2] = bad
+    got = kernels.powder_run(n, H, Z, B, p, np.full(S, 1 / S), slot, 3, times, precision=prec)[0]
+    got, good = got.cpu().numpy(), good.cpu().numpy()
+    assert not np.isfinite(got[1]).any()
+    assert np.abs(got[[0, 2]] - good[[0, 2]]).max() <= 1e-11
