@@ -56,6 +56,15 @@ def test_sample_counts(nt, t0):
     assert _compare(["mu", "e"], {1: 2.0}, t0 + 0.004 * np.arange(nt), 20.0) <= 1e-10
 
 
+# few samples of long steps: up to five squarings of the step are left out
+@pytest.mark.parametrize("spins,diss", [(["mu", "e"], {1: 2.0}), (["mu", "N"], {1: 0.7}),
+                                        (["mu", "e", "H"], {0: 0.1, 2: 0.3})])
+@pytest.mark.parametrize("nt", [2, 3, 5, 9, 17, 33, 40])
+@pytest.mark.parametrize("t0", [0.0, 0.6])
+def test_long_steps(spins, diss, nt, t0):
+    assert _compare(spins, diss, t0 + 0.3 * np.arange(nt), 20.0) <= 1e-10
+
+
 @pytest.mark.parametrize("temperature", [np.inf, 0.0])
 @pytest.mark.parametrize("rate", [0.0, 50.0])
 def test_rates_and_temperatures(temperature, rate):

@@ -32,6 +32,13 @@ def test_expectation_series(n, nt, nops):
     assert (np.abs(got - ref) / scale).max() <= 1e-11 * np.sqrt(n)
 
 
+# up to n = 4, 128 times per CTA
+@pytest.mark.parametrize("n", [1, 2, 3, 4, 5])
+@pytest.mark.parametrize("nt", [127, 128, 129, 300])
+def test_expectation_series_of_few_levels(n, nt):
+    test_expectation_series(n, nt, 2)
+
+
 @pytest.mark.parametrize("n", [1, 2, 4, 5, 24, 63, 64])
 @pytest.mark.parametrize("batch", [1, 3])
 @pytest.mark.parametrize("shared", ["none", "u", "m"])
