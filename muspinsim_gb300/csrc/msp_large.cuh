@@ -41,13 +41,11 @@ __host__ __device__ inline size_t large_scratch_doubles(int n) {
     return (size_t)5 * n * n + 5 * (size_t)n + 64;
 }
 
-template <typename T>
-struct LargeScratchT {
-    cx<T> *A, *U;
-    T *Zt, *d, *e, *lam;
-    cx<T> *tau;
+struct LargeScratch {
+    cx<double> *A, *U;
+    double *Zt, *d, *e, *lam;
+    cx<double> *tau;
 };
-using LargeScratch = LargeScratchT<double>;
 
 template <typename T>
 struct LargeEps;
@@ -135,28 +133,19 @@ __host__ __device__ inline size_t large_smem_bytes(int n, int threads) {
 // the relative error (2^-23 -> 2^-46 -> 2^-92), so the result is correct to
 // the last bit or two, in a dozen dependent FP64 operations.  Callers keep
 // x inside the seed's range (1e-36 .. 1e36).
-template <typename T>
-__device__ __forceinline__ T rsqrt_newton(T x);
-template <>
-__device__ __forceinline__ double rsqrt_newton<double>(double x) {
+__device__ __forceinline__ double rsqrt_newton(double x) {
     double y = (double)rsqrtf((float)x);
     const double h = 0.5 * x;
     y = y * fma(-h * y, y, 1.5);
     y = y * fma(-h * y, y, 1.5);
     return y;
 }
-// FP32: the hardware approximation and one Newton step
-template <>
-__device__ __forceinline__ float rsqrt_newton<float>(float x) {
-    const float y = rsqrtf(x);
-    return y * fmaf(-0.5f * x * y, y, 1.5f);
-}
 
 // Eigenpairs of the Hermitian matrix already in s.A (full, row-major):
 // eigenvalues into s.lam, eigenvectors (columns) into s.U.  Returns
 // MSP_ITEM_OK or MSP_ITEM_NOT_CONVERGED (QL iteration cap).
-template <typename T>
-__device__ int large_eigh(LargeScratchT<T> s, int n, char *smem) {
+inline __device__ int large_eigh(LargeScratch s, int n, char *smem) {
+    typedef double T;
     const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5;
     const int nw = nt >> 5;
     const int RW = nt < 64 ? nt : 64, G = nt / RW, pr = tid % RW, pg = tid / RW;
@@ -323,7 +312,7 @@ __device__ int large_eigh(LargeScratchT<T> s, int n, char *smem) {
                 h = c * pp;
                 const T x2 = fma(pp, pp, ei * ei);
                 if (x2 > T(1e-36) && x2 < T(1e36)) {
-                    const T y = rsqrt_newton<T>(x2);
+                    const T y = rsqrt_newton(x2);
                     r = x2 * y;
                     e[i + 1] = sn * r;
                     sn = ei * y;

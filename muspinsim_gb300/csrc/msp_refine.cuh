@@ -238,18 +238,18 @@ __device__ __forceinline__ void field_dw(const double *b, float2 &bx, float2 &by
     bz = make_float2(__shfl_sync(0xffffffffu, v.x, 2), __shfl_sync(0xffffffffu, v.y, 2));
 }
 
-// H = Hsys + b . Z into the Jacobi buffer (precision T, padded to m); in
-// MIXED mode also its split H = Hh + Hl into two FP32 matrices.  MIXED
-// with Hdw / Zdw (Hsys and Z pre-split into double-words, (re_hi, im_hi,
+// H = Hsys + b . Z into the Jacobi buffer (FP32, padded to m) unless PRE, and its split
+// H = Hh + Hl into two FP32 matrices.
+// With Hdw / Zdw (Hsys and Z pre-split into double-words, (re_hi, im_hi,
 // re_lo, im_lo) per entry) assembles in double-word FP32 (~2^-47 relative),
 // otherwise in FP64 (split exactly).  blockDim.x is a multiple of 32.
-template <typename T, bool REFINE, bool PRE = false>
+template <bool PRE>
 __device__ void load_hamiltonian(const cx<double> *Hsys, const cx<double> *Z, const float4 *Hdw,
                                  const float4 *Zdw, const double *b, int n, int m,
-                                 SnapSmem<T> &s) {
+                                 SnapSmem<float> &s) {
     const int tid = threadIdx.x, nt = blockDim.x, ld = m + 1, ldh = jacobi_ldh(m);
     const size_t nn = (size_t)n * n;
-    if (REFINE && Hdw != nullptr) {
+    if (Hdw != nullptr) {
         float2 bx, by, bz;
         field_dw(b, bx, by, bz);
         for (int e = tid; e < m * m; e += nt) {
@@ -268,7 +268,7 @@ __device__ void load_hamiltonian(const cx<double> *Hsys, const cx<double> *Z, co
                 hr = dw_two_sum(sr, cr);
                 hi = dw_two_sum(si, ci);
             }
-            if (!PRE) s.w.H[i * ldh + j] = mk<T>((T)hr.x, (T)hi.x);
+            if (!PRE) s.w.H[i * ldh + j] = mk<float>(hr.x, hi.x);
             s.Hh[i * ld + j] = mk<float>(hr.x, hi.x);
             s.Hl[i * ld + j] = mk<float>(hr.y, hi.y);
         }
@@ -283,31 +283,28 @@ __device__ void load_hamiltonian(const cx<double> *Hsys, const cx<double> *Z, co
                 h.re = hs.re + bx * z0.re + by * z1.re + bz * z2.re;
                 h.im = hs.im + bx * z0.im + by * z1.im + bz * z2.im;
             }
-            if (!PRE) s.w.H[i * ldh + j] = mk<T>((T)h.re, (T)h.im);
-            if (REFINE) {
-                const float hr = (float)h.re, hi = (float)h.im;
-                s.Hh[i * ld + j] = mk<float>(hr, hi);
-                s.Hl[i * ld + j] =
-                    mk<float>((float)(h.re - (double)hr), (float)(h.im - (double)hi));
-            }
+            const float hr = (float)h.re, hi = (float)h.im;
+            if (!PRE) s.w.H[i * ldh + j] = mk<float>(hr, hi);
+            s.Hh[i * ld + j] = mk<float>(hr, hi);
+            s.Hl[i * ld + j] = mk<float>((float)(h.re - (double)hr), (float)(h.im - (double)hi));
         }
     }
     __syncthreads();
-    if (REFINE) hamiltonian_row_norms(s, n, m);
+    hamiltonian_row_norms(s, n, m);
 }
 
-// The eigensolve of a snapshot: FP64 or FP32 Jacobi in this CTA, or (PRE)
+// The FP32 eigensolve of a snapshot: Jacobi in this CTA, or (PRE)
 // the FP32 eigenvectors the warp Jacobi stage left in a.evec, with the
 // status it wrote.  Leaves the eigenvectors in s.w.U (row stride ld; m + 1 after Jacobi).
-template <typename T, bool PRE>
+template <bool PRE>
 __device__ __forceinline__ int snap_eigvecs(const SnapArgs &a, int sn, int g, int n, int m, int ld,
-                                            SnapSmem<T> &s) {
-    if (!PRE) return jacobi_sweeps<T>(s.w, m, a.max_sweeps);
+                                            SnapSmem<float> &s) {
+    if (!PRE) return jacobi_sweeps<float>(s.w, m, a.max_sweeps);
     const float2 *X = reinterpret_cast<const float2 *>(a.evec) + (size_t)sn * n * n;
     for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
         const int i = FastDiv(n).div(e), j = e - i * n;
         const float2 x = X[e];
-        s.w.U[i * ld + j] = mk<T>((T)x.x, (T)x.y);
+        s.w.U[i * ld + j] = mk<float>(x.x, x.y);
     }
     const int st = a.status[g];
     __syncthreads();
@@ -499,12 +496,10 @@ __device__ void apply_digit(const cx<TF> *F, int dim, int stride, const cx<T> *X
     __syncthreads();
 }
 
-// Y[j][k] = sum_i conj(U_ij) X_ik for j >= k (row stride ld = n + (n & 1) + 1);
-// NN > 0: n = NN at compile time.
-template <typename T, int NN>
-__device__ __forceinline__ void tri_conj_products(const cx<T> *U, const cx<T> *X, cx<T> *Y,
-                                                  int n_rt) {
-    const int n = NN > 0 ? NN : n_rt, ld = n + (n & 1) + 1, ntri = n * (n + 1) / 2;
+// Y[j][k] = sum_i conj(U_ij) X_ik for j >= k (row stride ld = n + (n & 1) + 1).
+template <typename T>
+__device__ __forceinline__ void tri_conj_products(const cx<T> *U, const cx<T> *X, cx<T> *Y, int n) {
+    const int ld = n + (n & 1) + 1, ntri = n * (n + 1) / 2;
     for (int e = threadIdx.x; e < ntri; e += blockDim.x) {
         int j, k;
         tri_index(e, j, k);

@@ -149,9 +149,8 @@ __global__ void __maxnreg__(64) msp_snap_fast_kernel(SnapArgs a) {
         if (PRE)
             load_hamiltonian_rows(src, a.field + 3 * g, n, s);
         else
-            load_hamiltonian<T, true, PRE>(src.Hsys, src.Z, src.Hdw, src.Zdw, a.field + 3 * g, n, m,
-                                           s);
-        int st = snap_eigvecs<T, PRE>(a, sn, (int)g, n, m, ld, s);
+            load_hamiltonian<PRE>(src.Hsys, src.Z, src.Hdw, src.Zdw, a.field + 3 * g, n, m, s);
+        int st = snap_eigvecs<PRE>(a, sn, (int)g, n, m, ld, s);
         st |= PRE ? eigenpairs_rows(n, false, 0, a.max_refine) : eigenpairs(s, n, m, a.max_refine);
 
         // sigma_p = p . sigma (Pauli), applied on the muon (slowest) digit
@@ -301,13 +300,12 @@ __global__ void __maxnreg__(PRE ? 64 : 96) msp_snap_rho_kernel(SnapArgs a) {
         if (PRE)
             load_hamiltonian_rows(snap_source(a, sn), a.field + 3 * (size_t)sn, n, s);
         else
-            load_hamiltonian<T, true, PRE>(a.Hsys, a.Z, a.Hsys_dw, a.Z_dw,
-                                           a.field + 3 * (size_t)sn, n, m, s);
+            load_hamiltonian<PRE>(a.Hsys, a.Z, a.Hsys_dw, a.Z_dw, a.field + 3 * (size_t)sn, n, m, s);
         // made visible by the eigensolve's barriers
         if (!hot)
             for (int e = tid; e < a.fac_len; e += nt)
                 s.facf[e] = mk<float>((float)s.fac[e].re, (float)s.fac[e].im);
-        int st = snap_eigvecs<T, PRE>(a, sn, sn, n, m, ld, s);
+        int st = snap_eigvecs<PRE>(a, sn, sn, n, m, ld, s);
         st |= PRE ? eigenpairs_rows(n, true, a.fac_len, a.max_refine)
                   : eigenpairs(s, n, m, a.max_refine);
         const cx<T> *U = s.w.U;
@@ -328,7 +326,7 @@ __global__ void __maxnreg__(PRE ? 64 : 96) msp_snap_rho_kernel(SnapArgs a) {
             }
             if (!PRE) {
                 // X holds rho0 U.  rho'_jk (j >= k) -> Y (the other buffer).
-                tri_conj_products<T, 0>(U, X, Y, n);
+                tri_conj_products<T>(U, X, Y, n);
                 __syncthreads();
                 cx<T> *t = Y;
                 Y = const_cast<cx<T> *>(X);

@@ -43,7 +43,7 @@ namespace {
 // entries after: D1 over the FP32 matrix and vectors, D0 next, D2 last, so
 // that D0 can be filled from the FP32 vectors in place.
 struct Snap64Layout {
-    size_t lam0, lam, gn, tdiag, nz, red, acc, dl, corr, rk, ord, cst, scal, fac;
+    size_t lam0, lam, gn, tdiag, nz, red, dl, corr, rk, ord, cst, scal, fac;
     size_t region, xl, total;
 };
 
@@ -59,7 +59,6 @@ __host__ __device__ inline Snap64Layout snap64_layout(int n, int fac_len, int nw
     L.tdiag = lay_take(off, m * 8);
     L.nz = lay_take(off, m * 8);
     L.red = lay_take(off, 2 * (size_t)nwarps * 8);
-    L.acc = lay_take(off, 16);
     L.dl = lay_take(off, m * 4);
     L.corr = lay_take(off, m * 4);
     L.rk = lay_take(off, m * 4);
@@ -88,7 +87,7 @@ __host__ __device__ inline Snap64Layout snap64_layout(int n, int fac_len, int nw
 
 struct S64 {
     cx<double> *D0, *D1, *D2;
-    double *lam0, *lam, *gn, *tdiag, *red, *acc;
+    double *lam0, *lam, *gn, *tdiag, *red;
     unsigned long long *nz;  // bit k of row i: H_ik is not zero
     float *dl, *corr;
     int *rk, *ord, *cst, *scal;
@@ -107,7 +106,6 @@ __device__ __forceinline__ S64 carve64(char *base, int n, int fac_len) {
     s.tdiag = reinterpret_cast<double *>(base + L.tdiag);
     s.nz = reinterpret_cast<unsigned long long *>(base + L.nz);
     s.red = reinterpret_cast<double *>(base + L.red);
-    s.acc = reinterpret_cast<double *>(base + L.acc);
     s.dl = reinterpret_cast<float *>(base + L.dl);
     s.corr = reinterpret_cast<float *>(base + L.corr);
     s.rk = reinterpret_cast<int *>(base + L.rk);
@@ -538,8 +536,8 @@ __device__ __forceinline__ int snapshot64(const SnapArgs &a, const SnapSource &s
     const HSource h = {src.Hsys, src.Z, a.field + 3 * (size_t)src.g};
     if (!PRE && n <= S64_DIRECT_MAX) return eigenpair64(n, fac_len, h, a.max_sweeps);
     SnapSmem<float> f = snap_carve<float, true>(s.region, n, false, 0);
-    load_hamiltonian<float, true, PRE>(src.Hsys, src.Z, src.Hdw, src.Zdw, h.b, n, m, f);
-    const int st = snap_eigvecs<float, PRE>(a, sn, src.g, n, m, m + 1, f);
+    load_hamiltonian<PRE>(src.Hsys, src.Z, src.Hdw, src.Zdw, h.b, n, m, f);
+    const int st = snap_eigvecs<PRE>(a, sn, src.g, n, m, m + 1, f);
     return eigenpairs64(n, fac_len, h, st, a.max_sweeps, !PRE);
 }
 
@@ -680,7 +678,7 @@ __global__ void __maxnreg__(96) msp_snap64_rho_kernel(SnapArgs a) {
                 Y = (Y == s.D1) ? s.D2 : s.D1;
             }
             // rho'_jk (j >= k) into the other buffer
-            tri_conj_products<double, 0>(U, X, Y, n);
+            tri_conj_products<double>(U, X, Y, n);
             __syncthreads();
         }
         // O = p . S on the muon digit: half of sigma_p.  V into the buffer X (free now)
