@@ -10,9 +10,8 @@ muspinsim_gb300/workloads.py.
 
 Metric: P(t) samples/s, one sample = one (orientation, time) value before the
 orientation average.  ``value`` is the mixed-precision pipeline (FP32
-Householder + QL eigensolve + double-word refinement + FP32 phase sum) with
-inputs resident in HBM; the
-all-FP64 pipeline is timed beside it (``fp64``) and the max |dP| between the
+Householder + QL eigensolve + double-word refinement + the phase sum as a
+nonuniform Fourier transform) with inputs resident in HBM; the all-FP64 pipeline is timed beside it (``fp64``) and the max |dP| between the
 two is reported.  ``e2e`` runs the public ``powder_average`` call on host
 inputs (host->device copies and the device->host result inside the timed
 region).
@@ -52,9 +51,9 @@ SMS, FP32_FMA_PER_SM = 152, 128
 # count.
 TRAFFIC_PER_SNAPSHOT = {"eigensolve": 0.117e6 / 2000, "snapshots": 9.458e6 / 2000,
                         "phase": 13.288e6 / 2000}
-# Batches of at least this many snapshots take the Householder + QL
-# eigensolve (smaller ones the warp Jacobi)
-QL_MIN_SNAPSHOTS = 4096
+# Batches of n = 24 of at least this many snapshots take the Householder + QL
+# eigensolve (smaller ones the warp Jacobi): more than two warps per scheduler
+QL_MIN_SNAPSHOTS = 1217
 
 
 def parse_args():
@@ -844,7 +843,7 @@ def run_config4(args, world, rank, local):
                  "samples/s", ms, args, world,
                  f"{min(dims)}_to_{max(dims)}_dim_systems_{n_sys}x{n_or}_orient_{T}_t", cfg,
                  dtype="f32 (Jacobi for n <= 64, Householder + QL for n > 64 and for "
-                       "n <= 32 buckets of 4,096+ snapshots; double-word refinement; phase sum)",
+                       "larger n <= 32 buckets; double-word refinement; phase sum)",
                  fp64=({"value": samples / (out["fp64"][0] * 1e-3),
                         "ms_per_step": out["fp64"][0]} if "fp64" in out else None),
                  max_abs_dP_mixed_vs_fp64=dP, buckets=buckets)
@@ -938,7 +937,7 @@ def run_lindblad(args, world, rank, local):
     """Dissipative powder average (the Lindbladian branch of run_single):
     mu, e, 1H (n = 8, superoperator 64 x 64), dissipation on the electron
     and the proton, B = 3 mT, T = 20 K, 500 ZCW-style orientations, 1000
-    times on 0-10 us.  FP64 (exp(2 pi L dt) propagation on the device)."""
+    times on 0-10 us.  FP64 in both precisions (the real form of L)."""
     import torch
 
     from muspinsim_gb300 import _lib, kernels, workloads
@@ -977,12 +976,12 @@ def run_lindblad(args, world, rank, local):
     ms64 = _events_ms(lambda: step(_lib.PREC_FP64), max(1, min(args.steps, 3)))
     out = step().cpu().numpy()[0]
     out64 = step(_lib.PREC_FP64).cpu().numpy()[0]
-    line = _line("dissipative powder P(t) samples/s, double-word FP32 propagation",
+    line = _line("dissipative powder P(t) samples/s, real FP64 form in both precisions",
                  N * T / (ms * 1e-3), "samples/s", ms,
                  args, world, "mu_e_H_lindblad_500_orient_1000_t",
                  {"orientations": N, "times": T, "dim": n, "superoperator": n * n,
                   "dissipation_MHz": {"e": 2.0, "H": 0.3}, "temperature_K": 20.0},
-                 dtype="f32 double-word (propagation), f64 (construction, measurement)",
+                 dtype="f64",
                  gpu_launches=5 * max(1, args.steps),
                  fp64={"value": N * T / (ms64 * 1e-3), "ms_per_step": ms64},
                  mixed_over_fp64=ms64 / ms,
@@ -1045,8 +1044,9 @@ def run_celio(args, world, rank, local):
     native fast variant, muspinsim/celio.py:318-476): mu + 4 51V (I = 7/2,
     dimension 8192), the shape of the reference's own Celio example;
     8 ZCW-style orientations x 19 random states = 152 states (one per SM),
-    k = 10, 50 times on 0-10 us.  States stay in shared memory; the line's
-    value is the double-word FP32 form, with the FP64 form beside it."""
+    k = 10, 50 times on 0-10 us.  States stay in shared memory, where both
+    precisions take the fixed-point form; larger ones (more nuclei) double-word
+    FP32 (the line's value) and FP64 in global memory."""
     from muspinsim_gb300 import celio, workloads
     from muspinsim_gb300 import quaternion as Q
     from muspinsim_gb300.orientations import orientation_rows_to_quats
@@ -1089,33 +1089,41 @@ def run_celio(args, world, rank, local):
     fp32_peak = 152 * 128 * 2 * 2.07  # GFLOP/s, nominal FP32 FMA rate at 2.07 GHz
     achieved = flops / (ms["mixed"] * 1e-3) / 1e9
     pipe_ops = cmacs * 24 / (ms["mixed"] * 1e-3) / 1e9  # FP32 ops issued per second (12 f32x2)
+    fixed = V <= 8192
     samples = N * T
     line = _line(f"Celio P(t) samples/s (orientation x time, {A} random states each), "
-                 "double-word FP32", samples / (ms["mixed"] * 1e-3), "samples/s", ms["mixed"],
+                 + ("64-bit fixed point" if fixed else "double-word FP32"),
+                 samples / (ms["mixed"] * 1e-3), "samples/s", ms["mixed"],
                  args, world,
                  f"celio_muV{args.celio_nuclei}_dim{V}_{N}_orient_{A}_states_{T}_t_k{k}",
                  {"orientations": N, "states_per_orientation": A, "times": T, "dim": V,
                   "trotter_k": k, "factors_per_pass": len(batch.digits),
                   "l2": ("states resident in shared memory; HBM traffic is the inputs only"
-                         if V <= 8192 else "states in global memory (L2-resident): one launch "
+                         if fixed else "states in global memory (L2-resident): one launch "
                                            "per factor application")},
-                 dtype="f32 double-word", gpu_launches=steps,
+                 dtype=("64-bit fixed point (f16 digits, exact sums)" if fixed
+                        else "f32 double-word"), gpu_launches=steps,
                  state_steps_per_s=N * A * (T - 1) / (ms["mixed"] * 1e-3),
                  fp64={"value": samples / (ms["fp64"] * 1e-3), "ms_per_step": ms["fp64"],
                        "achieved_gflops": flops / (ms["fp64"] * 1e-3) / 1e9,
-                       "fp64_peak_gflops": 1250.0,
-                       "frac": flops / (ms["fp64"] * 1e-3) / 1e9 / 1250.0},
+                       **({} if fixed else {"fp64_peak_gflops": 1250.0,
+                                            "frac": flops / (ms["fp64"] * 1e-3) / 1e9 / 1250.0})},
                  mixed_over_fp64=ms["fp64"] / ms["mixed"],
                  max_abs_dP_mixed_vs_fp64=float(np.abs(outs["mixed"] - outs["fp64"]).max()),
-                 roofline={"bound": "fp32", "achieved": pipe_ops, "peak": fp32_peak,
-                           "unit": "GFLOP/s", "frac": pipe_ops / fp32_peak, "traffic": None,
-                           "algorithmic_gflops": achieved,
-                           "note": "achieved = FP32 operations issued (12 packed f32x2 "
-                                   "instructions = 24 FP32 ops per complex multiply-add of "
-                                   "the anchored double-word product) per second; peak = "
-                                   "nominal FP32 "
-                                   "(152 SMs x 128 lanes x 2 x 2.07 GHz), no measured FP32 "
-                                   "figure on this pool"},
+                 roofline=({"bound": "shared memory and digit handling around the MMAs",
+                            "achieved": achieved, "peak": None, "unit": "GFLOP/s", "frac": None,
+                            "traffic": None, "algorithmic_gflops": achieved,
+                            "note": "achieved = 8 flops per complex multiply-add of the factor "
+                                    "applications; the exact products take 104 FP16 MMAs each"}
+                           if fixed else
+                           {"bound": "fp32", "achieved": pipe_ops, "peak": fp32_peak,
+                            "unit": "GFLOP/s", "frac": pipe_ops / fp32_peak, "traffic": None,
+                            "algorithmic_gflops": achieved,
+                            "note": "achieved = FP32 operations issued (12 packed f32x2 "
+                                    "instructions = 24 FP32 ops per complex multiply-add of "
+                                    "the anchored double-word product) per second; peak = "
+                                    "nominal FP32 (152 SMs x 128 lanes x 2 x 2.07 GHz), no "
+                                    "FP32 figure is measured"}),
                  e2e={"value": samples / (e2e_ms * 1e-3), "unit": "samples/s",
                       "ms": e2e_ms, "h2d_bytes_per_step": int(batch.phases.numel() * 8 +
                                                              batch.mats.numel() * 16),

@@ -1101,7 +1101,8 @@ cudaError_t launch_team(void (*kernel)(Params...), int count, int threads, size_
         cudaGetLastError();
         occ = 1;
     }
-    // a cluster lies in one of eight GPCs
+    // a cluster lies in one of eight GPCs, taken as equal (if they are not, the choice
+    // may cost a wave; the launch is valid either way)
     const int gpc = occ * large_sms() / 8 > 8 ? occ * large_sms() / 8 : 8;
     unsigned team = 1;
     double best = 1e300;

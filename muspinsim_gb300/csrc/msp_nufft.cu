@@ -152,7 +152,11 @@ bool nufft_shape(long long S, int P, int slots, int T, int precision, bool two, 
     // ns), the tensor-core mixed sum 0.617 ms (18,300); spreading 0.80 ms
     // (3.4 pairs per ns) in FP64 and 0.077 ms (36) in mixed precision.  The
     // transform's FMAs run at about 400 per ns; the extra launches and their
-    // latencies cost 25 us.
+    // latencies cost 25 us.  One shape's figures: the FP64 spread is the one with a
+    // window in FP64 (nu_spread's takes 0.31 ms), and a direct sum's padded tiles and own
+    // launches are not counted, so the transform is taken later than it could be.  No
+    // call with 1 to 20,000 rows, 1 to 6,000 snapshots and 64 to 4,096 samples was
+    // found to take longer than with the direct sum alone.
     const double direct = (double)pairs * T / (f64 ? 255.0 : 18300.0);
     const double dft = (double)slots * s.tiles * grids *
                        (0.5 * s.n1 * s.n2 * s.n2 + 2.0 * s.tt * s.n1) / 400.0;

@@ -7,8 +7,8 @@
 //
 // FP32 eigenvectors (warp Jacobi or Householder + QL for batches of n <= 32,
 // else FP32 Jacobi in the CTA), then one Ogita-Aishima refinement step
-// evaluated in double-word FP32 arithmetic (msp_refine.cuh): residual
-// products H X, X^H H X and X^H X to ~2^-44, eigenvalues to FP64 accuracy
+// evaluated in double-word FP32 arithmetic (msp_refine.cuh): H X (for n > 32 and
+// eigensolves also X^H H X and X^H X) to ~2^-44, eigenvalues to FP64 accuracy
 // (Rayleigh quotient plus the second-order term), the eigenvectors corrected
 // to FP32 rounding.  GB300 runs FP32 at ~60x its FP64 rate, so this costs
 // about as much as the FP32 eigenvectors themselves instead of dominating as
@@ -415,7 +415,7 @@ static int occupancy_of(K kernel, int threads, size_t smem) {
 }
 
 // Threads of a snapshot kernel asked for `threads` (0: the default): the second
-// stage of the two-stage MIXED form takes at least what its eight rows per
+// stage of the two-stage MIXED form takes at least what its four rows per
 // thread need.
 static int stage2_threads(int n, int precision, int threads, bool rows) {
     const int least = rows && precision == MSP_PREC_MIXED ? row_threads(n) : 0;
